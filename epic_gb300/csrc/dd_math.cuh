@@ -14,14 +14,16 @@
 // series; pow = exp(y log x) with the double-double logarithm.  The tables are built on the
 // host from slow, long double-double series (2 atanh((c-1)/(c+1)) and exp(y/2^10)^(2^10)).
 //
-// Each function first takes a fast path (Ziv's strategy): the same reductions with a shorter
-// evaluation whose error is bounded well below 2^-69 of the result, then a rounding test that
+// Each function first takes a fast path (Ziv's strategy) in fixed point on the integer pipe
+// (fix_math.cuh), whose error is bounded below 2^-69 of the result, with a rounding test that
 // returns the result only if both ends of the error interval round to the same double.  About
-// one call in 2^16 fails the test and goes on to the double-double evaluation above.
+// one call in 2^15 fails the test and goes on, out of line, to the double-double evaluations
+// below: a short one (error below 2^-69, the same test), then the one above.
 #pragma once
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include "fix_math.cuh"
 
 namespace epic {
 
@@ -129,7 +131,16 @@ struct MathTable {
   double invc[LOG_N];      // 1024/k rounded
   dd exp2j[EXP_N];         // 2^(j/1024)
   dd atanc[ATAN_N];        // atan(k/32)
+  FixTable fix;            // the fixed-point paths' tables
 };
+
+// v in [0, 2) in units of 2^-s (s <= 127): v.hi scaled is an integer below 2^128
+inline u128 dd_to_fixed(dd v, int s) {
+  const unsigned __int128 h = (unsigned __int128)ldexp(v.hi, s);
+  const __int128 l = (__int128)rint(ldexp(v.lo, s));
+  const unsigned __int128 t = h + (unsigned __int128)l;
+  return {(uint64_t)(t >> 64), (uint64_t)t};
+}
 
 inline void fill_math_table(MathTable &t) {
   const dd third = dd_div({1., 0.}, {3., 0.});
@@ -142,6 +153,26 @@ inline void fill_math_table(MathTable &t) {
   }
   for (int j = 0; j < EXP_N; j++) t.exp2j[j] = slow_exp(dd_mul_d(t.ln2_1024, (double)j));
   for (int k = 0; k < ATAN_N; k++) t.atanc[k] = slow_atan({(double)k / 32., 0.});
+  for (int i = 0; i < FIX_N; i++) {
+    const uint32_t inv = (uint32_t)(((1u << 30) + FIX_N + i - 1) / (uint32_t)(FIX_N + i));
+    t.fix.inv[i] = inv;
+    // -log2(inv / 2^20): inv / 2^20 in (1/2, 1], doubled where it is below 0.7
+    double c = ldexp((double)inv, -20);
+    const int up = c < 0.7 ? 1 : 0;
+    if (up) c *= 2.;
+    const dd l2 = dd_div(dd_neg(slow_log(c)), t.ln2);
+    t.fix.lg[i] = c == 1. ? u128{up ? 1ull << 32 : 0, 0} : dd_to_fixed(dd_add_d(l2, (double)up), 96);
+    t.fix.e2[i] = dd_to_fixed(t.exp2j[i], 127);
+  }
+}
+// The table is a constant: built once per process, by the first call.
+inline const MathTable &math_table() {
+  static const MathTable *t = [] {
+    MathTable *p = new MathTable;
+    fill_math_table(*p);
+    return p;
+  }();
+  return *t;
 }
 
 // log(x) in double-double, x > 0 finite and normal.  Relative error ~2^-84.
@@ -268,7 +299,9 @@ __host__ __device__ __forceinline__ bool round_test(dd v, double err, double &ou
   return a == b;
 }
 
-__host__ __device__ __forceinline__ double cr_log(double x, const MathTable &T) {
+// ---- out of line: what the fixed-point paths leave ----
+
+static __host__ __device__ EPIC_COLD double cr_log_cold(double x, const MathTable &T) {
   if (!(x > 0.) || !(x < INFINITY) || x < 2.2250738585072014e-308) return log(x);
   if (x == 1.) return 0.;
   const dd v = fast_log(x, T);
@@ -276,40 +309,20 @@ __host__ __device__ __forceinline__ double cr_log(double x, const MathTable &T) 
   if (round_test(v, fabs(v.hi) * 0x1p-69, r)) return r;
   return dd_log(x, T).hi;
 }
-__host__ __device__ __forceinline__ double cr_exp(double x, const MathTable &T) {
+static __host__ __device__ EPIC_COLD double cr_exp_cold(double x, const MathTable &T) {
   if (!(fabs(x) < 700.)) return exp(x);
   if (x == 0.) return 1.;
   int q;
   const dd v = fast_exp(x, 0., T, q);
   double r;
-  if (round_test(v, fabs(v.hi) * 0x1p-69, r)) return r * pow2i(q);
+  // x's part below ulp(x) times r^2/2, left out of the sum, grows with |x|: below |x| 2^-77
+  if (round_test(v, fabs(v.hi) * (0x1p-69 + fabs(x) * 0x1p-76), r)) return r * pow2i(q);
   return dd_exp_round({x, 0.}, T);
 }
-// pow(x, y) and log(x) of one argument, sharing the fast logarithm; each result equals the
-// separate cr_pow / cr_log call.
-__host__ __device__ __forceinline__ double cr_pow(double x, double y, const MathTable &T);
-__host__ __device__ __forceinline__ double cr_log_pow(double x, double y, const MathTable &T, double &lg) {
-  if (!(x > 0.) || !(x < INFINITY) || x < 2.2250738585072014e-308 || x == 1. || y == 0. || y == 2. || !(fabs(y) < 1e6)) {
-    lg = cr_log(x, T);
-    return cr_pow(x, y, T);
-  }
-  const dd l = fast_log(x, T);
-  double r;
-  lg = round_test(l, fabs(l.hi) * 0x1p-69, r) ? r : dd_log(x, T).hi;
-  dd yl = two_prod(y, l.hi);
-  yl.lo += y * l.lo;
-  if (!(fabs(yl.hi) < 700.)) return pow(x, y);
-  yl = fast_two_sum(yl.hi, yl.lo);
-  int q;
-  const dd v = fast_exp(yl.hi, yl.lo, T, q);
-  if (round_test(v, fabs(v.hi) * (0x1p-69 + fabs(yl.hi) * 0x1p-68), r)) return r * pow2i(q);
-  const dd ls = dd_mul_d(dd_log(x, T), y);
-  return dd_exp_round(ls, T);
-}
-
-__host__ __device__ __forceinline__ double cr_pow(double x, double y, const MathTable &T) {
+static __host__ __device__ EPIC_COLD double cr_pow_cold(double x, double y, const MathTable &T) {
   if (y == 0. || x == 1.) return 1.;
   if (y == 2.) return x * x;   // the square rounded once: the correctly rounded x^2 for every x
+  if (y == -1.) return 1. / x;   // may lie within 2^-106 of a rounding boundary, beyond the evaluations below
   if (!(x > 0.) || !(x < INFINITY) || x < 2.2250738585072014e-308 || !(fabs(y) < 1e6)) return pow(x, y);
   const dd l = fast_log(x, T);
   dd yl = two_prod(y, l.hi);
@@ -323,6 +336,83 @@ __host__ __device__ __forceinline__ double cr_pow(double x, double y, const Math
   if (round_test(v, fabs(v.hi) * (0x1p-69 + fabs(yl.hi) * 0x1p-68), r)) return r * pow2i(q);
   const dd ls = dd_mul_d(dd_log(x, T), y);
   return dd_exp_round(ls, T);
+}
+
+// ---- the functions ----
+
+__host__ __device__ __forceinline__ bool positive_normal(uint64_t u) {
+  return u - 0x0010000000000000ull < 0x7FE0000000000000ull;
+}
+// ln from log2 (units of 2^-96, two's complement) where |ln| >= 2^-12 and the rounding is certain
+__host__ __device__ __forceinline__ bool fix_ln_round(u128 l2, double &out) {
+  const bool neg = (int64_t)l2.hi < 0;
+  if (neg) l2 = neg128(l2);
+  // |log2| ln 2: |log2| < 2^10, so the high word is below 2^42
+  const u128 ln = add128(mul128_64(l2, FIX_LN2_HI), {0, mulhi64(l2.hi, FIX_LN2_LO)});
+  if (ln.hi < (1ull << 20)) return false;
+  const int s = clz64(ln.hi), n = 31 - s;
+  uint64_t bits;
+  // the error below 2^-79 in units of 2^(n-116)
+  const bool ok = fix_round(shl128(ln, s), n, 1ull << (37 - n), bits);
+  out = dfrom(bits | (neg ? 0x8000000000000000ull : 0));
+  return ok;
+}
+// x^y from log2(x), where 2^-20 <= |y| < 16, |y log2 x| < 1000 and the rounding is certain
+__host__ __device__ __forceinline__ bool fix_pow_round(u128 l2, double y, const MathTable &T, double &out) {
+  const uint64_t uy = dbits(y);
+  const int s = (int)(uy >> 52 & 0x7FF) - 1022;   // |y| = Y 2^s, Y in [1/2, 1)
+  if ((unsigned)(s + 19) > 23u) return false;
+  bool neg = (int64_t)l2.hi < 0;
+  if (neg) l2 = neg128(l2);
+  u128 z = mul128_64(l2, (uy << 11) | 0x8000000000000000ull);
+  if (s > 0) z = shl128(z, s);
+  else if (s < 0) z = shr128(z, -s);
+  if (z.hi >= (1000ull << 32)) return false;
+  neg = neg != ((int64_t)uy < 0);
+  if (neg) z = neg128(z);
+  uint64_t bits;
+  // log2's error, 2^-79 |y| ln 2 of the result: below 2^41 units of 2^-116
+  const bool ok = fix_exp2(z, 1ull << 41, T.fix, bits);
+  out = dfrom(bits);
+  return ok;
+}
+
+__host__ __device__ __forceinline__ double cr_log(double x, const MathTable &T) {
+  const uint64_t u = dbits(x);
+  double r;
+  if (positive_normal(u) && fix_ln_round(fix_log2(u, T.fix), r)) return r;
+  return cr_log_cold(x, T);
+}
+__host__ __device__ __forceinline__ double cr_exp(double x, const MathTable &T) {
+  const uint64_t u = dbits(x), a = u & 0x7FFFFFFFFFFFFFFFull;
+  const int e = (int)(a >> 52) - 1023;
+  // 2^-30 <= |x| < 690: x / ln 2 in units of 2^(e-126), then of 2^-96
+  if (e >= -30 && a < 0x4085900000000000ull) {
+    u128 z = shr128(mul128_64({FIX_LOG2E_HI, FIX_LOG2E_LO}, (a << 11) | 0x8000000000000000ull), 30 - e);
+    if ((int64_t)u < 0) z = neg128(z);
+    uint64_t bits;
+    if (fix_exp2(z, 0, T.fix, bits)) return dfrom(bits);
+  }
+  return cr_exp_cold(x, T);
+}
+__host__ __device__ __forceinline__ double cr_pow(double x, double y, const MathTable &T) {
+  if (dbits(y) == 0x4000000000000000ull) return x * x;   // y = 2: the square rounded once, for every x
+  const uint64_t u = dbits(x);
+  double r;
+  if (positive_normal(u) && fix_pow_round(fix_log2(u, T.fix), y, T, r)) return r;
+  return cr_pow_cold(x, y, T);
+}
+// pow(x, y) and log(x) of one argument, sharing the logarithm; each result equals the separate
+// cr_pow / cr_log call.
+__host__ __device__ __forceinline__ double cr_log_pow(double x, double y, const MathTable &T, double &lg) {
+  const uint64_t u = dbits(x);
+  u128 l2 = {0, 0};
+  const bool ok = positive_normal(u);
+  if (ok) l2 = fix_log2(u, T.fix);
+  if (!ok || !fix_ln_round(l2, lg)) lg = cr_log_cold(x, T);
+  double r;
+  if (ok && fix_pow_round(l2, y, T, r)) return r;
+  return cr_pow_cold(x, y, T);
 }
 
 // ---- atan and cos (the turbulence closure's wall function and fv1 inversion) ----

@@ -617,16 +617,15 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
   std::vector<double> cl(g->nj + 1);
   for (int J = 0; J <= g->nj; J++) cl[J] = cos(g->lat[2 * J + 1] * kDeg);
   up(coslat, cl.data(), cl.size());
-  std::vector<epic::MathTable> host_lt(1);   // ~34 KB, built per model in a few ms
-  epic::fill_math_table(host_lt[0]);
+  const epic::MathTable &host_lt = epic::math_table();
   // t_rad's pow(cos(lat), 4.) once per row, with the device's correctly rounded pow (host-compiled)
   std::vector<double> cl4(g->nj + 1);
-  for (int J = 0; J <= g->nj; J++) cl4[J] = epic::cr_pow(cl[J], 4., host_lt[0]);
+  for (int J = 0; J <= g->nj; J++) cl4[J] = epic::cr_pow(cl[J], 4., host_lt);
   up(coslat4, cl4.data(), cl4.size());
-  cudaMemcpyAsync(lt, host_lt.data(), sizeof(epic::MathTable), cudaMemcpyHostToDevice, m->stream);
+  cudaMemcpyAsync(lt, &host_lt, sizeof(epic::MathTable), cudaMemcpyHostToDevice, m->stream);
   std::vector<double> thermo_host;   // hydrogen thermodynamics (x_h2 > 0)
   if (g->x_h2 > 0.) {
-    thermo_tables(*g, host_lt[0], thermo_host);
+    thermo_tables(*g, host_lt, thermo_host);
     cudaMemcpyAsync(thermo_d, thermo_host.data(), thermo_host.size() * sizeof(double), cudaMemcpyHostToDevice, m->stream);
   }
   d.thermo = thermo_d;
@@ -637,7 +636,7 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
     // correctly rounded pow (host-compiled)
     maxnu2.resize(g->nj + 1);
     for (int J = 0; J <= g->nj; J++) {
-      const double p2 = epic::cr_pow(g->dy0 * g->m[2 * J + 1], -2., host_lt[0]);
+      const double p2 = epic::cr_pow(g->dy0 * g->m[2 * J + 1], -2., host_lt);
       maxnu2[J] = T.max_nu[2] * (1. < p2 ? 1. : p2);
     }
     cudaMemcpyAsync((void *)d.turb_maxnu2, maxnu2.data(), maxnu2.size() * sizeof(double), cudaMemcpyHostToDevice, m->stream);
