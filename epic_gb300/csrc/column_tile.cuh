@@ -125,7 +125,7 @@ __device__ __forceinline__ float log_ratio_f(double a, double b) { return log1pf
 template <class R>
 __device__ __forceinline__ R sigmatheta_lp(const DevModel &M, R theta, R p, R pbot, R ptop, R lp) {
   if (p <= ptop) return theta;
-  const R s = RMath<R>::log(M, p / pbot) / lp;
+  const R s = qdiv(RMath<R>::log(M, qdiv(p, pbot)), lp);
   R g;
   const R f = f_and_g_sigma_r<R>(M, s, g);
   return f + g * theta;

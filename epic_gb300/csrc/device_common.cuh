@@ -230,10 +230,10 @@ __device__ __forceinline__ double xlog(const DevModel &M, double x) { return M.c
 __device__ __forceinline__ double xexp(const DevModel &M, double x) { return M.cr ? cr_exp(x, *M.lt) : ::exp(x); }
 __device__ __forceinline__ double xpow(const DevModel &M, double x, double y) { return M.cr ? cr_pow(x, y, *M.lt) : ::pow(x, y); }
 __device__ __forceinline__ double get_sigma(const DevModel &M, double pbot, double p, double ptop) {
-  return xlog(M, p / pbot) / xlog(M, ptop / pbot);
+  return div_rn(xlog(M, div_rn(p, pbot)), xlog(M, div_rn(ptop, pbot)));
 }
 __device__ __forceinline__ double get_p_sigma(const DevModel &M, double pbot, double sigma, double ptop) {
-  return pbot * xexp(M, sigma * xlog(M, ptop / pbot));
+  return pbot * xexp(M, sigma * xlog(M, div_rn(ptop, pbot)));
 }
 __device__ __forceinline__ double g_sigma(const DevModel &M, double s) {
   if (s <= M.sigma_sigma) return 0.;
@@ -283,13 +283,13 @@ __device__ __forceinline__ double hydrogen_temp(const DevModel &M, double theta1
     return xexp(M, (M.cpr * xlog(M, theta1) - 2.5 * M.x_h2 * ((1. - TH_FP) * -2.105769 + TH_FP * -1.666421)) /
                        (2.5 * M.x_he + 3.5 * (1. - M.x_he)));
   const double *fpdat = th_fpdat(M), *thg = th_thgrid(M), *t = th_t(M);
-  const double en = (double)(TH_N - 1) * (TH_FP - fpdat[0]) / (fpdat[TH_N - 1] - fpdat[0]);
+  const double en = div_rn((double)(TH_N - 1) * (TH_FP - fpdat[0]), fpdat[TH_N - 1] - fpdat[0]);
   int n = (int)en;
   double ffp, fth;
   if (n > TH_N - 2) { n = TH_N - 2; ffp = 1.; }
   else if (n < 0) { n = 0; ffp = 0.; }
   else ffp = fmod(en, 1.);
-  const double em = (double)(TH_M - 1) * (theta1 - thg[0]) / (thg[TH_M - 1] - thg[0]);
+  const double em = div_rn((double)(TH_M - 1) * (theta1 - thg[0]), thg[TH_M - 1] - thg[0]);
   int m = (int)em;
   if (m > TH_M - 2) { m = TH_M - 2; fth = 1.; }
   else if (m < 0) { m = 0; fth = 0.; }
@@ -298,10 +298,10 @@ __device__ __forceinline__ double hydrogen_temp(const DevModel &M, double theta1
          t[n * TH_M + m + 1] * (fth) * (1. - ffp) + t[(n + 1) * TH_M + m + 1] * (fth) * (ffp);
 }
 __device__ __forceinline__ double return_temp(const DevModel &M, double p, double theta) {
-  if (M.x_h2 == 0.) return theta * xpow(M, p / M.press0, M.kappa);
-  return hydrogen_temp(M, theta * xpow(M, p / M.press0, M.kappa));
+  if (M.x_h2 == 0.) return theta * xpow(M, div_rn(p, M.press0), M.kappa);
+  return hydrogen_temp(M, theta * xpow(M, div_rn(p, M.press0), M.kappa));
 }
-__device__ __forceinline__ double return_density(double p, double t, double mu) { return p * mu / (8.314472e+3 * t); }
+__device__ __forceinline__ double return_density(double p, double t, double mu) { return div_rn(p * mu, 8.314472e+3 * t); }
 __device__ __forceinline__ double return_enthalpy(const DevModel &M, double t) {
   if (M.x_h2 == 0. || t <= 20.) return (M.cpr * t) * M.rgas;
   double enthalpy;
@@ -310,7 +310,7 @@ __device__ __forceinline__ double return_enthalpy(const DevModel &M, double t) {
     enthalpy = (M.x_h2) * ((1. - TH_FP) * ho + TH_FP * hp) + (M.x_he * 2.5 + M.x_3 * 3.5) * t;
   } else {          // :6713-6735
     const double *tg = th_tgrid(M), *ho = th_h(M, 0), *hp = th_h(M, 1);
-    const double em = (double)(TH_M - 1) * (t - tg[0]) / (tg[TH_M - 1] - tg[0]);
+    const double em = div_rn((double)(TH_M - 1) * (t - tg[0]), tg[TH_M - 1] - tg[0]);
     int m = (int)em;
     double fract;
     if (m == TH_M - 1) { m--; fract = 1.; }
@@ -324,7 +324,7 @@ __device__ __forceinline__ double return_enthalpy(const DevModel &M, double t) {
 __device__ __forceinline__ double layer_p(const DevModel &M, double top, double bot) {
   if (fcmp(bot, top) == 0) return .5 * (bot + top);
   const double kp1 = M.kappa + 1.;
-  return xpow(M, (xpow(M, bot, kp1) - xpow(M, top, kp1)) / (kp1 * (bot - top)), 1. / M.kappa);
+  return xpow(M, div_rn(xpow(M, bot, kp1) - xpow(M, top, kp1), kp1 * (bot - top)), div_rn(1., M.kappa));
 }
 
 // ---- binary64 <-> binary32 conversions on the integer pipe ----
@@ -420,6 +420,9 @@ __device__ __forceinline__ double to_d(dfl x) { return df2d(x); }
 
 template <class R> __device__ __forceinline__ R rmax(R x, R y) { return x > y ? x : y; }
 template <class R> __device__ __forceinline__ R rmin(R x, R y) { return x < y ? x : y; }
+// a / b: the IEEE quotient (binary64 on the integer pipe)
+template <class R> __device__ __forceinline__ R qdiv(R a, R b) { return a / b; }
+template <> __device__ __forceinline__ double qdiv<double>(double a, double b) { return div_rn(a, b); }
 template <class R> struct RMath;
 template <> struct RMath<double> {
   static __device__ __forceinline__ double log(const DevModel &M, double x) { return xlog(M, x); }

@@ -16,6 +16,7 @@
 // series in r ln 2.  The tables are built on the host from the double-double series of dd_math.cuh.
 #pragma once
 #include <cstdint>
+#include <cstring>
 
 #ifdef __CUDACC__
 #define EPIC_COLD __noinline__
@@ -122,6 +123,67 @@ __host__ __device__ __forceinline__ bool fix_exp2(u128 z, uint64_t rel, const Fi
   const uint64_t g = a + (((a2 >> 1) + (a3s >> 12)) >> 10);                      // 2^r - 1, 2^-74
   const uint64_t p = mulhi64(t.hi, g);                                           // 2^-73
   return fix_round(add128(t, {p >> 10, p << 54}), n, (1ull << 47) + rel, bits);
+}
+
+// ---- division ----
+
+// A reciprocal estimate 2^31 y of b in [1, 2), y within 2^-22 of 1/b.
+__host__ __device__ __forceinline__ uint32_t recip31(uint32_t b24) {   // b's leading 24 bits
+#ifdef __CUDA_ARCH__
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(0x3f000000u + b24)));
+  const uint32_t q = __float2uint_rz(y * 2147483648.f);
+#else
+  const uint32_t q = (uint32_t)(0x1p54 / (double)b24);
+#endif
+  return q < 0x7fffffffu ? q : 0x7fffffffu;
+}
+
+static __host__ __device__ EPIC_COLD double div_cold(double a, double b) { return a / b; }
+
+// a / b rounded to nearest, the IEEE quotient, by long division of the significands in two digits of
+// 26 bits with a 32-bit reciprocal: about 60 integer instructions (30 clocks a warp) where the
+// binary64 pipe takes about ten operations (160 clocks).  Measured (FP64 form): 12 steps of 128x64x20
+// with transfers 20.5 -> 17.2 ms, 3 steps of 256x128x32 29.1 -> 23.5 ms.  The second digit is within 0.71 of the exact
+// quotient, so one comparison of the exact remainder with half the divisor rounds it; a quotient of
+// two 53-bit significands is never half way.  Zero dividends are answered here too (differences of
+// equal values are common in the fields); infinities, NaN, subnormals, zero divisors and quotients at
+// the ends of the range go to the division itself.
+__host__ __device__ __forceinline__ double div_rn(double a, double b) {
+  uint64_t ua, ub;
+#ifdef __CUDA_ARCH__
+  ua = (uint64_t)__double_as_longlong(a);
+  ub = (uint64_t)__double_as_longlong(b);
+#else
+  memcpy(&ua, &a, 8);
+  memcpy(&ub, &b, 8);
+#endif
+  const uint32_t ea = (uint32_t)(ua >> 52) & 0x7FFu, eb = (uint32_t)(ub >> 52) & 0x7FFu;
+  const uint64_t ma = (ua & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
+  const uint64_t mb = (ub & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
+  const int s = ma < mb ? 1 : 0;               // the significands' quotient 2^s ma / mb in [1, 2)
+  const uint32_t e = ea - eb + 1023u - (uint32_t)s;
+  const uint64_t sign = (ua ^ ub) & 0x8000000000000000ull;
+  const bool zero = (ua << 1) == 0 && eb - 1u < 2046u;
+  if (!zero && (ea - 1u >= 2046u || eb - 1u >= 2046u || e - 1u >= 2045u)) return div_cold(a, b);
+  const uint32_t y0 = recip31((uint32_t)(mb >> 29));                          // 1/b, units of 2^-31
+  const int t = (int)(((int64_t)1 << 52) - (int64_t)(((mb >> 21) * (uint64_t)y0) >> 10));   // 1 - b y0, 2^-52
+  const uint32_t y = 2u * y0 + (uint32_t)(((int64_t)t * (int)y0) >> 51);      // one Newton step, 2^-32
+  const uint32_t q1 = mulhi32((uint32_t)(ma >> (22 - s)), y) >> 4;            // the quotient, 2^-26
+  const int64_t r1 = (int64_t)((ma << (26 + s)) - mb * q1);
+  const int q2 = (int)(((int64_t)(int)(r1 >> 23) * (int64_t)(uint64_t)y + ((int64_t)1 << 34)) >> 35);   // 2^-52
+  const int64_t r2 = 2 * (int64_t)(((uint64_t)r1 << 26) - mb * (uint64_t)(int64_t)q2);
+  uint64_t q = ((uint64_t)q1 << 26) + (uint64_t)(int64_t)q2;
+  q += r2 > (int64_t)mb ? 1 : 0;
+  q -= r2 < -(int64_t)mb ? 1 : 0;
+  const uint64_t u = (zero ? 0 : ((uint64_t)(e - 1u) << 52) + q) | sign;
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double((long long)u);
+#else
+  double r;
+  memcpy(&r, &u, 8);
+  return r;
+#endif
 }
 
 }  // namespace epic

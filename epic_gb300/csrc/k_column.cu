@@ -25,7 +25,7 @@ __global__ void k_source_sink(DevModel M) {
   if (!col_index(M, j, i)) return;
   for (int k = M.k_sigma - 1; k <= M.nk; k++) {
     const long long x = M.at(k, j, i);
-    M.theta[x] += M.dt * M.heat3[x] / M.exner3[x];
+    M.theta[x] += qdiv(M.dt * M.heat3[x], M.exner3[x]);
   }
 }
 
@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(CT_THREADS, 3) k_calc_w(DevModel M, int source
   // TILE_SLOTS levels of each warp are issued together so that their latencies overlap.
   auto stage = [&](int k, double p3, double dv, double th, double ht, double ex) {
     if (source_sink && k >= ks - 1) {   // epic_funcs_diag.c:4768-4778
-      th += M.dt * ht / ex;
+      th += qdiv(M.dt * ht, ex);
       M.theta[c.base + k * n2] = th;
     }
     CT(P, k) = cv<R>(p3); CT(DV, k) = cv<R>(dv); CT(DS, k) = cv<R>(th); CT(W, k) = cv<R>(ht); CT(DF, k) = cv<R>(ex);
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(CT_THREADS, 3) k_calc_w(DevModel M, int source
   __syncthreads();
   const R ptop = CT(P, 0), pbot = CT(P, nk), psigma = CT(P, ks - 1);
   if (c.valid) {
-    for (int k = c.warp; k < nk; k += CT_WARPS) CT(LG, k) = RMath<R>::log(M, CT(P, k + 1) / CT(P, k));
+    for (int k = c.warp; k < nk; k += CT_WARPS) CT(LG, k) = RMath<R>::log(M, qdiv(CT(P, k + 1), CT(P, k)));
     if (c.warp == CT_WARPS - 1) s_lp[c.lane] = RMath<R>::log(M, ptop / pbot);
   }
   __syncthreads();
@@ -88,10 +88,10 @@ __global__ void __launch_bounds__(CT_THREADS, 3) k_calc_w(DevModel M, int source
       const R theta3 = CT(DS, k), heat = CT(W, k), exner = CT(DF, k);
       R w = R(0.);
       if (k < ks - 1) {
-        const R sigma = RMath<R>::log(M, p3 / pbot) / lp;
+        const R sigma = qdiv(RMath<R>::log(M, qdiv(p3, pbot)), lp);
         R g;
         f_and_g_sigma_r<R>(M, sigma, g);
-        w = g * heat / exner;
+        w = qdiv(g * heat, exner);
       }
       if (k >= 2) {
         const R P0 = CT(P, k - 2), P1 = CT(P, k - 1), P2 = p3, P3 = CT(P, k + 1);
@@ -101,11 +101,11 @@ __global__ void __launch_bounds__(CT_THREADS, 3) k_calc_w(DevModel M, int source
         const R df1 = P1 * CT(DV, k - 1);
         const R df2 = P2 * CT(DV, k);
         const R df3 = P3 * CT(DV, k + 1);
-        CT(DS, k) = -(df0 * (dz21 * dz21 * dz21 * (dz31 + dz32)) / (dz10 * dz20 * dz30) +
-                      df1 * (dz21 * (dz21 * (dz21 + R(2.) * (dz10 - dz31)) - R(6.) * dz10 * dz31)) / (dz10 * dz31) +
-                      df2 * (dz21 * (dz21 * (dz21 + R(2.) * (dz32 - dz20)) - R(6.) * dz20 * dz32)) / (dz20 * dz32) +
-                      df3 * (dz21 * dz21 * dz21 * (dz10 + dz20)) / (dz30 * dz31 * dz32)) /
-                    R(12.);
+        CT(DS, k) = -qdiv(qdiv(df0 * (dz21 * dz21 * dz21 * (dz31 + dz32)), dz10 * dz20 * dz30) +
+                            qdiv(df1 * (dz21 * (dz21 * (dz21 + R(2.) * (dz10 - dz31)) - R(6.) * dz10 * dz31)), dz10 * dz31) +
+                            qdiv(df2 * (dz21 * (dz21 * (dz21 + R(2.) * (dz32 - dz20)) - R(6.) * dz20 * dz32)), dz20 * dz32) +
+                            qdiv(df3 * (dz21 * dz21 * dz21 * (dz10 + dz20)), dz30 * dz31 * dz32),
+                        R(12.));
       }
       if constexpr (std::is_same_v<R, double>) {
         // dF/dp by a centred difference of return_sigmatheta at fixed theta and pbot
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(CT_THREADS, 3) k_calc_w(DevModel M, int source
         const R p4 = rmin(p3 + dp * R(.5), pbot);
         if (p2 < psigma && p4 >= psigma) p2 = p3;
         if (!(p2 < p4)) flag_error(M.ctl, ERR_CALC_W_P, k, c.j, c.i, p2);
-        CT(DF, k) = (sigmatheta_lp<R>(M, theta3, p2, pbot, ptop, lp) - sigmatheta_lp<R>(M, theta3, p4, pbot, ptop, lp)) / (p2 - p4);
+        CT(DF, k) = qdiv(sigmatheta_lp<R>(M, theta3, p2, pbot, ptop, lp) - sigmatheta_lp<R>(M, theta3, p4, pbot, ptop, lp), p2 - p4);
       } else {
         // The mixed forms differentiate return_sigmatheta analytically: in binary32 the centred
         // difference loses ~1e-5 of the derivative to rounding and truncation, and W3's error
@@ -167,7 +167,7 @@ __global__ void k_uv_drag(DevModel M) {
   const R pbot = R(0.5) * (cv<R>(M.p3[M.at(nk, j, i)]) + cv<R>(M.p3[M.at(nk, jm, im)]));
   for (int k = nk - 1; k >= 1; k--) {
     const R p3 = R(.5) * (cv<R>(M.p3[M.at(k, j, i)]) + cv<R>(M.p3[M.at(k, jm, im)]));
-    const R amp = (p3 / pbot - R(0.7)) / (R(1.) - R(0.7));
+    const R amp = qdiv(qdiv(p3, pbot) - R(0.7), R(1.) - R(0.7));
     if (amp < R(0.)) break;
     const R nu0 = cv<R>(M.hs_kf) * amp;
     const long long x = M.at(k, j, i);
@@ -242,13 +242,14 @@ __global__ void __launch_bounds__(CT_THREADS) k_hsu_vertical(DevModel M, double 
         const R whatp = sqrt(wpk * CT(WP, k + 1));
         const R whatm = -sqrt(wmk * CT(WM, k - 1));
         const R mu = (wpk - wmk) * dsi(2 * k + 1) * DT;
-        const R al = (R(1.) + mu) / R(6.);
+        const R al = qdiv(R(1.) + mu, R(6.));
         const R prod = (wa(k + 1) - amin(k + 1)) * (wa(k) - amin(k));
         const R aap = aa(k + 1), aak = aa(k);
-        R gap = aap / (aap + prod); gap = gap * gap;
-        R gam = aak / (aak + prod); gam = gam * gam;
-        const R bep = R(1.) + (R(1.) / (R(2.) * al) - R(1.)) * gap;
-        const R bem = R(1.) + (R(1.) / (R(2.) * al) - R(1.)) * gam;
+        R gap = qdiv(aap, aap + prod); gap = gap * gap;
+        R gam = qdiv(aak, aak + prod); gam = gam * gam;
+        const R hal = qdiv(R(1.), R(2.) * al) - R(1.);
+        const R bep = R(1.) + hal * gap;
+        const R bem = R(1.) + hal * gam;
         f += -al * (wpk * bep * d1(k) - whatp * (R(1.) - gap) * d1(k + 1) + wmk * bem * d2(k + 1) - whatm * (R(1.) - gam) * d2(k));
         CT(FF, k) = f;
       }
@@ -299,13 +300,14 @@ __global__ void __launch_bounds__(CT_THREADS) k_hsu_vertical(DevModel M, double 
         const R whatm = (k == 1 || k - 1 < kf) ? R(0.) : -sqrt(wmk * CT(WM, k - 1));
         const R whatp = (k == nk) ? R(0.) : sqrt(wpk * CT(WP, k + 1));
         const R mu = (wpk - wmk) * dsi(2 * k) * DT;
-        const R al = (R(1.) + mu) / R(6.);
+        const R al = qdiv(R(1.) + mu, R(6.));
         const R prod = (wa(k) - amin(k)) * (wa(k - 1) - amin(k - 1));
         const R aak = aa(k), aam = aa(k - 1);
-        R gap = aak / (aak + prod); gap = gap * gap;
-        R gam = aam / (aam + prod); gam = gam * gam;
-        const R bep = R(1.) + (R(1.) / (R(2.) * al) - R(1.)) * gap;
-        const R bem = R(1.) + (R(1.) / (R(2.) * al) - R(1.)) * gam;
+        R gap = qdiv(aak, aak + prod); gap = gap * gap;
+        R gam = qdiv(aam, aam + prod); gam = gam * gam;
+        const R hal = qdiv(R(1.), R(2.) * al) - R(1.);
+        const R bep = R(1.) + hal * gap;
+        const R bem = R(1.) + hal * gam;
         R g;
         if (k < nk) g = -al * (wpk * bep * d1(k) - whatp * (R(1.) - gap) * d1(k + 1) + wmk * bem * d2(k) - whatm * (R(1.) - gam) * d2(k - 1));
         else g = -al * (wpk * bep * d1(k) + wmk * bem * d2(k) - whatm * (R(1.) - gam) * d2(k - 1));
@@ -325,7 +327,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_hsu_vertical(DevModel M, double 
 template <class R>
 __device__ __forceinline__ R akima_dela(R d0, R d1) {
   const R tmp = d0 * d1;
-  return (tmp > R(0.)) ? R(2.) * tmp / (d0 + d1) : R(0.);
+  return (tmp > R(0.)) ? qdiv(R(2.) * tmp, d0 + d1) : R(0.);
 }
 
 // Vertical pass of akima_advection, epic_flux.c:1549-1744 (mass fluxes through the model top
@@ -364,7 +366,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_akima_vertical(DevModel M, doubl
     if (c.valid)
       for (int k = kf - 1 + c.warp; k <= nk; k += CT_WARPS) {
         if (k == kf - 1 || k == nk) { CT(FF, k) = R(0.); continue; }   // mass_flux_top, mass_flux_bot
-        const R aval = R(.5) * (wa(k) + wa(k + 1)) - (CT(DL, k) - CT(DL, k + 1)) / R(6.);
+        const R aval = R(.5) * (wa(k) + wa(k + 1)) - qdiv(CT(DL, k) - CT(DL, k + 1), R(6.));
         CT(FF, k) = CT(W, k) * aval;
       }
     __syncthreads();
@@ -389,7 +391,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_akima_vertical(DevModel M, doubl
     if (c.valid)
       for (int k = kf + c.warp; k <= nk + 1; k += CT_WARPS) {
         if (k == nk + 1) { CT(FF, k) = R(0.); continue; }
-        const R aval = R(.5) * (wa(k - 1) + wa(k)) - (CT(DL, k - 1) - CT(DL, k)) / R(6.);
+        const R aval = R(.5) * (wa(k - 1) + wa(k)) - qdiv(CT(DL, k - 1) - CT(DL, k), R(6.));
         CT(FF, k) = CT(W, k) * aval;
       }
     __syncthreads();
@@ -440,33 +442,33 @@ __global__ void __launch_bounds__(CT_THREADS) k_set_p2etc(DevModel M, int update
       p = p + M.dsgth[2 * k] * g * CT(HL, k);
       CT(P, k) = p;
     }
-    s_lp[c.lane] = xlog(M, CT(P, 0) / p);   // log(ptop/pbot)
+    s_lp[c.lane] = xlog(M, qdiv(CT(P, 0), p));   // log(ptop/pbot)
   }
   __syncthreads();
   const double ptop = CT(P, 0), pbot = CT(P, nk), lp = s_lp[c.lane];
   if (c.valid)   // pure-sigma interfaces: get_p_sigma
     for (int k = ks - 1 + c.warp; k < nk; k += CT_WARPS) {
-      const double sigma = (M.sgth[2 * k + 1] - M.zeta0) / (M.zeta1 - M.zeta0);
+      const double sigma = qdiv(M.sgth[2 * k + 1] - M.zeta0, M.zeta1 - M.zeta0);
       CT(P, k) = pbot * xexp(M, sigma * lp);
     }
   __syncthreads();
-  const double kp1 = M.kappa + 1.;
+  const double kp1 = M.kappa + 1., kinv = qdiv(1., M.kappa);
   if (c.valid)
     for (int k = c.warp; k <= nk; k += CT_WARPS) {
       const double pk = CT(P, k);
       if (k >= 1) {
         const long long x = c.base + k * n2;
         M.p3[x] = pk;
-        const double hl = (pk - CT(P, k - 1)) / (g * M.dsgth[2 * k]);
+        const double hl = qdiv(pk - CT(P, k - 1), g * M.dsgth[2 * k]);
         CT(HL, k) = hl;
         M.hdry[x] = dmaxr(M.h_min[k], hl);
       }
       CT(PP, k) = xpow(M, pk, kp1);
       if (update_theta && k < ks - 1) {   // the diagnostic THETA above k_sigma-1
-        const double sigma = xlog(M, pk / pbot) / lp;
+        const double sigma = qdiv(xlog(M, qdiv(pk, pbot)), lp);
         double gs;
         const double fs = f_and_g_sigma(M, sigma, gs);
-        const double th = (M.sgth[2 * k + 1] - fs) / gs;
+        const double th = qdiv(M.sgth[2 * k + 1] - fs, gs);
         CT(TH, k) = th;
         M.theta[c.base + k * n2] = th;
       }
@@ -478,24 +480,24 @@ __global__ void __launch_bounds__(CT_THREADS) k_set_p2etc(DevModel M, int update
     const double top = CT(P, k - 1), bot = CT(P, k);
     double p2;   // onto_kk(P2_INDEX) at the layer, epic_funcs_diag.c:2601-2618
     if (fcmp(bot, top) == 0) p2 = .5 * (bot + top);
-    else p2 = xpow(M, (CT(PP, k) - CT(PP, k - 1)) / (kp1 * (bot - top)), 1. / M.kappa);
+    else p2 = xpow(M, qdiv(CT(PP, k) - CT(PP, k - 1), kp1 * (bot - top)), kinv);
     M.p2[x] = p2;
-    if (k == 1) M.p2[c.base] = top * top / p2;
+    if (k == 1) M.p2[c.base] = qdiv(top * top, p2);
     double h;
     if (k == nk) h = CT(HL, nk);
     else {
       const double topwt = M.dsgth[2 * k], botwt = M.dsgth[2 * k + 2];
-      h = (topwt * CT(HL, k) + botwt * CT(HL, k + 1)) / (topwt + botwt);
+      h = qdiv(topwt * CT(HL, k) + botwt * CT(HL, k + 1), topwt + botwt);
     }
     M.h3[x] = h;
     if (k == 1) M.h3[c.base] = h;
     if (!update_theta) continue;
     double t2;
     if (k < ks - 1) {
-      const double sigma = xlog(M, p2 / pbot) / lp;
+      const double sigma = qdiv(xlog(M, qdiv(p2, pbot)), lp);
       double gs;
       const double fs = f_and_g_sigma(M, sigma, gs);
-      t2 = (M.sgth[2 * k] - fs) / gs;
+      t2 = qdiv(M.sgth[2 * k] - fs, gs);
     } else if (k == ks - 1) {
       t2 = .5 * (CT(TH, ks - 1) + CT(TH, ks - 2));
     } else {
@@ -506,7 +508,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_set_p2etc(DevModel M, int update
       auto Y = [&](int kay) { return CT(TH, nk - kay); };
       const int kay = s_kay[k];
       const double dx = X(kay + 1) - X(kay);
-      t2 = Y(kay) + (Y(kay + 1) - Y(kay)) * (sg - X(kay)) / dx;
+      t2 = Y(kay) + qdiv((Y(kay + 1) - Y(kay)) * (sg - X(kay)), dx);
     }
     M.theta2[x] = t2;
   }
@@ -515,7 +517,8 @@ __global__ void __launch_bounds__(CT_THREADS) k_set_p2etc(DevModel M, int update
 // store_pgrad_vars, column part (epic_funcs_diag.c:3595-3895): T3, EXNER3, RHO3, T2, RHO2,
 // the k = 0 extrapolations, GZ3 and MONT3 from the surface up, the monotone-GZ check, and
 // the first DZDT3 terms.  Shared arrays: P, R (RHO3), T3, LG (log of successive pressure
-// ratios), GZ (the Leslie-Purser increments, then the running sum in place).
+// ratios), GZ (the Leslie-Purser increments, then the running sum in place), Q (P/RHO3, each
+// level's quotient once for the four increments that read it).
 __global__ void __launch_bounds__(CT_THREADS) k_pgrad_vars_column(DevModel M) {
   if (epic_member(M)) return;
   extern __shared__ double sm[];
@@ -524,19 +527,20 @@ __global__ void __launch_bounds__(CT_THREADS) k_pgrad_vars_column(DevModel M) {
   const int nk = M.nk, L = nk + 1;
   const long long n2 = M.n2;
   const double mu = M.mu_dry;
-  double *P = sm, *R = P + 32 * L, *T3 = R + 32 * L, *LG = T3 + 32 * L, *GZ = LG + 32 * L;
+  double *P = sm, *R = P + 32 * L, *T3 = R + 32 * L, *LG = T3 + 32 * L, *GZ = LG + 32 * L, *Q = GZ + 32 * L;
   if (c.valid)
     for (int k = c.warp; k <= nk; k += CT_WARPS) {
       const long long x = c.base + k * n2;
       const double theta = M.theta[x], p = M.p3[x];
       const double t3 = return_temp(M, p, theta);
       M.t3[x] = t3;
-      M.exner3[x] = M.cp * t3 / theta;
+      M.exner3[x] = qdiv(M.cp * t3, theta);
       const double rho = return_density(p, t3, mu);
       M.rho3[x] = rho;
       CT(P, k) = p;
       CT(R, k) = rho;
       CT(T3, k) = t3;
+      CT(Q, k) = qdiv(p, rho);
       if (k >= 1) {
         const double pr = M.p2[x];
         const double t2 = return_temp(M, pr, M.theta2[x]);
@@ -548,9 +552,9 @@ __global__ void __launch_bounds__(CT_THREADS) k_pgrad_vars_column(DevModel M) {
     }
   __syncthreads();
   if (c.valid) {
-    for (int k = c.warp; k < nk; k += CT_WARPS) CT(LG, k) = xlog(M, CT(P, k + 1) / CT(P, k));
+    for (int k = c.warp; k < nk; k += CT_WARPS) CT(LG, k) = xlog(M, qdiv(CT(P, k + 1), CT(P, k)));
     if (c.warp == CT_WARPS - 1) {
-      M.rho2[c.base] = CT(R, 0) * CT(R, 0) / s_rho2_1[c.lane];
+      M.rho2[c.base] = qdiv(CT(R, 0) * CT(R, 0), s_rho2_1[c.lane]);
       M.theta2[c.base] = M.sgth[0];
       M.t2[c.base] = CT(T3, 0);
     }
@@ -560,25 +564,24 @@ __global__ void __launch_bounds__(CT_THREADS) k_pgrad_vars_column(DevModel M) {
     for (int k = 2 + c.warp; k <= nk - 1; k += CT_WARPS) {
       const double dz10 = CT(LG, k), dz21 = CT(LG, k - 1), dz32 = CT(LG, k - 2);
       const double dz20 = dz21 + dz10, dz30 = dz32 + dz20, dz31 = dz32 + dz21;
-      const double df0 = CT(P, k + 1) / CT(R, k + 1), df1 = CT(P, k) / CT(R, k), df2 = CT(P, k - 1) / CT(R, k - 1),
-                   df3 = CT(P, k - 2) / CT(R, k - 2);
-      CT(GZ, k - 1) = -(df0 * (dz21 * dz21 * dz21 * (dz31 + dz32)) / (dz10 * dz20 * dz30) +
-                        df1 * (dz21 * (dz21 * (dz21 + 2. * (dz10 - dz31)) - 6. * dz10 * dz31)) / (dz10 * dz31) +
-                        df2 * (dz21 * (dz21 * (dz21 + 2. * (dz32 - dz20)) - 6. * dz20 * dz32)) / (dz20 * dz32) +
-                        df3 * (dz21 * dz21 * dz21 * (dz10 + dz20)) / (dz30 * dz31 * dz32)) /
-                      12.;
+      const double df0 = CT(Q, k + 1), df1 = CT(Q, k), df2 = CT(Q, k - 1), df3 = CT(Q, k - 2);
+      CT(GZ, k - 1) = -qdiv(qdiv(df0 * (dz21 * dz21 * dz21 * (dz31 + dz32)), dz10 * dz20 * dz30) +
+                              qdiv(df1 * (dz21 * (dz21 * (dz21 + 2. * (dz10 - dz31)) - 6. * dz10 * dz31)), dz10 * dz31) +
+                              qdiv(df2 * (dz21 * (dz21 * (dz21 + 2. * (dz32 - dz20)) - 6. * dz20 * dz32)), dz20 * dz32) +
+                              qdiv(df3 * (dz21 * dz21 * dz21 * (dz10 + dz20)), dz30 * dz31 * dz32),
+                          12.);
     }
   __syncthreads();
   if (c.warp == 0 && c.valid) {   // GZ3 from the surface up
     double gz = M.topo_scale * M.gz_surface[M.at2(c.j, c.i)];
     CT(GZ, nk) = gz;
-    gz = gz + ((CT(P, nk) + CT(P, nk - 1)) / (CT(R, nk) + CT(R, nk - 1))) * CT(LG, nk - 1);
+    gz = gz + qdiv(CT(P, nk) + CT(P, nk - 1), CT(R, nk) + CT(R, nk - 1)) * CT(LG, nk - 1);
     CT(GZ, nk - 1) = gz;
     for (int k = nk - 1; k >= 2; k--) {
       gz = gz + CT(GZ, k - 1);
       CT(GZ, k - 1) = gz;
     }
-    CT(GZ, 0) = gz + ((CT(P, 1) + CT(P, 0)) / (CT(R, 1) + CT(R, 0))) * CT(LG, 0);
+    CT(GZ, 0) = gz + qdiv(CT(P, 1) + CT(P, 0), CT(R, 1) + CT(R, 0)) * CT(LG, 0);
   }
   __syncthreads();
   if (!c.valid) return;
@@ -594,10 +597,10 @@ __global__ void __launch_bounds__(CT_THREADS) k_pgrad_vars_column(DevModel M) {
       // DZDT3 = -(GZ3_new - GZ3_old)/(dt*g) from the third step on, 0 before (:3679-3693, :3897-3909)
       double dz = 0.;
       if (itime > 1) {
-        const double dtg_inv = -1. / (M.dt * M.grav[2 * c.j + 1]);
+        const double dtg_inv = qdiv(-1., M.dt * M.grav[2 * c.j + 1]);
         dz = (old - gzk) * dtg_inv;
       }
-      dz += M.w3[x] * M.h3[x] / CT(R, k);
+      dz += qdiv(M.w3[x] * M.h3[x], CT(R, k));
       M.dzdt3[x] = dz;
       if (gzk >= CT(GZ, k - 1)) flag_error(M.ctl, ERR_GZ_MONOTONE, k, c.j, c.i, gzk);
     }
@@ -714,8 +717,8 @@ __global__ void __launch_bounds__(CT_THREADS, 4) k_set_p2etc_mixed(DevModel M, i
     M.p2[x] = p2;
     put_split(M.work2, x, p2);
     if (k == 1) {
-      M.p2[c.base] = top * top / p2;
-      put_split(M.work2, c.base, top * top / p2);
+      M.p2[c.base] = qdiv(top * top, p2);
+      put_split(M.work2, c.base, qdiv(top * top, p2));
     }
     double h;
     if (k == nk) h = CT(HL, nk);
@@ -782,7 +785,7 @@ __global__ void __launch_bounds__(CT_THREADS, 4) k_pgrad_vars_column_mixed(DevMo
       CT(T3, k) = t3;
       if (!FULL) return;
       M.t3[x] = t3;
-      M.exner3[x] = H2 ? M.cp * t3 / theta : f2d(cpf * pf);
+      M.exner3[x] = H2 ? qdiv(M.cp * t3, theta) : f2d(cpf * pf);
       M.rho3[x] = rho;
       if (k >= 1) {
         double r2;
@@ -822,7 +825,7 @@ __global__ void __launch_bounds__(CT_THREADS, 4) k_pgrad_vars_column_mixed(DevMo
   if (c.valid) {
     for (int k = c.warp; k < nk; k += CT_WARPS) CT(LG, k) = log_ratio_f(CT(P, k), CT(P, k + 1));
     if (FULL && c.warp == CT_WARPS - 1) {
-      M.rho2[c.base] = CT(R, 0) * CT(R, 0) / s_rho2_1[c.lane];
+      M.rho2[c.base] = qdiv(CT(R, 0) * CT(R, 0), s_rho2_1[c.lane]);
       M.theta2[c.base] = M.sgth[0];
       M.t2[c.base] = CT(T3, 0);
     }
@@ -833,8 +836,8 @@ __global__ void __launch_bounds__(CT_THREADS, 4) k_pgrad_vars_column_mixed(DevMo
   if (c.valid) {
     if (c.warp == 0) CT(GZ, nk) = M.topo_scale * M.gz_surface[M.at2(c.j, c.i)];
     if (c.warp == CT_WARPS - 1) {
-      CT(GZ, nk - 1) = ((CT(P, nk) + CT(P, nk - 1)) / (CT(R, nk) + CT(R, nk - 1))) * f2d(CT(LG, nk - 1));
-      CT(GZ, 0) = ((CT(P, 1) + CT(P, 0)) / (CT(R, 1) + CT(R, 0))) * f2d(CT(LG, 0));
+      CT(GZ, nk - 1) = qdiv(CT(P, nk) + CT(P, nk - 1), CT(R, nk) + CT(R, nk - 1)) * f2d(CT(LG, nk - 1));
+      CT(GZ, 0) = qdiv(CT(P, 1) + CT(P, 0), CT(R, 1) + CT(R, 0)) * f2d(CT(LG, 0));
     }
     for (int k = 2 + c.warp; k <= nk - 1; k += CT_WARPS) {
       const float dz10 = CT(LG, k), dz21 = CT(LG, k - 1), dz32 = CT(LG, k - 2);
@@ -910,9 +913,9 @@ __global__ void k_pgrad_dzdt(DevModel M) {
   const int jj = 2 * j;
   const Ctl *c = M.ctl;
   const double *U = M.u + (long long)c->it_uv * M.n3, *V = M.v + (long long)c->it_uv * M.n3;
-  const R gdx_inv3 = R(.5) * cv<R>(M.m[jj + 1]) / cv<R>(M.grav[jj + 1]);
-  const R gdy_inv2 = R(.5) * cv<R>(M.n[jj]) / cv<R>(M.grav[jj]);
-  const R gdy_inv4 = R(.5) * cv<R>(M.n[jj + 2]) / cv<R>(M.grav[jj + 2]);
+  const R gdx_inv3 = qdiv(R(.5) * cv<R>(M.m[jj + 1]), cv<R>(M.grav[jj + 1]));
+  const R gdy_inv2 = qdiv(R(.5) * cv<R>(M.n[jj]), cv<R>(M.grav[jj]));
+  const R gdy_inv4 = qdiv(R(.5) * cv<R>(M.n[jj + 2]), cv<R>(M.grav[jj + 2]));
   const double *G = M.gz3;
   const long long x = M.at(k, j, i);
   // geopotential differences are formed in FP64 in both forms
@@ -960,14 +963,14 @@ __global__ void k_calc_heating(DevModel M) {
     const R ka = R(1.) / (R(40.) * R(60.) * R(60.) * R(24.)), ks = R(1.) / (R(4.) * R(60.) * R(60.) * R(24.));
     const R pressure = cv<R>(M.p3[x]);
     const R pbot = cv<R>(M.p3[M.at(M.nk, j, ii)]);
-    const R amp = (pressure / pbot - R(0.7)) / (R(1.) - R(0.7));
+    const R amp = qdiv(qdiv(pressure, pbot) - R(0.7), R(1.) - R(0.7));
     R kt = ka;
     if (amp > R(0.)) kt += (ks - ka) * RMath<R>::cos4(M, j) * amp;   // pow(cos(lat), 4.), per row
-    const R cp_over_time = R(1004.) / (R(1.) / kt);
+    const R cp_over_time = qdiv(R(1004.), qdiv(R(1.), kt));
     R c2 = cv<R>(M.coslat[j]);
     c2 *= c2;
     const R s2 = R(1.) - c2;
-    const R p_p0 = pressure / (R(1000.) * R(100.));
+    const R p_p0 = qdiv(pressure, R(1000.) * R(100.));
     R lg;
     const R pw = RMath<R>::log_pow(M, p_p0, cv<R>(M.kappa), lg);
     R teq = (R(315.) - R(60.) * s2 - R(10.) * lg * c2) * pw;
@@ -1164,7 +1167,7 @@ int launch_store_pgrad_vars(const DevModel &M, cudaStream_t s, bool early) {
   }
   if (M.col64) (h2 ? k_pgrad_vars_column_acc_h2 : k_pgrad_vars_column_acc)<<<grid, CT_THREADS, smem, s>>>(M);
   else if (M.mixed) (h2 ? k_pgrad_vars_column_mixed<true, true> : k_pgrad_vars_column_mixed<true, false>)<<<grid, CT_THREADS, smem, s>>>(M);
-  else k_pgrad_vars_column<<<grid, CT_THREADS, smem, s>>>(M);
+  else k_pgrad_vars_column<<<grid, CT_THREADS, tile_smem(M, 6), s>>>(M);
   EPIC_LAUNCH_R(M.mixed, k_pgrad_dzdt, epic_blocks((long long)M.nk * (M.nj + 1) * M.ni, TB(M, TB_UPDATE)), TB(M, TB_UPDATE), 0, s, M);
   return 0;
 }

@@ -255,7 +255,7 @@ __global__ void k_varz_tables(DevModel M, const double *buff, int sel, int index
   }
   if (n == 2) {
     if (lane == 0) {
-      const double del1 = (t[1].y - t[0].y) / (t[1].x - t[0].x);
+      const double del1 = div_rn(t[1].y - t[0].y, t[1].x - t[0].x);
       t[0].z = del1;
       t[1].z = del1;
     }
@@ -265,7 +265,7 @@ __global__ void k_varz_tables(DevModel M, const double *buff, int sel, int index
     // the two intervals around point q (the first two for q = 0, the last two for q = n-1)
     const int m = q == 0 ? 1 : (q == n - 1 ? n - 2 : q);
     const double h1 = t[m].x - t[m - 1].x, h2 = t[m + 1].x - t[m].x;
-    const double del1 = (t[m].y - t[m - 1].y) / h1, del2 = (t[m + 1].y - t[m].y) / h2;
+    const double del1 = div_rn(t[m].y - t[m - 1].y, h1), del2 = div_rn(t[m + 1].y - t[m].y, h2);
     const double hsum = h1 + h2;
     double z;
     if (q == 0) {
@@ -288,9 +288,9 @@ __global__ void k_varz_tables(DevModel M, const double *buff, int sel, int index
       z = 0.0;
       if (pchst(del1, del2) > 0.0) {
         const double hsumt3 = 3.0 * hsum;
-        const double w1 = (hsum + h1) / hsumt3, w2 = (hsum + h2) / hsumt3;
+        const double w1 = div_rn(hsum + h1, hsumt3), w2 = div_rn(hsum + h2, hsumt3);
         const double dmx = dmaxr(fabs(del1), fabs(del2)), dmn = dminr(fabs(del1), fabs(del2));
-        z = dmn / (w1 * (del1 / dmx) + w2 * (del2 / dmx));
+        z = div_rn(dmn, w1 * div_rn(del1, dmx) + w2 * div_rn(del2, dmx));
       }
     }
     t[q].z = z;
@@ -330,9 +330,9 @@ __device__ __forceinline__ void varz_intervals_mixed(const Trip *t, int n, int i
     v.c2 = v.c3 = make_float2(0.f, 0.f);
     if (q + 1 < n) {   // splint_pchip's cubic, epic_funcs_util.c:926-946
       const double h = t[q + 1].x - t[q].x;
-      const double delta = (t[q + 1].y - t[q].y) / h;
-      const double del1 = (t[q].z - delta) / h, del2 = (t[q + 1].z - delta) / h;
-      v.c3 = split_df((del1 + del2) / h);
+      const double delta = div_rn(t[q + 1].y - t[q].y, h);
+      const double del1 = div_rn(t[q].z - delta, h), del2 = div_rn(t[q + 1].z - delta, h);
+      v.c3 = split_df(div_rn(del1 + del2, h));
       v.c2 = split_df(-(del1 + del1 + del2));
     }
     iv[q] = v;
@@ -439,10 +439,10 @@ __global__ void k_varz_filter_rows(DevModel M, double *buff, int sel, int index,
     }
     const Trip *tk = t + kay;
     const R h = cv<R>(tk[1].x) - cv<R>(tk[0].x);
-    const R delta = (cv<R>(tk[1].y) - cv<R>(tk[0].y)) / h;
-    const R del1 = (cv<R>(tk[0].z) - delta) / h;
-    const R del2 = (cv<R>(tk[1].z) - delta) / h;
-    const R c3 = (del1 + del2) / h;
+    const R delta = qdiv(cv<R>(tk[1].y) - cv<R>(tk[0].y), h);
+    const R del1 = qdiv(cv<R>(tk[0].z) - delta, h);
+    const R del2 = qdiv(cv<R>(tk[1].z) - delta, h);
+    const R c3 = qdiv(del1 + del2, h);
     const R c2 = -(del1 + del1 + del2);
     const R xx = gzz - cv<R>(tk[0].x);
     R v = cv<R>(tk[0].y) + xx * (cv<R>(tk[0].z) + xx * (c2 + xx * c3));
@@ -479,7 +479,7 @@ __global__ void k_hsu_zonal(DevModel M, double *buff, int kind, int kstart) {
   const bool filt = row_is_filtered(M, j, 0);
   if (filt) load_twiddles(M, fs);
   const double *U = M.u + (long long)M.ctl->it_uv * M.n3;
-  const R n_inv = R(1.) / cv<R>(M.n[2 * j + 1]);
+  const R n_inv = qdiv(R(1.), cv<R>(M.n[2 * j + 1]));
   const R mn1 = cv<R>(M.mn[2 * j + 1]);
   for (int i = threadIdx.x; i <= ni + 1; i += blockDim.x) {
     a[i] = cv<R>(buff[base + i]);
@@ -521,13 +521,14 @@ __global__ void k_hsu_zonal(DevModel M, double *buff, int kind, int kstart) {
     const R uhatp = sqrt(up[i] * up[i - 1]);
     const R uhatm = -sqrt(um[i] * um[i + 1]);
     const R mu = (up[i] - um[i]) * mn1 * DT;
-    const R al = (R(1.) + mu) / R(6.);
-    R gap = aa[i - 1] / (aa[i - 1] + (a[i - 1] - a_min) * (a[i] - a_min));
+    const R al = qdiv(R(1.) + mu, R(6.));
+    R gap = qdiv(aa[i - 1], aa[i - 1] + (a[i - 1] - a_min) * (a[i] - a_min));
     gap = gap * gap;
-    R gam = aa[i] / (aa[i] + (a[i - 1] - a_min) * (a[i] - a_min));
+    R gam = qdiv(aa[i], aa[i] + (a[i - 1] - a_min) * (a[i] - a_min));
     gam = gam * gam;
-    const R bep = R(1.) + (R(1.) / (R(2.) * al) - R(1.)) * gap;
-    const R bem = R(1.) + (R(1.) / (R(2.) * al) - R(1.)) * gam;
+    const R hal = qdiv(R(1.), R(2.) * al) - R(1.);
+    const R bep = R(1.) + hal * gap;
+    const R bem = R(1.) + hal * gam;
     const R behatp = R(1.) - gap, behatm = R(1.) - gam;
     const R g = -al * (up[i] * bep * d1[i] - uhatp * behatp * d1[i - 1] + um[i] * bem * d2[i - 1] - uhatm * behatm * d2[i]);
     ff[i] += g;
@@ -562,7 +563,7 @@ __global__ void k_akima_zonal(DevModel M, double *buff, int kind, int kstart) {
   const bool filt = row_is_filtered(M, j, 0);
   if (filt) load_twiddles(M, fs);
   const double *U = M.u + (long long)M.ctl->it_uv * M.n3;
-  const R n_inv = R(1.) / cv<R>(M.n[2 * j + 1]);
+  const R n_inv = qdiv(R(1.), cv<R>(M.n[2 * j + 1]));
   const R mn1 = cv<R>(M.mn[2 * j + 1]);
   for (int i = threadIdx.x; i <= ni + 1; i += blockDim.x) {
     a[i] = cv<R>(buff[base + i]);
@@ -580,13 +581,13 @@ __global__ void k_akima_zonal(DevModel M, double *buff, int kind, int kstart) {
   __syncthreads();
   for (int i = threadIdx.x + 1; i <= ni; i += blockDim.x) {
     const R tmp = da[i] * da[i + 1];
-    dl[i] = (tmp > R(0.)) ? R(2.) * tmp / (da[i] + da[i + 1]) : R(0.);
+    dl[i] = (tmp > R(0.)) ? qdiv(R(2.) * tmp, da[i] + da[i + 1]) : R(0.);
   }
   __syncthreads();
   if (threadIdx.x == 0) { dl[0] = dl[ni]; dl[ni + 1] = dl[1]; }
   __syncthreads();
   for (int i = threadIdx.x + 1; i <= ni; i += blockDim.x) {
-    const R aval = R(.5) * (a[i] + a[i - 1]) - (dl[i] - dl[i - 1]) / R(6.);
+    const R aval = R(.5) * (a[i] + a[i - 1]) - qdiv(dl[i] - dl[i - 1], R(6.));
     ff[i] = u2d[i] * aval * n_inv;
   }
   __syncthreads();

@@ -63,7 +63,7 @@ __device__ __forceinline__ R uh_at(const DevModel &M, const double *Uk, const do
   if (j < 0 || j > M.nj) return R(0.);
   i = wrap_i(M, i);
   const R havg = R(.5) * (cv<R>(Hk[M.at2(j, i)]) + cv<R>(Hk[M.at2(j, i - 1)]));
-  return cv<R>(Uk[M.at2(j, i)]) * havg * (R(1.) / cv<R>(M.n[2 * j + 1]));
+  return cv<R>(Uk[M.at2(j, i)]) * havg * qdiv(R(1.), cv<R>(M.n[2 * j + 1]));
 }
 // VH(j,i) for j = 1..nj (0 at the poles), periodic in i
 template <class R>
@@ -71,7 +71,7 @@ __device__ __forceinline__ R vh_at(const DevModel &M, const double *Vk, const do
   if (j < 1 || j > M.nj) return R(0.);
   i = wrap_i(M, i);
   const R havg = R(.5) * (cv<R>(Hk[M.at2(j, i)]) + cv<R>(Hk[M.at2(j - 1, i)]));
-  return cv<R>(Vk[M.at2(j, i)]) * havg * (R(1.) / cv<R>(M.m[2 * j]));
+  return cv<R>(Vk[M.at2(j, i)]) * havg * qdiv(R(1.), cv<R>(M.m[2 * j]));
 }
 
 // Kinetic energy per mass on the h grid, planes k = 1..nk-1, into work0 (with pads).
@@ -257,7 +257,7 @@ __device__ __forceinline__ LonFace<R> lon_face(const DevModel &M, const R (&z)[3
   const R a1 = f.ztne + f.ztse, b1 = f.ztne * f.ztse, a2 = f.zbne + f.zbse, b2 = f.zbne * f.zbse;
   const R terms1 = a1 * a1 - b1 - (a2 * a2 - b2);
   const R terms2 = R(3.) * (a1 - a2);
-  f.east = (-terms1 * (f.pbe - f.pte) + terms2 * (f.zte * f.pbe - f.zbe * f.pte)) / (f.zte - f.zbe);
+  f.east = qdiv(-terms1 * (f.pbe - f.pte) + terms2 * (f.zte * f.pbe - f.zbe * f.pte), f.zte - f.zbe);
   return f;
 }
 
@@ -316,27 +316,27 @@ __global__ void k_pgrad_lon(DevModel M) {
   const R rlns = cv<R>(M.rln[2 * j]), rlnn = cv<R>(M.rln[2 * j + 2]);
   R a1 = e.ztne + e.ztse, a2 = w.ztne + w.ztse;
   R terms2 = R(3.) * (a1 - a2), top, bottom;
-  if (fabs(R(2.) * (e.zte - w.zte) / (e.zte + w.zte - e.zbe - w.zbe)) > DLOGZ_TOL) {
+  if (fabs(qdiv(R(2.) * (e.zte - w.zte), e.zte + w.zte - e.zbe - w.zbe)) > DLOGZ_TOL) {
     const R b1 = e.ztne * e.ztse, b2 = w.ztne * w.ztse;
     const R terms1 = a1 * a1 - b1 - (a2 * a2 - b2);
-    top = (-terms1 * (w.pte - e.pte) + terms2 * (e.zte * w.pte - w.zte * e.pte)) / (e.zte - w.zte);
+    top = qdiv(-terms1 * (w.pte - e.pte) + terms2 * (e.zte * w.pte - w.zte * e.pte), e.zte - w.zte);
   } else {
     top = Pow2{.5f} * (w.pte + e.pte) * terms2;
   }
   a1 = e.zbne + e.zbse;
   a2 = w.zbne + w.zbse;
   terms2 = R(3.) * (a1 - a2);
-  if (fabs(R(2.) * (e.zbe - w.zbe) / (e.zte + w.zte - e.zbe - w.zbe)) > DLOGZ_TOL) {
+  if (fabs(qdiv(R(2.) * (e.zbe - w.zbe), e.zte + w.zte - e.zbe - w.zbe)) > DLOGZ_TOL) {
     const R b1 = e.zbne * e.zbse, b2 = w.zbne * w.zbse;
     const R terms1 = a1 * a1 - b1 - (a2 * a2 - b2);
-    bottom = (-terms1 * (w.pbe - e.pbe) + terms2 * (e.zbe * w.pbe - w.zbe * e.pbe)) / (e.zbe - w.zbe);
+    bottom = qdiv(-terms1 * (w.pbe - e.pbe) + terms2 * (e.zbe * w.pbe - w.zbe * e.pbe), e.zbe - w.zbe);
   } else {
     bottom = Pow2{.5f} * (w.pbe + e.pbe) * terms2;
   }
   R pgflon = top - bottom + R(0.) - R(0.) + w.east - e.east;
   const R dzn = e.ztne - e.zbne + w.ztne - w.zbne;
   const R dzs = e.ztse - e.zbse + w.ztse - w.zbse;
-  pgflon /= face_width<R>(M.lon, 2 * i - 1, 2 * i + 1) * rho * (rlns * (dzs + Pow2{.5f} * dzn) + rlnn * (dzn + Pow2{.5f} * dzs));
+  pgflon = qdiv(pgflon, face_width<R>(M.lon, 2 * i - 1, 2 * i + 1) * rho * (rlns * (dzs + Pow2{.5f} * dzn) + rlnn * (dzn + Pow2{.5f} * dzs)));
   const long long x = plane_offset(M, PL_UV_TEND) + M.at(k, j, i);
   M.dudt[x] = M.dudt[x] + to_d(pgflon);
 }
@@ -358,7 +358,7 @@ __device__ __forceinline__ LatFace<R> lat_face(const DevModel &M, const R (&z)[3
   const R a1 = f.ztne + f.ztnw, b1 = f.ztne * f.ztnw, a2 = f.zbne + f.zbnw, b2 = f.zbne * f.zbnw;
   const R terms1 = a1 * a1 - b1 - (a2 * a2 - b2);
   const R terms2 = R(3.) * (a1 - a2);
-  f.north = f.rln * (-terms1 * (f.pbn - f.ptn) + terms2 * (f.ztn * f.pbn - f.zbn * f.ptn)) / (f.ztn - f.zbn);
+  f.north = qdiv(f.rln * (-terms1 * (f.pbn - f.ptn) + terms2 * (f.ztn * f.pbn - f.zbn * f.ptn)), f.ztn - f.zbn);
   return f;
 }
 
@@ -422,15 +422,15 @@ __global__ void k_pgrad_lat(DevModel M) {
   a1 = n.ztne + ztse; b1 = n.ztne * ztse; a2 = n.zbne + zbse; b2 = n.zbne * zbse;
   terms1 = a1 * a1 - b1 - (a2 * a2 - b2);
   terms2 = R(3.) * (a1 - a2);
-  const R east = Pow2{.5f} * (rlns - rlnn) * (-terms1 * (pbe - pte) + terms2 * (zte * pbe - zbe * pte)) / (zte - zbe);
+  const R east = qdiv(Pow2{.5f} * (rlns - rlnn) * (-terms1 * (pbe - pte) + terms2 * (zte * pbe - zbe * pte)), zte - zbe);
   a1 = n.ztnw + ztsw; b1 = n.ztnw * ztsw; a2 = n.zbnw + zbsw; b2 = n.zbnw * zbsw;
   terms1 = a1 * a1 - b1 - (a2 * a2 - b2);
   terms2 = R(3.) * (a1 - a2);
-  const R west = Pow2{.5f} * (rlns - rlnn) * (-terms1 * (pbw - ptw) + terms2 * (ztw * pbw - zbw * ptw)) / (ztw - zbw);
+  const R west = qdiv(Pow2{.5f} * (rlns - rlnn) * (-terms1 * (pbw - ptw) + terms2 * (ztw * pbw - zbw * ptw)), ztw - zbw);
   R top, bottom;
   a1 = n.ztne + n.ztnw; a2 = ztse + ztsw;
   terms2 = R(3.) * (a1 - a2);
-  if (fabs(R(2.) * (n.ztn - zts) / (n.ztn + zts - n.zbn - zbs)) > DLOGZ_TOL) {
+  if (fabs(qdiv(R(2.) * (n.ztn - zts), n.ztn + zts - n.zbn - zbs)) > DLOGZ_TOL) {
     b1 = n.ztne * n.ztnw; b2 = ztse * ztsw; b3 = n.ztne * ztse + n.ztnw * ztsw;
     terms1 = a1 * a1 - b1 - (a2 * a2 - b2);
     top = Pow2{.5f} * ((n.ptn - pts) * ((rlnn + rlns) * terms1 + (rlnn - rlns) * (b1 + b2 - b3)) + (rlnn + rlns) * terms2 * (n.ztn * pts - zts * n.ptn)) /
@@ -440,7 +440,7 @@ __global__ void k_pgrad_lat(DevModel M) {
   }
   a1 = n.zbne + n.zbnw; a2 = zbse + zbsw;
   terms2 = R(3.) * (a1 - a2);
-  if (fabs(R(2.) * (n.zbn - zbs) / (n.ztn + zts - n.zbn - zbs)) > DLOGZ_TOL) {
+  if (fabs(qdiv(R(2.) * (n.zbn - zbs), n.ztn + zts - n.zbn - zbs)) > DLOGZ_TOL) {
     b1 = n.zbne * n.zbnw; b2 = zbse * zbsw; b3 = n.zbne * zbse + n.zbnw * zbsw;
     terms1 = a1 * a1 - b1 - (a2 * a2 - b2);
     bottom = Pow2{.5f} * ((n.pbn - pbs) * ((rlnn + rlns) * terms1 + (rlnn - rlns) * (b1 + b2 - b3)) + (rlnn + rlns) * terms2 * (n.zbn * pbs - zbs * n.pbn)) /
@@ -451,7 +451,7 @@ __global__ void k_pgrad_lat(DevModel M) {
   R pgflat = top - bottom + south - (north + west + east);
   const R dzn = n.ztne - n.zbne + n.ztnw - n.zbnw;
   const R dzs = ztse - zbse + ztsw - zbsw;
-  pgflat /= face_width<R>(M.lat, 2 * j - 1, 2 * j + 1) * rho * rlt * (rlns * (dzs + Pow2{.5f} * dzn) + rlnn * (dzn + Pow2{.5f} * dzs));
+  pgflat = qdiv(pgflat, face_width<R>(M.lat, 2 * j - 1, 2 * j + 1) * rho * rlt * (rlns * (dzs + Pow2{.5f} * dzn) + rlnn * (dzn + Pow2{.5f} * dzs)));
   const long long x = plane_offset(M, PL_UV_TEND) + M.at(k, j, i);
   M.dvdt[x] = M.dvdt[x] + to_d(pgflat);
 }
@@ -467,7 +467,7 @@ __device__ __forceinline__ void vmp(const DevModel &M, const double *V, int kind
   if (j < 0 || j > M.nj + 1) { vm = vp = R(0.); return; }
   if (kind == 2) v2d = (j >= 1 && j <= M.nj) ? R(.5) * (cv<R>(V[M.at(k, j, i)]) + cv<R>(V[M.at(k - 1, j, i)])) : R(0.);
   else v2d = cv<R>(V[M.at(k, j, i)]);
-  const R mi = (fabs(M.lat[2 * j]) == 90.) ? R(0.) : R(1.) / cv<R>(M.m[2 * j]);
+  const R mi = (fabs(M.lat[2 * j]) == 90.) ? R(0.) : qdiv(R(1.), cv<R>(M.m[2 * j]));
   vm = rmin(R(0.), v2d * mi);
   vp = rmax(R(0.), v2d * mi);
 }
@@ -529,13 +529,14 @@ __global__ void k_hsu_merid_corr(DevModel M, const double *A, int kind, int k0) 
     const R vhatp = sqrt(vp * vpm);
     const R vhatm = -sqrt(vm * vmp1);
     const R mu = (vp - vm) * cv<R>(M.mn[2 * j]) * DT;
-    const R al = (R(1.) + mu) / R(6.);
+    const R al = qdiv(R(1.) + mu, R(6.));
     const R am1 = aaa(j - 1), a0 = aaa(j);
     const R prod = (a(j - 1) - a_min) * (a(j) - a_min);
-    R gap = am1 / (am1 + prod); gap = gap * gap;
-    R gam = a0 / (a0 + prod); gam = gam * gam;
-    const R bep = R(1.) + (R(1.) / (R(2.) * al) - R(1.)) * gap;
-    const R bem = R(1.) + (R(1.) / (R(2.) * al) - R(1.)) * gam;
+    R gap = qdiv(am1, am1 + prod); gap = gap * gap;
+    R gam = qdiv(a0, a0 + prod); gam = gam * gam;
+    const R hal = qdiv(R(1.), R(2.) * al) - R(1.);
+    const R bep = R(1.) + hal * gap;
+    const R bem = R(1.) + hal * gam;
     ffv += -al * (vp * bep * diff1(j) - vhatp * (R(1.) - gap) * diff1(j - 1) + vm * bem * diff2(j - 1) - vhatm * (R(1.) - gam) * diff2(j));
   }
   write_with_pads(M.work3, M, M.at(k, j, 0), i, ffv);
@@ -620,13 +621,14 @@ __global__ void k_hsu_meridional(DevModel M, double *A, int kind, int k0) {
       const R vhatp = sqrt(vp_1 * vp_0);
       const R vhatm = -sqrt(vm_1 * vm_2);
       const R mu = (vp_1 - vm_1) * cv<R>(M.mn[2 * jj]) * DT;
-      const R al = (R(1.) + mu) / R(6.);
+      const R al = qdiv(R(1.) + mu, R(6.));
       const R am1 = aaa(jj - 1, a_m1, a_0, a_1), a0 = aaa(jj, a_0, a_1, a_2);
       const R prod = (a_0 - a_min) * (a_1 - a_min);
-      R gap = am1 / (am1 + prod); gap = gap * gap;
-      R gam = a0 / (a0 + prod); gam = gam * gam;
-      const R bep = R(1.) + (R(1.) / (R(2.) * al) - R(1.)) * gap;
-      const R bem = R(1.) + (R(1.) / (R(2.) * al) - R(1.)) * gam;
+      R gap = qdiv(am1, am1 + prod); gap = gap * gap;
+      R gam = qdiv(a0, a0 + prod); gam = gam * gam;
+      const R hal = qdiv(R(1.), R(2.) * al) - R(1.);
+    const R bep = R(1.) + hal * gap;
+      const R bem = R(1.) + hal * gam;
       f += -al * (vp_1 * bep * diff1_jj - vhatp * (R(1.) - gap) * diff1_jm + vm_1 * bem * diff2_jm - vhatm * (R(1.) - gam) * diff2_jj);
       ffv_1 = f;
     }
@@ -656,7 +658,7 @@ __global__ void k_hsu_meridional(DevModel M, double *A, int kind, int k0) {
 template <class R>
 __device__ __forceinline__ R akima_mean(R d0, R d1) {   // the dela of akima_advection
   const R tmp = d0 * d1;
-  return (tmp > R(0.)) ? R(2.) * tmp / (d0 + d1) : R(0.);
+  return (tmp > R(0.)) ? qdiv(R(2.) * tmp, d0 + d1) : R(0.);
 }
 
 template <class R>
@@ -672,8 +674,8 @@ __global__ void k_akima_merid_flux(DevModel M, const double *A, int kind, int k0
   const R dl_jm = akima_mean<R>(deltaa(j - 1), deltaa(j));
   const double *V = M.v + plane_offset(M, PL_UV);
   const R v2d = kind == 2 ? R(.5) * (cv<R>(V[M.at(k, j, i)]) + cv<R>(V[M.at(k - 1, j, i)])) : cv<R>(V[M.at(k, j, i)]);
-  const R m_2j_inv = (fabs(M.lat[2 * j]) == 90.) ? R(0.) : R(1.) / cv<R>(M.m[2 * j]);
-  const R aval = R(.5) * (a(j) + a(j - 1)) - (dl_j - dl_jm) / R(6.);
+  const R m_2j_inv = (fabs(M.lat[2 * j]) == 90.) ? R(0.) : qdiv(R(1.), cv<R>(M.m[2 * j]));
+  const R aval = R(.5) * (a(j) + a(j - 1)) - qdiv(dl_j - dl_jm, R(6.));
   write_with_pads(M.work3, M, M.at(k, j, 0), i, to_d(v2d * aval * m_2j_inv));
 }
 
@@ -865,10 +867,10 @@ __global__ void k_zonal_visc(DevModel M, double *A, int sel, int jbot, int jhalf
 template <class R>
 __device__ __forceinline__ R div_at(const DevModel &M, const double *UU, const double *VV, int k, int j, int i) {
   const int jj = 2 * j + 1;
-  const R n_inv = R(1.) / cv<R>(M.n[jj]);
+  const R n_inv = qdiv(R(1.), cv<R>(M.n[jj]));
   const R mn1 = cv<R>(M.mn[jj]);
-  const R m2j_inv = (j == 0) ? R(0.) : R(1.) / cv<R>(M.m[jj - 1]);
-  const R m2jp2_inv = (j == M.nj) ? R(0.) : R(1.) / cv<R>(M.m[jj + 1]);
+  const R m2j_inv = (j == 0) ? R(0.) : qdiv(R(1.), cv<R>(M.m[jj - 1]));
+  const R m2jp2_inv = (j == M.nj) ? R(0.) : qdiv(R(1.), cv<R>(M.m[jj + 1]));
   return mn1 * ((cv<R>(UU[M.at(k, j, i + 1)]) * n_inv - cv<R>(UU[M.at(k, j, i)]) * n_inv) +
                 (cv<R>(VV[M.at(k, j + 1, i)]) * m2jp2_inv - cv<R>(VV[M.at(k, j, i)]) * m2j_inv));
 }
@@ -892,15 +894,15 @@ __global__ void k_pv_interior(DevModel M, const double *VV) {
   const double *UU = M.u + plane_offset(M, PL_UV);
   const double *HH = M.h3;
   const R f2j = cv<R>(M.f[2 * j]), m2j = cv<R>(M.m[2 * j]), n2j = cv<R>(M.n[2 * j]);
-  const R m_m1_inv = R(1.) / cv<R>(M.m[2 * j - 1]), m_p1_inv = R(1.) / cv<R>(M.m[2 * j + 1]);
-  const R mn_m1_inv = R(1.) / cv<R>(M.mn[2 * j - 1]), mn_p1_inv = R(1.) / cv<R>(M.mn[2 * j + 1]);
-  const R mn_pv = R(.5) / (mn_m1_inv + mn_p1_inv);
+  const R m_m1_inv = qdiv(R(1.), cv<R>(M.m[2 * j - 1])), m_p1_inv = qdiv(R(1.), cv<R>(M.m[2 * j + 1]));
+  const R mn_m1_inv = qdiv(R(1.), cv<R>(M.mn[2 * j - 1])), mn_p1_inv = qdiv(R(1.), cv<R>(M.mn[2 * j + 1]));
+  const R mn_pv = qdiv(R(.5), mn_m1_inv + mn_p1_inv);
   const R ze = m2j * ((cv<R>(VV[M.at(k, j, i)]) - cv<R>(VV[M.at(k, j, i - 1)])) +
                       n2j * (cv<R>(UU[M.at(k, j - 1, i)]) * m_m1_inv - cv<R>(UU[M.at(k, j, i)]) * m_p1_inv));
   R pv = (ze + f2j);
   const R h_pv = ((cv<R>(HH[M.at(k, j, i)]) + cv<R>(HH[M.at(k, j, i - 1)])) * mn_p1_inv +
                   (cv<R>(HH[M.at(k, j - 1, i)]) + cv<R>(HH[M.at(k, j - 1, i - 1)])) * mn_m1_inv) * mn_pv;
-  pv /= h_pv;
+  pv = qdiv(pv, h_pv);
   write_with_pads(M.pv3, M, M.at(k, j, 0), i, pv);
 }
 
@@ -965,13 +967,13 @@ __global__ void k_ri2(DevModel M) {
     const R pressure = cv<R>(M.p2[x]), temperature = cv<R>(M.t2[x]), density = cv<R>(M.rho2[x]);
     const R cp = R(1004.), mu = cv<R>(M.mu_dry);
     const R deltap = R(0.001) * pressure, deltaT = R(0.001) * temperature;
-    auto dens = [&](R p, R t) { return p * mu / (R(8.314472e+3) * t); };   // return_density
-    const R drho_dp_T = (dens(pressure + deltap, temperature) - dens(pressure - deltap, temperature)) / (R(2.) * deltap);
-    const R drho_dT_p = (dens(pressure, temperature + deltaT) - dens(pressure, temperature - deltaT)) / (R(2.) * deltaT);
-    const R Drho_Dp = (cv<R>(M.rho3[x]) - cv<R>(M.rho3[M.at(k - 1, j, i)])) / (cv<R>(M.p3[x]) - cv<R>(M.p3[M.at(k - 1, j, i)]));
+    auto dens = [&](R p, R t) { return qdiv(p * mu, R(8.314472e+3) * t); };   // return_density
+    const R drho_dp_T = qdiv(dens(pressure + deltap, temperature) - dens(pressure - deltap, temperature), R(2.) * deltap);
+    const R drho_dT_p = qdiv(dens(pressure, temperature + deltaT) - dens(pressure, temperature - deltaT), R(2.) * deltaT);
+    const R Drho_Dp = qdiv(cv<R>(M.rho3[x]) - cv<R>(M.rho3[M.at(k - 1, j, i)]), cv<R>(M.p3[x]) - cv<R>(M.p3[M.at(k - 1, j, i)]));
     const R g = cv<R>(M.grav[2 * j + 1]);
-    const R brunt2 = g * g * (Drho_Dp - drho_dp_T + temperature / (cp * density * density) * drho_dT_p * drho_dT_p);
-    ri = brunt2 / (dudz2 + dvdz2);
+    const R brunt2 = g * g * (Drho_Dp - drho_dp_T + qdiv(temperature, cp * density * density) * drho_dT_p * drho_dT_p);
+    ri = qdiv(brunt2, dudz2 + dvdz2);
   } else {
     ri = R(1.e+6);
   }
