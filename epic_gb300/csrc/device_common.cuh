@@ -22,6 +22,10 @@ enum TuneGroup { TB_UV_CORE = 0, TB_PGRAD, TB_HSU, TB_VISC, TB_DIAG, TB_UPDATE, 
 
 namespace epic {
 
+constexpr int SCRATCH_SETS = 3;   // work0..3, once per branch of the step that uses them concurrently
+constexpr int TABLE_SETS = 4;     // ptable, once per field of the 3-D filter
+constexpr int SCRATCH_VOLUMES = 3 + 4 * SCRATCH_SETS;   // gz, unity, old and the sets of work0..3
+
 // Time-plane indices and step counters live on the device so that one captured CUDA graph
 // serves every step (the reference rotates IT_ZERO/IT_MINUS1/IT_MINUS2 on the host,
 // src/shared/epic_timestep.c:257-274).
@@ -97,6 +101,9 @@ struct DevModel {
   double *gz3, *mont3, *heat3, *pv3, *ri2, *div_uv3, *w3, *dzdt3, *u_spinup, *gz_surface;
   // scratch
   double *gz, *unity, *old, *work0, *work1, *work2, *work3, *ptable;
+  int wset, tset;   // which of the SCRATCH_SETS copies of work0..3 and of the TABLE_SETS copies of
+                    // ptable this launch's work0..3 and ptable are (concurrent branches of a step
+                    // keep theirs apart; on a member's own description both are 0)
   float2 *lp3;   // log P3 at every interface as a double-float: written by set_p2etc of the mixed
                  // form (stage 11), read by its store_pgrad_vars (stage 19); P3 does not change
                  // between the two
@@ -124,7 +131,7 @@ struct DevModel {
 // A pointer into member 0's arrays, moved to the same place in member `to`'s arrays.  The pool of
 // a model (epic_model_create) packs the state arrays back to back as planes of n3 values (u and v
 // value planes, the tendency planes, then the single fields), and carves the scratch volumes gz,
-// unity, old, work0..3 one after another, each rounded up to 256 bytes (and, with the turbulence
+// unity, old and the sets of work0..3 one after another, each rounded up to 256 bytes (and, with the turbulence
 // closure, NU_TURB and the three diffusivities the same way); so the plane (or volume) index and
 // the offset inside it follow from the address by integer arithmetic, and map to the member's
 // pool with its own n3.  A pointer outside these regions (a table) is returned as is.
@@ -135,7 +142,7 @@ __device__ __forceinline__ P *relocate_field(const DevModel &from, const DevMode
   const long long n3 = from.reloc_n3;
   const char *s0 = reinterpret_cast<const char *>(from.gz);
   const long long st0 = scratch_stride(n3);
-  if (c >= s0 && c < s0 + 7 * st0) {
+  if (c >= s0 && c < s0 + SCRATCH_VOLUMES * st0) {
     const long long o = c - s0, q = o / st0;
     return reinterpret_cast<P *>(reinterpret_cast<char *>(to.gz) + q * scratch_stride(to.n3) + (o - q * st0));
   }
@@ -167,12 +174,27 @@ __device__ __forceinline__ P *member_ptr(const DevModel &M, const DevModel &mem,
   if (M.hetero) return relocate_field(M, mem, p);
   return (P *)(mem.pool_base + ((const char *)p - M.pool_base));
 }
+// Point work0..3 and ptable of a description that has sets 0 at sets ws and ts; n3: the field size
+// of the model whose arrays it carries.
+__host__ __device__ __forceinline__ void scratch_sets(DevModel &M, int ws, int ts, long long n3) {
+  if (ws) {
+    const long long st = 4LL * ws * (scratch_stride(n3) / 8);
+    M.work0 += st; M.work1 += st; M.work2 += st; M.work3 += st;
+    M.wset = ws;
+  }
+  if (ts) {
+    M.ptable += (long long)ts * 3 * (M.nj + 3) * (M.nk + 2);
+    M.tset = ts;
+  }
+}
 template <class... P>
 __device__ __forceinline__ bool epic_member(DevModel &M, P *&...ptrs) {
   if (M.batch) {
     const DevModel &mem = M.batch[blockIdx.z];
     ((ptrs = member_ptr(M, mem, ptrs)), ...);
+    const int ws = M.wset, ts = M.tset;
     M = mem;
+    scratch_sets(M, ws, ts, M.n3);
   }
   return M.ctl->halted != 0;
 }

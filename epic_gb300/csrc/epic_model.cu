@@ -226,9 +226,17 @@ int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
       }
       break;
     case 11: launch_set_p2etc(M, 1, s); break;
-    case 12: launch_uv_pgrad(M, s); break;
+    case 12:
+      launch_pgrad_poles(M, s);
+      launch_pgrad_lon(M, s);
+      launch_pgrad_lat(M, s);
+      break;
     case 13: launch_divergence_damping(M, s); break;
-    case 14: launch_uv_update(M, s); break;
+    case 14:
+      launch_uv_decide(M, s);
+      launch_uv_update(M, s);
+      launch_uv_rotate(M, s);
+      break;
     case 15:
       launch_meridional_hyperviscosity(M, 0, M.u, PL_UV, s);
       launch_meridional_hyperviscosity(M, 1, M.v, PL_UV, s);
@@ -236,7 +244,12 @@ int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
       launch_zonal_hyperviscosity(M, 1, M.v, PL_UV, s);
       break;
     case 16:
-      launch_store_diag(M, s);
+      launch_diag_filter_v(M, s);
+      launch_diag_pv(M, s);
+      launch_diag_pv_poles(M, s);
+      launch_diag_filter_u(M, s);
+      launch_diag_div(M, s);
+      launch_diag_ri2(M, s);
       if (M.turb) launch_set_diffusion_coef(M, s);
       break;
     case 17: launch_calc_heating(M, s); break;
@@ -256,23 +269,184 @@ int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
 
 int run_stage(epic_model *m, int stage) { return run_stage_on(m->d, m->stream, stage); }
 
-int enqueue_step_on(const DevModel &M, cudaStream_t s) {
-  static const int step[] = {0, 20, 3, 4, 5, 6, 7, 8, 9, 10, 11, 19, 12, 13, 14, 15, 16, 17};
-  // with the turbulence closure (timestep, epic_timestep.c:130-290): source_sink_turb after
-  // calc_w; the scalar subgrid diffusion around the scalars' hyperviscosity; uv_horizontal_subgrid
-  // before divergence damping, uv_vertical_subgrid after the time update (grid.diffusion_direction
-  // chooses which diffusions run)
-  static const int step_turb[] = {0, 20, 21, 3, 4, 22, 5, 23, 6, 7, 8, 9, 10, 11, 19, 12, 24, 13, 14, 25, 15, 16, 17};
-  const int *seq = M.turb ? step_turb : step;
-  const int n = M.turb ? (int)(sizeof(step_turb) / sizeof(int)) : (int)(sizeof(step) / sizeof(int));
-  for (int q = 0; q < n; q++) {
-    const int st = seq[q];
-    if ((st == 22 || st == 24) && !M.turb_h) continue;
-    if ((st == 23 || st == 25) && !M.turb_v) continue;
-    int rc = run_stage_on(M, s, st);
-    if (rc) return rc;
+// The branches of a step.  Many of its kernels do not depend on one another (the momentum
+// tendencies, UNITY, THETA and HDRY until the pressure is integrated; the four fields of the 3-D
+// filter; DUDT and DVDT; U and V), and on all but the largest grids one of them leaves most of the
+// GPU idle, so a captured step runs them as up to LANES branches: lane 0 is the capturing stream,
+// the others join it before the step ends.  Without `side` (a step enqueued directly) every lane
+// is the one stream, and the order of the calls is the order of the kernels.
+constexpr int LANES = 4;
+struct Lanes {
+  cudaStream_t lane[LANES];
+  std::vector<cudaEvent_t> events;
+  bool side = false;
+  int rc = EPIC_OK;
+  explicit Lanes(cudaStream_t s) { for (auto &l : lane) l = s; }
+  Lanes(const Lanes &) = delete;
+  ~Lanes() {
+    for (auto e : events) cudaEventDestroy(e);
+    if (side)
+      for (int q = 1; q < LANES; q++) cudaStreamDestroy(lane[q]);
   }
-  return EPIC_OK;
+  // side streams of their own; false leaves one stream
+  bool open() {
+    for (int q = 1; q < LANES; q++)
+      if (cudaStreamCreateWithFlags(&lane[q], cudaStreamNonBlocking) != cudaSuccess) {
+        while (--q >= 1) cudaStreamDestroy(lane[q]);
+        for (int r = 1; r < LANES; r++) lane[r] = lane[0];
+        return false;
+      }
+    return side = true;
+  }
+  cudaStream_t operator[](int q) const { return lane[q]; }
+  // the point that a lane has reached, and a lane made to go on only after such a point
+  cudaEvent_t point(int from) {
+    if (!side || rc) return nullptr;
+    cudaEvent_t e = nullptr;
+    if (check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming))) {
+      events.push_back(e);
+      check(cudaEventRecord(e, lane[from]));
+    }
+    return e;
+  }
+  void after(int to, cudaEvent_t e) { if (side && !rc) check(cudaStreamWaitEvent(lane[to], e, 0)); }
+  void after(int to, int from) { after(to, point(from)); }
+  bool check(cudaError_t c) {
+    if (c != cudaSuccess) rc = set_error(EPIC_ERR_CUDA, "step branches: %s", cudaGetErrorString(c));
+    return c == cudaSuccess;
+  }
+  void fork() { for (int q = 1; q < LANES; q++) after(q, 0); }
+};
+
+// The launch description with work0..3 of set ws and ptable of set ts.
+DevModel with_scratch(const DevModel &M, int ws, int ts) {
+  DevModel d = M;
+  epic::scratch_sets(d, ws, ts, M.batch ? M.reloc_n3 : M.n3);
+  return d;
+}
+
+// One step (timestep(STEP_PROGS_AND_SYNC_DIAGS), epic_timestep.c:130-390), the stages of
+// run_stage_on in an order of the same dependences.  Scratch: lanes 0, 1 / 3 and 2 hold sets 0, 1
+// and 2 of work0..3 (lane 1's uv_core takes work0 alone, lane 3's scalars work1..3).
+int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
+  using namespace epic;
+  Lanes one(s);
+  Lanes &L = lanes ? *lanes : one;
+  const DevModel M1 = with_scratch(M, 1, 1), M2 = with_scratch(M, 2, 2), M3 = with_scratch(M, 1, 3);
+  auto vertical = M.akima ? launch_akima_vertical : launch_hsu_vertical;
+  auto meridional = M.akima ? launch_akima_meridional : launch_hsu_meridional;
+  auto zonal = M.akima ? launch_akima_zonal : launch_hsu_zonal;
+
+  L.fork();
+  launch_zero_tend(M, L[1]);
+  launch_uv_decide(M, L[1]);
+  launch_advection_prep(M, 0, L[2]);   // UNITY = 1
+  launch_calc_w(M, L[0], true);        // source_sink and calc_w: THETA, W3
+  L.fork();
+  // lane 1: DUDT, DVDT of uv_core and uv_drag
+  launch_uv_core(M1, L[1]);
+  launch_uv_drag(M1, L[1]);
+  // lane 2: UNITY advected
+  vertical(M2, M.unity, 0, L[2]);
+  meridional(M2, M.unity, 0, L[2]);
+  zonal(M2, M.unity, 0, 1, L[2]);
+  if (M.turb) {
+    launch_source_sink_turb(M, L[0]);
+    L.after(0, 1);   // the subgrid diffusion's set_p2etc rewrites P3 and H3, which lane 1 reads
+    if (M.turb_h) launch_scalar_hdiff(M, L[0]);
+    L.after(3, 0);
+  }
+  // lane 3: THETA's hyperviscosity; lane 0: HDRY's
+  launch_meridional_hyperviscosity(M3, 3, M.theta, PL_NONE, L[3]);
+  launch_zonal_hyperviscosity(M3, 3, M.theta, PL_NONE, L[3]);
+  launch_meridional_hyperviscosity(M, 2, M.hdry, PL_NONE, L[0]);
+  launch_zonal_hyperviscosity(M, 2, M.hdry, PL_NONE, L[0]);   // then restore_mass, in the same kernel
+  if (M.turb) {
+    launch_meridional_hyperviscosity(M3, 4, M.nu_turb, PL_NONE, L[3]);
+    launch_zonal_hyperviscosity(M3, 4, M.nu_turb, PL_NONE, L[3]);
+    launch_restore_nu(M, L[3]);
+    if (M.turb_v) {
+      L.after(0, 3);
+      launch_scalar_vdiff(M, L[0]);
+      L.after(3, 0);
+    }
+  }
+  // lane 3: THETA's advection (and NU_TURB's) corrected by UNITY's; lane 0: HDRY's
+  launch_advection_prep(M, 1, L[3]);
+  vertical(M3, M.theta, 1, L[3]);
+  meridional(M3, M.theta, 1, L[3]);
+  zonal(M3, M.theta, 0, M.k_sigma - 1, L[3]);
+  L.after(3, 2);
+  launch_advection_prep(M, 2, L[3]);
+  if (M.turb) {
+    launch_advection_prep(M, 3, L[3]);
+    vertical(M3, M.nu_turb, 3, L[3]);
+    meridional(M3, M.nu_turb, 3, L[3]);
+    zonal(M3, M.nu_turb, 2, 1, L[3]);
+    launch_advection_prep(M, 4, L[3]);
+  }
+  vertical(M, M.hdry, 2, L[0]);
+  meridional(M, M.hdry, 2, L[0]);
+  zonal(M, M.hdry, 1, 1, L[0]);   // then restore_mass, in the same kernel
+  L.after(0, 1);                  // lane 1 has read P3 and H3
+  launch_set_p2etc(M, 0, L[0], true);
+  L.after(0, 3);
+  launch_store_pgrad_vars(M, L[0], true);
+  int rc = run_stage_on(M, L[0], 8);   // the filtered GZ
+  if (rc) return rc;
+  // the 3-D filter: lane 1 DUDT, lane 2 DVDT, lane 3 THETA (and NU_TURB), lane 0 HDRY
+  L.fork();
+  launch_varz_filter(M1, M.dudt, PL_UV_TEND, 0, 1, M.nk, L[1]);
+  launch_varz_filter(M2, M.dvdt, PL_UV_TEND, 1, 1, M.nk, L[2]);
+  launch_varz_filter(M3, M.theta, PL_NONE, 3, M.k_sigma - 1, M.nk, L[3]);
+  if (M.turb) {
+    launch_varz_filter(M3, M.nu_turb, PL_NONE, 4, 0, M.nk, L[3]);
+    launch_restore_nu(M, L[3]);
+  }
+  launch_varz_filter(M, M.hdry, PL_NONE, 2, 1, M.nk, L[0]);   // then restore_mass, in the same kernel
+  L.after(0, 3);
+  launch_set_p2etc(M, 1, L[0]);
+  launch_store_pgrad_vars(M, L[0], false, false);
+  launch_pgrad_poles(M, L[0]);
+  L.after(3, 0);
+  launch_pgrad_dzdt(M, L[3]);      // the rest of store_pgrad_vars
+  launch_calc_heating(M, L[3]);    // of P3 and T3
+  // lane 1: DUDT's pressure gradient, lane 0: DVDT's
+  L.after(1, 0);
+  launch_pgrad_lon(M, L[1]);
+  L.after(0, 2);
+  launch_pgrad_lat(M, L[0]);
+  L.after(0, 1);
+  if (M.turb && M.turb_h) launch_uv_hdiff(M, L[0]);
+  launch_divergence_damping(M, L[0]);
+  L.after(0, 3);                   // DZDT3 reads the winds before their update
+  launch_uv_update(M, L[0]);
+  // Adams-Bashforth: nothing after the update reads the indices that turn (the winds have one plane)
+  if (M.uv_scheme == EPIC_UV_AB3) L.after(3, 0);
+  launch_uv_rotate(M, L[M.uv_scheme == EPIC_UV_AB3 ? 3 : 0]);
+  if (M.turb && M.turb_v) launch_uv_vdiff(M, L[0]);
+  // lane 0: U, lane 1: V; the filtered copies go on in the same lanes
+  L.after(1, 0);
+  launch_meridional_hyperviscosity(M, 0, M.u, PL_UV, L[0]);
+  launch_zonal_hyperviscosity(M, 0, M.u, PL_UV, L[0]);
+  launch_meridional_hyperviscosity(M1, 1, M.v, PL_UV, L[1]);
+  launch_zonal_hyperviscosity(M1, 1, M.v, PL_UV, L[1]);
+  const cudaEvent_t u_done = L.point(0), v_done = L.point(1);
+  launch_diag_filter_u(M, L[0]);
+  launch_diag_filter_v(M1, L[1]);
+  L.after(2, u_done);
+  launch_diag_pv_poles(M, L[2]);
+  L.after(2, v_done);
+  launch_diag_ri2(M, L[2]);
+  L.after(0, v_done);
+  launch_diag_div(M, L[0]);
+  L.after(1, u_done);
+  launch_diag_pv(M1, L[1]);
+  L.after(0, 1);
+  L.after(0, 2);
+  L.after(0, 3);
+  if (M.turb) launch_set_diffusion_coef(M, L[0]);
+  return L.rc ? L.rc : check_launch("step launch");
 }
 
 int enqueue_sync_on(const DevModel &M, cudaStream_t s) {
@@ -292,8 +466,10 @@ int enqueue_sync(epic_model *m) { return enqueue_sync_on(m->d, m->stream); }
 cudaGraphExec_t capture_step(const DevModel &M, cudaStream_t s, int *kernels) {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  Lanes lanes(s);
+  lanes.open();
   if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-    int rc = enqueue_step_on(M, s);
+    int rc = enqueue_step_on(M, s, &lanes);
     if (!rc) rc = epic::launch_itime_advance(M, s);
     cudaError_t e = cudaStreamEndCapture(s, &graph);
     if (rc == EPIC_OK && e == cudaSuccess && graph) {
@@ -419,11 +595,11 @@ size_t model_pool_bytes(const epic_grid &g) {
   const size_t n3 = (size_t)L.n3, n2 = (size_t)L.n2;
   const size_t nvp = g.uv_scheme == EPIC_UV_AB3 ? 1 : 2, ntp = g.uv_scheme == EPIC_UV_AB3 ? 3 : 1;
   const size_t n_state3 = 2 * nvp + 2 * ntp + 20;   // u,v planes + tendencies + 20 single fields
-  const size_t n_scratch3 = 8;                      // gz, unity, old, work0..3, lp3 (float2)
+  const size_t n_scratch3 = epic::SCRATCH_VOLUMES + 1;   // gz, unity, old, the sets of work0..3; lp3 (float2)
   const size_t nj1 = 2 * (g.nj + 1) + 1, ni1 = 2 * (g.ni + 1) + 1, nk1 = 2 * (g.nk + 1) + 1;
   const size_t ntw = epic::twiddle_doubles(g.ni);
   auto rnd = [](size_t b) { return ((b + 255) / 256) * 256; };
-  return rnd(sizeof(Ctl)) + (n_state3 + n_scratch3) * rnd(n3 * 8) + 3 * rnd(n2 * 8) + rnd((size_t)(g.nj + 3) * (g.nk + 2) * 3 * 8) +
+  return rnd(sizeof(Ctl)) + (n_state3 + n_scratch3) * rnd(n3 * 8) + 3 * rnd(n2 * 8) + rnd((size_t)epic::TABLE_SETS * (g.nj + 3) * (g.nk + 2) * 3 * 8) +
          rnd(ni1 * 8) + 10 * rnd(nj1 * 8) + 3 * rnd(nk1 * 8) + rnd((g.nk + 2) * 8) + rnd((g.k_sponge + 1) * 8) +
          2 * rnd(3 * (g.nj + 2) * 8) + rnd(ntw * 8) + rnd(ntw * 4) + 2 * rnd((g.nj + 1) * 8) + rnd(sizeof(epic::MathTable)) +
          rnd(32 * sizeof(float2)) + rnd(((size_t)epic::TH_N * epic::TH_M + 4 * epic::TH_M + epic::TH_N) * 8) +
@@ -559,10 +735,11 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
   p += (256 - ((size_t)(p - m->pool) & 255)) & 255;   // the scratch and tables start 256-aligned
   double **s3[] = {&d.gz, &d.unity, &d.old, &d.work0, &d.work1, &d.work2, &d.work3};
   for (double **q : s3) *q = carve<double>(p, n3);
+  for (int q = 0; q < 4 * (epic::SCRATCH_SETS - 1); q++) carve<double>(p, n3);   // work0..3 of the other sets
   d.lp3 = carve<float2>(p, n3);
   d.gz_surface = carve<double>(p, n2);
   double *hlh = carve<double>(p, n2), *hlpv = carve<double>(p, n2);
-  d.ptable = carve<double>(p, (size_t)(g->nj + 3) * (g->nk + 2) * 3);
+  d.ptable = carve<double>(p, (size_t)epic::TABLE_SETS * (g->nj + 3) * (g->nk + 2) * 3);
   double *lon = carve<double>(p, ni1);
   double *j1[10];
   for (int i = 0; i < 10; i++) j1[i] = carve<double>(p, nj1);
@@ -594,9 +771,9 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
     return set_error(EPIC_ERR_NOMEM, "internal pool layout overflow");
   }
   // the layout relocate_field (batches of mixed sizes) relies on: packed state planes, then the
-  // seven scratch volumes at one stride
+  // scratch volumes at one stride
   if ((const char *)d.u_spinup - (const char *)d.u != (long long)(2 * d.nvp + 2 * d.ntp + 19) * d.n3 * 8 ||
-      (const char *)d.work3 - (const char *)d.gz != 6 * epic::scratch_stride(d.n3)) {
+      (const char *)d.lp3 - (const char *)d.gz != epic::SCRATCH_VOLUMES * epic::scratch_stride(d.n3)) {
     epic_model_destroy(m);
     return set_error(EPIC_ERR_STATE, "internal pool layout differs from the batch relocation's");
   }

@@ -1152,7 +1152,7 @@ __global__ void __launch_bounds__(256) k_gz_from_u(DevModel M) {
   }
 }
 
-int launch_store_pgrad_vars(const DevModel &M, cudaStream_t s, bool early) {
+int launch_store_pgrad_vars(const DevModel &M, cudaStream_t s, bool early, bool dzdt) {
   if (M.gas_giant) {
     k_gz_means<<<zg(M.nj + 1, M), 256, (size_t)3 * M.ni * sizeof(double), s>>>(M);
     k_gz_from_u<<<zg(1, M), 256, (size_t)(7 * M.nj + 8) * sizeof(double), s>>>(M);
@@ -1168,6 +1168,9 @@ int launch_store_pgrad_vars(const DevModel &M, cudaStream_t s, bool early) {
   if (M.col64) (h2 ? k_pgrad_vars_column_acc_h2 : k_pgrad_vars_column_acc)<<<grid, CT_THREADS, smem, s>>>(M);
   else if (M.mixed) (h2 ? k_pgrad_vars_column_mixed<true, true> : k_pgrad_vars_column_mixed<true, false>)<<<grid, CT_THREADS, smem, s>>>(M);
   else k_pgrad_vars_column<<<grid, CT_THREADS, tile_smem(M, 6), s>>>(M);
+  return dzdt ? launch_pgrad_dzdt(M, s) : 0;
+}
+int launch_pgrad_dzdt(const DevModel &M, cudaStream_t s) {
   EPIC_LAUNCH_R(M.mixed, k_pgrad_dzdt, epic_blocks((long long)M.nk * (M.nj + 1) * M.ni, TB(M, TB_UPDATE)), TB(M, TB_UPDATE), 0, s, M);
   return 0;
 }

@@ -1086,9 +1086,7 @@ __global__ void k_uv_rotate(DevModel M) {
     c->it_minus2 = c->it_minus1;
     c->it_minus1 = c->it_zero;
     c->it_zero = itmp;
-    c->it_uv = 0;
-    c->it_uv_dis = 0;
-    c->it_uv_tend = c->it_zero;
+    c->it_uv_tend = c->it_zero;   // it_uv and it_uv_dis stay 0: one plane (branches of the step read them meanwhile)
   } else {
     const int itmp = c->it_minus1;
     c->it_minus1 = c->it_zero;
@@ -1139,22 +1137,23 @@ int launch_uv_core(const DevModel &M, cudaStream_t s) {
 // k_pgrad_lon's face exchange: one face per thread of the block
 static size_t lon_smem(const DevModel &M, size_t face_bytes) { return (size_t)TB(M, TB_PGRAD) * face_bytes; }
 
-int launch_uv_pgrad(const DevModel &M, cudaStream_t s) {
+int launch_pgrad_poles(const DevModel &M, cudaStream_t s) {
   k_gz_pole_rows<<<zg(M.nk + 1, M), 128, 0, s>>>(M);
-  // FP64 form: binary64; mixed: double-float on the splits; fast mixed: binary32 on the splits
-  const dim3 glon = zg(cells_blocks(M, M.nk - 1, M.nj + 1, TB(M, TB_PGRAD)), M), glat = zg(cells_blocks(M, M.nk - 1, M.nj, TB(M, TB_PGRAD)), M);
-  if (!M.mixed) {
-    k_pgrad_lon<double><<<glon, TB(M, TB_PGRAD), lon_smem(M, sizeof(LonFace<double>)), s>>>(M);
-    k_pgrad_lat<double><<<glat, TB(M, TB_PGRAD), 0, s>>>(M);
-    return 0;
-  }
-  if (M.col64) {
-    k_pgrad_lon<dfl><<<glon, TB(M, TB_PGRAD), lon_smem(M, sizeof(LonFace<dfl>)), s>>>(M);
-    k_pgrad_lat<dfl><<<glat, TB(M, TB_PGRAD), 0, s>>>(M);
-  } else {
-    k_pgrad_lon<float><<<glon, TB(M, TB_PGRAD), 0, s>>>(M);
-    k_pgrad_lat<float><<<glat, TB(M, TB_PGRAD), 0, s>>>(M);
-  }
+  return 0;
+}
+// FP64 form: binary64; mixed: double-float on the splits; fast mixed: binary32 on the splits
+int launch_pgrad_lon(const DevModel &M, cudaStream_t s) {
+  const dim3 grid = zg(cells_blocks(M, M.nk - 1, M.nj + 1, TB(M, TB_PGRAD)), M);
+  if (!M.mixed) k_pgrad_lon<double><<<grid, TB(M, TB_PGRAD), lon_smem(M, sizeof(LonFace<double>)), s>>>(M);
+  else if (M.col64) k_pgrad_lon<dfl><<<grid, TB(M, TB_PGRAD), lon_smem(M, sizeof(LonFace<dfl>)), s>>>(M);
+  else k_pgrad_lon<float><<<grid, TB(M, TB_PGRAD), 0, s>>>(M);
+  return 0;
+}
+int launch_pgrad_lat(const DevModel &M, cudaStream_t s) {
+  const dim3 grid = zg(cells_blocks(M, M.nk - 1, M.nj, TB(M, TB_PGRAD)), M);
+  if (!M.mixed) k_pgrad_lat<double><<<grid, TB(M, TB_PGRAD), 0, s>>>(M);
+  else if (M.col64) k_pgrad_lat<dfl><<<grid, TB(M, TB_PGRAD), 0, s>>>(M);
+  else k_pgrad_lat<float><<<grid, TB(M, TB_PGRAD), 0, s>>>(M);
   return 0;
 }
 
@@ -1269,21 +1268,38 @@ int launch_divergence_damping(const DevModel &M, cudaStream_t s) {
   return 0;
 }
 
-int launch_uv_update(const DevModel &M, cudaStream_t s) {
+int launch_uv_decide(const DevModel &M, cudaStream_t s) {
   k_uv_decide<<<zg(1, M), 1, 0, s>>>(M);
+  return 0;
+}
+int launch_uv_update(const DevModel &M, cudaStream_t s) {
   k_uv_update<<<zg(epic_blocks(2LL * (M.nk - 1) * (M.nj + 1) * M.ni, TB(M, TB_UPDATE)), M), TB(M, TB_UPDATE), 0, s>>>(M);
+  return 0;
+}
+int launch_uv_rotate(const DevModel &M, cudaStream_t s) {
   k_uv_rotate<<<zg(1, M), 1, 0, s>>>(M);
   return 0;
 }
 
-int launch_store_diag(const DevModel &M, cudaStream_t s) {
-  // PV3: filtered copy of V (v rows), then the interior and polar values.
-  launch_filter_planes(M, M.v, PL_UV, M.work1, 0, M.nk + 1, 1, s, M.mixed);
+int launch_diag_filter_v(const DevModel &M, cudaStream_t s) {
+  return launch_filter_planes(M, M.v, PL_UV, M.work1, 0, M.nk + 1, 1, s, M.mixed);
+}
+int launch_diag_filter_u(const DevModel &M, cudaStream_t s) {
+  return launch_filter_planes(M, M.u, PL_UV, M.work2, 0, M.nk + 1, 0, s, M.mixed);
+}
+int launch_diag_pv(const DevModel &M, cudaStream_t s) {
   EPIC_LAUNCH_R(M.mixed, k_pv_interior, cells_blocks(M, M.nk + 1, M.nj, TB(M, TB_DIAG)), TB(M, TB_DIAG), 0, s, M, M.work1);
+  return 0;
+}
+int launch_diag_pv_poles(const DevModel &M, cudaStream_t s) {
   k_pv_poles<<<zg(M.nk + 1, M), 128, 4 * M.ni * sizeof(double), s>>>(M);
-  // DIV_UV3 from a filtered copy of U.
-  launch_filter_planes(M, M.u, PL_UV, M.work2, 0, M.nk + 1, 0, s, M.mixed);
+  return 0;
+}
+int launch_diag_div(const DevModel &M, cudaStream_t s) {
   EPIC_LAUNCH_R(M.mixed, k_divergence, cells_blocks(M, M.nk + 1, M.nj + 1, TB(M, TB_DIAG)), TB(M, TB_DIAG), 0, s, M, M.work2, M.v, PL_UV, M.div_uv3, 0, M.nk + 1);
+  return 0;
+}
+int launch_diag_ri2(const DevModel &M, cudaStream_t s) {
   EPIC_LAUNCH_R(M.mixed, k_ri2, cells_blocks(M, M.nk, M.nj + 1, TB(M, TB_DIAG)), TB(M, TB_DIAG), 0, s, M);
   return 0;
 }

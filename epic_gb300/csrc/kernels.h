@@ -83,7 +83,9 @@ int launch_restore_mass(const DevModel &M, cudaStream_t s);
 // GZ3 places the 3-D filter's profiles, so it needs their accuracy; EPIC_PREC_MIXED_FAST with
 // its FP32 ones).  The FP64 form writes everything in every call, as the reference does.
 int launch_set_p2etc(const DevModel &M, int update_theta, cudaStream_t s, bool early = false);
-int launch_store_pgrad_vars(const DevModel &M, cudaStream_t s, bool early = false);
+// dzdt: its horizontal part of DZDT3 too (launch_pgrad_dzdt).
+int launch_store_pgrad_vars(const DevModel &M, cudaStream_t s, bool early = false, bool dzdt = true);
+int launch_pgrad_dzdt(const DevModel &M, cudaStream_t s);
 int launch_gz_monotone(const DevModel &M, cudaStream_t s);
 int launch_calc_heating(const DevModel &M, cudaStream_t s);
 int launch_advection_prep(const DevModel &M, int phase, cudaStream_t s);
@@ -93,7 +95,10 @@ int column_kernels_init(int nk);
 int launch_copy_gz(const DevModel &M, cudaStream_t s);
 int launch_zero_tend(const DevModel &M, cudaStream_t s);
 int launch_uv_core(const DevModel &M, cudaStream_t s);
-int launch_uv_pgrad(const DevModel &M, cudaStream_t s);
+// uv_pgrad_finite_volume: GZ3's pole rows, then DUDT (lon) and DVDT (lat), independent of each other
+int launch_pgrad_poles(const DevModel &M, cudaStream_t s);
+int launch_pgrad_lon(const DevModel &M, cudaStream_t s);
+int launch_pgrad_lat(const DevModel &M, cudaStream_t s);
 int launch_hsu_meridional(const DevModel &M, double *buff, int kind, cudaStream_t s);
 // akima_advection (epic_flux.c:1502-1940), the other advection scheme: vertical (k_column.cu),
 // meridional (k_stencil.cu) and zonal (k_filter.cu) passes, arguments as their Hsu counterparts
@@ -103,8 +108,19 @@ int launch_akima_zonal(const DevModel &M, double *buff, int kind, int kstart, cu
 int launch_meridional_hyperviscosity(const DevModel &M, int index, double *var, int sel, cudaStream_t s);
 int launch_zonal_hyperviscosity(const DevModel &M, int index, double *var, int sel, cudaStream_t s);
 int launch_divergence_damping(const DevModel &M, cudaStream_t s);
+// the time update: which scheme coefficients this step takes (decide: from the tendency planes of
+// earlier steps alone), the update, the rotation of the time-plane indices
+int launch_uv_decide(const DevModel &M, cudaStream_t s);
 int launch_uv_update(const DevModel &M, cudaStream_t s);
-int launch_store_diag(const DevModel &M, cudaStream_t s);
+int launch_uv_rotate(const DevModel &M, cudaStream_t s);
+// store_diag: the filtered copies of V (into work1) and U (into work2), PV3 from the first with its
+// polar values, DIV_UV3 from the second, RI2
+int launch_diag_filter_v(const DevModel &M, cudaStream_t s);
+int launch_diag_filter_u(const DevModel &M, cudaStream_t s);
+int launch_diag_pv(const DevModel &M, cudaStream_t s);
+int launch_diag_pv_poles(const DevModel &M, cudaStream_t s);
+int launch_diag_div(const DevModel &M, cudaStream_t s);
+int launch_diag_ri2(const DevModel &M, cudaStream_t s);
 int launch_itime_advance(const DevModel &M, cudaStream_t s);
 int launch_set_itime(const DevModel &M, long long itime, cudaStream_t s);
 
