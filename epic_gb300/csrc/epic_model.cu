@@ -202,15 +202,14 @@ int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
     // EPIC_PREC_MIXED computes it in double-float like stage 19 (the FP32 kernel made the wind
     // error after a day ~2x larger); EPIC_PREC_MIXED_FAST keeps the FP32 kernel.
     case 7: launch_store_pgrad_vars(M, s, true); break;
-    case 8:
-      launch_copy_gz(M, s);
+    case 8:   // from GZ3 into its copy GZ (epic_timestep.c:176-195)
       // The 3-D filter's profiles interpolate in the filtered GZ: filtering GZ itself in FP32
       // makes the mixed form's V error after a day grow from 4e-5 to 7e-5 (leapfrog: 1.7e-4 ->
       // 1.6e-3).  The mixed forms filter it on the tensor cores as GZ - GZ(i=1) per row (FP32
       // rounding of the zonal variations only) where the operator product applies, the FP64 form
       // in binary64.
-      if (M.mixed && filter_gemm_usable(M)) launch_filter_planes(M, M.gz, PL_NONE, M.gz, 0, M.nk, 0, s, 1, 1);
-      else launch_filter_planes(M, M.gz, PL_NONE, M.gz, 0, M.nk, 0, s);
+      if (M.mixed && filter_gemm_usable(M)) launch_filter_planes(M, M.gz3, PL_NONE, M.gz, 0, M.nk, 0, s, 1, 1);
+      else launch_filter_planes(M, M.gz3, PL_NONE, M.gz, 0, M.nk, 0, s);
       launch_gz_monotone(M, s);
       break;
     case 9:
@@ -847,6 +846,7 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
   epic::filter_kernels_init(g->ni);
   epic::column_kernels_init(g->nk);
   epic::column_acc_kernels_init();
+  epic::stencil_kernels_init();
   epic::filter_gemm_init(g->ni);
   e = cudaStreamSynchronize(m->stream);
   if (e != cudaSuccess) {

@@ -925,22 +925,35 @@ __global__ void k_pgrad_dzdt(DevModel M) {
 }
 
 // Monotone fix of the filtered GZ copy, epic_timestep.c:182-195 (the zonal filter of planes
-// 0..nk-1 has already run; each plane's fix only needs the finished plane below it).
+// 0..nk-1, from GZ3 into GZ, has already run; each plane's fix only needs the finished plane below
+// it, the lowest being GZ3's own).  A column's levels are loaded eight at a time before the chain
+// that uses them: one load after another, each waiting behind the store of the level before, took
+// 15 us at 128x64x20.
 __global__ void k_gz_monotone(DevModel M) {
   if (epic_member(M)) return;
   int j, i;
   if (!col_index(M, j, i)) return;
-  double below = M.gz[M.at(M.nk, j, i)];
-  for (int k = M.nk - 1; k >= 0; k--) {
-    const long long x = M.at(k, j, i);
-    double g;
-    // fcmp(below, 0.) == 0 holds exactly when below is +-0 or NaN (for any other value the
-    // tolerance, DBL_EPSILON times 2^exponent, is below |below|): tested without frexp/ldexp,
-    // which cost ten FP64 instructions a level
-    if (below == 0. || below != below) g = 1.e-3;
-    else g = dmaxr(M.gz[x], below + fabs(below) * 1.e-5);
-    M.gz[x] = g;
-    below = g;
+  constexpr int NL = 8;
+  const int base = M.at(0, j, i), n2 = (int)M.n2;
+  double below = M.gz3[base + M.nk * n2];
+  M.gz[base + M.nk * n2] = below;
+  for (int kt = M.nk - 1; kt >= 0; kt -= NL) {
+    double v[NL];
+#pragma unroll
+    for (int q = 0; q < NL; q++) v[q] = M.gz[base + max(kt - q, 0) * n2];
+#pragma unroll
+    for (int q = 0; q < NL; q++) {
+      if (kt - q < 0) break;
+      double g;
+      // fcmp(below, 0.) == 0 holds exactly when below is +-0 or NaN (for any other value the
+      // tolerance, DBL_EPSILON times 2^exponent, is below |below|): tested on its bits, since
+      // frexp/ldexp and comparisons are binary64 operations
+      const unsigned long long u = (unsigned long long)__double_as_longlong(below) << 1;
+      if (u - 1 >= 0xffe0000000000000ull) g = 1.e-3;
+      else g = dmaxr(v[q], below + fabs(below) * 1.e-5);
+      M.gz[base + (kt - q) * n2] = g;
+      below = g;
+    }
   }
 }
 

@@ -35,13 +35,6 @@ static inline unsigned cells_blocks(const DevModel &M, int nkk, int njj, int th)
 }
 __device__ __forceinline__ int wrap_i(const DevModel &M, int i) { return i == 0 ? M.ni : (i == M.ni + 1 ? 1 : i); }
 
-// The copy of GZ3 that the filtered geopotential starts from, epic_timestep.c:176-181.
-__global__ void k_copy_gz(DevModel M) {
-  if (epic_member(M)) return;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < M.n3) M.gz[t] = M.gz3[t];
-}
-
 // memset of DUDT, DVDT(it_uv_tend), epic_timestep.c:107-108
 __global__ void k_zero_tend(DevModel M) {
   if (epic_member(M)) return;
@@ -145,26 +138,44 @@ __global__ void k_uv_core_u(DevModel M) {
 // uv_pgrad_finite_volume, epic_timestep.c:909-1273
 // ---------------------------------------------------------------------------------------------
 
+// Row sums in the reference's order (one addition after another) occupy the binary64 pipe for a
+// whole warp instruction per addition whatever the number of active lanes, so the kernels that need
+// them stage several rows in shared memory and sum one row per lane.  Rows lie ni+1 (an odd number
+// of) values apart, which keeps the lanes on different banks.  ROW_SUM_SMEM bounds a block's rows.
+constexpr size_t ROW_SUM_SMEM = 48 * 1024;
+static __device__ __forceinline__ double row_sum(const double *row, int n) {
+  double sum = 0.;
+#pragma unroll 8
+  for (int i = 0; i < n; i++) sum += row[i];
+  return sum;
+}
+// levels per block of a kernel that sums `rows` rows of each, one per lane of a warp
+static int row_sum_levels(const DevModel &M, int rows) {
+  const int fit = (int)(ROW_SUM_SMEM / ((size_t)rows * (M.ni + 1) * sizeof(double)));
+  return fit < 1 ? 1 : (fit > 32 / rows ? 32 / rows : fit);
+}
+
 // Pole boundary rows of GZ3 (zonal means of the adjacent row), epic_timestep.c:930-998.
-// One block per k; thread 0 sums in the reference order.
-__global__ void k_gz_pole_rows(DevModel M) {
+// One block per lv levels, the two rows of each summed in the reference's order, a row per lane.
+// With the rows read from global memory by one thread of a block per level it took 14 us at
+// 128x64x20 (row_sum's comment).
+__global__ void __launch_bounds__(256) k_gz_pole_rows(DevModel M, int lv) {
   if (epic_member(M)) return;
-  const int k = blockIdx.x;
-  __shared__ double avg[2];
-  if (threadIdx.x < 2) {
-    const int j = threadIdx.x == 0 ? 0 : M.nj;
-    double tmp = 0.;
-    for (int i = 1; i <= M.ni; i++) tmp += M.gz3[M.at(k, j, i)];
-    avg[threadIdx.x] = tmp / M.ni;
+  extern __shared__ double rows[];   // [lv][2][ni+1]: rows 0 and nj of each level
+  __shared__ double avg[32];
+  const int ni = M.ni, k0 = (int)blockIdx.x * lv, nl = min(lv, M.nk + 1 - k0);
+  for (int t = (int)threadIdx.x; t < 2 * nl * ni; t += (int)blockDim.x) {
+    const int r = t / ni, i = t - r * ni;
+    rows[r * (ni + 1) + i] = M.gz3[M.at(k0 + (r >> 1), (r & 1) ? M.nj : 0, i + 1)];
   }
   __syncthreads();
-  for (int i = threadIdx.x; i <= M.ni + 1; i += blockDim.x) {
-    M.gz3[M.at(k, -1, i)] = avg[0];
-    M.gz3[M.at(k, M.nj + 1, i)] = avg[1];
-    if (M.mixed) {
-      put_split(M.work1, M.at(k, -1, i), avg[0]);
-      put_split(M.work1, M.at(k, M.nj + 1, i), avg[1]);
-    }
+  if ((int)threadIdx.x < 2 * nl) avg[threadIdx.x] = row_sum(rows + (int)threadIdx.x * (ni + 1), ni) / ni;
+  __syncthreads();
+  for (int t = (int)threadIdx.x; t < 2 * nl * (ni + 2); t += (int)blockDim.x) {
+    const int r = t / (ni + 2), i = t - r * (ni + 2);
+    const int x = M.at(k0 + (r >> 1), (r & 1) ? M.nj + 1 : -1, i);
+    M.gz3[x] = avg[r];
+    if (M.mixed) put_split(M.work1, x, avg[r]);
   }
 }
 
@@ -777,11 +788,85 @@ __global__ void k_visc_apply(DevModel M, double *A, int sel, const double *D, in
   write_with_pads(A, M, M.at(c.k, c.j, 0), c.i, A[x] + to_d(cv<R>(M.dt) * cv<R>(sign) * cv<R>(D[x])));
 }
 
-// zonal_hyperviscosity, epic_subgrid.c:715-808: one warp per row (j, k), rows_per_block rows
-// per block.  The updated row stays in FP64 in both forms.  The FP64 form sums the row mean in
-// the reference's order on lane 0; the mixed form sums it in FP64 with a warp reduction.
-template <class R>
-__global__ void k_zonal_visc(DevModel M, double *A, int sel, int jbot, int jhalf, int k0, int restore) {
+// zonal_hyperviscosity, epic_subgrid.c:715-808, in the FP64 form: `rows` rows per block, a warp per
+// row at a time; the row means, in the reference's order, by one warp with a row per lane (row_sum).
+// Bound by those additions: with one lane of each row's warp summing it, 4 orders x ni additions a row
+// held the binary64 pipe (71% busy) for 36 us a field at 128x64x20.
+__global__ void __launch_bounds__(256) k_zonal_visc_rows(DevModel M, double *A, int sel, int jbot, int jhalf, int k0, int nkk, int restore, int rows) {
+  if (epic_member(M, A)) return;
+  extern __shared__ double vr[];
+  __shared__ double s_mean[32];
+  const int ni = M.ni, W = ni + 3, lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
+  const int nr = M.nj - jbot + 1;
+  const int row0 = (int)blockIdx.x * rows, nl = min(rows, nr * nkk - row0);
+  if (nl <= 0) return;   // a member with fewer rows than the launch
+  A += plane_offset(M, sel);
+  double *a = vr, *h = a + rows * W, *d = h + rows * W;
+  auto row_at = [&](int r, int &j, int &k) {
+    const int q = (row0 + r) / nr;
+    k = k0 + q;
+    j = jbot + row0 + r - q * nr;
+  };
+  for (int r = w; r < nl; r += nw) {
+    int j, k;
+    row_at(r, j, k);
+    const int base = M.at(k, j, 0);
+    for (int i = lane; i <= ni + 1; i += 32) a[r * W + i] = h[r * W + i] = A[base + i];
+  }
+  __syncwarp();
+  double sign = 1.;
+  bool any_applied = false;
+  // fully unrolled so that M.coef[], M.nu[] are indexed by constants (M stays in registers)
+#pragma unroll
+  for (int itmp = 2; itmp <= 8; itmp += 2) {
+    for (int r = w; r < nl; r += nw) {
+      int j, k;
+      row_at(r, j, k);
+      const double mm = M.m[2 * j + jhalf];
+      const double dc = fabs(M.lat[2 * j + jhalf]) > M.lat0 ? M.coef[itmp] * M.m0 * M.m0 : M.coef[itmp] * mm * mm;
+      const double *hr = h + r * W;
+      for (int i = lane + 1; i <= ni; i += 32) d[r * W + i] = dc * (hr[i - 1] - 2. * hr[i] + hr[i + 1]);
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < nl) s_mean[threadIdx.x] = row_sum(d + (int)threadIdx.x * W + 1, ni) / ni;
+    __syncthreads();
+    for (int r = w; r < nl; r += nw) {
+      const double mean = s_mean[r];
+      double *dr = d + r * W;
+      for (int i = lane + 1; i <= ni; i += 32) {
+        const double v = dr[i] - mean;
+        dr[i] = v;
+        if (i == 1) dr[ni + 1] = v;
+        if (i == ni) dr[0] = v;
+        if (M.nu[itmp] > 0.) a[r * W + i] += M.dt * sign * v;
+      }
+    }
+    __syncwarp();
+    if (M.nu[itmp] > 0.) any_applied = true;
+    sign = -sign;
+    double rest = 0.;
+#pragma unroll
+    for (int q = itmp + 2; q <= 8; q += 2) rest += M.nu[q];
+    if (!(rest > 0.)) break;
+    double *t = h; h = d; d = t;   // swap roles
+  }
+  // restore (HDRY): restore_mass, which the hyperviscosity step calls next (epic_subgrid.c:240),
+  // on the new row -- the same max per cell, one pass fewer
+  if (any_applied || restore)
+    for (int r = w; r < nl; r += nw) {
+      int j, k;
+      row_at(r, j, k);
+      const int base = M.at(k, j, 0);
+      for (int i = lane + 1; i <= ni; i += 32) {
+        const double v = a[r * W + i];
+        write_with_pads(A, M, base, i, restore ? dmaxr(M.h_min[k], v) : v);
+      }
+    }
+}
+
+// The same in the mixed forms: one warp per row (j, k), blockDim.x / 32 rows per block.  The updated
+// row stays in FP64; the row mean is an FP32 warp reduction.
+__global__ void k_zonal_visc_mixed(DevModel M, double *A, int sel, int jbot, int jhalf, int k0, int restore) {
   if (epic_member(M, A)) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int ni = M.ni, lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
@@ -790,71 +875,51 @@ __global__ void k_zonal_visc(DevModel M, double *A, int sel, int jbot, int jhalf
   if (j > M.nj) return;
   A += plane_offset(M, sel);
   const long long base = M.at(k, j, 0);
-  const size_t row_bytes = (size_t)(ni + 2) * (sizeof(double) + 2 * sizeof(R));
+  const size_t row_bytes = (size_t)(ni + 2) * (sizeof(double) + 2 * sizeof(float));
   double *a = reinterpret_cast<double *>(smraw + w * row_bytes);
-  R *hh = reinterpret_cast<R *>(a + (ni + 2)), *d = hh + (ni + 2);
+  float *hh = reinterpret_cast<float *>(a + (ni + 2)), *d = hh + (ni + 2);
   const unsigned full = 0xffffffffu;
-  for (int i = lane; i <= ni + 1; i += 32) { a[i] = A[base + i]; hh[i] = cv<R>(a[i]); }
+  for (int i = lane; i <= ni + 1; i += 32) a[i] = A[base + i];
   __syncwarp();
-  if (!std::is_same_v<R, double>) {
-    // the mixed forms' first second difference is of the field itself: its neighbour
-    // differences a(i+1) - a(i) in binary64, one per point (k_d2dy2)
-    for (int i = lane; i <= ni; i += 32) hh[i] = cv<R>(a[i + 1] - a[i]);
-    __syncwarp();
-  }
+  // the first second difference is of the field itself: its neighbour differences a(i+1) - a(i) in
+  // binary64, one per point (k_d2dy2)
+  for (int i = lane; i <= ni; i += 32) hh[i] = d2f(a[i + 1] - a[i]);
+  __syncwarp();
   const bool taper = fabs(M.lat[2 * j + jhalf]) > M.lat0;
   const double mm = M.m[2 * j + jhalf];
-  R sign = R(1.);
+  float sign = 1.f;
   bool any_applied = false;
   // fully unrolled so that M.coef[], M.nu[] are indexed by constants (M stays in registers)
 #pragma unroll
   for (int itmp = 2; itmp <= 8; itmp += 2) {
-    const R dc = cv<R>(taper ? M.coef[itmp] * M.m0 * M.m0 : M.coef[itmp] * mm * mm);
-    if (!std::is_same_v<R, double> && itmp == 2)   // differences of the neighbour differences
-      for (int i = lane + 1; i <= ni; i += 32) d[i] = dc * (hh[i] - hh[i - 1]);
-    else
-      for (int i = lane + 1; i <= ni; i += 32) d[i] = dc * (hh[i - 1] - R(2.) * hh[i] + hh[i + 1]);
+    const float dc = d2f(taper ? M.coef[itmp] * M.m0 * M.m0 : M.coef[itmp] * mm * mm);
+    // the row sum of a periodic second difference vanishes but for rounding: FP32 suffices
+    float fm = 0.f;
+    for (int i = lane + 1; i <= ni; i += 32) {
+      const float v = itmp == 2 ? dc * (hh[i] - hh[i - 1]) : dc * (hh[i - 1] - 2.f * hh[i] + hh[i + 1]);
+      d[i] = v;
+      fm += v;
+    }
+    for (int o = 16; o > 0; o >>= 1) fm += __shfl_xor_sync(full, fm, o);
+    const float mean = fm / (float)ni;
     __syncwarp();
-    R mean;
-    if (sizeof(R) == sizeof(double)) {
-      double mv = 0.;
-      if (lane == 0) {
-        d[ni + 1] = d[1];
-        d[0] = d[ni];
-        double fm = 0.;
-        for (int i = 1; i <= ni; i++) fm += d[i];
-        mv = fm / ni;
-      }
-      mean = cv<R>(__shfl_sync(full, mv, 0));
-    } else {
-      // the row sum of a periodic second difference vanishes but for rounding: FP32 suffices
-      float fm = 0.f;
-      for (int i = lane + 1; i <= ni; i += 32) fm += d[i];
-      for (int o = 16; o > 0; o >>= 1) fm += __shfl_xor_sync(full, fm, o);
-      mean = fm / (float)ni;
-      if (lane == 0) {
-        d[ni + 1] = d[1];
-        d[0] = d[ni];
-      }
+    for (int i = lane + 1; i <= ni; i += 32) {
+      const float v = d[i] - mean;
+      d[i] = v;
+      if (i == 1) d[ni + 1] = v;
+      if (i == ni) d[0] = v;
+      if (M.nu[itmp] > 0.) a[i] += f2d(d2f(M.dt) * sign * v);
     }
     __syncwarp();
-    for (int i = lane; i <= ni + 1; i += 32) d[i] -= mean;
-    __syncwarp();
-    if (M.nu[itmp] > 0.) {
-      for (int i = lane + 1; i <= ni; i += 32) a[i] += to_d(cv<R>(M.dt) * sign * d[i]);
-      any_applied = true;
-    }
+    if (M.nu[itmp] > 0.) any_applied = true;
     sign = -sign;
     double rest = 0.;
 #pragma unroll
     for (int q = itmp + 2; q <= 8; q += 2) rest += M.nu[q];
     if (!(rest > 0.)) break;
-    for (int i = lane; i <= ni + 1; i += 32) hh[i] = d[i];   // swap roles
-    __syncwarp();
+    float *t = hh; hh = d; d = t;   // swap roles
   }
-  __syncwarp();
-  // restore (HDRY): restore_mass, which the hyperviscosity step calls next (epic_subgrid.c:240),
-  // on the new row -- the same max per cell, one pass fewer
+  // restore (HDRY): restore_mass too (k_zonal_visc_rows)
   if (any_applied || restore)
     for (int i = lane + 1; i <= ni; i += 32) write_with_pads(A, M, base, i, restore ? dmaxr(M.h_min[k], a[i]) : a[i]);
 }
@@ -907,41 +972,36 @@ __global__ void k_pv_interior(DevModel M, const double *VV) {
 }
 
 // Polar potential vorticity from the circulation of the adjacent u row, :4279-4341.
-// One block per plane; thread 0 forms the sums in the reference order.
-__global__ void k_pv_poles(DevModel M) {
+// One block per lv planes: the four rows of each staged by every thread, then summed in the
+// reference's order, a row per lane.  One thread summing a plane's four rows one after another took
+// 27 us at 128x64x20.
+__global__ void __launch_bounds__(256) k_pv_poles(DevModel M, int lv) {
   if (epic_member(M)) return;
-  const int k = blockIdx.x;
+  extern __shared__ double rows[];   // [lv][4][ni+1]: U(j=0), H(j=0), U(j=nj), H(j=nj) of each plane
+  __shared__ double sum[32], pole[16];
+  const int ni = M.ni, J = M.nj, k0 = (int)blockIdx.x * lv, nl = min(lv, M.nk + 1 - k0);
   const double *UU = M.u + plane_offset(M, PL_UV);
   const double *HH = M.h3;
-  __shared__ double pole[2];
-  // the four rows are staged by every thread, then summed by one thread in the reference's order
-  extern __shared__ double rows[];   // [4][ni]: U(j=0), H(j=0), U(j=nj), H(j=nj)
-  const int ni = M.ni, J = M.nj;
-  for (int i = threadIdx.x; i < ni; i += blockDim.x) {
-    rows[i] = UU[M.at(k, 0, i + 1)];
-    rows[ni + i] = HH[M.at(k, 0, i + 1)];
-    rows[2 * ni + i] = UU[M.at(k, J, i + 1)];
-    rows[3 * ni + i] = HH[M.at(k, J, i + 1)];
+  for (int t = (int)threadIdx.x; t < 4 * nl * ni; t += (int)blockDim.x) {
+    const int r = t / ni, i = t - r * ni;
+    const double v = ((r & 1) ? HH : UU)[M.at(k0 + (r >> 2), (r & 2) ? J : 0, i + 1)];
+    rows[r * (ni + 1) + i] = (r & 3) == 0 ? -v : v;   // the south's circulation is the negated sum
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double ze = 0., h = 0.;
-    for (int i = 0; i < ni; i++) ze -= rows[i];
-    ze *= M.mn[0] / ((M.m[1]) * (double)(M.ni));
-    for (int i = 0; i < ni; i++) h += rows[ni + i];
+  const int t = (int)threadIdx.x;
+  if (t < 4 * nl) sum[t] = row_sum(rows + t * (ni + 1), ni);
+  __syncthreads();
+  if (t < 2 * nl) {
+    const int north = t & 1;
+    double ze = sum[2 * t], h = sum[2 * t + 1];
+    ze *= north ? M.mn[2 * (J + 1)] / (M.m[2 * J + 1] * (double)(M.ni)) : M.mn[0] / ((M.m[1]) * (double)(M.ni));
     h /= (double)(M.ni);
-    pole[0] = (ze + M.f[0]) / h;
-    ze = 0.; h = 0.;
-    for (int i = 0; i < ni; i++) ze += rows[2 * ni + i];
-    ze *= M.mn[2 * (J + 1)] / (M.m[2 * J + 1] * (double)(M.ni));
-    for (int i = 0; i < ni; i++) h += rows[3 * ni + i];
-    h /= (double)(M.ni);
-    pole[1] = (ze + M.f[2 * (J + 1)]) / h;
+    pole[t] = (ze + (north ? M.f[2 * (J + 1)] : M.f[0])) / h;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i <= M.ni + 1; i += blockDim.x) {
-    M.pv3[M.at(k, 0, i)] = pole[0];
-    M.pv3[M.at(k, M.nj + 1, i)] = pole[1];
+  for (int q = (int)threadIdx.x; q < 2 * nl * (ni + 2); q += (int)blockDim.x) {
+    const int r = q / (ni + 2), i = q - r * (ni + 2);
+    M.pv3[M.at(k0 + (r >> 1), (r & 1) ? M.nj + 1 : 0, i)] = pole[r];
   }
 }
 
@@ -1115,11 +1175,6 @@ __global__ void k_set_itime(DevModel M, long long itime) {
 
 // ---- launchers ----
 
-int launch_copy_gz(const DevModel &M, cudaStream_t s) {
-  k_copy_gz<<<zg(epic_blocks(M.n3, TB(M, TB_POINT)), M), TB(M, TB_POINT), 0, s>>>(M);
-  return 0;
-}
-
 int launch_zero_tend(const DevModel &M, cudaStream_t s) {
   k_zero_tend<<<zg(epic_blocks(M.n3, TB(M, TB_POINT)), M), TB(M, TB_POINT), 0, s>>>(M);
   return 0;
@@ -1138,7 +1193,8 @@ int launch_uv_core(const DevModel &M, cudaStream_t s) {
 static size_t lon_smem(const DevModel &M, size_t face_bytes) { return (size_t)TB(M, TB_PGRAD) * face_bytes; }
 
 int launch_pgrad_poles(const DevModel &M, cudaStream_t s) {
-  k_gz_pole_rows<<<zg(M.nk + 1, M), 128, 0, s>>>(M);
+  const int lv = row_sum_levels(M, 2);
+  k_gz_pole_rows<<<zg(epic_blocks(M.nk + 1, lv), M), 256, (size_t)2 * lv * (M.ni + 1) * sizeof(double), s>>>(M, lv);
   return 0;
 }
 // FP64 form: binary64; mixed: double-float on the splits; fast mixed: binary32 on the splits
@@ -1245,19 +1301,37 @@ int launch_meridional_hyperviscosity(const DevModel &M, int index, double *var, 
   return 0;
 }
 
+constexpr size_t VISC_ROWS_SMEM = 101 * 1024;   // two blocks per SM; 4 rows of EPIC_MAX_NI fit
+
 // index 2 (HDRY) applies restore_mass as well (in the kernel, or alone without hyperviscosity)
 int launch_zonal_hyperviscosity(const DevModel &M, int index, double *var, int sel, cudaStream_t s) {
   if (M.ni < 2 || !(M.nu[4] + M.nu[6] + M.nu[8] > 0.)) return index == 2 ? launch_restore_mass(M, s) : 0;
   int k0, k1;
   visc_krange(M, index, k0, k1);
   const int jbot = index == 1 ? 1 : 0, jhalf = index == 1 ? 0 : 1;
-  const size_t row_bytes = (size_t)(M.ni + 2) * (sizeof(double) + 2 * (M.mixed ? sizeof(float) : sizeof(double)));
+  const int nrows = M.nj - jbot + 1, nkk = k1 - k0 + 1;
+  if (!M.mixed) {
+    // rows per block: a power of 2, the fewest that leave two blocks per SM or fewer (each order's
+    // sums are one chain of ni additions per block), up to a warp's lanes and VISC_ROWS_SMEM
+    const size_t row_bytes = (size_t)3 * (M.ni + 3) * sizeof(double);
+    const long long total = (long long)nrows * nkk * (M.nbatch > 1 ? M.nbatch : 1);
+    int rows = 4;
+    while (rows < 32 && total > 2LL * 152 * rows && 2 * rows * row_bytes <= VISC_ROWS_SMEM) rows *= 2;
+    k_zonal_visc_rows<<<zg(epic_blocks((long long)nrows * nkk, rows), M), 256, rows * row_bytes, s>>>(M, var, sel, jbot, jhalf, k0, nkk,
+                                                                                                     index == 2, rows);
+    return 0;
+  }
+  const size_t row_bytes = (size_t)(M.ni + 2) * (sizeof(double) + 2 * sizeof(float));
   int rows = (int)((40 * 1024) / row_bytes);
   rows = rows < 1 ? 1 : (rows > 4 ? 4 : rows);
-  const int nrows = M.nj - jbot + 1;
-  dim3 grid((nrows + rows - 1) / rows, k1 - k0 + 1);
-  EPIC_LAUNCH_R(M.mixed, k_zonal_visc, grid, 32 * rows, rows * row_bytes, s, M, var, sel, jbot, jhalf, k0, index == 2);
+  dim3 grid((nrows + rows - 1) / rows, nkk);
+  k_zonal_visc_mixed<<<zg(grid, M), 32 * rows, rows * row_bytes, s>>>(M, var, sel, jbot, jhalf, k0, index == 2);
   return 0;
+}
+
+// the largest dynamic shared memory of a launch, raised once for the process (models of all sizes)
+int stencil_kernels_init() {
+  return cudaFuncSetAttribute(k_zonal_visc_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VISC_ROWS_SMEM) == cudaSuccess ? 0 : -1;
 }
 
 int launch_divergence_damping(const DevModel &M, cudaStream_t s) {
@@ -1292,7 +1366,8 @@ int launch_diag_pv(const DevModel &M, cudaStream_t s) {
   return 0;
 }
 int launch_diag_pv_poles(const DevModel &M, cudaStream_t s) {
-  k_pv_poles<<<zg(M.nk + 1, M), 128, 4 * M.ni * sizeof(double), s>>>(M);
+  const int lv = row_sum_levels(M, 4);
+  k_pv_poles<<<zg(epic_blocks(M.nk + 1, lv), M), 256, (size_t)4 * lv * (M.ni + 1) * sizeof(double), s>>>(M, lv);
   return 0;
 }
 int launch_diag_div(const DevModel &M, cudaStream_t s) {

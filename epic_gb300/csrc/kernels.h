@@ -92,7 +92,6 @@ int launch_advection_prep(const DevModel &M, int phase, cudaStream_t s);
 int column_kernels_init(int nk);
 
 // k_stencil.cu -- horizontal stencils and the time update
-int launch_copy_gz(const DevModel &M, cudaStream_t s);
 int launch_zero_tend(const DevModel &M, cudaStream_t s);
 int launch_uv_core(const DevModel &M, cudaStream_t s);
 // uv_pgrad_finite_volume: GZ3's pole rows, then DUDT (lon) and DVDT (lat), independent of each other
@@ -107,6 +106,7 @@ int launch_akima_meridional(const DevModel &M, double *buff, int kind, cudaStrea
 int launch_akima_zonal(const DevModel &M, double *buff, int kind, int kstart, cudaStream_t s);
 int launch_meridional_hyperviscosity(const DevModel &M, int index, double *var, int sel, cudaStream_t s);
 int launch_zonal_hyperviscosity(const DevModel &M, int index, double *var, int sel, cudaStream_t s);
+int stencil_kernels_init();
 int launch_divergence_damping(const DevModel &M, cudaStream_t s);
 // the time update: which scheme coefficients this step takes (decide: from the tendency planes of
 // earlier steps alone), the update, the rotation of the time-plane indices

@@ -1,0 +1,20 @@
+"""Kernels that work on whole latitude rows (the zonal filter, the 3-D filter, the zonal advection pass,
+zonal hyperviscosity, the polar row sums), the column kernels beside them and the meridional passes, in
+the FP64 form at the ends of their range of row lengths: every stage equals the correctly rounded
+restatement bit for bit."""
+import pytest
+
+from epic_gb300 import EPIC_ADV_AKIMA, EPIC_ADV_HSU, EPIC_PROFILE_N2, HSConfig
+from test_gpu_parity import _stage_by_stage
+
+pytestmark = pytest.mark.gpu
+
+
+# the shortest and longest rows, levels that do and do not fill the
+# last block, more rows than a block sums at once
+@pytest.mark.parametrize("ni,nj,nk", [(4, 7, 5), (8, 9, 6), (16, 40, 9), (32, 12, 17), (64, 33, 21), (128, 9, 8), (256, 12, 5), (1024, 8, 5)])
+@pytest.mark.parametrize("adv", [EPIC_ADV_HSU, EPIC_ADV_AKIMA])
+def test_rows(gpu, ni, nj, nk, adv):
+    a = min(1., 2. * nj / ni)   # hyperviscosity stable at the shorter of the two spacings
+    _stage_by_stage(HSConfig(ni=ni, nj=nj, nk=nk, dt=max(1, 600 // ni), seed=ni + nk, advection_scheme=adv, nu4=0.5 * a**4,
+                             nu6=0.05 * a**6, nu8=0.02 * a**8, state="jet", profile=EPIC_PROFILE_N2, turbulence=ni == 32))
