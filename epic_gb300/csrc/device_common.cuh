@@ -204,13 +204,25 @@ __device__ __forceinline__ bool epic_member(DevModel &M, P *&...ptrs) {
 __device__ __forceinline__ double dmaxr(double x, double y) { return x > y ? x : y; }   // MAX, include/epic.h:144
 __device__ __forceinline__ double dminr(double x, double y) { return x < y ? x : y; }   // MIN, include/epic.h:138
 
-// fcmp, src/shared/epic_funcs_util.c:4275-4330
-__device__ __forceinline__ int fcmp(double x1, double x2) {
+// fcmp, src/shared/epic_funcs_util.c:4275-4330.  delta is two units of the last place of the larger
+// magnitude, so values of one sign whose bit patterns lie more than 8 apart are ordered as their
+// patterns are, and opposite signs as their signs: the usual answers, on the integer pipe (the
+// comparison itself is four binary64 operations, 16 clocks a warp each).  The rest -- near neighbours,
+// zeros, very small or infinite magnitudes, NaN -- takes the reference's own arithmetic.
+static __device__ __noinline__ int fcmp_near(double x1, double x2) {
   int e;
   frexp(fabs(x1) > fabs(x2) ? x1 : x2, &e);
   const double delta = ldexp(DBL_EPSILON, e);
   const double d = x1 - x2;
   return d > delta ? 1 : (d < -delta ? -1 : 0);
+}
+__device__ __forceinline__ int fcmp(double x1, double x2) {
+  const long long u1 = __double_as_longlong(x1), u2 = __double_as_longlong(x2);
+  const unsigned e1 = (unsigned)(u1 >> 52) & 0x7ffu, e2 = (unsigned)(u2 >> 52) & 0x7ffu;
+  const long long d = u1 - u2;
+  const bool same = (u1 ^ u2) >= 0, apart = same ? d > 8 || d < -8 : true;
+  if (e1 - 64u < 1983u && e2 - 64u < 1983u && apart) return (same ? (d > 0) != (u1 < 0) : u2 < 0) ? 1 : -1;
+  return fcmp_near(x1, x2);
 }
 
 // THETA2 at an isentropic layer (set_p2etc, K > k_sigma-1) interpolates linearly in the table
@@ -445,6 +457,17 @@ template <class R> __device__ __forceinline__ R rmin(R x, R y) { return x < y ? 
 // a / b: the IEEE quotient (binary64 on the integer pipe)
 template <class R> __device__ __forceinline__ R qdiv(R a, R b) { return a / b; }
 template <> __device__ __forceinline__ double qdiv<double>(double a, double b) { return div_rn(a, b); }
+// x / 2 in the compute type: binary64 on the integer pipe (the exponent less one; zeros as they are,
+// magnitudes at the ends of the range by the multiplication)
+static __device__ __noinline__ double half_cold(double x) { return .5 * x; }
+template <class R> __device__ __forceinline__ R half_of(R x) { return R(.5) * x; }
+template <> __device__ __forceinline__ double half_of<double>(double x) {
+  const int hi = __double2hiint(x), lo = __double2loint(x);
+  const unsigned e = (unsigned)hi & 0x7ff00000u;
+  const bool zero = (((unsigned)hi << 1) | (unsigned)lo) == 0u;
+  if (!zero && e - 0x00200000u >= 0x7fd00000u) return half_cold(x);
+  return __hiloint2double(zero ? hi : hi - 0x00100000, lo);
+}
 template <class R> struct RMath;
 template <> struct RMath<double> {
   static __device__ __forceinline__ double log(const DevModel &M, double x) { return xlog(M, x); }
@@ -480,6 +503,40 @@ template <> struct RMath<float> {
     return d > delta ? 1 : (d < -delta ? -1 : 0);
   }
 };
+
+// ---- the corrector of hsu_advection at one face (epic_flux.c:717-1484, all three directions) ----
+//
+// The reference splits the face's velocity into max(0, w) and min(0, w) and sums the corrections of
+// both; one of the two is zero, and so (for finite fields) is every term it multiplies.  hsu_face
+// evaluates the upwind side alone: one square root and two quotients a face instead of two and
+// three, half the products -- the same value, a zero term added nowhere changing it.
+// w: the face's velocity; w_up: the velocity at the next face upstream; a_u, a_d: the field in the
+// cells upstream and downstream; ap_d: the predicted field downstream; d_up: predicted minus field
+// across the upstream face; aa: the squared second difference in the upstream cell; min_u, min_d: the
+// field's floor in the two cells; c: the metric
+// factor of the Courant number (times dt in the reference's order: |w| c DT).
+template <class R> __device__ __forceinline__ bool is_neg(R w);   // the sign bit
+template <> __device__ __forceinline__ bool is_neg<double>(double w) { return __double2hiint(w) < 0; }
+template <> __device__ __forceinline__ bool is_neg<float>(float w) { return __float_as_int(w) < 0; }
+template <class R> __device__ __forceinline__ R qsqrt(R x) { return sqrt(x); }
+template <> __device__ __forceinline__ double qsqrt<double>(double x) { return sqrt_rn(x); }
+template <class R>
+__device__ __forceinline__ R hsu_face(R w, R w_up, R a_u, R a_d, R ap_d, R d_up, R aa, R min_u, R min_d, R c, R DT) {
+  const bool neg = is_neg(w);
+  const R wu = is_neg(w_up) == neg ? w_up : R(0.);
+  R f = R(.5) * (w * (ap_d + a_u));
+  R what = qsqrt<R>(w * wu);
+  what = neg ? -what : what;
+  const R mu = fabs(w) * c * DT;
+  const R al = qdiv(R(1.) + mu, R(6.));
+  R g = qdiv(aa, aa + (a_u - min_u) * (a_d - min_d));
+  g = g * g;
+  const R be = R(1.) + (qdiv(R(1.), R(2.) * al) - R(1.)) * g;
+  return f + -al * (w * be * (ap_d - a_u) - what * (R(1.) - g) * d_up);
+}
+// the predictor's flux: the upwind cell's value carried by w (the other side's term is zero)
+template <class R>
+__device__ __forceinline__ R hsu_upwind(R w, R a_minus, R a_plus) { return w * (is_neg(w) ? a_minus : a_plus); }
 
 struct Trip { double x, y, z; };
 

@@ -1415,7 +1415,6 @@ extern "C" int epic_batch_autotune(epic_batch *b, int32_t trial_steps, int32_t *
     int best = b->d.tb[g];
     float best_ms = 3.4e38f;
     for (int c = 0; c < ncand && rc == EPIC_OK; c++) {
-      if (g == TB_ROW && c > 0 && cand[c] > b->d.ni / 2) continue;   // more threads than butterflies
       b->d.tb[g] = cand[c];
       float ms = 0.f;
       rc = time_steps(&ms);

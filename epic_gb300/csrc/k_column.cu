@@ -180,9 +180,9 @@ __global__ void k_uv_drag(DevModel M) {
 // interface variable, with the layer variables' predictor and corrector, :876-960, and the floor
 // NU_TURB_MIN).  A column tile (32 columns j = 0..nj, i = 0..ni+1 per block): every pass
 // of the predictor-corrector is pointwise in k given the previous pass, so the levels are
-// spread over the warps with a barrier between passes; d1, d2 and the smoothness weights are
-// recomputed where used (the same expressions, so the same values).  Shared arrays [k][lane]:
-// WA (the field), WM, WP (the split vertical velocity), PR (the predictor), FF (the fluxes).
+// spread over the warps with a barrier between passes; the smoothness weights are recomputed where
+// used.  Shared arrays [k][lane]: WA (the field), W (the vertical velocity; positive is towards
+// smaller k), PR (the predictor), FF (the fluxes).
 template <class R>
 __global__ void __launch_bounds__(CT_THREADS) k_hsu_vertical(DevModel M, double *buff, int kind) {
   if (epic_member(M, buff)) return;
@@ -194,64 +194,45 @@ __global__ void __launch_bounds__(CT_THREADS) k_hsu_vertical(DevModel M, double 
   const bool layer = kind == 2, nuk = kind == 3;
   const int kf = kind == 1 ? M.k_sigma - 1 : 1;
   const R ep = R(1.e-10), DT = cv<R>(M.dt);
-  R *WA = sm, *WM = WA + 32 * L, *WP = WM + 32 * L, *PR = WP + 32 * L, *FF = PR + 32 * L;
-  auto amin = [&](int k) { return layer ? cv<R>(M.h_min[k]) : (nuk && k >= 1 ? cv<R>(1.e-3 * M.kinvisc) : R(0.)); };
+  R *WA = sm, *W = WA + 32 * L, *PR = W + 32 * L, *FF = PR + 32 * L;
   auto dsi = [&](int kk) { return cv<R>(M.dsgth_inv[kk]); };
   auto wa = [&](int k) { return CT(WA, k); };
+  // W3 at the layer's middle, 0 in the top and bottom layers
+  auto w_layer = [&](int k) {
+    return (k == 1 || k == nk) ? R(0.) : R(.5) * (cv<R>(M.w3[c.base + k * n2]) + cv<R>(M.w3[c.base + (k - 1) * n2]));
+  };
   if (c.valid)
     for (int k = (layer ? kf : kf - 1) + c.warp; k <= nk; k += CT_WARPS) CT(WA, k) = cv<R>(buff[c.base + k * n2]);
   if (layer || nuk) {
     if (c.valid && layer)
-      for (int k = kf - 1 + c.warp; k <= nk; k += CT_WARPS) {
-        const R w = cv<R>(M.w3[c.base + k * n2]);
-        CT(WM, k) = rmin(R(0.), w);
-        CT(WP, k) = rmax(R(0.), w);
-      }
+      for (int k = kf - 1 + c.warp; k <= nk; k += CT_WARPS) CT(W, k) = cv<R>(M.w3[c.base + k * n2]);
     if (c.valid && nuk) {
-      for (int k = kf + c.warp; k <= nk; k += CT_WARPS) {
-        const R w = (k == 1 || k == nk) ? R(0.) : R(.5) * (cv<R>(M.w3[c.base + k * n2]) + cv<R>(M.w3[c.base + (k - 1) * n2]));
-        CT(WM, k) = rmin(R(0.), w);
-        CT(WP, k) = rmax(R(0.), w);
-      }
+      for (int k = kf + c.warp; k <= nk; k += CT_WARPS) CT(W, k) = w_layer(k);
       // entry 0 is never loaded for NU_TURB; the corrector reads it only against d2(1) = 0
-      if (c.warp == 0) { CT(WM, 0) = R(0.); CT(WP, 0) = R(0.); }
+      if (c.warp == 0) CT(W, 0) = R(0.);
     }
     __syncthreads();
     if (c.valid)
       for (int k = kf - 1 + c.warp; k <= nk; k += CT_WARPS)
-        CT(FF, k) = (k == kf - 1 || k == nk) ? R(0.) : CT(WP, k) * wa(k + 1) + CT(WM, k) * wa(k);
+        CT(FF, k) = (k == kf - 1 || k == nk) ? R(0.) : hsu_upwind<R>(CT(W, k), wa(k), wa(k + 1));
     __syncthreads();
     if (c.valid)
       for (int k = kf + c.warp; k <= nk; k += CT_WARPS) CT(PR, k) = wa(k) + (CT(FF, k) - CT(FF, k - 1)) * dsi(2 * k) * DT;
     __syncthreads();
-    // d1, d2 and the smoothness weight aa of level k (epic_flux.c's first corrector loop)
-    auto d1 = [&](int k) { return k == nk ? R(0.) : CT(PR, k) - wa(k + 1); };
-    auto d2 = [&](int k) { return k == 1 ? R(0.) : CT(PR, k) - wa(k - 1); };
-    auto aa = [&](int k) {
-      R tmp;
-      if (k == 1) tmp = fabs(wa(k + 1) - wa(k)) + ep;
-      else if (k == nk) tmp = fabs(-wa(k) + wa(k - 1)) + ep;
-      else tmp = fabs(wa(k + 1) - R(2.) * wa(k) + wa(k - 1)) + ep;
-      return tmp * tmp;
-    };
-    // the corrector reads PR, WA, WM and WP only, so it rewrites FF in place
+    // the corrector reads PR, WA and W only, so it rewrites FF in place
     if (c.valid)
       for (int k = kf + c.warp; k < nk; k += CT_WARPS) {
-        const R wpk = CT(WP, k), wmk = CT(WM, k);
-        R f = R(.5) * (wpk * (CT(PR, k) + wa(k + 1)) + wmk * (CT(PR, k + 1) + wa(k)));
-        const R whatp = sqrt(wpk * CT(WP, k + 1));
-        const R whatm = -sqrt(wmk * CT(WM, k - 1));
-        const R mu = (wpk - wmk) * dsi(2 * k + 1) * DT;
-        const R al = qdiv(R(1.) + mu, R(6.));
-        const R prod = (wa(k + 1) - amin(k + 1)) * (wa(k) - amin(k));
-        const R aap = aa(k + 1), aak = aa(k);
-        R gap = qdiv(aap, aap + prod); gap = gap * gap;
-        R gam = qdiv(aak, aak + prod); gam = gam * gam;
-        const R hal = qdiv(R(1.), R(2.) * al) - R(1.);
-        const R bep = R(1.) + hal * gap;
-        const R bem = R(1.) + hal * gam;
-        f += -al * (wpk * bep * d1(k) - whatp * (R(1.) - gap) * d1(k + 1) + wmk * bem * d2(k + 1) - whatm * (R(1.) - gam) * d2(k));
-        CT(FF, k) = f;
+        const R w = CT(W, k);
+        const bool neg = is_neg(w);   // from layer k down to k+1, else from k+1 up to k
+        const int u = neg ? k : k + 1, d = neg ? k + 1 : k;   // the layers upstream and downstream
+        const bool edge = neg ? k == 1 : k + 1 == nk;         // no layer beyond the upstream one
+        const R au = wa(u), ad = wa(d), auu = edge ? R(0.) : wa(neg ? k - 1 : k + 2);
+        R t;
+        if (edge) t = fabs(neg ? ad - au : -au + ad) + ep;
+        else t = fabs((neg ? ad : auu) - R(2.) * au + (neg ? auu : ad)) + ep;
+        auto amin = [&](int q) { return layer ? cv<R>(M.h_min[q]) : cv<R>(1.e-3 * M.kinvisc); };   // HDRY's and NU_TURB's floors
+        CT(FF, k) = hsu_face<R>(w, CT(W, neg ? k - 1 : k + 1), au, ad, CT(PR, d), edge ? R(0.) : CT(PR, u) - auu, t * t, amin(u), amin(d),
+                                dsi(2 * k + 1), DT);
       }
     __syncthreads();
     if (c.valid && layer)
@@ -267,15 +248,11 @@ __global__ void __launch_bounds__(CT_THREADS) k_hsu_vertical(DevModel M, double 
       }
   } else {
     if (c.valid)
-      for (int k = kf + c.warp; k <= nk; k += CT_WARPS) {
-        const R w = (k == 1 || k == nk) ? R(0.) : R(.5) * (cv<R>(M.w3[c.base + k * n2]) + cv<R>(M.w3[c.base + (k - 1) * n2]));
-        CT(WM, k) = rmin(R(0.), w);
-        CT(WP, k) = rmax(R(0.), w);
-      }
+      for (int k = kf + c.warp; k <= nk; k += CT_WARPS) CT(W, k) = w_layer(k);
     __syncthreads();
     if (c.valid)
       for (int k = kf + c.warp; k <= nk + 1; k += CT_WARPS)
-        CT(FF, k) = k == nk + 1 ? R(0.) : CT(WP, k) * wa(k) + CT(WM, k) * wa(k - 1);
+        CT(FF, k) = k == nk + 1 ? R(0.) : hsu_upwind<R>(CT(W, k), wa(k - 1), wa(k));
     __syncthreads();
     if (c.valid)
       for (int k = kf - 1 + c.warp; k <= nk; k += CT_WARPS)
@@ -291,27 +268,16 @@ __global__ void __launch_bounds__(CT_THREADS) k_hsu_vertical(DevModel M, double 
       else tmp = fabs(wa(k + 1) - R(2.) * wa(k) + wkm1) + ep;
       return tmp * tmp;
     };
-    auto d1 = [&](int k) { return CT(PR, k - 1) - wa(k); };
-    auto d2 = [&](int k) { return k == kf - 1 ? R(0.) : CT(PR, k) - wa(k - 1); };
     if (c.valid)
       for (int k = kf + c.warp; k <= nk; k += CT_WARPS) {
-        const R wpk = CT(WP, k), wmk = CT(WM, k);
-        R f = R(.5) * (wpk * (CT(PR, k - 1) + wa(k)) + wmk * (CT(PR, k) + wa(k - 1)));
-        const R whatm = (k == 1 || k - 1 < kf) ? R(0.) : -sqrt(wmk * CT(WM, k - 1));
-        const R whatp = (k == nk) ? R(0.) : sqrt(wpk * CT(WP, k + 1));
-        const R mu = (wpk - wmk) * dsi(2 * k) * DT;
-        const R al = qdiv(R(1.) + mu, R(6.));
-        const R prod = (wa(k) - amin(k)) * (wa(k - 1) - amin(k - 1));
-        const R aak = aa(k), aam = aa(k - 1);
-        R gap = qdiv(aak, aak + prod); gap = gap * gap;
-        R gam = qdiv(aam, aam + prod); gam = gam * gam;
-        const R hal = qdiv(R(1.), R(2.) * al) - R(1.);
-        const R bep = R(1.) + hal * gap;
-        const R bem = R(1.) + hal * gam;
-        R g;
-        if (k < nk) g = -al * (wpk * bep * d1(k) - whatp * (R(1.) - gap) * d1(k + 1) + wmk * bem * d2(k) - whatm * (R(1.) - gam) * d2(k - 1));
-        else g = -al * (wpk * bep * d1(k) + wmk * bem * d2(k) - whatm * (R(1.) - gam) * d2(k - 1));
-        CT(FF, k) = f + g;
+        const R w = CT(W, k);
+        const bool neg = is_neg(w);   // from interface k-1 down to k, else from k up to k-1
+        const int u = neg ? k - 1 : k, d = neg ? k : k - 1;
+        // no velocity upstream of the last layer's, and none below the first one's interface (for
+        // k = 1 and k - 1 < kf); the predictor keeps the field at interface kf - 1
+        const R w_up = neg ? ((k == 1 || k - 1 < kf) ? R(0.) : CT(W, k - 1)) : (k == nk ? R(0.) : CT(W, k + 1));
+        const R d_up = neg ? (k - 1 == kf - 1 ? R(0.) : CT(PR, k - 1) - wa(k - 2)) : (k == nk ? R(0.) : CT(PR, k) - wa(k + 1));
+        CT(FF, k) = hsu_face<R>(w, w_up, wa(u), wa(d), CT(PR, d), d_up, aa(u), R(0.), R(0.), dsi(2 * k), DT);
       }
     __syncthreads();
     if (c.valid)
@@ -1031,7 +997,7 @@ int launch_uv_drag(const DevModel &M, cudaStream_t s) {
 }
 int launch_hsu_vertical(const DevModel &M, double *buff, int kind, cudaStream_t s) {
   EPIC_LAUNCH_R(M.mixed, k_hsu_vertical, ntile_blocks(M), CT_THREADS,
-                (size_t)5 * 32 * (M.nk + 2) * (M.mixed ? sizeof(float) : sizeof(double)), s, M, buff, kind);
+                (size_t)4 * 32 * (M.nk + 2) * (M.mixed ? sizeof(float) : sizeof(double)), s, M, buff, kind);
   return 0;
 }
 int launch_akima_vertical(const DevModel &M, double *buff, int kind, cudaStream_t s) {
@@ -1202,7 +1168,7 @@ int launch_advection_prep(const DevModel &M, int phase, cudaStream_t s) {
 // models of different sizes in one process never lower it for one another.
 int column_kernels_init(int) {
   const int big = (int)(6 * 32 * (EPIC_MAX_NK + 1) * sizeof(double));
-  const int hv = (int)(5 * 32 * (EPIC_MAX_NK + 2) * sizeof(double));
+  const int hv = (int)(4 * 32 * (EPIC_MAX_NK + 2) * sizeof(double));
   if (cudaFuncSetAttribute(k_calc_w<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
       cudaFuncSetAttribute(k_calc_w<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
       cudaFuncSetAttribute(k_set_p2etc, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||

@@ -3,8 +3,8 @@
 // The reference filters one latitude row at a time: realft() forward, multiply wavenumber m by
 // HIGH_LAT(J,m+1), realft() inverse and scale by 2/ni (epic_adjust.c:412-456), where realft and
 // four1 are the Numerical Recipes in C (2nd ed., pp. 507, 513) real and complex radix-2 FFTs
-// (epic_funcs_util.c:4023-4132).  Here one thread block owns one row and carries out the same
-// arithmetic in parallel: every butterfly of a four1 stage and every iteration of realft's
+// (epic_funcs_util.c:4023-4132).  Here a group of lanes of one warp owns one row and carries out the
+// same arithmetic in parallel: every butterfly of a four1 stage and every iteration of realft's
 // post-processing loop touches its own data, so they run concurrently; the twiddle factors,
 // which NR builds by a recurrence, are computed once on the host with exactly that recurrence.
 // Compiled without FMA contraction, each filtered row is bit-identical to the reference's.
@@ -15,7 +15,7 @@
 
 namespace epic {
 
-template <class R> struct Cplx { R re, im; };
+template <class R> struct __align__(2 * sizeof(R)) Cplx { R re, im; };
 
 // Twiddle table layout (pairs), N = ni/2 complex points:
 //   [0, N-1)              four1 isign=+1, stage with half h at offset h-1, entries p = 0..h-1
@@ -29,59 +29,100 @@ __host__ __device__ inline size_t nr_twiddle_pairs(int ni) {
   return 2 * (size_t)(N - 1) + 2 * (size_t)(N / 2 - 1);
 }
 
-template <class R>
-struct FilterSmem {
-  Cplx<R> *z, *w;   // row as N complex points; twiddles
+// ---- rows by lane groups ----
+//
+// A row belongs to G lanes of one warp (RowShape): 32, or fewer where a row has fewer butterflies, so
+// that a warp instruction is full either way -- a binary64 one costs the pipe the same 16 clocks
+// whatever the number of active lanes.  A block takes `rows` levels of one latitude row, so its rows
+// are all filtered or all not and share what depends on the latitude; a row's passes are separated by
+// __syncwarp alone.  With a block of two warps a row, its passes separated by block barriers and the
+// twiddles copied to shared memory by each, the FP64 form's filters ran at 43-66% of the binary64 pipe
+// with 3 warps resident per scheduler.
+struct RowShape { int G, rows, stride; };   // lanes a row, rows a block, compute-type values a row in shared memory
+struct RowLane {
+  int gl, G, r, k;
+  bool live;   // the row exists (the last block of a launch may have rows to spare)
 };
-
-template <class R>
-__device__ __forceinline__ FilterSmem<R> carve_filter(R *base, int ni) {
-  const int N = ni / 2;
-  FilterSmem<R> s;
-  s.z = reinterpret_cast<Cplx<R> *>(base);
-  s.w = s.z + N;
-  return s;
-}
-// shared-memory elements (of the compute type) one row filter needs
-__host__ __device__ inline size_t filter_smem_elems(int ni) {
-  return 2 * ((size_t)(ni / 2) + nr_twiddle_pairs(ni));
+__device__ __forceinline__ RowLane row_lane(const RowShape &S, int k0, int kend) {
+  RowLane L;
+  L.G = S.G;
+  L.gl = (int)threadIdx.x & (S.G - 1);
+  L.r = (int)threadIdx.x / S.G;
+  const int k = k0 + (int)blockIdx.y * S.rows + L.r;
+  L.live = k <= kend;
+  L.k = L.live ? k : kend;
+  return L;
 }
 
-template <class R> __device__ __forceinline__ const R *twiddle_table(const DevModel &M);
-template <> __device__ __forceinline__ const double *twiddle_table<double>(const DevModel &M) { return M.tw; }
-template <> __device__ __forceinline__ const float *twiddle_table<float>(const DevModel &M) { return M.twf; }
+template <class R> __device__ __forceinline__ const Cplx<R> *twiddle_table(const DevModel &M);
+template <> __device__ __forceinline__ const Cplx<double> *twiddle_table<double>(const DevModel &M) { return reinterpret_cast<const Cplx<double> *>(M.tw); }
+template <> __device__ __forceinline__ const Cplx<float> *twiddle_table<float>(const DevModel &M) { return reinterpret_cast<const Cplx<float> *>(M.twf); }
 
-template <class R>
-__device__ __forceinline__ void load_twiddles(const DevModel &M, FilterSmem<R> &s) {
-  const int n = (int)nr_twiddle_pairs(M.ni);
-  const Cplx<R> *g = reinterpret_cast<const Cplx<R> *>(twiddle_table<R>(M));
-  for (int k = threadIdx.x; k < n; k += blockDim.x) s.w[k] = g[k];
-}
+// The place of row value e = i-1 among the N complex points in bit-reversed order, which
+// filter_row takes its input in.
+__device__ __forceinline__ int fft_place(int e, int lg) { return 2 * (int)(__brev((unsigned)(e >> 1)) >> (32 - lg)) + (e & 1); }
+__device__ __forceinline__ int fft_log(int ni) { return 31 - __clz(ni / 2); }
 
-// four1's Danielson-Lanczos stages on z (already bit-reversed); tw = this direction's table.
+// four1's Danielson-Lanczos stages on z (already bit-reversed); tw = this direction's table.  The
+// first stage's only twiddle is (1, 0).
 template <class R>
-__device__ __forceinline__ void four1_stages(Cplx<R> *z, const Cplx<R> *tw, int N) {
-  for (int h = 1; h < N; h <<= 1) {
+__device__ __forceinline__ void four1_stages(Cplx<R> *z, const Cplx<R> *tw, int N, const RowLane &L) {
+  for (int b = L.gl; b < N / 2; b += L.G) {
+    const Cplx<R> u = z[2 * b], v = z[2 * b + 1];
+    z[2 * b] = {u.re + v.re, u.im + v.im};
+    z[2 * b + 1] = {u.re - v.re, u.im - v.im};
+  }
+  __syncwarp();
+  for (int h = 2; h < N; h <<= 1) {
     const Cplx<R> *wt = tw + (h - 1);
-    for (int b = threadIdx.x; b < N / 2; b += blockDim.x) {
-      const int p = b & (h - 1);
-      const int i0 = (b / h) * 2 * h + p;
-      const int j0 = i0 + h;
-      const R wr = wt[p].re, wi = wt[p].im;
-      const R tempr = wr * z[j0].re - wi * z[j0].im;
-      const R tempi = wr * z[j0].im + wi * z[j0].re;
-      z[j0].re = z[i0].re - tempr;
-      z[j0].im = z[i0].im - tempi;
-      z[i0].re += tempr;
-      z[i0].im += tempi;
+    for (int b = L.gl; b < N / 2; b += L.G) {
+      const int p = b & (h - 1), i0 = 2 * (b - p) + p, j0 = i0 + h;
+      const Cplx<R> w = wt[p], u = z[i0], v = z[j0];
+      const R tempr = w.re * v.re - w.im * v.im;
+      const R tempi = w.re * v.im + w.im * v.re;
+      z[j0] = {u.re - tempr, u.im - tempi};
+      z[i0] = {u.re + tempr, u.im + tempi};
     }
-    __syncthreads();
+    __syncwarp();
   }
 }
 
+// Filter a row with weights h(I) = hl[I], I = 1..ni/2+1 (HIGH_LAT(J,I)): z holds the row's values in
+// bit-reversed order (fft_place), on return the filtered row in order, to be multiplied by
+// filter_scale.  Every lane of the warp must call this.  realft forward, the weights and realft
+// inverse (epic_adjust.c:412-456) meet in one pass between the two four1 calls: both split loops and
+// the weights act on the pair (q, N-q).  The reference's factors 1/2 (c1, c2, two per value) and 2/ni
+// are powers of 2, which commute with every rounding in between (the values being far from the ends
+// of the range), so they are left to the one final multiplication.
+template <class R> __device__ __forceinline__ R filter_scale(int ni) { return R(.5) / R(ni); }
 template <class R>
-__device__ __forceinline__ void bitrev_permute(Cplx<R> *z, int N, int lg) {
-  for (int k = threadIdx.x; k < N; k += blockDim.x) {
+__device__ __forceinline__ void filter_row(const DevModel &M, Cplx<R> *z, const double *hl, const RowLane &L) {
+  const int N = M.ni / 2, lg = fft_log(M.ni);
+  const Cplx<R> *t4p = twiddle_table<R>(M), *t4m = t4p + (N - 1), *trp = t4p + 2 * (N - 1), *trm = trp + (N / 2 - 1);
+  four1_stages(z, t4p, N, L);
+  for (int q = L.gl; q < N / 2; q += L.G) {
+    if (q == 0) {   // wavenumbers 0 and ni/2 share z[0]; ni/4 has no partner
+      const Cplx<R> a = z[0], b = z[N / 2];
+      const R s = (a.re + a.im) * cv<R>(hl[1]), d = (a.re - a.im) * cv<R>(hl[N + 1]);
+      z[0] = {R(2.) * (s + d), R(2.) * (s - d)};
+      const R h = R(4.) * cv<R>(hl[N / 2 + 1]);
+      if (N > 1) z[N / 2] = {b.re * h, b.im * h};
+      continue;
+    }
+    Cplx<R> a = z[q], b = z[N - q], w = trp[q - 1];
+    R x = a.re + b.re, y = a.im - b.im, s = a.im + b.im, d = a.re - b.re;
+    R ws = w.re * s, id = w.im * d, wd = w.re * d, is = w.im * s;
+    const R hq = cv<R>(hl[q + 1]), hn = cv<R>(hl[N - q + 1]);
+    a = {(x + ws + id) * hq, (y - wd + is) * hq};
+    b = {(x - ws - id) * hn, (-y - wd + is) * hn};
+    w = trm[q - 1];
+    x = a.re + b.re; y = a.im - b.im; s = a.im + b.im; d = a.re - b.re;
+    ws = w.re * s; id = w.im * d; wd = w.re * d; is = w.im * s;
+    z[q] = {x - ws - id, y + wd - is};
+    z[N - q] = {x + ws + id, -y + wd - is};
+  }
+  __syncwarp();
+  for (int k = L.gl; k < N; k += L.G) {
     const int r = (int)(__brev((unsigned)k) >> (32 - lg));
     if (r > k) {
       const Cplx<R> t = z[k];
@@ -89,117 +130,44 @@ __device__ __forceinline__ void bitrev_permute(Cplx<R> *z, int N, int lg) {
       z[r] = t;
     }
   }
-  __syncthreads();
-}
-
-// realft's split loop (i = 2..n/4, here q = i-1): c2 = -0.5 forward, +0.5 inverse.
-template <class R>
-__device__ __forceinline__ void realft_split(Cplx<R> *z, const Cplx<R> *tw, int N, R c2) {
-  const R c1 = R(0.5);
-  for (int q = 1 + threadIdx.x; q < N / 2; q += blockDim.x) {
-    const Cplx<R> a = z[q], b = z[N - q];
-    const R wr = tw[q - 1].re, wi = tw[q - 1].im;
-    const R h1r = c1 * (a.re + b.re);
-    const R h1i = c1 * (a.im - b.im);
-    const R h2r = -c2 * (a.im + b.im);
-    const R h2i = c2 * (a.re - b.re);
-    z[q].re = h1r + wr * h2r - wi * h2i;
-    z[q].im = h1i + wr * h2i + wi * h2r;
-    z[N - q].re = h1r - wr * h2r + wi * h2i;
-    z[N - q].im = -h1i + wr * h2i + wi * h2r;
-  }
-  __syncthreads();
-}
-
-// Filter row x[1..ni] (1-based, shared memory) in place with weights h(I) = hl[rowbase + I],
-// I = 1..ni/2+1 (HIGH_LAT(J,I)).  Every thread of the block must call this.
-template <class R>
-__device__ void filter_row_smem(const DevModel &M, R *x, const double *hl, long long rowbase, FilterSmem<R> &s) {
-  const int ni = M.ni, N = ni / 2;
-  const int lg = 31 - __clz(N);
-  const Cplx<R> *t4p = s.w, *t4m = s.w + (N - 1), *trp = s.w + 2 * (N - 1), *trm = trp + (N / 2 - 1);
-  Cplx<R> *z = s.z;
-  // realft(data, n, 1): four1(data, n/2, 1) -- bit reversal, stages -- then the split loop
-  for (int k = threadIdx.x; k < N; k += blockDim.x) {
-    const int r = (int)(__brev((unsigned)k) >> (32 - lg));
-    z[r].re = x[2 * k + 1];
-    z[r].im = x[2 * k + 2];
-  }
-  __syncthreads();
-  four1_stages(z, t4p, N);
-  realft_split(z, trp, N, R(-0.5));
-  if (threadIdx.x == 0) {
-    const R h1r = z[0].re;
-    z[0].re = h1r + z[0].im;
-    z[0].im = h1r - z[0].im;
-  }
-  __syncthreads();
-  // spectral weights (epic_adjust.c:447-453)
-  for (int q = threadIdx.x; q < N; q += blockDim.x) {
-    if (q == 0) {
-      z[0].re *= cv<R>(hl[rowbase + 1]);
-      z[0].im *= cv<R>(hl[rowbase + N + 1]);
-    } else {
-      const R h = cv<R>(hl[rowbase + q + 1]);
-      z[q].re *= h;
-      z[q].im *= h;
-    }
-  }
-  __syncthreads();
-  // realft(data, n, -1): split loop, then four1(data, n/2, -1)
-  realft_split(z, trm, N, R(0.5));
-  if (threadIdx.x == 0) {
-    const R h1r = z[0].re;
-    z[0].re = R(0.5) * (h1r + z[0].im);
-    z[0].im = R(0.5) * (h1r - z[0].im);
-  }
-  __syncthreads();
-  bitrev_permute(z, N, lg);
-  four1_stages(z, t4m, N);
-  const R scale = R(2.) / R(ni);
-  for (int k = threadIdx.x; k < N; k += blockDim.x) {
-    x[2 * k + 1] = z[k].re * scale;
-    x[2 * k + 2] = z[k].im * scale;
-  }
-  __syncthreads();
+  __syncwarp();
+  four1_stages(z, t4m, N, L);
 }
 
 __device__ __forceinline__ bool row_is_filtered(const DevModel &M, int j, int vgrid) {
   return fabs(M.lat[vgrid ? 2 * j : 2 * j + 1]) >= M.lat0;
 }
 
-// zonal_filter(index, plane, NULL, TWODIM) of planes k0..k0+gridDim.y-1, from src into dst
-// (dst may equal src).  Block = one row j in -1..nj+1; rows outside the filtered set are
+// zonal_filter(index, plane, NULL, TWODIM) of planes k0..k0+nplanes-1, from src into dst
+// (dst may equal src).  blockIdx.x = row j + 1, j in -1..nj+1; rows outside the filtered set are
 // copied; rows 0..nj+1 get periodic pads (bc_lateral).
 template <class R>
-__global__ void k_filter_planes(DevModel M, const double *src, int src_sel, double *dst, int k0, int vgrid) {
+__global__ void k_filter_planes(DevModel M, const double *src, int src_sel, double *dst, int k0, int nplanes, int vgrid, RowShape S) {
   if (epic_member(M, src, dst)) return;
   extern __shared__ __align__(16) unsigned char smraw[];
-  R *sm = reinterpret_cast<R *>(smraw);
   src += plane_offset(M, src_sel);
-  const int j = (int)blockIdx.x - 1;
+  const int j = (int)blockIdx.x - 1, ni = M.ni;
   if (j > M.nj + 1) return;   // a member with fewer rows than the launch (batches of mixed sizes)
-  const int k = k0 + (int)blockIdx.y;
-  const long long base = M.at(k, j, 0);
-  R *x = sm;
-  FilterSmem<R> fs = carve_filter(sm + (M.ni + 2), M.ni);
+  const RowLane L = row_lane(S, k0, k0 + nplanes - 1);
+  const int base = M.at(L.k, j, 0);
   const bool valid = vgrid ? (j >= 1 && j <= M.nj) : (j >= 0 && j <= M.nj);
-  const bool filt = valid && row_is_filtered(M, j, vgrid);
-  if (!filt) {
-    if (src != dst)
-      for (int i = threadIdx.x; i <= M.ni + 1; i += blockDim.x) dst[base + i] = src[base + i];
-    __syncthreads();
-    if (j >= 0 && threadIdx.x == 0) {
-      dst[base] = dst[base + M.ni];
-      dst[base + M.ni + 1] = dst[base + 1];
+  if (!(valid && row_is_filtered(M, j, vgrid))) {
+    if (!L.live) return;
+    const bool pads = j >= 0;
+    for (int i = L.gl; i <= ni + 1; i += L.G) {
+      if (pads && (i == 0 || i == ni + 1)) dst[base + i] = src[base + (i == 0 ? ni : 1)];
+      else if (src != dst) dst[base + i] = src[base + i];
     }
     return;
   }
-  load_twiddles(M, fs);
-  for (int i = threadIdx.x; i <= M.ni + 1; i += blockDim.x) x[i] = cv<R>(src[base + i]);
-  __syncthreads();
-  filter_row_smem(M, x, vgrid ? M.high_lat_pv : M.high_lat_h, M.at2(j, 0), fs);
-  for (int i = threadIdx.x + 1; i <= M.ni; i += blockDim.x) write_with_pads(dst, M, base, i, x[i]);
+  R *x = reinterpret_cast<R *>(smraw) + L.r * S.stride;
+  const int lg = fft_log(ni);
+  for (int e = L.gl; e < ni; e += L.G) x[fft_place(e, lg)] = L.live ? cv<R>(src[base + e + 1]) : R(0.);
+  __syncwarp();
+  filter_row<R>(M, reinterpret_cast<Cplx<R> *>(x), (vgrid ? M.high_lat_pv : M.high_lat_h) + M.at2(j, 0), L);
+  if (!L.live) return;
+  const R scale = filter_scale<R>(ni);
+  for (int e = L.gl; e < ni; e += L.G) write_with_pads(dst, M, base, e + 1, to_d(x[e] * scale));
 }
 
 
@@ -269,7 +237,7 @@ __global__ void k_varz_tables(DevModel M, const double *buff, int sel, int index
     const double hsum = h1 + h2;
     double z;
     if (q == 0) {
-      const double w1 = (h1 + hsum) / hsum, w2 = -h1 / hsum;
+      const double w1 = div_rn(h1 + hsum, hsum), w2 = div_rn(-h1, hsum);
       z = w1 * del1 + w2 * del2;
       if (pchst(z, del1) <= 0.0) z = 0.0;
       else if (pchst(del1, del2) < 0.0) {
@@ -277,7 +245,7 @@ __global__ void k_varz_tables(DevModel M, const double *buff, int sel, int index
         if (fabs(dmx) < fabs(z)) z = dmx;
       }
     } else if (q == n - 1) {
-      const double w1 = -h2 / hsum, w2 = (h2 + hsum) / hsum;
+      const double w1 = div_rn(-h2, hsum), w2 = div_rn(h2 + hsum, hsum);
       z = w1 * del1 + w2 * del2;
       if (pchst(z, del2) <= 0.0) z = 0.0;
       else if (pchst(del1, del2) < 0.0) {
@@ -360,242 +328,217 @@ __device__ __forceinline__ dfl varz_profile_mixed(const Trip *t, const double *k
   return index == 2 ? d2df(knot[kay]) * exp_df(inc, exp2tab) : d2df(knot[kay]) + inc;
 }
 
+// The FP64 form's profile of one latitude: the knots, and splint_pchip's cubic (epic_funcs_util.c:926-946)
+// of every interval, whose coefficients depend on the interval alone -- computed once per block, not
+// once per column.
+struct VarzKnot { double x, y, z, c2, c3; };
+__device__ __forceinline__ void varz_intervals(const Trip *t, int n, VarzKnot *kn) {
+  for (int q = threadIdx.x; q < n; q += blockDim.x) {
+    VarzKnot v = {t[q].x, t[q].y, t[q].z, 0., 0.};
+    if (q + 1 < n) {
+      const double h = t[q + 1].x - t[q].x;
+      const double delta = div_rn(t[q + 1].y - t[q].y, h);
+      const double del1 = div_rn(t[q].z - delta, h), del2 = div_rn(t[q + 1].z - delta, h);
+      v.c3 = div_rn(del1 + del2, h);
+      v.c2 = -(del1 + del1 + del2);
+    }
+    kn[q] = v;
+  }
+}
+__device__ __forceinline__ double varz_profile(const VarzKnot *kn, int n, double g) {
+  int kay;   // find_place_in_table (epic_funcs_util.c:2908-2967)
+  if (fcmp(g, kn[0].x) <= 0) kay = 0;
+  else if (fcmp(g, kn[n - 1].x) >= 0) kay = n - 2;
+  else {
+    int il = -1, iu = n;
+    while (iu - il > 1) {
+      const int im = (iu + il) >> 1;
+      if (fcmp(g, kn[im].x) >= 0) il = im; else iu = im;
+    }
+    kay = il < 0 ? 0 : il;
+  }
+  const VarzKnot v = kn[kay];
+  const double xx = g - v.x;
+  return v.y + xx * (v.z + xx * (v.c2 + xx * v.c3));
+}
+// doubles of the block's table: knots and cubics (FP64), knot values and VarzInterval (mixed)
+__host__ __device__ inline size_t varz_table_doubles(int nk, bool mixed) {
+  return (size_t)(nk + 2) * (mixed ? 1 + sizeof(VarzInterval) / 8 : sizeof(VarzKnot) / 8) + (((nk + 2) & 1) ? 1 : 0);
+}
+
 // The rest of the THREEDIM zonal_filter: subtract var(gz), filter, add it back.
-// Block = one row (k = kstart + blockIdx.y, j = jstart + blockIdx.x).
+// blockIdx.x = row j - jstart, levels kstart.. by blockIdx.y.  Shared memory: the table, then per row
+// the profile's values (binary64) and the deviation (the compute type).
 template <class R>
-__global__ void k_varz_filter_rows(DevModel M, double *buff, int sel, int index, int kstart, int kend) {
+__global__ void k_varz_filter_rows(DevModel M, double *buff, int sel, int index, int kstart, int kend, RowShape S) {
   if (epic_member(M, buff)) return;
-  extern __shared__ __align__(16) unsigned char smraw[];
+  extern __shared__ __align__(16) double smd[];
   buff += plane_offset(M, sel);
-  const int jstart = index == 1 ? 1 : 0;
+  constexpr bool exact = std::is_same_v<R, double>;
+  const int jstart = index == 1 ? 1 : 0, ni = M.ni;
   const int j = jstart + (int)blockIdx.x;
   if (j > M.nj) return;   // a member with fewer rows than the launch (batches of mixed sizes)
-  const int k = kstart + (int)blockIdx.y;
   const int vgrid = index == 1;
   const Trip *t = reinterpret_cast<const Trip *>(M.ptable) + (long long)(j + 1) * (M.nk + 2);
   const int n = kend - kstart + 1;
   const double *gz = M.gz;
-  const long long base = M.at(k, j, 0);
   const bool filt = row_is_filtered(M, j, vgrid);
   // The mixed forms leave unfiltered rows untouched (their subtract-and-add-back is the identity
   // up to one rounding); the FP64 form repeats the reference's arithmetic on them.
-  if (!filt && !std::is_same_v<R, double>) return;
-  if constexpr (!std::is_same_v<R, double>) {
-    double *vzd = reinterpret_cast<double *>(smraw), *knot = vzd + (M.ni + 2);
-    VarzInterval *iv = reinterpret_cast<VarzInterval *>(knot + (M.nk + 2));
-    R *x = reinterpret_cast<R *>(iv + (M.nk + 2));
-    FilterSmem<R> fs = carve_filter(x + (M.ni + 2), M.ni);
-    load_twiddles(M, fs);
-    varz_intervals_mixed(t, n, index, knot, iv);
-    __syncthreads();
-    // the profile's argument, its value and the deviation in double-float (integer and FP32
-    // pipes: this kernel had the FP64 unit half busy); the deviation is filtered in binary32 and
-    // added back to the profile in binary64 below, the profile's own rounding cancelling
-    for (int i = threadIdx.x + 1; i <= M.ni; i += blockDim.x) {
-      dfl gzd;
-      switch (index) {
-        case 0: gzd = df_ldexp(d2df(gz[M.at(k, j, i)]) + d2df(gz[M.at(k, j, i - 1)]), -1); break;
-        case 1: gzd = df_ldexp(d2df(gz[M.at(k, j, i)]) + d2df(gz[M.at(k, j - 1, i)]), -1); break;
-        case 2: gzd = df_ldexp(d2df(gz[M.at(k, j, i)]) + d2df(gz[M.at(k - 1, j, i)]), -1); break;
-        default: gzd = d2df(gz[M.at(k, j, i)]); break;
-      }
-      const dfl v = varz_profile_mixed(t, knot, iv, n, index, gzd, M.exp2tab);
-      vzd[i] = df2d(v);
-      x[i] = (d2df(buff[base + i]) - v).hi;
-    }
-    __syncthreads();
-    filter_row_smem(M, x, vgrid ? M.high_lat_pv : M.high_lat_h, M.at2(j, 0), fs);
-    // HDRY (index 2): restore_mass, which timestep() calls next (epic_timestep.c:212), on the
-    // filtered value; unfiltered rows are untouched here and already restored
-    for (int i = threadIdx.x + 1; i <= M.ni; i += blockDim.x) {
-      const double v = f2d(x[i]) + vzd[i];
-      write_with_pads(buff, M, base, i, index == 2 ? dmaxr(M.h_min[k], v) : v);
-    }
-    return;
-  }
-  R *sm = reinterpret_cast<R *>(smraw);
-  R *x = sm, *vz = sm + (M.ni + 2);
-  FilterSmem<R> fs = carve_filter(sm + 2 * (M.ni + 2), M.ni);
-  if (filt) load_twiddles(M, fs);
-  for (int i = threadIdx.x + 1; i <= M.ni; i += blockDim.x) {
-    R gzz;
-    switch (index) {
-      case 0: gzz = R(.5) * (cv<R>(gz[M.at(k, j, i)]) + cv<R>(gz[M.at(k, j, i - 1)])); break;
-      case 1: gzz = R(.5) * (cv<R>(gz[M.at(k, j, i)]) + cv<R>(gz[M.at(k, j - 1, i)])); break;
-      case 2: gzz = R(.5) * (cv<R>(gz[M.at(k, j, i)]) + cv<R>(gz[M.at(k - 1, j, i)])); break;
-      default: gzz = cv<R>(gz[M.at(k, j, i)]); break;
-    }
-    // find_place_in_table (epic_funcs_util.c:2908-2967) and splint_pchip (:926-946)
-    int kay;
-    if (RMath<R>::cmp(gzz, cv<R>(t[0].x)) <= 0) kay = 0;
-    else if (RMath<R>::cmp(gzz, cv<R>(t[n - 1].x)) >= 0) kay = n - 2;
-    else {
-      int il = -1, iu = n;
-      while (iu - il > 1) {
-        const int im = (iu + il) >> 1;
-        if (RMath<R>::cmp(gzz, cv<R>(t[im].x)) >= 0) il = im; else iu = im;
-      }
-      kay = il < 0 ? 0 : il;
-    }
-    const Trip *tk = t + kay;
-    const R h = cv<R>(tk[1].x) - cv<R>(tk[0].x);
-    const R delta = qdiv(cv<R>(tk[1].y) - cv<R>(tk[0].y), h);
-    const R del1 = qdiv(cv<R>(tk[0].z) - delta, h);
-    const R del2 = qdiv(cv<R>(tk[1].z) - delta, h);
-    const R c3 = qdiv(del1 + del2, h);
-    const R c2 = -(del1 + del1 + del2);
-    const R xx = gzz - cv<R>(tk[0].x);
-    R v = cv<R>(tk[0].y) + xx * (cv<R>(tk[0].z) + xx * (c2 + xx * c3));
-    if (index == 2) v = RMath<R>::exp(M, v);
-    vz[i] = v;
-    x[i] = cv<R>(buff[base + i] - to_d(v));
-  }
+  if (!filt && !exact) return;
+  VarzKnot *kn = reinterpret_cast<VarzKnot *>(smd);
+  VarzInterval *iv = reinterpret_cast<VarzInterval *>(smd);
+  double *knot = smd + (size_t)(M.nk + 2) * (sizeof(VarzInterval) / 8);
+  if constexpr (exact) varz_intervals(t, n, kn);
+  else varz_intervals_mixed(t, n, index, knot, iv);
   __syncthreads();
-  if (filt) filter_row_smem(M, x, vgrid ? M.high_lat_pv : M.high_lat_h, M.at2(j, 0), fs);
-  for (int i = threadIdx.x + 1; i <= M.ni; i += blockDim.x) {   // HDRY (index 2): restore_mass too
-    const double v = to_d(x[i]) + to_d(vz[i]);
-    write_with_pads(buff, M, base, i, index == 2 ? dmaxr(M.h_min[k], v) : v);
+  const RowLane L = row_lane(S, kstart, kend);
+  const int k = L.k, base = M.at(k, j, 0), lg = fft_log(ni);
+  double *vz = smd + varz_table_doubles(M.nk, !exact) + (size_t)L.r * S.stride;
+  R *x = reinterpret_cast<R *>(vz + ni);
+  // the other value of the mean that gives the profile's argument: U, V and layer variables lie
+  // half-way between GZ's points
+  const int other = index == 0 ? -1 : (index == 1 ? -M.iadim : (index == 2 ? -(int)M.n2 : 0));
+  for (int e = L.gl; e < ni; e += L.G) {
+    const int p = base + e + 1;
+    double v = 0.;
+    R dev = R(0.);
+    if (L.live) {
+      if constexpr (exact) {
+        const double g = other ? half_of(gz[p] + gz[p + other]) : gz[p];
+        v = varz_profile(kn, n, g);
+        if (index == 2) v = xexp(M, v);
+        dev = buff[p] - v;
+      } else {
+        // the profile's argument, its value and the deviation in double-float (integer and FP32
+        // pipes: this kernel had the FP64 unit half busy); the deviation is filtered in binary32 and
+        // added back to the profile in binary64 below, the profile's own rounding cancelling
+        const dfl g = other ? df_ldexp(d2df(gz[p]) + d2df(gz[p + other]), -1) : d2df(gz[p]);
+        const dfl pv = varz_profile_mixed(t, knot, iv, n, index, g, M.exp2tab);
+        v = df2d(pv);
+        dev = (d2df(buff[p]) - pv).hi;
+      }
+    }
+    vz[e] = v;
+    x[filt ? fft_place(e, lg) : e] = dev;
+  }
+  __syncwarp();
+  if (filt) filter_row<R>(M, reinterpret_cast<Cplx<R> *>(x), (vgrid ? M.high_lat_pv : M.high_lat_h) + M.at2(j, 0), L);
+  if (!L.live) return;
+  const R scale = filter_scale<R>(ni);
+  // HDRY (index 2): restore_mass, which timestep() calls next (epic_timestep.c:212), on the new value
+  for (int e = L.gl; e < ni; e += L.G) {
+    const double v = to_d(filt ? x[e] * scale : x[e]) + vz[e];
+    write_with_pads(buff, M, base, e + 1, index == 2 ? dmaxr(M.h_min[k], v) : v);
   }
 }
 
-// Zonal pass of hsu_advection (epic_flux.c:1316-1484) for one row: the fluxes come from a
+// Row j of a zonal advection pass in shared memory: the zonally filtered copy that the fluxes come
+// from, in order, a[0..ni-1] for i = 1..ni.
+template <class R>
+__device__ __forceinline__ void zonal_filtered_row(const DevModel &M, const double *buff, int base, int j, R *a, const RowLane &L) {
+  const bool filt = row_is_filtered(M, j, 0);   // of the whole block
+  const int ni = M.ni, lg = fft_log(ni);
+  for (int e = L.gl; e < ni; e += L.G) a[filt ? fft_place(e, lg) : e] = L.live ? cv<R>(buff[base + e + 1]) : R(1.);
+  __syncwarp();
+  if (!filt) return;
+  filter_row<R>(M, reinterpret_cast<Cplx<R> *>(a), M.high_lat_h + M.at2(j, 0), L);
+  const R scale = filter_scale<R>(ni);
+  for (int e = L.gl; e < ni; e += L.G) a[e] = a[e] * scale;
+  __syncwarp();
+}
+
+// Zonal pass of hsu_advection (epic_flux.c:1316-1484), a row per lane group: the fluxes come from a
 // zonally filtered copy of the row, the update goes to the unfiltered field.
 // kind: 0 = interface variable (unity, THETA), 1 = HDRY (layer; u averaged to the layer),
 // 2 = NU_TURB (interface variable with the floor NU_TURB_MIN).
+// Shared arrays by i - 1: a (the filtered row), ff (the flux through the west face), ap (the
+// predicted row); w (the velocity) by i, with the field's own pads.
 template <class R>
-__global__ void k_hsu_zonal(DevModel M, double *buff, int kind, int kstart) {
+__global__ void k_hsu_zonal(DevModel M, double *buff, int kind, int kstart, RowShape S) {
   if (epic_member(M, buff)) return;
   extern __shared__ __align__(16) unsigned char smraw[];
-  R *sm = reinterpret_cast<R *>(smraw);
-  const int ni = M.ni, W = ni + 2;
+  const int ni = M.ni;
   const int j = (int)blockIdx.x;
   if (j > M.nj) return;   // a member with fewer rows than the launch (batches of mixed sizes)
-  const int k = kstart + (int)blockIdx.y;
-  R *a = sm, *um = a + W, *up = um + W, *ff = up + W, *ap = ff + W, *d1 = ap + W, *d2 = d1 + W, *aa = d2 + W;
-  FilterSmem<R> fs = carve_filter(aa + W, ni);
-  const R ep = R(1.e-10), DT = cv<R>(M.dt);
+  const RowLane L = row_lane(S, kstart, M.nk);
+  const int k = L.k, base = M.at(k, j, 0);
+  R *a = reinterpret_cast<R *>(smraw) + L.r * S.stride, *ff = a + ni, *ap = ff + ni, *w = ap + ni;
+  const R DT = cv<R>(M.dt);
   const R a_min = kind == 1 ? cv<R>(M.h_min[k]) : (kind == 2 ? cv<R>(1.e-3 * M.kinvisc) : R(0.));
-  const long long base = M.at(k, j, 0);
-  const bool filt = row_is_filtered(M, j, 0);
-  if (filt) load_twiddles(M, fs);
   const double *U = M.u + (long long)M.ctl->it_uv * M.n3;
   const R n_inv = qdiv(R(1.), cv<R>(M.n[2 * j + 1]));
   const R mn1 = cv<R>(M.mn[2 * j + 1]);
-  for (int i = threadIdx.x; i <= ni + 1; i += blockDim.x) {
-    a[i] = cv<R>(buff[base + i]);
+  for (int i = L.gl; i <= ni + 1; i += L.G) {
     // u2d, with periodic pads for the layer average (bc_lateral(u2d))
     const int ii = kind == 1 ? (i == 0 ? ni : (i == ni + 1 ? 1 : i)) : i;
-    const R u2d = kind == 1 ? R(.5) * (cv<R>(U[M.at(k, j, ii)]) + cv<R>(U[M.at(k - 1, j, ii)])) : cv<R>(U[M.at(k, j, i)]);
-    um[i] = rmin(R(0.), u2d * n_inv);
-    up[i] = rmax(R(0.), u2d * n_inv);
+    R u2d = R(0.);
+    if (L.live) u2d = kind == 1 ? half_of(cv<R>(U[M.at(k, j, ii)]) + cv<R>(U[M.at(k - 1, j, ii)])) : cv<R>(U[M.at(k, j, i)]);
+    w[i] = u2d * n_inv;
   }
-  __syncthreads();
-  if (filt) filter_row_smem(M, a, M.high_lat_h, M.at2(j, 0), fs);
-  if (threadIdx.x == 0) { a[0] = a[ni]; a[ni + 1] = a[1]; }
-  __syncthreads();
-  // predictor
-  for (int i = threadIdx.x + 1; i <= ni; i += blockDim.x) ff[i] = up[i] * a[i - 1] + um[i] * a[i];
-  __syncthreads();
-  if (threadIdx.x == 0) { ff[0] = ff[ni]; ff[ni + 1] = ff[1]; }
-  __syncthreads();
-  for (int i = threadIdx.x + 1; i <= ni; i += blockDim.x) ap[i] = a[i] + (ff[i] - ff[i + 1]) * mn1 * DT;
-  __syncthreads();
-  if (threadIdx.x == 0) { ap[0] = ap[ni]; ap[ni + 1] = ap[1]; }
-  __syncthreads();
-  // corrector
-  for (int i = threadIdx.x + 1; i <= ni; i += blockDim.x) {
-    ff[i] = R(.5) * (up[i] * (ap[i] + a[i - 1]) + um[i] * (ap[i - 1] + a[i]));
-    d1[i] = ap[i] - a[i - 1];
-    d2[i] = ap[i] - a[i + 1];
-    const R tmp = fabs(a[i - 1] - R(2.) * a[i] + a[i + 1]) + ep;
-    aa[i] = tmp * tmp;
+  zonal_filtered_row<R>(M, buff, base, j, a, L);
+  const int mask = ni - 1;   // ni is a power of 2: rows wrap
+  for (int e = L.gl; e < ni; e += L.G) ff[e] = hsu_upwind<R>(w[e + 1], a[e], a[(e - 1) & mask]);
+  __syncwarp();
+  for (int e = L.gl; e < ni; e += L.G) ap[e] = a[e] + (ff[e] - ff[(e + 1) & mask]) * mn1 * DT;
+  __syncwarp();
+  for (int e = L.gl; e < ni; e += L.G) {
+    const R v = w[e + 1];
+    const bool neg = is_neg(v);   // from cell e west to e-1, else from e-1 east to e
+    const int west = (e - 1) & mask, u = neg ? e : west, d = neg ? west : e, uu = (neg ? e + 1 : e - 2) & mask;
+    const R au = a[u], ad = a[d], auu = a[uu];
+    const R t = fabs((neg ? ad : auu) - R(2.) * au + (neg ? auu : ad)) + R(1.e-10);
+    ff[e] = hsu_face<R>(v, w[neg ? e + 2 : e], au, ad, ap[d], ap[u] - auu, t * t, a_min, a_min, mn1, DT);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    d1[0] = d1[ni]; d1[ni + 1] = d1[1];
-    d2[0] = d2[ni]; d2[ni + 1] = d2[1];
-    aa[0] = aa[ni]; aa[ni + 1] = aa[1];
-  }
-  __syncthreads();
-  for (int i = threadIdx.x + 1; i <= ni; i += blockDim.x) {
-    const R uhatp = sqrt(up[i] * up[i - 1]);
-    const R uhatm = -sqrt(um[i] * um[i + 1]);
-    const R mu = (up[i] - um[i]) * mn1 * DT;
-    const R al = qdiv(R(1.) + mu, R(6.));
-    R gap = qdiv(aa[i - 1], aa[i - 1] + (a[i - 1] - a_min) * (a[i] - a_min));
-    gap = gap * gap;
-    R gam = qdiv(aa[i], aa[i] + (a[i - 1] - a_min) * (a[i] - a_min));
-    gam = gam * gam;
-    const R hal = qdiv(R(1.), R(2.) * al) - R(1.);
-    const R bep = R(1.) + hal * gap;
-    const R bem = R(1.) + hal * gam;
-    const R behatp = R(1.) - gap, behatm = R(1.) - gam;
-    const R g = -al * (up[i] * bep * d1[i] - uhatp * behatp * d1[i - 1] + um[i] * bem * d2[i - 1] - uhatm * behatm * d2[i]);
-    ff[i] += g;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) { ff[0] = ff[ni]; ff[ni + 1] = ff[1]; }
-  __syncthreads();
+  __syncwarp();
+  if (!L.live) return;
   // HDRY (kind 1): restore_mass (epic_adjust.c:45-96), which advection() calls next
   // (epic_flux.c:623), on the new value -- the same max per cell, one pass fewer
-  for (int i = threadIdx.x + 1; i <= ni; i += blockDim.x) {
-    const double v = buff[base + i] + to_d((ff[i] - ff[i + 1]) * mn1 * DT);
-    write_with_pads(buff, M, base, i, kind == 1 ? dmaxr(M.h_min[k], v) : v);
+  for (int e = L.gl; e < ni; e += L.G) {
+    const double v = buff[base + e + 1] + to_d((ff[e] - ff[(e + 1) & mask]) * mn1 * DT);
+    write_with_pads(buff, M, base, e + 1, kind == 1 ? dmaxr(M.h_min[k], v) : v);
   }
 }
 
-// Zonal pass of akima_advection (epic_flux.c:1826-1932) for one row: the fluxes come from a
+// Zonal pass of akima_advection (epic_flux.c:1826-1932), a row per lane group: the fluxes come from a
 // zonally filtered copy of the row, the update goes to the unfiltered field.
 // kind: 0 = interface variable (unity, THETA), 1 = HDRY (layer; u averaged to the layer).
+// Shared arrays by i - 1: a (the filtered row), dl (the limited slopes), ff (the fluxes).
 template <class R>
-__global__ void k_akima_zonal(DevModel M, double *buff, int kind, int kstart) {
+__global__ void k_akima_zonal(DevModel M, double *buff, int kind, int kstart, RowShape S) {
   if (epic_member(M, buff)) return;
   extern __shared__ __align__(16) unsigned char smraw[];
-  R *sm = reinterpret_cast<R *>(smraw);
-  const int ni = M.ni, W = ni + 2;
+  const int ni = M.ni;
   const int j = (int)blockIdx.x;
   if (j > M.nj) return;   // a member with fewer rows than the launch (batches of mixed sizes)
-  const int k = kstart + (int)blockIdx.y;
-  R *a = sm, *u2d = a + W, *da = u2d + W, *dl = da + W, *ff = dl + W;
-  FilterSmem<R> fs = carve_filter(ff + W, ni);
+  const RowLane L = row_lane(S, kstart, M.nk);
+  const int k = L.k, base = M.at(k, j, 0), mask = ni - 1;
+  R *a = reinterpret_cast<R *>(smraw) + L.r * S.stride, *dl = a + ni, *ff = dl + ni;
   const R DT = cv<R>(M.dt);
-  const long long base = M.at(k, j, 0);
-  const bool filt = row_is_filtered(M, j, 0);
-  if (filt) load_twiddles(M, fs);
   const double *U = M.u + (long long)M.ctl->it_uv * M.n3;
   const R n_inv = qdiv(R(1.), cv<R>(M.n[2 * j + 1]));
   const R mn1 = cv<R>(M.mn[2 * j + 1]);
-  for (int i = threadIdx.x; i <= ni + 1; i += blockDim.x) {
-    a[i] = cv<R>(buff[base + i]);
-    // u2d, with periodic pads for the layer average (bc_lateral(u2d))
-    const int ii = kind == 1 ? (i == 0 ? ni : (i == ni + 1 ? 1 : i)) : i;
-    u2d[i] = kind == 1 ? R(.5) * (cv<R>(U[M.at(k, j, ii)]) + cv<R>(U[M.at(k - 1, j, ii)])) : cv<R>(U[M.at(k, j, i)]);
+  zonal_filtered_row<R>(M, buff, base, j, a, L);
+  for (int e = L.gl; e < ni; e += L.G) {
+    const R d0 = a[e] - a[(e - 1) & mask], d1 = a[(e + 1) & mask] - a[e];
+    const R tmp = d0 * d1;
+    dl[e] = (tmp > R(0.)) ? qdiv(R(2.) * tmp, d0 + d1) : R(0.);
   }
-  __syncthreads();
-  if (filt) filter_row_smem(M, a, M.high_lat_h, M.at2(j, 0), fs);
-  if (threadIdx.x == 0) { a[0] = a[ni]; a[ni + 1] = a[1]; }
-  __syncthreads();
-  for (int i = threadIdx.x + 1; i <= ni; i += blockDim.x) da[i] = a[i] - a[i - 1];
-  __syncthreads();
-  if (threadIdx.x == 0) { da[0] = da[ni]; da[ni + 1] = da[1]; }
-  __syncthreads();
-  for (int i = threadIdx.x + 1; i <= ni; i += blockDim.x) {
-    const R tmp = da[i] * da[i + 1];
-    dl[i] = (tmp > R(0.)) ? qdiv(R(2.) * tmp, da[i] + da[i + 1]) : R(0.);
+  __syncwarp();
+  for (int e = L.gl; e < ni; e += L.G) {
+    const R aval = half_of(a[e] + a[(e - 1) & mask]) - qdiv(dl[e] - dl[(e - 1) & mask], R(6.));
+    R u2d = R(0.);
+    if (L.live) {
+      const int p = base + e + 1;
+      u2d = kind == 1 ? half_of(cv<R>(U[p]) + cv<R>(U[p - (int)M.n2])) : cv<R>(U[p]);
+    }
+    ff[e] = u2d * aval * n_inv;
   }
-  __syncthreads();
-  if (threadIdx.x == 0) { dl[0] = dl[ni]; dl[ni + 1] = dl[1]; }
-  __syncthreads();
-  for (int i = threadIdx.x + 1; i <= ni; i += blockDim.x) {
-    const R aval = R(.5) * (a[i] + a[i - 1]) - qdiv(dl[i] - dl[i - 1], R(6.));
-    ff[i] = u2d[i] * aval * n_inv;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) { ff[0] = ff[ni]; ff[ni + 1] = ff[1]; }
-  __syncthreads();
-  for (int i = threadIdx.x + 1; i <= ni; i += blockDim.x) {   // HDRY (kind 1): restore_mass too
-    const double v = buff[base + i] + to_d((ff[i] - ff[i + 1]) * mn1 * DT);
-    write_with_pads(buff, M, base, i, kind == 1 ? dmaxr(M.h_min[k], v) : v);
+  __syncwarp();
+  if (!L.live) return;
+  for (int e = L.gl; e < ni; e += L.G) {   // HDRY (kind 1): restore_mass too
+    const double v = buff[base + e + 1] + to_d((ff[e] - ff[(e + 1) & mask]) * mn1 * DT);
+    write_with_pads(buff, M, base, e + 1, kind == 1 ? dmaxr(M.h_min[k], v) : v);
   }
 }
 
@@ -623,14 +566,24 @@ __global__ void k_filter_rows_unfiltered(DevModel M, const double *src, int src_
 
 // ---- launchers ----
 
-static int row_threads(const DevModel &M) { return M.tb[TB_ROW] > 0 ? M.tb[TB_ROW] : (M.ni >= 256 ? 128 : 64); }
+// The shape of a row kernel whose rows take `stride` values of `elem` bytes each: lanes a row as above;
+// 128 threads a block (or the tuning table's choice), fewer where its rows would take more than 48 KB,
+// so that several blocks share an SM.
+static RowShape row_shape(const DevModel &M, int stride, size_t elem, unsigned &threads) {
+  RowShape S;
+  S.G = M.ni >= 128 ? 32 : (M.ni >= 64 ? 16 : 8);
+  S.stride = stride;
+  threads = M.tb[TB_ROW] > 0 ? (unsigned)M.tb[TB_ROW] : 128u;
+  while (threads > 32 && threads / (unsigned)S.G * (unsigned)stride * elem > 48 * 1024) threads /= 2;
+  S.rows = (int)threads / S.G;
+  return S;
+}
+static size_t row_bytes(const RowShape &S, size_t elem) { return (size_t)S.rows * (size_t)S.stride * elem; }
 static size_t relem(int fp32) { return fp32 ? sizeof(float) : sizeof(double); }
 
 int launch_filter_planes(const DevModel &M, const double *src, int src_sel, double *dst, int k0, int nplanes, int vgrid, cudaStream_t s,
                          int fp32, int shift, int pads_set) {
   if (nplanes <= 0) return 0;
-  const size_t smem = ((size_t)(M.ni + 2) + filter_smem_elems(M.ni)) * relem(fp32);
-  dim3 grid(M.nj + 3, nplanes);
   if (fp32 && filter_gemm_usable(M)) {
     // The rows the operator leaves alone are copied (and padded) by a light kernel of their own:
     // done by the operator's blocks, each reserving the product's ~83 KB of shared memory, they
@@ -641,7 +594,10 @@ int launch_filter_planes(const DevModel &M, const double *src, int src_sel, doub
       k_filter_rows_unfiltered<<<zg(epic_blocks(32 * warps, 128), M), 128, 0, s>>>(M, src, src_sel, dst, k0, nplanes, vgrid);
     return launch_filter_planes_gemm(M, src, src_sel, dst, k0, nplanes, vgrid, s, shift);
   }
-  EPIC_LAUNCH_R(fp32, k_filter_planes, grid, row_threads(M), smem, s, M, src, src_sel, dst, k0, vgrid);
+  unsigned th;
+  const RowShape S = row_shape(M, M.ni, relem(fp32), th);
+  const dim3 grid(M.nj + 3, epic_blocks(nplanes, S.rows));
+  EPIC_LAUNCH_R(fp32, k_filter_planes, grid, th, row_bytes(S, relem(fp32)), s, M, src, src_sel, dst, k0, nplanes, vgrid, S);
   return 0;
 }
 
@@ -649,25 +605,27 @@ int launch_varz_filter(const DevModel &M, double *buff, int sel, int index, int 
   const int jstart = index == 1 ? 1 : 0;
   const int nrows = M.nj - jstart + 1;
   k_varz_tables<<<zg(epic_blocks(32LL * nrows, 128), M), 128, 0, s>>>(M, buff, sel, index, kstart, kend);
-  const size_t smem = M.mixed ? ((size_t)(M.ni + 2) + (M.nk + 2)) * sizeof(double) + (size_t)(M.nk + 2) * sizeof(VarzInterval) +
-                                    ((size_t)(M.ni + 2) + filter_smem_elems(M.ni)) * sizeof(float)
-                             : (2 * (size_t)(M.ni + 2) + filter_smem_elems(M.ni)) * sizeof(double);
-  dim3 grid(nrows, kend - kstart + 1);
-  EPIC_LAUNCH_R(M.mixed, k_varz_filter_rows, grid, row_threads(M), smem, s, M, buff, sel, index, kstart, kend);
+  unsigned th;
+  const RowShape S = row_shape(M, M.mixed ? M.ni + M.ni / 2 : 2 * M.ni, sizeof(double), th);
+  const size_t smem = varz_table_doubles(M.nk, M.mixed) * sizeof(double) + row_bytes(S, sizeof(double));
+  const dim3 grid(nrows, epic_blocks(kend - kstart + 1, S.rows));
+  EPIC_LAUNCH_R(M.mixed, k_varz_filter_rows, grid, th, smem, s, M, buff, sel, index, kstart, kend, S);
   return 0;
 }
 
 int launch_akima_zonal(const DevModel &M, double *buff, int kind, int kstart, cudaStream_t s) {
-  const size_t smem = (5 * (size_t)(M.ni + 2) + filter_smem_elems(M.ni)) * relem(M.mixed);
-  dim3 grid(M.nj + 1, M.nk - kstart + 1);
-  EPIC_LAUNCH_R(M.mixed, k_akima_zonal, grid, row_threads(M), smem, s, M, buff, kind, kstart);
+  unsigned th;
+  const RowShape S = row_shape(M, 3 * M.ni, relem(M.mixed), th);
+  const dim3 grid(M.nj + 1, epic_blocks(M.nk - kstart + 1, S.rows));
+  EPIC_LAUNCH_R(M.mixed, k_akima_zonal, grid, th, row_bytes(S, relem(M.mixed)), s, M, buff, kind, kstart, S);
   return 0;
 }
 
 int launch_hsu_zonal(const DevModel &M, double *buff, int kind, int kstart, cudaStream_t s) {
-  const size_t smem = (8 * (size_t)(M.ni + 2) + filter_smem_elems(M.ni)) * relem(M.mixed);
-  dim3 grid(M.nj + 1, M.nk - kstart + 1);
-  EPIC_LAUNCH_R(M.mixed, k_hsu_zonal, grid, row_threads(M), smem, s, M, buff, kind, kstart);
+  unsigned th;
+  const RowShape S = row_shape(M, 4 * M.ni + 2, relem(M.mixed), th);
+  const dim3 grid(M.nj + 1, epic_blocks(M.nk - kstart + 1, S.rows));
+  EPIC_LAUNCH_R(M.mixed, k_hsu_zonal, grid, th, row_bytes(S, relem(M.mixed)), s, M, buff, kind, kstart, S);
   return 0;
 }
 
@@ -679,10 +637,10 @@ static void filter_attrs(int bytes) {
   cudaFuncSetAttribute(k_filter_planes<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-// Raised once to the largest row (ni = EPIC_MAX_NI), so models of different sizes in one process
-// never lower the limit for one another.
+// Raised once to the most a launch takes (row_shape's 48 KB and the varz kernels' table), so models of
+// different sizes in one process never lower the limit for one another.
 int filter_kernels_init(int) {
-  const size_t big = (8 * (size_t)(EPIC_MAX_NI + 2) + filter_smem_elems(EPIC_MAX_NI)) * sizeof(double);
+  const size_t big = 48 * 1024 + varz_table_doubles(EPIC_MAX_NK, false) * sizeof(double);
   filter_attrs<double>((int)big);
   filter_attrs<float>((int)big);
   return 0;

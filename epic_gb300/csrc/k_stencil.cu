@@ -472,15 +472,33 @@ __global__ void k_pgrad_lat(DevModel M) {
 // THETA), 2 = HDRY (v averaged to the layer), 3 = NU_TURB (interface, floor NU_TURB_MIN).  Four launches over all planes k0..nk.
 // ---------------------------------------------------------------------------------------------
 
+// the velocity through the v point over its map factor; 0 outside the rows 0..nj+1
 template <class R>
-__device__ __forceinline__ void vmp(const DevModel &M, const double *V, int kind, int k, int j, int i, R &vm, R &vp) {
+__device__ __forceinline__ R vm_at(const DevModel &M, const double *V, int kind, int k, int j, int i) {
+  if (j < 0 || j > M.nj + 1) return R(0.);
   R v2d;
-  if (j < 0 || j > M.nj + 1) { vm = vp = R(0.); return; }
   if (kind == 2) v2d = (j >= 1 && j <= M.nj) ? R(.5) * (cv<R>(V[M.at(k, j, i)]) + cv<R>(V[M.at(k - 1, j, i)])) : R(0.);
   else v2d = cv<R>(V[M.at(k, j, i)]);
   const R mi = (fabs(M.lat[2 * j]) == 90.) ? R(0.) : qdiv(R(1.), cv<R>(M.m[2 * j]));
-  vm = rmin(R(0.), v2d * mi);
-  vp = rmax(R(0.), v2d * mi);
+  return v2d * mi;
+}
+template <class R>
+__device__ __forceinline__ R hsu_floor(const DevModel &M, int kind, int k) {
+  return kind == 2 ? cv<R>(M.h_min[k]) : (kind == 3 ? cv<R>(1.e-3 * M.kinvisc) : R(0.));
+}
+// The corrector flux through v row j (1..nj) by velocity w: the rows u and d are upstream and
+// downstream of it, uu the row beyond u.  a, ap: the field and the predicted field by row.
+template <class R, class FA, class FP>
+__device__ __forceinline__ R hsu_merid_flux(const DevModel &M, R w, R w_up, int j, R a_min, R DT, FA a, FP ap) {
+  const int nj = M.nj;
+  const bool neg = is_neg(w);            // from row j south to j-1, else from j-1 north to j
+  const int u = neg ? j : j - 1, d = neg ? j - 1 : j, uu = neg ? j + 1 : j - 2;
+  const bool edge = neg ? u == nj : u == 0;
+  const R au = a(u), ad = a(d), auu = edge ? R(0.) : a(uu);
+  R t;
+  if (edge) t = fabs(neg ? ad - au : -au + ad) + R(1.e-10);
+  else t = fabs((neg ? ad : auu) - R(2.) * au + (neg ? auu : ad)) + R(1.e-10);
+  return hsu_face<R>(w, w_up, au, ad, ap(d), edge ? R(0.) : ap(u) - auu, t * t, a_min, a_min, cv<R>(M.mn[2 * j]), DT);
 }
 
 template <class R>
@@ -491,9 +509,8 @@ __global__ void k_hsu_merid_pred(DevModel M, const double *A, int kind, int k0) 
   const double *V = M.v + plane_offset(M, PL_UV);
   R ff = R(0.);
   if (c.j >= 1 && c.j <= M.nj) {
-    R vm, vp;
-    vmp<R>(M, V, kind, c.k, c.j, c.i, vm, vp);
-    ff = vp * cv<R>(A[M.at(c.k, c.j - 1, c.i)]) + vm * cv<R>(A[M.at(c.k, c.j, c.i)]);
+    const R w = vm_at<R>(M, V, kind, c.k, c.j, c.i);
+    ff = w * cv<R>(A[M.at(c.k, is_neg(w) ? c.j : c.j - 1, c.i)]);
   }
   write_with_pads(M.work1, M, M.at(c.k, c.j, 0), c.i, ff);
 }
@@ -517,38 +534,12 @@ __global__ void k_hsu_merid_corr(DevModel M, const double *A, int kind, int k0) 
   const int k = c.k, j = c.j, i = c.i, nj = M.nj;
   R ffv = R(0.);
   if (j >= 1 && j <= nj) {
-    const R ep = R(1.e-10), DT = cv<R>(M.dt);
-    const R a_min = kind == 2 ? cv<R>(M.h_min[k]) : (kind == 3 ? cv<R>(1.e-3 * M.kinvisc) : R(0.));
     const double *V = M.v + plane_offset(M, PL_UV);
     const double *AP = M.work2;
-    auto a = [&](int jj) { return cv<R>(A[M.at(k, jj, i)]); };
-    auto ap = [&](int jj) { return cv<R>(AP[M.at(k, jj, i)]); };
-    auto diff1 = [&](int jj) { return jj == 0 ? R(0.) : ap(jj) - a(jj - 1); };
-    auto diff2 = [&](int jj) { return jj == nj ? R(0.) : ap(jj) - a(jj + 1); };
-    auto aaa = [&](int jj) {
-      R t;
-      if (jj == 0) t = fabs(-a(0) + a(1)) + ep;
-      else if (jj == nj) t = fabs(a(nj - 1) - a(nj)) + ep;
-      else t = fabs(a(jj - 1) - R(2.) * a(jj) + a(jj + 1)) + ep;
-      return t * t;
-    };
-    R vm, vp, vmm, vpm, vmp1, vpp1;
-    vmp<R>(M, V, kind, k, j, i, vm, vp);
-    vmp<R>(M, V, kind, k, j - 1, i, vmm, vpm);
-    vmp<R>(M, V, kind, k, j + 1, i, vmp1, vpp1);
-    ffv = R(.5) * (vp * (ap(j) + a(j - 1)) + vm * (ap(j - 1) + a(j)));
-    const R vhatp = sqrt(vp * vpm);
-    const R vhatm = -sqrt(vm * vmp1);
-    const R mu = (vp - vm) * cv<R>(M.mn[2 * j]) * DT;
-    const R al = qdiv(R(1.) + mu, R(6.));
-    const R am1 = aaa(j - 1), a0 = aaa(j);
-    const R prod = (a(j - 1) - a_min) * (a(j) - a_min);
-    R gap = qdiv(am1, am1 + prod); gap = gap * gap;
-    R gam = qdiv(a0, a0 + prod); gam = gam * gam;
-    const R hal = qdiv(R(1.), R(2.) * al) - R(1.);
-    const R bep = R(1.) + hal * gap;
-    const R bem = R(1.) + hal * gam;
-    ffv += -al * (vp * bep * diff1(j) - vhatp * (R(1.) - gap) * diff1(j - 1) + vm * bem * diff2(j - 1) - vhatm * (R(1.) - gam) * diff2(j));
+    const R w = vm_at<R>(M, V, kind, k, j, i);
+    const R w_up = vm_at<R>(M, V, kind, k, is_neg(w) ? j + 1 : j - 1, i);
+    ffv = hsu_merid_flux<R>(M, w, w_up, j, hsu_floor<R>(M, kind, k), cv<R>(M.dt), [&](int jj) { return cv<R>(A[M.at(k, jj, i)]); },
+                            [&](int jj) { return cv<R>(AP[M.at(k, jj, i)]); });
   }
   write_with_pads(M.work3, M, M.at(k, j, 0), i, ffv);
 }
@@ -565,9 +556,9 @@ __global__ void k_hsu_merid_update(DevModel M, double *A, int k0) {
 }
 
 // The four meridional passes fused: one thread per (k, i) marches j = 0..nj and keeps, in a
-// sliding register window, the original field A at rows j-2..j+2 (A is updated in place behind
-// the march), the split velocity at rows j-1..j+2, the predictor fluxes FF at j+1, j+2, the
-// predicted field AP at j-1..j+1 and the corrector flux FFV at j.  Every value is the same
+// sliding register window, the original field A at rows j-1..j+2 (A is updated in place behind
+// the march), the velocity at rows j..j+2, the predictor fluxes FF at j+1, j+2, the
+// predicted field AP at j, j+1 and the corrector flux FFV at j.  Every value is the same
 // expression on the same operands as in the four passes (k_hsu_merid_pred/apred/corr/update),
 // so the results are identical bit for bit, with no scratch traffic.  Row j+3's loads are issued
 // at the top of iteration j, ahead of the arithmetic that does not need them.
@@ -579,85 +570,58 @@ __global__ void k_hsu_meridional(DevModel M, double *A, int kind, int k0) {
   if (i > M.ni) return;
   const int nj = M.nj;
   const double *V = M.v + plane_offset(M, PL_UV);
-  const R ep = R(1.e-10), DT = cv<R>(M.dt);
-  const R a_min = kind == 2 ? cv<R>(M.h_min[k]) : (kind == 3 ? cv<R>(1.e-3 * M.kinvisc) : R(0.));
+  const R DT = cv<R>(M.dt), a_min = hsu_floor<R>(M, kind, k);
   auto ld = [&](int jj) { return A[M.at(k, jj, i)]; };
-  auto ff_of = [&](int jj, R vm, R vp, R am1, R a0) { return (jj >= 1 && jj <= nj) ? vp * am1 + vm * a0 : R(0.); };
+  auto ff_of = [&](int jj, R w, R am1, R a0) { return (jj >= 1 && jj <= nj) ? hsu_upwind<R>(w, a0, am1) : R(0.); };
   auto ap_of = [&](int jj, double ad, R ff0, R ff1) { return cv<R>(ad + to_d((ff0 - ff1) * cv<R>(M.mn[2 * jj + 1]) * DT)); };
   // window at the top of iteration j
-  R a_m2 = R(0.), a_m1 = R(0.), a_0, a_1, a_2;   // A(j-2..j+2)
-  double ad_0, ad_1, ad_2;                       // A(j..j+2) in binary64
-  R vm_m1 = R(0.), vp_m1 = R(0.), vm_0, vp_0, vm_1, vp_1, vm_2, vp_2;   // split velocity at j-1..j+2
-  R ff_1, ff_2;                                  // FF(j+1), FF(j+2)
-  R ap_m1 = R(0.), ap_0, ap_1;                   // AP(j-1..j+1)
-  R ffv_0 = R(0.);                               // FFV(j); FFV(0) = 0
+  R a_m1 = R(0.), a_0, a_1, a_2;   // A(j-1..j+2)
+  double ad_0, ad_1, ad_2;         // A(j..j+2) in binary64
+  R w_0, w_1, w_2;                 // velocity at j..j+2
+  R ff_1, ff_2;                    // FF(j+1), FF(j+2)
+  R ap_0, ap_1;                    // AP(j), AP(j+1)
+  R ffv_0 = R(0.);                 // FFV(j); FFV(0) = 0
   ad_0 = ld(0); ad_1 = ld(1); ad_2 = ld(2);
   a_0 = cv<R>(ad_0); a_1 = cv<R>(ad_1); a_2 = cv<R>(ad_2);
-  vmp<R>(M, V, kind, k, 0, i, vm_0, vp_0);
-  vmp<R>(M, V, kind, k, 1, i, vm_1, vp_1);
-  vmp<R>(M, V, kind, k, 2, i, vm_2, vp_2);
+  w_0 = vm_at<R>(M, V, kind, k, 0, i);
+  w_1 = vm_at<R>(M, V, kind, k, 1, i);
+  w_2 = vm_at<R>(M, V, kind, k, 2, i);
   {
     const R ff_0 = R(0.);   // FF(0): row 0 is outside 1..nj
-    ff_1 = ff_of(1, vm_1, vp_1, a_0, a_1);
-    ff_2 = ff_of(2, vm_2, vp_2, a_1, a_2);
+    ff_1 = ff_of(1, w_1, a_0, a_1);
+    ff_2 = ff_of(2, w_2, a_1, a_2);
     ap_0 = ap_of(0, ad_0, ff_0, ff_1);
     ap_1 = ap_of(1, ad_1, ff_1, ff_2);
   }
-  // aaa(jj) of the reference from a(jj-1), a(jj), a(jj+1)
-  auto aaa = [&](int jj, R am, R a0v, R ap1) {
-    R t;
-    if (jj == 0) t = fabs(-a0v + ap1) + ep;
-    else if (jj == nj) t = fabs(am - a0v) + ep;
-    else t = fabs(am - R(2.) * a0v + ap1) + ep;
-    return t * t;
-  };
   for (int j = 0; j <= nj; j++) {
     // row j+3's inputs (rows beyond nj+1 do not exist and are not used)
     const int j3 = j + 3;
     double ad_3 = 0.;
-    R vm_3 = R(0.), vp_3 = R(0.);
+    R w_3 = R(0.);
     if (j3 <= nj + 1) {
       ad_3 = ld(j3);
-      vmp<R>(M, V, kind, k, j3, i, vm_3, vp_3);
+      w_3 = vm_at<R>(M, V, kind, k, j3, i);
     }
-    // FFV(j+1): the corrector flux of row jj = j+1 (k_hsu_merid_corr)
+    // FFV(j+1): the corrector flux of row j+1 (k_hsu_merid_corr), its rows j-1..j+2 in the window
     R ffv_1 = R(0.);
-    const int jj = j + 1;
-    if (jj >= 1 && jj <= nj) {
-      const R diff1_jj = ap_1 - a_0;                              // diff1(jj), jj >= 1
-      const R diff1_jm = (jj - 1 == 0) ? R(0.) : ap_0 - a_m1;     // diff1(jj-1)
-      const R diff2_jm = (jj - 1 == nj) ? R(0.) : ap_0 - a_1;     // diff2(jj-1)
-      const R diff2_jj = (jj == nj) ? R(0.) : ap_1 - a_2;         // diff2(jj)
-      R f = R(.5) * (vp_1 * (ap_1 + a_0) + vm_1 * (ap_0 + a_1));
-      const R vhatp = sqrt(vp_1 * vp_0);
-      const R vhatm = -sqrt(vm_1 * vm_2);
-      const R mu = (vp_1 - vm_1) * cv<R>(M.mn[2 * jj]) * DT;
-      const R al = qdiv(R(1.) + mu, R(6.));
-      const R am1 = aaa(jj - 1, a_m1, a_0, a_1), a0 = aaa(jj, a_0, a_1, a_2);
-      const R prod = (a_0 - a_min) * (a_1 - a_min);
-      R gap = qdiv(am1, am1 + prod); gap = gap * gap;
-      R gam = qdiv(a0, a0 + prod); gam = gam * gam;
-      const R hal = qdiv(R(1.), R(2.) * al) - R(1.);
-    const R bep = R(1.) + hal * gap;
-      const R bem = R(1.) + hal * gam;
-      f += -al * (vp_1 * bep * diff1_jj - vhatp * (R(1.) - gap) * diff1_jm + vm_1 * bem * diff2_jm - vhatm * (R(1.) - gam) * diff2_jj);
-      ffv_1 = f;
-    }
+    if (j + 1 <= nj)
+      ffv_1 = hsu_merid_flux<R>(
+          M, w_1, is_neg(w_1) ? w_2 : w_0, j + 1, a_min, DT,
+          [&](int jj) { return jj <= j ? (jj < j ? a_m1 : a_0) : (jj > j + 1 ? a_2 : a_1); }, [&](int jj) { return jj <= j ? ap_0 : ap_1; });
     // the update of row j (k_hsu_merid_update)
     const R da = (ffv_0 - ffv_1) * cv<R>(M.mn[2 * j + 1]) * cv<R>(M.dt);
     write_with_pads(A, M, M.at(k, j, 0), i, ad_0 + to_d(da));
     // advance the window to j+1: FF(j+3), AP(j+2)
     const R a_3 = cv<R>(ad_3);
-    const R ff_3 = ff_of(j3, vm_3, vp_3, a_2, a_3);
+    const R ff_3 = ff_of(j3, w_3, a_2, a_3);
     const R ap_2 = (j + 2 <= nj) ? ap_of(j + 2, ad_2, ff_2, ff_3) : R(0.);
-    a_m2 = a_m1; a_m1 = a_0; a_0 = a_1; a_1 = a_2; a_2 = a_3;
+    a_m1 = a_0; a_0 = a_1; a_1 = a_2; a_2 = a_3;
     ad_0 = ad_1; ad_1 = ad_2; ad_2 = ad_3;
-    vm_m1 = vm_0; vp_m1 = vp_0; vm_0 = vm_1; vp_0 = vp_1; vm_1 = vm_2; vp_1 = vp_2; vm_2 = vm_3; vp_2 = vp_3;
+    w_0 = w_1; w_1 = w_2; w_2 = w_3;
     ff_1 = ff_2; ff_2 = ff_3;
-    ap_m1 = ap_0; ap_0 = ap_1; ap_1 = ap_2;
+    ap_0 = ap_1; ap_1 = ap_2;
     ffv_0 = ffv_1;
   }
-  (void)a_m2; (void)vm_m1; (void)vp_m1; (void)ap_m1;
 }
 
 // ---------------------------------------------------------------------------------------------
