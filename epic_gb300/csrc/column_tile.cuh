@@ -15,11 +15,14 @@ namespace epic {
 // running sum, in the reference's order, so the results are those of one thread per column.
 constexpr int CT_WARPS = 8;
 constexpr int CT_THREADS = 32 * CT_WARPS;
+// The kernels of the FP64 form, whose pointwise phases are long chains of integer instructions, take
+// twice the warps when the launch has too few tiles to fill the GPU with eight each (tile_threads).
+constexpr int CT_THREADS_WIDE = 2 * CT_THREADS;
 // levels per warp whose loads a column kernel issues together before using them
 constexpr int TILE_SLOTS = 4;
 
 struct ColTile {
-  int lane, warp, j, i;
+  int lane, warp, nw, j, i;   // nw: the block's warps
   bool valid;
   long long base;   // M.at(0, j, i)
 };
@@ -27,6 +30,7 @@ __device__ __forceinline__ ColTile col_tile(const DevModel &M) {
   ColTile c;
   c.lane = (int)(threadIdx.x & 31);
   c.warp = (int)(threadIdx.x >> 5);
+  c.nw = (int)(blockDim.x >> 5);
   const int t = (int)blockIdx.x * 32 + c.lane;
   c.valid = t < (M.nj + 1) * M.iadim;
   c.j = c.valid ? t / M.iadim : 0;
@@ -36,6 +40,26 @@ __device__ __forceinline__ ColTile col_tile(const DevModel &M) {
 }
 // level k of a [k][lane] shared array
 #define CT(a, k) (a)[(k) * 32 + c.lane]
+
+// One column's running sum in the reference's order, by one warp: A[k] becomes acc + A[k0] + A[k0+dk]
+// + ... + A[k].  Eight increments are read ahead of the chain that adds them (the compiler cannot
+// move a read of the shared array over the write of the sum before it).
+__device__ __forceinline__ double ct_serial_sum(double *A, int k0, int k1, int dk, int lane, double acc) {
+  constexpr int NL = 8;
+  const int n = (k1 - k0) / dk + 1;
+  for (int q0 = 0; q0 < n; q0 += NL) {
+    double v[NL];
+#pragma unroll
+    for (int q = 0; q < NL; q++) v[q] = A[(k0 + min(q0 + q, n - 1) * dk) * 32 + lane];
+#pragma unroll
+    for (int q = 0; q < NL; q++) {
+      if (q0 + q >= n) break;
+      acc = acc + v[q];
+      A[(k0 + (q0 + q) * dk) * 32 + lane] = acc;
+    }
+  }
+  return acc;
+}
 
 // Running sum over the levels of every column of a tile, by all CT_WARPS warps: on entry
 // A[k] (k = 1..n) holds the increments and A[0] the starting value, on exit

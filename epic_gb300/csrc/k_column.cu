@@ -39,7 +39,7 @@ __global__ void k_source_sink(DevModel M) {
 // source_sink = 1: the step's source_sink (k_source_sink) first, in the same pass over the
 // columns: THETA(k >= k_sigma-1) += dt*HEAT3/EXNER3 in binary64, written back and then used.
 template <class R>
-__global__ void __launch_bounds__(CT_THREADS, 3) k_calc_w(DevModel M, int source_sink) {
+__global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : CT_THREADS, std::is_same_v<R, double> ? 2 : 3) k_calc_w(DevModel M, int source_sink) {
   if (epic_member(M)) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   R *sm = reinterpret_cast<R *>(smraw);
@@ -62,14 +62,14 @@ __global__ void __launch_bounds__(CT_THREADS, 3) k_calc_w(DevModel M, int source
     double v[TILE_SLOTS][5];
 #pragma unroll
     for (int r = 0; r < TILE_SLOTS; r++) {
-      const long long x = c.base + min(c.warp + r * CT_WARPS, nk) * n2;
+      const long long x = c.base + min(c.warp + r * c.nw, nk) * n2;
       v[r][0] = __ldg(M.p3 + x); v[r][1] = __ldg(M.div_uv3 + x); v[r][2] = __ldg(M.theta + x);
       v[r][3] = __ldg(M.heat3 + x); v[r][4] = __ldg(M.exner3 + x);
     }
 #pragma unroll
     for (int r = 0; r < TILE_SLOTS; r++)
-      if (c.warp + r * CT_WARPS <= nk) stage(c.warp + r * CT_WARPS, v[r][0], v[r][1], v[r][2], v[r][3], v[r][4]);
-    for (int k = c.warp + TILE_SLOTS * CT_WARPS; k <= nk; k += CT_WARPS) {
+      if (c.warp + r * c.nw <= nk) stage(c.warp + r * c.nw, v[r][0], v[r][1], v[r][2], v[r][3], v[r][4]);
+    for (int k = c.warp + TILE_SLOTS * c.nw; k <= nk; k += c.nw) {
       const long long x = c.base + k * n2;
       stage(k, M.p3[x], M.div_uv3[x], M.theta[x], M.heat3[x], M.exner3[x]);
     }
@@ -77,13 +77,13 @@ __global__ void __launch_bounds__(CT_THREADS, 3) k_calc_w(DevModel M, int source
   __syncthreads();
   const R ptop = CT(P, 0), pbot = CT(P, nk), psigma = CT(P, ks - 1);
   if (c.valid) {
-    for (int k = c.warp; k < nk; k += CT_WARPS) CT(LG, k) = RMath<R>::log(M, qdiv(CT(P, k + 1), CT(P, k)));
-    if (c.warp == CT_WARPS - 1) s_lp[c.lane] = RMath<R>::log(M, ptop / pbot);
+    for (int k = c.warp; k < nk; k += c.nw) CT(LG, k) = RMath<R>::log(M, qdiv(CT(P, k + 1), CT(P, k)));
+    if (c.warp == c.nw - 1) s_lp[c.lane] = RMath<R>::log(M, qdiv(ptop, pbot));
   }
   __syncthreads();
   const R lp = s_lp[c.lane];
   if (c.valid)
-    for (int k = 1 + c.warp; k < nk; k += CT_WARPS) {
+    for (int k = 1 + c.warp; k < nk; k += c.nw) {
       const R p3 = CT(P, k);
       const R theta3 = CT(DS, k), heat = CT(W, k), exner = CT(DF, k);
       R w = R(0.);
@@ -127,13 +127,22 @@ __global__ void __launch_bounds__(CT_THREADS, 3) k_calc_w(DevModel M, int source
       CT(W, k) = w;
     }
   __syncthreads();
-  if (c.warp == 0 && c.valid) {
+  // SUM_DIV(nk) = 0, so the dF/dpbot term contributes nothing.
+  if constexpr (std::is_same_v<R, double>) {
+    if (c.warp == 0 && c.valid) {
+      CT(DS, 1) = 0.;
+      if (nk > 2) ct_serial_sum(DS, 2, nk - 1, 1, c.lane, 0.);
+    }
+    __syncthreads();
+    if (c.valid)
+      for (int k = c.warp; k <= nk; k += c.nw)
+        M.w3[c.base + k * n2] = k == 0 || k == nk ? 0. : CT(W, k) - (CT(DS, k) * CT(DF, k) + 0.);
+  } else if (c.warp == 0 && c.valid) {
     M.w3[c.base] = 0.;
     M.w3[c.base + nk * n2] = 0.;
     double sum_div = 0.;
     for (int k = 1; k < nk; k++) {
       if (k >= 2) sum_div = sum_div + to_d(CT(DS, k));
-      // SUM_DIV(nk) = 0, so the dF/dpbot term contributes nothing.
       M.w3[c.base + k * n2] = to_d(CT(W, k)) - (sum_div * to_d(CT(DF, k)) + 0.);
     }
   }
@@ -184,7 +193,7 @@ __global__ void k_uv_drag(DevModel M) {
 // used.  Shared arrays [k][lane]: WA (the field), W (the vertical velocity; positive is towards
 // smaller k), PR (the predictor), FF (the fluxes).
 template <class R>
-__global__ void __launch_bounds__(CT_THREADS) k_hsu_vertical(DevModel M, double *buff, int kind) {
+__global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : CT_THREADS) k_hsu_vertical(DevModel M, double *buff, int kind) {
   if (epic_member(M, buff)) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   R *sm = reinterpret_cast<R *>(smraw);
@@ -202,26 +211,26 @@ __global__ void __launch_bounds__(CT_THREADS) k_hsu_vertical(DevModel M, double 
     return (k == 1 || k == nk) ? R(0.) : R(.5) * (cv<R>(M.w3[c.base + k * n2]) + cv<R>(M.w3[c.base + (k - 1) * n2]));
   };
   if (c.valid)
-    for (int k = (layer ? kf : kf - 1) + c.warp; k <= nk; k += CT_WARPS) CT(WA, k) = cv<R>(buff[c.base + k * n2]);
+    for (int k = (layer ? kf : kf - 1) + c.warp; k <= nk; k += c.nw) CT(WA, k) = cv<R>(buff[c.base + k * n2]);
   if (layer || nuk) {
     if (c.valid && layer)
-      for (int k = kf - 1 + c.warp; k <= nk; k += CT_WARPS) CT(W, k) = cv<R>(M.w3[c.base + k * n2]);
+      for (int k = kf - 1 + c.warp; k <= nk; k += c.nw) CT(W, k) = cv<R>(M.w3[c.base + k * n2]);
     if (c.valid && nuk) {
-      for (int k = kf + c.warp; k <= nk; k += CT_WARPS) CT(W, k) = w_layer(k);
+      for (int k = kf + c.warp; k <= nk; k += c.nw) CT(W, k) = w_layer(k);
       // entry 0 is never loaded for NU_TURB; the corrector reads it only against d2(1) = 0
       if (c.warp == 0) CT(W, 0) = R(0.);
     }
     __syncthreads();
     if (c.valid)
-      for (int k = kf - 1 + c.warp; k <= nk; k += CT_WARPS)
+      for (int k = kf - 1 + c.warp; k <= nk; k += c.nw)
         CT(FF, k) = (k == kf - 1 || k == nk) ? R(0.) : hsu_upwind<R>(CT(W, k), wa(k), wa(k + 1));
     __syncthreads();
     if (c.valid)
-      for (int k = kf + c.warp; k <= nk; k += CT_WARPS) CT(PR, k) = wa(k) + (CT(FF, k) - CT(FF, k - 1)) * dsi(2 * k) * DT;
+      for (int k = kf + c.warp; k <= nk; k += c.nw) CT(PR, k) = wa(k) + (CT(FF, k) - CT(FF, k - 1)) * dsi(2 * k) * DT;
     __syncthreads();
     // the corrector reads PR, WA and W only, so it rewrites FF in place
     if (c.valid)
-      for (int k = kf + c.warp; k < nk; k += CT_WARPS) {
+      for (int k = kf + c.warp; k < nk; k += c.nw) {
         const R w = CT(W, k);
         const bool neg = is_neg(w);   // from layer k down to k+1, else from k+1 up to k
         const int u = neg ? k : k + 1, d = neg ? k + 1 : k;   // the layers upstream and downstream
@@ -236,26 +245,26 @@ __global__ void __launch_bounds__(CT_THREADS) k_hsu_vertical(DevModel M, double 
       }
     __syncthreads();
     if (c.valid && layer)
-      for (int k = kf + c.warp; k <= nk; k += CT_WARPS) {
+      for (int k = kf + c.warp; k <= nk; k += c.nw) {
         const long long x = c.base + k * n2;
         buff[x] = buff[x] + to_d((CT(FF, k) - CT(FF, k - 1)) * dsi(2 * k) * DT);
       }
     if (c.valid && nuk)   // the interface update; w_ff[nk+1] is the 0 the THETA call left there
-      for (int k = kf + c.warp; k <= nk; k += CT_WARPS) {
+      for (int k = kf + c.warp; k <= nk; k += c.nw) {
         const long long x = c.base + k * n2;
         const R ffk1 = k == nk ? R(0.) : CT(FF, k + 1);
         buff[x] = buff[x] + to_d((ffk1 - CT(FF, k)) * dsi(2 * k + 1) * DT);
       }
   } else {
     if (c.valid)
-      for (int k = kf + c.warp; k <= nk; k += CT_WARPS) CT(W, k) = w_layer(k);
+      for (int k = kf + c.warp; k <= nk; k += c.nw) CT(W, k) = w_layer(k);
     __syncthreads();
     if (c.valid)
-      for (int k = kf + c.warp; k <= nk + 1; k += CT_WARPS)
+      for (int k = kf + c.warp; k <= nk + 1; k += c.nw)
         CT(FF, k) = k == nk + 1 ? R(0.) : hsu_upwind<R>(CT(W, k), wa(k - 1), wa(k));
     __syncthreads();
     if (c.valid)
-      for (int k = kf - 1 + c.warp; k <= nk; k += CT_WARPS)
+      for (int k = kf - 1 + c.warp; k <= nk; k += c.nw)
         CT(PR, k) = k == kf - 1 ? wa(kf - 1) : wa(k) + (CT(FF, k + 1) - CT(FF, k)) * dsi(2 * k + 1) * DT;
     __syncthreads();
     // For THETA (kf > 1) the entry below the first loaded one is the value the reference's
@@ -269,7 +278,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_hsu_vertical(DevModel M, double 
       return tmp * tmp;
     };
     if (c.valid)
-      for (int k = kf + c.warp; k <= nk; k += CT_WARPS) {
+      for (int k = kf + c.warp; k <= nk; k += c.nw) {
         const R w = CT(W, k);
         const bool neg = is_neg(w);   // from interface k-1 down to k, else from k up to k-1
         const int u = neg ? k - 1 : k, d = neg ? k : k - 1;
@@ -281,7 +290,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_hsu_vertical(DevModel M, double 
       }
     __syncthreads();
     if (c.valid)
-      for (int k = kf + c.warp; k <= nk; k += CT_WARPS) {
+      for (int k = kf + c.warp; k <= nk; k += c.nw) {
         const long long x = c.base + k * n2;
         const R ffk1 = k == nk ? R(0.) : CT(FF, k + 1);
         buff[x] = buff[x] + to_d((ffk1 - CT(FF, k)) * dsi(2 * k + 1) * DT);
@@ -384,7 +393,7 @@ __global__ void k_restore_mass(DevModel M) {
 // set_p2etc, epic_funcs_diag.c:3352-3569 (nq = 0: H2 is HDRY, PDRY3 is P3, HDRY3 is H3).
 // Shared arrays: P (interface pressure), HL (get_h at the layers), TH (THETA), PP (P^(kappa+1),
 // each interface's power computed once for the two layers that share it).
-__global__ void __launch_bounds__(CT_THREADS) k_set_p2etc(DevModel M, int update_theta) {
+__global__ void __launch_bounds__(CT_THREADS_WIDE) k_set_p2etc(DevModel M, int update_theta) {
   if (epic_member(M)) return;
   extern __shared__ double sm[];
   __shared__ double s_lp[32];
@@ -395,32 +404,27 @@ __global__ void __launch_bounds__(CT_THREADS) k_set_p2etc(DevModel M, int update
   __shared__ int s_kay[EPIC_MAX_NK + 1];
   if (update_theta) theta2_intervals(M, s_kay, nullptr);
   const double g = M.grav[2 * c.j + 1];
-  if (c.valid)   // stage H2 (in HL until the prefix sum is done) and THETA
-    for (int k = c.warp; k <= nk; k += CT_WARPS) {
+  if (c.valid)   // stage THETA and the layers' pressure thicknesses
+    for (int k = c.warp; k <= nk; k += c.nw) {
       CT(TH, k) = M.theta[c.base + k * n2];
-      if (k >= 1) CT(HL, k) = M.hdry[c.base + k * n2];
+      CT(P, k) = k == 0 ? M.p3[c.base] : M.dsgth[2 * k] * g * M.hdry[c.base + k * n2];
     }
   __syncthreads();
   if (c.warp == 0 && c.valid) {   // P3 top-down: P3(K) = P3(K-1) + dsgth*g*H2
-    double p = M.p3[c.base];
-    CT(P, 0) = p;
-    for (int k = 1; k <= nk; k++) {
-      p = p + M.dsgth[2 * k] * g * CT(HL, k);
-      CT(P, k) = p;
-    }
+    const double p = ct_serial_sum(P, 1, nk, 1, c.lane, CT(P, 0));
     s_lp[c.lane] = xlog(M, qdiv(CT(P, 0), p));   // log(ptop/pbot)
   }
   __syncthreads();
   const double ptop = CT(P, 0), pbot = CT(P, nk), lp = s_lp[c.lane];
   if (c.valid)   // pure-sigma interfaces: get_p_sigma
-    for (int k = ks - 1 + c.warp; k < nk; k += CT_WARPS) {
+    for (int k = ks - 1 + c.warp; k < nk; k += c.nw) {
       const double sigma = qdiv(M.sgth[2 * k + 1] - M.zeta0, M.zeta1 - M.zeta0);
       CT(P, k) = pbot * xexp(M, sigma * lp);
     }
   __syncthreads();
   const double kp1 = M.kappa + 1., kinv = qdiv(1., M.kappa);
   if (c.valid)
-    for (int k = c.warp; k <= nk; k += CT_WARPS) {
+    for (int k = c.warp; k <= nk; k += c.nw) {
       const double pk = CT(P, k);
       if (k >= 1) {
         const long long x = c.base + k * n2;
@@ -441,7 +445,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_set_p2etc(DevModel M, int update
     }
   __syncthreads();
   if (!c.valid) return;
-  for (int k = 1 + c.warp; k <= nk; k += CT_WARPS) {
+  for (int k = 1 + c.warp; k <= nk; k += c.nw) {
     const long long x = c.base + k * n2;
     const double top = CT(P, k - 1), bot = CT(P, k);
     double p2;   // onto_kk(P2_INDEX) at the layer, epic_funcs_diag.c:2601-2618
@@ -485,7 +489,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_set_p2etc(DevModel M, int update
 // the first DZDT3 terms.  Shared arrays: P, R (RHO3), T3, LG (log of successive pressure
 // ratios), GZ (the Leslie-Purser increments, then the running sum in place), Q (P/RHO3, each
 // level's quotient once for the four increments that read it).
-__global__ void __launch_bounds__(CT_THREADS) k_pgrad_vars_column(DevModel M) {
+__global__ void __launch_bounds__(CT_THREADS_WIDE) k_pgrad_vars_column(DevModel M) {
   if (epic_member(M)) return;
   extern __shared__ double sm[];
   __shared__ double s_rho2_1[32];
@@ -495,7 +499,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_pgrad_vars_column(DevModel M) {
   const double mu = M.mu_dry;
   double *P = sm, *R = P + 32 * L, *T3 = R + 32 * L, *LG = T3 + 32 * L, *GZ = LG + 32 * L, *Q = GZ + 32 * L;
   if (c.valid)
-    for (int k = c.warp; k <= nk; k += CT_WARPS) {
+    for (int k = c.warp; k <= nk; k += c.nw) {
       const long long x = c.base + k * n2;
       const double theta = M.theta[x], p = M.p3[x];
       const double t3 = return_temp(M, p, theta);
@@ -518,16 +522,21 @@ __global__ void __launch_bounds__(CT_THREADS) k_pgrad_vars_column(DevModel M) {
     }
   __syncthreads();
   if (c.valid) {
-    for (int k = c.warp; k < nk; k += CT_WARPS) CT(LG, k) = xlog(M, qdiv(CT(P, k + 1), CT(P, k)));
-    if (c.warp == CT_WARPS - 1) {
+    for (int k = c.warp; k < nk; k += c.nw) CT(LG, k) = xlog(M, qdiv(CT(P, k + 1), CT(P, k)));
+    if (c.warp == c.nw - 1) {
       M.rho2[c.base] = qdiv(CT(R, 0) * CT(R, 0), s_rho2_1[c.lane]);
       M.theta2[c.base] = M.sgth[0];
       M.t2[c.base] = CT(T3, 0);
     }
   }
   __syncthreads();
-  if (c.valid)
-    for (int k = 2 + c.warp; k <= nk - 1; k += CT_WARPS) {
+  if (c.valid)   // GZ3's value at the surface and the increments upwards
+    for (int k = 1 + c.warp; k <= nk + 1; k += c.nw) {
+      if (k == nk + 1) { CT(GZ, nk) = M.topo_scale * M.gz_surface[M.at2(c.j, c.i)]; continue; }
+      if (k == 1 || k == nk) {   // at the two ends
+        CT(GZ, k - 1) = qdiv(CT(P, k) + CT(P, k - 1), CT(R, k) + CT(R, k - 1)) * CT(LG, k - 1);
+        continue;
+      }
       const double dz10 = CT(LG, k), dz21 = CT(LG, k - 1), dz32 = CT(LG, k - 2);
       const double dz20 = dz21 + dz10, dz30 = dz32 + dz20, dz31 = dz32 + dz21;
       const double df0 = CT(Q, k + 1), df1 = CT(Q, k), df2 = CT(Q, k - 1), df3 = CT(Q, k - 2);
@@ -538,22 +547,13 @@ __global__ void __launch_bounds__(CT_THREADS) k_pgrad_vars_column(DevModel M) {
                           12.);
     }
   __syncthreads();
-  if (c.warp == 0 && c.valid) {   // GZ3 from the surface up
-    double gz = M.topo_scale * M.gz_surface[M.at2(c.j, c.i)];
-    CT(GZ, nk) = gz;
-    gz = gz + qdiv(CT(P, nk) + CT(P, nk - 1), CT(R, nk) + CT(R, nk - 1)) * CT(LG, nk - 1);
-    CT(GZ, nk - 1) = gz;
-    for (int k = nk - 1; k >= 2; k--) {
-      gz = gz + CT(GZ, k - 1);
-      CT(GZ, k - 1) = gz;
-    }
-    CT(GZ, 0) = gz + qdiv(CT(P, 1) + CT(P, 0), CT(R, 1) + CT(R, 0)) * CT(LG, 0);
-  }
+  if (c.warp == 0 && c.valid)   // GZ3 from the surface up
+    ct_serial_sum(GZ, nk - 1, 0, -1, c.lane, CT(GZ, nk));
   __syncthreads();
   if (!c.valid) return;
   const bool interior = c.i >= 1 && c.i <= M.ni;
   const long long itime = M.ctl->itime;
-  for (int k = c.warp; k <= nk; k += CT_WARPS) {
+  for (int k = c.warp; k <= nk; k += c.nw) {
     const long long x = c.base + k * n2;
     const double gzk = CT(GZ, k);
     const double old = M.gz3[x];
@@ -986,8 +986,14 @@ static inline unsigned ncol_blocks(const DevModel &M, int th) { return epic_bloc
 int launch_source_sink(const DevModel &M, cudaStream_t s) { k_source_sink<<<zg(ncol_blocks(M, TB(M, TB_COLUMN)), M), TB(M, TB_COLUMN), 0, s>>>(M); return 0; }
 static inline unsigned ntile_blocks(const DevModel &M) { return epic_blocks((long long)(M.nj + 1) * (M.ni + 2), 32); }
 static inline size_t tile_smem(const DevModel &M, int arrays) { return (size_t)arrays * 32 * (M.nk + 1) * sizeof(double); }
+// 16 warps a tile for the FP64 form's column kernels while the launch has at most a tile per SM:
+// each warp then takes one or two levels of a 20-level column instead of two or three.
+static inline int tile_threads(const DevModel &M) {
+  const long long tiles = (long long)ntile_blocks(M) * (M.nbatch > 1 ? M.nbatch : 1);
+  return !M.mixed && M.nk > CT_WARPS && tiles <= 152 ? CT_THREADS_WIDE : CT_THREADS;
+}
 int launch_calc_w(const DevModel &M, cudaStream_t s, bool with_source_sink) {
-  EPIC_LAUNCH_R(M.mixed, k_calc_w, ntile_blocks(M), CT_THREADS, tile_smem(M, 6), s, M, (int)with_source_sink);
+  EPIC_LAUNCH_R(M.mixed, k_calc_w, ntile_blocks(M), tile_threads(M), tile_smem(M, 6), s, M, (int)with_source_sink);
   return 0;
 }
 int launch_uv_drag(const DevModel &M, cudaStream_t s) {
@@ -996,7 +1002,7 @@ int launch_uv_drag(const DevModel &M, cudaStream_t s) {
   return 0;
 }
 int launch_hsu_vertical(const DevModel &M, double *buff, int kind, cudaStream_t s) {
-  EPIC_LAUNCH_R(M.mixed, k_hsu_vertical, ntile_blocks(M), CT_THREADS,
+  EPIC_LAUNCH_R(M.mixed, k_hsu_vertical, ntile_blocks(M), tile_threads(M),
                 (size_t)4 * 32 * (M.nk + 2) * (M.mixed ? sizeof(float) : sizeof(double)), s, M, buff, kind);
   return 0;
 }
@@ -1012,7 +1018,7 @@ int launch_restore_mass(const DevModel &M, cudaStream_t s) {
 int launch_set_p2etc(const DevModel &M, int update_theta, cudaStream_t s, bool early) {
   if (M.col64) k_set_p2etc_acc<<<zg(ntile_blocks(M), M), CT_THREADS, tile_smem(M, 4), s>>>(M, update_theta, !early);
   else if (M.mixed) k_set_p2etc_mixed<<<zg(ntile_blocks(M), M), CT_THREADS, tile_smem(M, 3), s>>>(M, update_theta, !early);
-  else k_set_p2etc<<<zg(ntile_blocks(M), M), CT_THREADS, tile_smem(M, 4), s>>>(M, update_theta);
+  else k_set_p2etc<<<zg(ntile_blocks(M), M), tile_threads(M), tile_smem(M, 4), s>>>(M, update_theta);
   return 0;
 }
 // The gas-giant lower boundary of store_pgrad_vars (epic_funcs_diag.c:3779-3811) with gz_from_u
@@ -1146,7 +1152,7 @@ int launch_store_pgrad_vars(const DevModel &M, cudaStream_t s, bool early, bool 
   }
   if (M.col64) (h2 ? k_pgrad_vars_column_acc_h2 : k_pgrad_vars_column_acc)<<<grid, CT_THREADS, smem, s>>>(M);
   else if (M.mixed) (h2 ? k_pgrad_vars_column_mixed<true, true> : k_pgrad_vars_column_mixed<true, false>)<<<grid, CT_THREADS, smem, s>>>(M);
-  else k_pgrad_vars_column<<<grid, CT_THREADS, tile_smem(M, 6), s>>>(M);
+  else k_pgrad_vars_column<<<grid, tile_threads(M), tile_smem(M, 6), s>>>(M);
   return dzdt ? launch_pgrad_dzdt(M, s) : 0;
 }
 int launch_pgrad_dzdt(const DevModel &M, cudaStream_t s) {

@@ -624,6 +624,48 @@ __global__ void k_hsu_meridional(DevModel M, double *A, int kind, int k0) {
   }
 }
 
+// The four passes in one kernel over tiles: a block takes TC neighbouring columns of one level, every
+// row, with the field, the velocity, the fluxes and the predicted field in shared memory [row][column]
+// and a barrier between the passes.  The same expressions on the same operands again.  On small and
+// middle grids the four passes are four launches with too few warps each (27 us in all at 128x64x20 in
+// the FP64 form), the march one thread a column in a chain of nj rows.
+template <class R>
+__global__ void __launch_bounds__(256) k_hsu_merid_tile(DevModel M, double *A, int kind, int k0, int TC) {
+  if (epic_member(M, A)) return;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int nj = M.nj, tx = (int)threadIdx.x & (TC - 1), ty = (int)threadIdx.x / TC, ny = (int)blockDim.x / TC;
+  const int i = (int)blockIdx.x * TC + tx + 1, k = k0 + (int)blockIdx.y;
+  if ((int)blockIdx.x * TC >= M.ni) return;   // a member narrower than the launch
+  const bool live = i <= M.ni;
+  R *a = reinterpret_cast<R *>(smraw) + tx, *w = a + (nj + 2) * TC, *ff = w + (nj + 2) * TC, *ap = ff + (nj + 2) * TC;
+  const double *V = M.v + plane_offset(M, PL_UV);
+  const R DT = cv<R>(M.dt), a_min = hsu_floor<R>(M, kind, k);
+  for (int j = ty; j <= nj + 1; j += ny) {
+    a[j * TC] = live && j <= nj ? cv<R>(A[M.at(k, j, i)]) : R(0.);
+    w[j * TC] = live ? vm_at<R>(M, V, kind, k, j, i) : R(0.);
+  }
+  __syncthreads();
+  for (int j = ty; j <= nj + 1; j += ny)
+    ff[j * TC] = j >= 1 && j <= nj ? hsu_upwind<R>(w[j * TC], a[j * TC], a[(j - 1) * TC]) : R(0.);
+  __syncthreads();
+  if (live)
+    for (int j = ty; j <= nj; j += ny)
+      ap[j * TC] = cv<R>(A[M.at(k, j, i)] + to_d((ff[j * TC] - ff[(j + 1) * TC]) * cv<R>(M.mn[2 * j + 1]) * DT));
+  __syncthreads();
+  if (live)
+    for (int j = 1 + ty; j <= nj; j += ny) {   // ff of rows 0 and nj+1 stays 0
+      const R v = w[j * TC];
+      ff[j * TC] = hsu_merid_flux<R>(M, v, w[(is_neg(v) ? j + 1 : j - 1) * TC], j, a_min, DT, [&](int jj) { return a[jj * TC]; },
+                                     [&](int jj) { return ap[jj * TC]; });
+    }
+  __syncthreads();
+  if (live)
+    for (int j = ty; j <= nj; j += ny) {
+      const R da = (ff[j * TC] - ff[(j + 1) * TC]) * cv<R>(M.mn[2 * j + 1]) * cv<R>(M.dt);
+      write_with_pads(A, M, M.at(k, j, 0), i, A[M.at(k, j, i)] + to_d(da));
+    }
+}
+
 // ---------------------------------------------------------------------------------------------
 // Meridional pass of akima_advection, epic_flux.c:1752-1820.  kind: 0/1 interface (unity,
 // THETA; V of the interface), 2 = HDRY (V averaged to the layer).  Two launches over planes
@@ -702,42 +744,45 @@ __global__ void k_d2dy2(DevModel M, const double *src, int src_sel, double *dst,
   write_with_pads(dst, M, M.at(k, j, 0), i, d);
 }
 
-// The mixed forms' first two d2dy2 passes of meridional_hyperviscosity in one kernel: the first
-// (of the state field, binary64 differences as in k_d2dy2) into shared memory, the second from
-// there into dst.  Block = 32 columns of one layer k0 + blockIdx.y, every row; the values are
-// those of two k_d2dy2<float> launches (the intermediate is a float either way), without the
+// The first two d2dy2 passes of meridional_hyperviscosity in one kernel: the first (of the state field;
+// binary64 differences in the mixed forms as in k_d2dy2) into shared memory, the second from
+// there into dst.  Block = TC columns of one layer k0 + blockIdx.y, every row; the values are
+// those of two k_d2dy2 launches (the mixed forms' intermediate is a float either way), without the
 // intermediate volume's write and read.
-__global__ void k_d2dy2_pair_mixed(DevModel M, const double *src, int src_sel, double *dst, int vgrid, int k0) {
+template <class R>
+__global__ void __launch_bounds__(256) k_d2dy2_pair(DevModel M, const double *src, int src_sel, double *dst, int vgrid, int k0, int TC) {
   if (epic_member(M, src, dst)) return;
+  constexpr bool exact = std::is_same_v<R, double>;
   const double coef1 = M.coef[2], coef2 = M.coef[4];
   extern __shared__ __align__(16) unsigned char smraw[];
-  float *d1 = reinterpret_cast<float *>(smraw);   // [row][lane]
   src += plane_offset(M, src_sel);
-  const int lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
-  const int i = (int)blockIdx.x * 32 + lane + 1;
+  const int tx = (int)threadIdx.x & (TC - 1), ty = (int)threadIdx.x / TC, ny = (int)blockDim.x / TC;
+  R *d1 = reinterpret_cast<R *>(smraw) + tx;   // [row][column]
+  const int i = (int)blockIdx.x * TC + tx + 1;
   const int k = k0 + (int)blockIdx.y;
   const int nj = M.nj, jlast = vgrid ? nj + 1 : nj;
   const double *cfa = vgrid ? M.v_coef : M.h_coef;
   const bool live = i <= M.ni;
-  for (int j = w; j <= jlast; j += nw) {
-    float d = 0.f;
+  for (int j = ty; j <= jlast; j += ny) {
+    R d = R(0.);
     if (live) {
       const double *cf = cfa + 3 * j;
-      const float a0 = d2f(coef1) * d2f(cf[0]), a2 = d2f(coef1) * d2f(cf[2]);
+      const R a0 = cv<R>(coef1) * cv<R>(cf[0]), a2 = cv<R>(coef1) * cv<R>(cf[2]);
       const int m = j == 0 ? 1 : (j == jlast ? j - 1 : j);
       const double hm = src[M.at(k, m, i)];
-      d = a0 * d2f(src[M.at(k, m - 1, i)] - hm) + a2 * d2f(src[M.at(k, m + 1, i)] - hm);
+      if constexpr (exact) d = a0 * src[M.at(k, m - 1, i)] + coef1 * cf[1] * hm + a2 * src[M.at(k, m + 1, i)];
+      else d = a0 * cv<R>(src[M.at(k, m - 1, i)] - hm) + a2 * cv<R>(src[M.at(k, m + 1, i)] - hm);
     }
-    d1[j * 32 + lane] = d;
+    d1[j * TC] = d;
   }
   __syncthreads();
   if (!live) return;
-  for (int j = w; j <= jlast; j += nw) {
+  for (int j = ty; j <= jlast; j += ny) {
     const double *cf = cfa + 3 * j;
-    const float a0 = d2f(coef2) * d2f(cf[0]), a1 = d2f(coef2) * d2f(cf[1]), a2 = d2f(coef2) * d2f(cf[2]);
+    const R a0 = cv<R>(coef2) * cv<R>(cf[0]), a1 = cv<R>(coef2) * cv<R>(cf[1]), a2 = cv<R>(coef2) * cv<R>(cf[2]);
     const int m = j == 0 ? 1 : (j == jlast ? j - 1 : j);
-    const float d = a0 * d1[(m - 1) * 32 + lane] + a1 * d1[m * 32 + lane] + a2 * d1[(m + 1) * 32 + lane];
-    write_with_pads(dst, M, M.at(k, j, 0), i, f2d(d));
+    const R d = a0 * d1[(m - 1) * TC] + a1 * d1[m * TC] + a2 * d1[(m + 1) * TC];
+    write_with_pads(dst, M, M.at(k, j, 0), i, to_d(d));
   }
 }
 
@@ -1177,12 +1222,6 @@ int launch_pgrad_lat(const DevModel &M, cudaStream_t s) {
   return 0;
 }
 
-// The fused march (k_hsu_meridional) has one thread per (k, i, member) walking nj+1 rows; it
-// wins once those threads fill the GPU (large batches).  Smaller launches take the four passes,
-// whose threads cover every cell.  Both give the same bits.  The tuning table's
-// TB_HSU_MERID_VARIANT entry overrides the choice (1 fused, 2 four passes).
-constexpr long long HSU_FUSED_MIN_THREADS = 65536;
-
 int launch_akima_meridional(const DevModel &M, double *buff, int kind, cudaStream_t s) {
   const int k0 = kind == 1 ? M.k_sigma - 1 : 1;
   const int nkk = M.nk - k0 + 1;
@@ -1191,6 +1230,14 @@ int launch_akima_meridional(const DevModel &M, double *buff, int kind, cudaStrea
   EPIC_LAUNCH_R(M.mixed, k_akima_merid_update, cells_blocks(M, nkk, M.nj + 1, th), th, 0, s, M, buff, k0);
   return 0;
 }
+
+// The meridional Hsu pass has three forms that give the same bits.  The tile (k_hsu_merid_tile) where
+// its four arrays of nj+2 rows fit MERID_SMEM with 32 columns, or 16 or 8 (64 bytes of a row); the march
+// (k_hsu_meridional, one thread per (k, i, member) walking nj+1 rows) once those threads fill the GPU
+// (large batches); else the four passes, whose threads cover every cell.  The tuning table's
+// TB_HSU_MERID_VARIANT entry overrides the choice (1 march, 2 four passes).
+constexpr long long HSU_FUSED_MIN_THREADS = 65536;
+constexpr size_t MERID_SMEM = 100 * 1024;   // two blocks per SM
 
 int launch_hsu_meridional(const DevModel &M, double *buff, int kind, cudaStream_t s) {
   const int k0 = kind == 1 ? M.k_sigma - 1 : 1;
@@ -1201,6 +1248,13 @@ int launch_hsu_meridional(const DevModel &M, double *buff, int kind, cudaStream_
                      (variant == 0 && (long long)M.ni * nkk * (M.nbatch > 1 ? M.nbatch : 1) >= HSU_FUSED_MIN_THREADS);
   if (fused) {
     EPIC_LAUNCH_R(M.mixed, k_hsu_meridional, dim3(epic_blocks(M.ni, th), nkk), th, 0, s, M, buff, kind, k0);
+    return 0;
+  }
+  const size_t col = (size_t)4 * (M.nj + 2) * (M.mixed ? sizeof(float) : sizeof(double));
+  int TC = 32;
+  while (TC >= 8 && TC * col > MERID_SMEM) TC /= 2;
+  if (variant == 0 && TC >= 8) {
+    EPIC_LAUNCH_R(M.mixed, k_hsu_merid_tile, dim3(epic_blocks(M.ni, TC), nkk), 256, TC * col, s, M, buff, kind, k0, TC);
     return 0;
   }
   EPIC_LAUNCH_R(M.mixed, k_hsu_merid_pred, cells_blocks(M, nkk, M.nj + 2, th), th, 0, s, M, buff, kind, k0);
@@ -1233,15 +1287,17 @@ int launch_meridional_hyperviscosity(const DevModel &M, int index, double *var, 
   double *bufs[2] = {M.work1, M.work2};
   int which = 0;
   double sign = 1.;
-  // the mixed forms fuse the first two passes when nothing is applied between them
-  const size_t pair_smem = (size_t)nrows * 32 * sizeof(float);
-  const bool pair = M.mixed && !(M.nu[2] > 0.) && M.nu[4] + M.nu[6] + M.nu[8] > 0. && pair_smem <= 48 * 1024;
+  // the first two passes in one kernel when nothing is applied between them
+  const size_t pair_col = (size_t)nrows * (M.mixed ? sizeof(float) : sizeof(double));
+  const int pair_tc = 16 * pair_col <= 48 * 1024 ? 16 : 8;
+  const bool pair = !(M.nu[2] > 0.) && M.nu[4] + M.nu[6] + M.nu[8] > 0. && pair_tc * pair_col <= 48 * 1024;
   for (int itmp = 2; itmp <= 8; itmp += 2) {
     double *dst = bufs[which];
     if (pair && itmp == 2) {
       // the second pass's output goes where the unfused loop leaves it
       dst = bufs[1];
-      k_d2dy2_pair_mixed<<<zg(dim3((unsigned)((M.ni + 31) / 32), (unsigned)nkk), M), 256, pair_smem, s>>>(M, var, sel, dst, vgrid, k0);
+      EPIC_LAUNCH_R(M.mixed, k_d2dy2_pair, dim3(epic_blocks(M.ni, pair_tc), (unsigned)nkk), 256, pair_tc * pair_col, s, M, var, sel, dst,
+                    vgrid, k0, pair_tc);
       itmp = 4;
       which = 1;
       sign = -sign;
@@ -1251,7 +1307,7 @@ int launch_meridional_hyperviscosity(const DevModel &M, int index, double *var, 
     }
     src_sel = PL_NONE;
     if (M.nu[itmp] > 0.) {
-      // k_d2dy2 / k_d2dy2_pair_mixed wrote every row of dst with its pads
+      // k_d2dy2 / k_d2dy2_pair wrote every row of dst with its pads
       launch_filter_planes(M, dst, PL_NONE, dst, k0, nkk, vgrid, s, M.mixed, 0, 1);
       EPIC_LAUNCH_R(M.mixed, k_visc_apply, cells_blocks(M, nkk, vgrid ? M.nj : M.nj + 1, TB(M, TB_VISC)), TB(M, TB_VISC), 0, s, M, var, sel, dst, vgrid, sign, k0, nkk);
     }
@@ -1295,7 +1351,11 @@ int launch_zonal_hyperviscosity(const DevModel &M, int index, double *var, int s
 
 // the largest dynamic shared memory of a launch, raised once for the process (models of all sizes)
 int stencil_kernels_init() {
-  return cudaFuncSetAttribute(k_zonal_visc_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VISC_ROWS_SMEM) == cudaSuccess ? 0 : -1;
+  if (cudaFuncSetAttribute(k_zonal_visc_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VISC_ROWS_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(k_hsu_merid_tile<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MERID_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(k_hsu_merid_tile<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MERID_SMEM) != cudaSuccess)
+    return -1;
+  return 0;
 }
 
 int launch_divergence_damping(const DevModel &M, cudaStream_t s) {

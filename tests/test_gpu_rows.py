@@ -2,9 +2,11 @@
 zonal hyperviscosity, the polar row sums), the column kernels beside them and the meridional passes, in
 the FP64 form at the ends of their range of row lengths: every stage equals the correctly rounded
 restatement bit for bit."""
+import numpy as np
 import pytest
 
-from epic_gb300 import EPIC_ADV_AKIMA, EPIC_ADV_HSU, EPIC_PROFILE_N2, HSConfig
+from epic_gb300 import (EPIC_ADV_AKIMA, EPIC_ADV_HSU, EPIC_PROFILE_N2, EPIC_SYNC_DIAGS_ONLY, HSConfig, Model, TUNE_HSU_MERID_VARIANT,
+                        hs_setup)
 from test_gpu_parity import _stage_by_stage
 
 pytestmark = pytest.mark.gpu
@@ -19,3 +21,21 @@ def test_rows(gpu, ni, nj, nk, adv):
     a = min(1., 2. * nj / ni)   # hyperviscosity stable at the shorter of the two spacings
     _stage_by_stage(HSConfig(ni=ni, nj=nj, nk=nk, dt=max(1, 600 // ni), seed=ni + nk, advection_scheme=adv, nu4=0.5 * a**4,
                              nu6=0.05 * a**6, nu8=0.02 * a**8, state="jet", profile=EPIC_PROFILE_N2, turbulence=ni == 32))
+
+
+# the meridional Hsu pass's forms (tiles of 32, 16 and 8 columns, the march, the four passes) on the last
+# and first number of rows of each
+@pytest.mark.parametrize("form,nj", [(0, 98), (0, 99), (0, 198), (0, 199), (0, 399), (1, 198), (1, 199), (1, 799)])
+def test_meridional_forms(gpu, form, nj):
+    ga, f = hs_setup(HSConfig(ni=16, nj=nj, nk=4, dt=5, seed=nj, state="jet", profile=EPIC_PROFILE_N2))
+    got = []
+    for variant in (0, 1, 2):
+        m = Model(ga, form)
+        m.set_tuning([0] * TUNE_HSU_MERID_VARIANT + [variant])
+        m.upload(f)
+        m.timestep(EPIC_SYNC_DIAGS_ONLY)
+        m.run(2)
+        got.append(m.download())
+    for n in ("hdry", "theta", "p3", "u"):
+        for g in got[1:]:
+            assert np.array_equal(got[0].arrays[n], g.arrays[n]), n
