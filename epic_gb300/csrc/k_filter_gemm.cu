@@ -24,7 +24,13 @@
 // the host, already split into TF32 hi and lo parts, and kept in HBM for the filtered rows only
 // (ni/32 x 32 KB per row); the TMA engine copies each step's pair into shared memory
 // (cp.async.bulk.tensor with the 128-byte swizzle, completion counted on an mbarrier) while the
-// threads convert and stage the planes' values.
+// threads convert and stage the planes' values.  At ni = 128 a row's four tiles stay in shared memory
+// and a CTA takes several groups of columns in turn.
+//
+// What bounds it: latency on a single model (a few dozen CTAs, each a chain of load, convert, multiply,
+// store), the staging and the plane traffic on a large batch.  So eight warps stage and store while one
+// more brings the operator tiles and issues the products, all through mbarriers (no block barrier in
+// the pipeline), with every tile of a short row and four chunks of plane values on their way at once.
 //
 // With shift set, each row of each plane is filtered as x - x(1), and x(1) is added back to the
 // output in binary64: the operator passes a constant unchanged (its wavenumber-0 weight is 1), so
@@ -52,8 +58,11 @@ namespace {
 constexpr int FG_M = 128;        // output points per tile (tensor-memory lanes)
 constexpr int FG_KC = 32;        // K elements per staged chunk: one 128-byte swizzle row of FP32
 constexpr int FG_NMAX = 64;      // columns per CTA ((member, plane) pairs), a multiple of 32
-constexpr int FG_THREADS = 128;  // four warps: one per 32-lane quarter of tensor memory
-constexpr unsigned FG_WAIT_LIMIT = 1u << 22;
+constexpr int FG_STAGE = 256;    // eight staging and epilogue warps: two per 32-lane quarter of tensor memory
+constexpr int FG_THREADS = FG_STAGE + 32;   // and one that issues the operator copies and the products
+constexpr int FG_BUFS = 4;       // operator tile pairs and chunks of plane values in shared memory, each
+constexpr int FG_GROUPS = 8;     // column groups a CTA takes in turn at most
+constexpr unsigned FG_WAIT_LIMIT = 1u << 20;
 constexpr unsigned FG_A_BYTES = FG_M * FG_KC * 4;   // one operator tile (hi or lo): 16 KB
 
 // Byte offset of element (r, e), 0 <= e < 32, in a 128B-swizzled K-major tile of FP32 rows.
@@ -103,7 +112,8 @@ __device__ __forceinline__ void tma_tile(unsigned dst, const void *map, int y, u
       : "memory");
 }
 
-__device__ __forceinline__ bool mbar_wait(unsigned mbar, unsigned phase) {
+// Bounded; gives up at once when another wait of the CTA has.
+__device__ __forceinline__ bool mbar_wait(unsigned mbar, unsigned phase, volatile int *fail) {
   for (unsigned it = 0; it < FG_WAIT_LIMIT; it++) {
     uint32_t done;
     asm volatile(
@@ -112,275 +122,326 @@ __device__ __forceinline__ bool mbar_wait(unsigned mbar, unsigned phase) {
         : "r"(mbar), "r"(phase)
         : "memory");
     if (done) return true;
+    if (*fail) return false;
   }
+  *fail = 1;
   return false;
+}
+__device__ __forceinline__ void mbar_arrive(unsigned mbar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
+}
+__device__ __forceinline__ void mma_commit(unsigned mbar) {   // arrives once the products issued so far are done
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
 }
 
 }  // namespace
 
-// Block = one row j in -1..nj+1 (x) and, in y, one group of G members times one chunk of pc
-// planes: column n = g pc + p is plane k0 + chunk pc + p of member q0 + g, N = G pc rounded up to
-// 32 (idle columns stay zero).  Rows outside the filtered set return at once
+// blockIdx.x = row j + 1, j in -1..nj+1.  The columns of a launch lie in `units` groups: group u is
+// plane chunk u % nch (pc planes) of G members from q0 = (u / nch) G; column n = g pc + p is plane
+// k0 + chunk pc + p of member q0 + g, N = G pc rounded up to 32 (idle columns stay zero).
+// blockIdx.y / msplit = the first group of a CTA, which takes every gs-th from there; msplit CTAs (a
+// cluster) share a row's 128-point output tiles.  Rows outside the filtered set return at once
 // (k_filter_rows_unfiltered copies them).  A member the batch has halted keeps its planes
-// untouched.  G > 1 only when the members share the launch's geometry and operator (fop_shared).
+// untouched.  G > 1, and several groups per CTA, only when the members share the launch's geometry and
+// operator (fop_shared).
 //
-// The product runs as a two-stage pipeline over steps t = (K chunk c, output tile mt): the
-// operator tiles are double-buffered by step, the planes' tile by K chunk (staged once per chunk,
-// read by its mtiles output tiles); while the tensor cores multiply step t, TMA brings step t+1's
-// operator tiles and the threads stage the next chunk, whose inputs are already on their way from
-// global memory into registers.  Each step's products are committed to the mbarrier of its buffer;
-// a buffer is refilled only after the commit of the step that last read it (commits complete in
-// issue order).
-__global__ void __launch_bounds__(FG_THREADS) k_filter_planes_gemm(DevModel M, const double *src, int src_sel, double *dst, int k0,
-                                                                     int nplanes, int vgrid, int shift, int pc, int G, int N, int msplit) {
+// Steps t count (group, K chunk c, output tile) in order.  The issuing thread waits for step t's
+// operator tiles and chunk, issues the products, commits them to the buffers they read, and refills the
+// operator buffer of step t-1 for step t-1+FG_BUFS; with `resident` (ni = 128, one tile per chunk) the
+// four buffers are filled once.  The staging threads keep FG_BUFS chunks of their columns' values in
+// registers ahead of the one they convert, across groups.  In place, the CTAs of a cluster have all read
+// a row before any writes it.
+__global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M, const double *src, int src_sel, double *dst, int k0,
+                                                                      int nplanes, int vgrid, int shift, int pc, int G, int N, int msplit,
+                                                                      int units, int gs, int resident) {
   extern __shared__ __align__(16) unsigned char fg_raw[];
-  __shared__ __align__(8) uint64_t bars[4];   // products of buffer 0 / 1 done; operator tiles of buffer 0 / 1 landed
+  // operator tiles landed / read (per buffer), plane chunk staged / read (per buffer), accumulator
+  // complete / read out
+  __shared__ __align__(8) uint64_t bars[4 * FG_BUFS + 2];
   __shared__ uint32_t tmem_base;
-  __shared__ int fail;
-  __shared__ const double *s_src[FG_NMAX];
-  __shared__ double *s_dst[FG_NMAX];
-  __shared__ int s_col[FG_NMAX];             // offset of the column's row (i = 0) in its member's field, -1 when idle
-  __shared__ unsigned char s_colg[FG_NMAX];  // the column's member slot g
-  __shared__ double s_x1[FG_NMAX];           // the subtracted value of each column's row (shift), else 0
-  const int tid = (int)threadIdx.x, warp = tid >> 5;
+  __shared__ volatile int fail;
+  __shared__ const double *s_src[FG_GROUPS][FG_NMAX];   // each column's row (i = 0), null when idle
+  __shared__ double *s_dst[FG_GROUPS][FG_NMAX];
+  __shared__ double s_x1[FG_GROUPS][FG_NMAX];           // the subtracted value of each column's row (shift), else 0
+  const int tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int j = (int)blockIdx.x - 1;
   const int nch = (nplanes + pc - 1) / pc;
-  const int yq = (int)blockIdx.y / msplit, msi = (int)blockIdx.y - yq * msplit;
-  const int chunk = yq % nch, q0 = (yq / nch) * G;
+  const int u0 = (int)blockIdx.y / msplit, msi = (int)blockIdx.y - u0 * msplit;
   const int members = M.batch ? M.nbatch : 1;
   // geometry: a one-member CTA takes its member's own (batches of mixed sizes); the members of
   // a larger group share the launch's
-  const DevModel &Mg = M.batch ? M.batch[q0] : M;
+  const DevModel &Mg = M.batch ? M.batch[(u0 / nch) * G] : M;
   const DevModel &opm = M.fop_shared ? M : Mg;
   const int ni = Mg.ni, mtiles = ni / FG_M, nchunks = ni / FG_KC, ntiles = ni / FG_KC;
-  // this CTA's output tiles: msplit CTAs share a row's mtiles (a member narrower than the launch
-  // may leave some of them without a tile)
+  // this CTA's output tiles (a member narrower than the launch may leave some CTAs without one)
   const int mts = mtiles >= msplit ? mtiles / msplit : 1, mt0 = msi * mts;
   if (mt0 >= mtiles) return;
   if (j > Mg.nj + 1) return;   // a member with fewer rows than the launch
   const int slot = opm.fop_slot[vgrid * (Mg.nj + 3) + j + 1];
   if (slot < 0) return;
-  if (tid < G) {
-    const int q = q0 + tid;
-    const double *sp = nullptr;
-    double *dp = nullptr;
-    if (q < members) {
-      const DevModel &mq = M.batch ? M.batch[q] : M;
-      if (!mq.ctl->halted) {
-        sp = member_ptr(M, mq, src) + plane_offset(mq, src_sel);
-        dp = member_ptr(M, mq, dst);
-      }
-    }
-    s_src[tid] = sp;
-    s_dst[tid] = dp;
-  }
-  __syncthreads();
-  int live = 0;
-  if (tid < N) {
-    const int g = tid / pc, p = tid - g * pc, plane = chunk * pc + p;
-    int base = -1;
-    if (g < G && plane < nplanes && s_src[g]) base = Mg.at(k0 + plane, j, 0);
-    s_col[tid] = base;
-    s_colg[tid] = (unsigned char)(g < G ? g : 0);
-    s_x1[tid] = shift && base >= 0 ? s_src[g][base + 1] : 0.;
-    live = base >= 0;
-  }
-  if (!__syncthreads_or(live)) return;   // every member of the group halted
+  const int ngroups = (units - u0 + gs - 1) / gs;   // of this CTA, at most FG_GROUPS
 
-  // two operator buffers of A_hi, A_lo (128 x 32 FP32 each), then two plane buffers of B_hi,
+  // FG_BUFS operator buffers of A_hi, A_lo (128 x 32 FP32 each), then FG_BUFS plane buffers of B_hi,
   // B_lo (N x 32 each); the swizzle atoms need a 1024-byte aligned base
   const unsigned b_bytes = (unsigned)N * FG_KC * 4;
   unsigned char *fg_smem = fg_raw + ((1024u - ((unsigned)__cvta_generic_to_shared(fg_raw) & 1023u)) & 1023u);
-  const unsigned smem_s = (unsigned)__cvta_generic_to_shared(fg_smem);
-  const unsigned a_s = smem_s, b_s = smem_s + 4 * FG_A_BYTES;
+  const unsigned a_s = (unsigned)__cvta_generic_to_shared(fg_smem), b_off = FG_BUFS * 2 * FG_A_BYTES;
   const unsigned bars_s = (unsigned)__cvta_generic_to_shared(&bars[0]);
+  const unsigned a_full = bars_s, a_free = bars_s + 8 * FG_BUFS, b_full = a_free + 8 * FG_BUFS, b_free = b_full + 8 * FG_BUFS;
+  const unsigned acc_full = b_free + 8 * FG_BUFS, acc_free = acc_full + 8;
   const uint32_t tcols = (uint32_t)(mts * N) <= 32 ? 32u : 1u << (32 - __clz(mts * N - 1));   // a power of 2 >= 32
-  if (tid == 0) {
+  if (tid == FG_STAGE) {
     fail = 0;
-    for (int b = 0; b < 4; b++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars_s + 8 * b));
+    for (int q = 0; q < FG_BUFS; q++) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(a_full + 8 * q));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(a_free + 8 * q));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(b_full + 8 * q), "r"(FG_STAGE));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b_free + 8 * q));
+    }
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(acc_full));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(acc_free), "r"(FG_STAGE));
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
-  if (warp == 0) {
+  __syncwarp();
+  if (warp == FG_STAGE / 32) {
     const unsigned dst_s = (unsigned)__cvta_generic_to_shared(&tmem_base);
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_s), "r"(tcols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  for (int t = tid; t < ngroups * N; t += FG_THREADS) {
+    const int gi = t / N, n = t - gi * N, u = u0 + gi * gs;
+    const int g = n / pc, plane = (u % nch) * pc + n - g * pc, q = (u / nch) * G + g;
+    const double *sp = nullptr;
+    double *dp = nullptr;
+    if (g < G && q < members && plane < nplanes) {
+      const DevModel &mq = M.batch ? M.batch[q] : M;
+      if (!mq.ctl->halted) {
+        const int row = Mg.at(k0 + plane, j, 0);
+        sp = member_ptr(M, mq, src) + plane_offset(mq, src_sel) + row;
+        dp = member_ptr(M, mq, dst) + row;
+      }
+    }
+    s_src[gi][n] = sp;
+    s_dst[gi][n] = dp;
+    s_x1[gi][n] = shift && sp ? sp[1] : 0.;
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t dtmem = tmem_base;
-  const uint32_t idesc = idesc_tf32(N);
 
-  // B[n][e] = x_n(kc + e + 1) - x1_n, zero in idle columns: N/16 16-byte chunks (4 values each)
-  // per thread and K chunk, loaded into registers two chunks ahead (two register sets, the chunks
-  // taken in pairs), so that a chunk's loads have two chunks' products to arrive in
-  constexpr int BQMAX = FG_NMAX * FG_KC / 4 / FG_THREADS;   // 4
-  const int nq = N * (FG_KC / 4) / FG_THREADS;
-  double breg0[BQMAX][4], breg1[BQMAX][4];
-  auto load_b = [&](int kc, double (&bn)[BQMAX][4]) {
-#pragma unroll
-    for (int u = 0; u < BQMAX; u++) {
-      if (u >= nq) break;
-      const int q = tid + u * FG_THREADS, n = q / (FG_KC / 4), e0 = 4 * (q % (FG_KC / 4));
-      const int base = s_col[n];
-      if (base >= 0) {
-        const double *row = s_src[s_colg[n]] + base + kc + e0 + 1;
-        const double c = s_x1[n];
-#pragma unroll
-        for (int v = 0; v < 4; v++) bn[u][v] = row[v] - c;
-      } else {
-#pragma unroll
-        for (int v = 0; v < 4; v++) bn[u][v] = 0.;
-      }
-    }
-  };
-  load_b(0, breg0);
-  if (nchunks > 1) load_b(FG_KC, breg1);
-  int last_tma = -1, last_commit = -1;
-  // step t = (K chunk c, output tile mt); false once the CTA must stop
-  auto step = [&](int c, int mt, double (&bn)[BQMAX][4]) -> bool {
-    const int t = c * mts + (mt - mt0), kc = c * FG_KC, abuf = t & 1, bbuf = c & 1;
-    // both buffers were last read by the products of step t-2 or earlier
-    if (t >= 2 && !mbar_wait(bars_s + 8 * abuf, (unsigned)(((t - 2) >> 1) & 1))) atomicExch(&fail, 1);
-    __syncthreads();
-    if (fail) return false;
-    const unsigned a_hi_s = a_s + abuf * 2 * FG_A_BYTES, a_lo_s = a_hi_s + FG_A_BYTES;
-    const unsigned b_hi_s = b_s + bbuf * 2 * b_bytes, b_lo_s = b_hi_s + b_bytes;
-    if (tid == 0) {
-      // the operator tile for offset (128 mt - kc) mod ni, hi then lo
-      const int tt = ((mt * FG_M - kc) & (ni - 1)) / FG_KC;
-      const int y = ((slot * ntiles + tt) * 2) * FG_M;
-      const unsigned tb = bars_s + 8 * (2 + abuf);
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tb), "r"(2 * FG_A_BYTES) : "memory");
-      tma_tile(a_hi_s, opm.fop_map, y, tb);
-      tma_tile(a_lo_s, opm.fop_map, y + FG_M, tb);
-      last_tma = t;
-    }
-    if (mt == mt0) {   // the planes' tile of this K chunk, then the loads of chunk c+2 into its registers
-      unsigned char *bh = fg_smem + (b_hi_s - smem_s), *bl = bh + b_bytes;
-#pragma unroll
-      for (int u = 0; u < BQMAX; u++) {
-        if (u >= nq) break;
-        const int q = tid + u * FG_THREADS, n = q / (FG_KC / 4), e0 = 4 * (q % (FG_KC / 4));
-        const float b0 = d2f(bn[u][0]), b1 = d2f(bn[u][1]), b2 = d2f(bn[u][2]), b3 = d2f(bn[u][3]);
-        const float4 hv = make_float4(tf32_hi(b0), tf32_hi(b1), tf32_hi(b2), tf32_hi(b3));
-        const float4 lv = make_float4(b0 - hv.x, b1 - hv.y, b2 - hv.z, b3 - hv.w);
-        const unsigned off = sw128(n, e0);
-        *reinterpret_cast<float4 *>(bh + off) = hv;
-        *reinterpret_cast<float4 *>(bl + off) = lv;
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      if (c + 2 < nchunks) load_b(kc + 2 * FG_KC, bn);
-    }
-    __syncthreads();
-    if (tid == 0) {
-      if (!mbar_wait(bars_s + 8 * (2 + abuf), (unsigned)((t >> 1) & 1))) {
-        fail = 1;
-      } else {
-        last_tma = -1;
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t d_mt = dtmem + (uint32_t)((mt - mt0) * N);
-        for (int ks = 0; ks < FG_KC / 8; ks++) {   // K = 8 TF32 (32 bytes) per instruction
-          const unsigned koff = (unsigned)ks * 32;
-          const uint32_t acc = (kc > 0 || ks > 0) ? 1u : 0u;
-          mma_tf32(d_mt, smem_desc(a_hi_s + koff), smem_desc(b_hi_s + koff), idesc, acc);
-          mma_tf32(d_mt, smem_desc(a_hi_s + koff), smem_desc(b_lo_s + koff), idesc, 1u);
-          mma_tf32(d_mt, smem_desc(a_lo_s + koff), smem_desc(b_hi_s + koff), idesc, 1u);
+  if (warp == FG_STAGE / 32) {
+    if (lane == 0) {
+      const uint32_t idesc = idesc_tf32(N);
+      const int steps = ngroups * nchunks * mts, loads = resident ? nchunks : steps;
+      auto load_a = [&](int t) {   // step t's operator tiles, for offset (128 mt - kc) mod ni, hi then lo
+        const int c = (t / mts) % nchunks, mt = mt0 + t % mts, buf = t % FG_BUFS;
+        const int tt = ((mt * FG_M - c * FG_KC) & (ni - 1)) / FG_KC, y = ((slot * ntiles + tt) * 2) * FG_M;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a_full + 8 * buf), "r"(2 * FG_A_BYTES) : "memory");
+        tma_tile(a_s + buf * 2 * FG_A_BYTES, opm.fop_map, y, a_full + 8 * buf);
+        tma_tile(a_s + buf * 2 * FG_A_BYTES + FG_A_BYTES, opm.fop_map, y + FG_M, a_full + 8 * buf);
+      };
+      int issued = 0;
+      for (; issued < loads && issued < FG_BUFS; issued++) load_a(issued);
+      bool ok = true;
+      int t = 0;
+      for (int n = 0; n < ngroups * nchunks && ok; n++) {   // chunks in order
+        const int gi = n / nchunks, c = n - gi * nchunks, bb = n % FG_BUFS;
+        if (c == 0 && gi > 0) {   // the accumulator read out
+          ok = mbar_wait(acc_free, (unsigned)((gi - 1) & 1), &fail);
+          asm volatile("tcgen05.fence::after_thread_sync;");
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bars_s + 8 * abuf) : "memory");
-        last_commit = t;
-      }
-    }
-    return true;
-  };
-  bool going = true;
-  for (int c = 0; c < nchunks && going; c += 2) {   // nchunks = ni/32 is even
-    for (int mt = mt0; mt < mt0 + mts && going; mt++) going = step(c, mt, breg0);
-    for (int mt = mt0; mt < mt0 + mts && going; mt++) going = step(c + 1, mt, breg1);
-  }
-  // drain: the last commit covers every earlier one; an operator copy whose wait gave up is
-  // waited for again (both bounded), so that nothing writes this CTA's shared or tensor memory
-  // after it is released
-  __shared__ int s_last_commit;
-  if (tid == 0) {
-    s_last_commit = last_commit;
-    if (last_tma >= 0 && !mbar_wait(bars_s + 8 * (2 + (last_tma & 1)), (unsigned)((last_tma >> 1) & 1))) fail = 1;
-  }
-  __syncthreads();
-  const int lc = s_last_commit;
-  if (lc >= 0 && !mbar_wait(bars_s + 8 * (lc & 1), (unsigned)((lc >> 1) & 1))) atomicExch(&fail, 1);
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;");
-  if (!fail) {
-    const int lane = tid & 31;
-    for (int mt = mt0; mt < mt0 + mts; mt++)
-      for (int cg = 0; cg < N; cg += 32) {
-        // warp w reads tensor-memory lanes 32w..32w+31: output point 128 mt + 32w + lane, columns cg..cg+31
-        uint32_t r[32];
-        const uint32_t taddr = dtmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((mt - mt0) * N + cg);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-            "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-              "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-              "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-              "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-            : "r"(taddr));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        const int i = mt * FG_M + warp * 32 + lane + 1;
-#pragma unroll
-        for (int n = 0; n < 32; n++) {
-          const int col = cg + n, base = s_col[col];
-          if (base >= 0) {
-            const double y = f2d(__uint_as_float(r[n]));
-            write_with_pads(s_dst[s_colg[col]], Mg, base, i, shift ? y + s_x1[col] : y);
+        ok = ok && mbar_wait(b_full + 8 * bb, (unsigned)((n / FG_BUFS) & 1), &fail);
+        for (int mt = 0; mt < mts && ok; mt++, t++) {
+          const int ab = t % FG_BUFS;
+          ok = mbar_wait(a_full + 8 * ab, resident ? 0u : (unsigned)((t / FG_BUFS) & 1), &fail);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;");
+          const unsigned a_hi = a_s + ab * 2 * FG_A_BYTES, a_lo = a_hi + FG_A_BYTES;
+          const unsigned b_hi = a_s + b_off + bb * 2 * b_bytes, b_lo = b_hi + b_bytes;
+          const uint32_t d_mt = dtmem + (uint32_t)(mt * N);
+          for (int ks = 0; ks < FG_KC / 8; ks++) {   // K = 8 TF32 (32 bytes) per instruction
+            const unsigned koff = (unsigned)ks * 32;
+            mma_tf32(d_mt, smem_desc(a_hi + koff), smem_desc(b_hi + koff), idesc, (c > 0 || ks > 0) ? 1u : 0u);
+            mma_tf32(d_mt, smem_desc(a_hi + koff), smem_desc(b_lo + koff), idesc, 1u);
+            mma_tf32(d_mt, smem_desc(a_lo + koff), smem_desc(b_hi + koff), idesc, 1u);
+          }
+          // commits complete in issue order: the accumulator's is the last of a group
+          if (!resident) mma_commit(a_free + 8 * ab);
+          if (mt == mts - 1) {
+            mma_commit(b_free + 8 * bb);
+            if (c == nchunks - 1) mma_commit(acc_full);
+          }
+          if (!resident && t >= 1 && issued < loads) {   // step t-1's buffer, its products done while step t's run
+            const int pb = (t - 1) % FG_BUFS;
+            ok = mbar_wait(a_free + 8 * pb, (unsigned)(((t - 1) / FG_BUFS) & 1), &fail);
+            if (ok) load_a(issued++);
           }
         }
       }
-  } else if (tid == 0) {
-    flag_error(Mg.ctl, ERR_TIMEOUT, k0 + chunk * pc, j, 0, 0.);
+      // an operator copy whose step was never reached is waited for (bounded by the limit), so that
+      // nothing writes this CTA's shared memory after it is released
+      if (!ok)
+        for (int q = 0; q < issued; q++)
+          if (q + FG_BUFS >= issued) {
+            int none = 0;
+            mbar_wait(a_full + 8 * (q % FG_BUFS), (unsigned)((q / FG_BUFS) & 1), &none);
+          }
+    }
+    __syncwarp();
+    if (msplit > 1)
+      for (int gi = 0; gi < ngroups; gi++) {   // the staging threads' cluster barriers
+        asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+      }
+  } else {
+    // B[n][e] = x_n(kc + e + 1) - x1_n, zero in idle columns: thread tid converts 4 neighbouring values of
+    // column tid/8 and, for N = 64, of column 32 + tid/8, in every chunk
+    constexpr int BQ = FG_NMAX * FG_KC / 4 / FG_STAGE;   // 2
+    const int nq = N * (FG_KC / 4) / FG_STAGE, e0 = 4 * (tid % (FG_KC / 4));
+    const int total = ngroups * nchunks;
+    double breg[FG_BUFS][BQ][4];
+    auto load_b = [&](int n, double (&bn)[BQ][4]) {
+      const int gi = n / nchunks, kc = (n - gi * nchunks) * FG_KC;
+#pragma unroll
+      for (int u = 0; u < BQ; u++) {
+        if (u >= nq) break;
+        const int col = tid / (FG_KC / 4) + u * (FG_STAGE / (FG_KC / 4));
+        const double *row = s_src[gi][col];
+#pragma unroll
+        for (int v = 0; v < 4; v++) bn[u][v] = row ? row[kc + e0 + 1 + v] : 0.;
+      }
+    };
+#pragma unroll
+    for (int q = 0; q < FG_BUFS; q++)
+      if (q < total) load_b(q, breg[q]);
+    auto epilogue = [&](int gi) {
+      __syncwarp();
+      if (msplit > 1) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");   // this CTA has read its row
+      const bool done = mbar_wait(acc_full, (unsigned)(gi & 1), &fail);
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      __syncwarp();
+      if (msplit > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+      if (__all_sync(0xffffffffu, done)) {
+        for (int mt = 0; mt < mts; mt++)
+          for (int cg = (warp >> 2) * 16; cg < N; cg += 32) {
+            __syncwarp();
+            // warp w reads tensor-memory lanes 32 (w % 4)..+31: output point 128 mt + 32 (w % 4) + lane, columns cg..cg+15
+            uint32_t r[16];
+            const uint32_t taddr = dtmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(mt * N + cg);
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                  "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                : "r"(taddr));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            const int i = (mt0 + mt) * FG_M + (warp & 3) * 32 + lane + 1;
+#pragma unroll
+            for (int n = 0; n < 16; n++) {
+              double *row = s_dst[gi][cg + n];
+              if (row) {
+                const double y = f2d(__uint_as_float(r[n]));
+                write_with_pads(row, Mg, 0, i, shift ? y + s_x1[gi][cg + n] : y);
+              }
+            }
+          }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;");
+      mbar_arrive(acc_free);
+    };
+    for (int n0 = 0; n0 < total; n0 += FG_BUFS) {
+#pragma unroll
+      for (int q = 0; q < FG_BUFS; q++) {   // chunk n in buffer q
+        const int n = n0 + q;
+        if (n >= total) break;
+        if (n >= FG_BUFS) mbar_wait(b_free + 8 * q, (unsigned)((n / FG_BUFS - 1) & 1), &fail);
+        unsigned char *bh = fg_smem + b_off + q * 2 * b_bytes, *bl = bh + b_bytes;
+        const int gi = n / nchunks;
+#pragma unroll
+        for (int u = 0; u < BQ; u++) {
+          if (u >= nq) break;
+          const int col = tid / (FG_KC / 4) + u * (FG_STAGE / (FG_KC / 4));
+          const double x1 = s_x1[gi][col];
+          float4 b4;
+          if (shift)
+            b4 = make_float4(d2f(breg[q][u][0] - x1), d2f(breg[q][u][1] - x1), d2f(breg[q][u][2] - x1), d2f(breg[q][u][3] - x1));
+          else b4 = make_float4(d2f(breg[q][u][0]), d2f(breg[q][u][1]), d2f(breg[q][u][2]), d2f(breg[q][u][3]));
+          const float4 hv = make_float4(tf32_hi(b4.x), tf32_hi(b4.y), tf32_hi(b4.z), tf32_hi(b4.w));
+          const unsigned off = sw128(col, e0);
+          *reinterpret_cast<float4 *>(bh + off) = hv;
+          *reinterpret_cast<float4 *>(bl + off) = make_float4(b4.x - hv.x, b4.y - hv.y, b4.z - hv.z, b4.w - hv.w);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_arrive(b_full + 8 * q);
+        if (n + FG_BUFS < total) load_b(n + FG_BUFS, breg[q]);
+        if (n + 1 == (gi + 1) * nchunks) epilogue(gi);
+      }
+    }
   }
+  // every wait of the other threads is over; the last group's products were waited for in its epilogue,
+  // unless a wait gave up: then the commits in flight are given their time (bounded)
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(dtmem), "r"(tcols));
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  if (fail) {
+    if (tid == 0) {
+      int none = 0;
+      mbar_wait(acc_full, (unsigned)((ngroups - 1) & 1), &none);
+      flag_error(Mg.ctl, ERR_TIMEOUT, k0, j, 0, 0.);
+    }
+    __syncthreads();
+  }
+  if (warp == FG_STAGE / 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(dtmem), "r"(tcols));
 }
 
-// dynamic shared memory of a CTA with N columns: two operator buffers, two plane buffers, the
-// alignment slack of the swizzle atoms
-size_t filter_gemm_smem_bytes(int n) { return 1024 + 4 * (size_t)FG_A_BYTES + 4 * (size_t)n * FG_KC * 4; }
+// dynamic shared memory of a CTA with N columns: operator buffers, plane buffers, the alignment slack of
+// the swizzle atoms
+size_t filter_gemm_smem_bytes(int n) { return 1024 + (size_t)FG_BUFS * 2 * (FG_A_BYTES + (size_t)n * FG_KC * 4); }
 
 static int g_sms = 0;   // SMs of the device (filter_gemm_init, at model creation: not during a graph capture)
 
 bool filter_gemm_usable(const DevModel &M) { return M.fop_map && M.ni % FG_M == 0 && M.ni <= 8 * FG_M; }
 
-// Columns per CTA: up to 64 (32 at ni = 1024), so that two CTAs fit an SM in shared memory
-// (~98 KB each) and in tensor memory (mtiles x N <= 256 columns each).  Planes beyond that split
-// into chunks; members of one operator fill the rest of the columns.
+// Columns per CTA: up to 64.  Planes beyond that split into chunks; members of one operator fill the
+// rest of the columns.  The accumulators of a CTA's output tiles take mts x N <= 512 tensor-memory columns.
 int launch_filter_planes_gemm(const DevModel &M, const double *src, int src_sel, double *dst, int k0, int nplanes, int vgrid, cudaStream_t s,
                               int shift) {
   const int members = M.batch ? M.nbatch : 1;
-  const int nmax = M.ni / FG_M <= 4 ? FG_NMAX : 32;
-  const int pc = nplanes < nmax ? nplanes : nmax;
+  const int pc = nplanes < FG_NMAX ? nplanes : FG_NMAX;
   const int nch = (nplanes + pc - 1) / pc;
-  int G = M.fop_shared ? nmax / pc : 1;
+  int G = M.fop_shared ? FG_NMAX / pc : 1;
   if (G > members) G = members;
   const int N = ((G * pc + 31) / 32) * 32;
-  const int groups = (members + G - 1) / G;
-  // Few members (a single model): about half of the nj+3 rows are filtered, and one CTA per
-  // (row, group, plane chunk) leaves SMs idle while each CTA walks all its output tiles; split a
-  // row's 128-point output tiles over up to mtiles CTAs (each tile's sums are unchanged) until
-  // there are two CTAs with work per SM.  Not in place: a CTA writes its tiles while the others
-  // of its row still read the whole row.
-  const int sms = g_sms > 0 ? g_sms : 152;
-  const int mtiles = M.ni / FG_M;
-  const long long working = (long long)(M.nj + 3) / 2 * nch * groups;
+  const int units = nch * ((members + G - 1) / G);
+  const int sms = g_sms > 0 ? g_sms : 152, mtiles = M.ni / FG_M, rows = (M.nj + 3) / 2;   // about half the rows are filtered
+  // one CTA per SM (its buffers fill the shared memory).  Few units: a cluster of CTAs shares a row's
+  // output tiles (each tile's sums are unchanged) until every SM has one.
   int msplit = 1;
-  if (src != dst)
-    while (2 * msplit <= mtiles && working * msplit < 2LL * sms) msplit *= 2;
-  dim3 grid((unsigned)(M.nj + 3), (unsigned)(nch * groups * msplit), 1u);
-  k_filter_planes_gemm<<<grid, FG_THREADS, filter_gemm_smem_bytes(N), s>>>(M, src, src_sel, dst, k0, nplanes, vgrid, shift, pc, G, N,
-                                                                          msplit);
-  return 0;
+  while (2 * msplit <= mtiles && (long long)rows * units * msplit < sms) msplit *= 2;
+  // many units, and the row's operator in the four buffers: a CTA takes several groups
+  const int resident = M.ni == FG_KC * FG_BUFS && (M.fop_shared || !M.batch);
+  int gs = units;
+  if (resident) {
+    gs = sms / rows > 1 ? sms / rows : 1;
+    if (gs > units) gs = units;
+    if ((units + gs - 1) / gs > FG_GROUPS) gs = (units + FG_GROUPS - 1) / FG_GROUPS;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(M.nj + 3), (unsigned)(gs * msplit), 1u);
+  cfg.blockDim = dim3(FG_THREADS);
+  cfg.dynamicSmemBytes = filter_gemm_smem_bytes(N);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1;
+  at[0].val.clusterDim.y = (unsigned)msplit;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_filter_planes_gemm, M, src, src_sel, dst, k0, nplanes, vgrid, shift, pc, G, N, msplit, units, gs, resident) ==
+                 cudaSuccess
+             ? 0
+             : -1;
 }
 
 int filter_gemm_init(int) {
