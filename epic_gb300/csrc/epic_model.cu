@@ -258,7 +258,12 @@ int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
     // the turbulence closure (epic_subgrid.c)
     case 21: if (M.turb) launch_source_sink_turb(M, s); break;
     case 22: if (M.turb) launch_scalar_hdiff(M, s); break;
-    case 23: if (M.turb) launch_scalar_vdiff(M, s); break;
+    case 23:
+      if (M.turb) {
+        launch_tau_wall_h(M, M.work0, s);
+        launch_scalar_vdiff(M, M.work0, s);
+      }
+      break;
     case 24: if (M.turb) launch_uv_hdiff(M, s); break;
     case 25: if (M.turb) launch_uv_vdiff(M, s); break;
     default: return set_error(EPIC_ERR_ARG, "unknown stage %d", stage);
@@ -350,6 +355,7 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
   meridional(M2, M.unity, 0, L[2]);
   zonal(M2, M.unity, 0, 1, L[2]);
   if (M.turb) {
+    if (M.turb_v) launch_tau_wall_h(M, M2.work0, L[2]);
     launch_source_sink_turb(M, L[0]);
     L.after(0, 1);   // the subgrid diffusion's set_p2etc rewrites P3 and H3, which lane 1 reads
     if (M.turb_h) launch_scalar_hdiff(M, L[0]);
@@ -366,7 +372,8 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
     launch_restore_nu(M, L[3]);
     if (M.turb_v) {
       L.after(0, 3);
-      launch_scalar_vdiff(M, L[0]);
+      L.after(0, 2);
+      launch_scalar_vdiff(M, M2.work0, L[0]);
       L.after(3, 0);
     }
   }
@@ -441,10 +448,14 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
   launch_diag_div(M, L[0]);
   L.after(1, u_done);
   launch_diag_pv(M1, L[1]);
+  if (M.turb) {   // of the winds and NU_TURB
+    L.after(3, u_done);
+    L.after(3, v_done);
+    launch_set_diffusion_coef(M, L[3]);
+  }
   L.after(0, 1);
   L.after(0, 2);
   L.after(0, 3);
-  if (M.turb) launch_set_diffusion_coef(M, L[0]);
   return L.rc ? L.rc : check_launch("step launch");
 }
 
@@ -847,6 +858,7 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
   epic::column_kernels_init(g->nk);
   epic::column_acc_kernels_init();
   epic::stencil_kernels_init();
+  epic::turb_kernels_init();
   epic::filter_gemm_init(g->ni);
   e = cudaStreamSynchronize(m->stream);
   if (e != cudaSuccess) {

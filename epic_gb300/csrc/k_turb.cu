@@ -10,8 +10,8 @@
 //     wavefronts K + J + I = d, one launch each, every point of a front independent of the others;
 //   - the Laplacians of laplacian_h are three pointwise passes around the row filter, all layers
 //     at once (each layer's Laplacian reads only its own plane);
-//   - the implicit vertical diffusions are one thread per column (crank_nicolson and the band
-//     solver with partial pivoting in registers and local memory);
+//   - the implicit vertical diffusions take a tile of 32 columns per block: the set-up of the bands and
+//     the residual are pointwise in the levels, the band solver's recurrences one warp's;
 //   - uv_horizontal_diffusion's stresses are recomputed where the wind updates read them.
 #include "device_common.cuh"
 #include "kernels.h"
@@ -23,7 +23,6 @@ namespace epic {
 namespace {
 
 constexpr double SA_CV1_3 = 7.1 * 7.1 * 7.1;   // cv1^3, epic_subgrid.c:2186-2187
-constexpr int TN = EPIC_TURB_MAX_NK + 4;        // crank_nicolson's column arrays (n + 2 <= nk + 3)
 enum { WALL_U, WALL_V, WALL_H };               // law_of_the_wall's grids: U_INDEX, V_INDEX, the h-grid
 
 __device__ __forceinline__ double nu_floor(const DevModel &M) { return 1.e-4 * M.kinvisc; }
@@ -32,7 +31,7 @@ __device__ __forceinline__ double nu_floor(const DevModel &M) { return 1.e-4 * M
 // FLOAT_MAX on a gas giant
 __device__ __forceinline__ double d_wall(const DevModel &M, int k, int j, int i) {
   if (M.gas_giant) return DBL_MAX;
-  return (M.gz3[M.at(k, j, i)] - M.topo_scale * M.gz_surface[M.at2(j, i)]) / M.grav[2 * j + 1];
+  return div_rn(M.gz3[M.at(k, j, i)] - M.topo_scale * M.gz_surface[M.at2(j, i)], M.grav[2 * j + 1]);
 }
 
 __device__ __forceinline__ double limit_range(double lo, double x, double hi) { return x < lo ? lo : (x > hi ? hi : x); }
@@ -43,15 +42,15 @@ __device__ double func_utau(const DevModel &M, double u_tau, double u_tan, doubl
   const double sqrt_one_third = sqrt(1. / 3.);
   const MathTable &T = *M.lt;
   double u_plus = 0.;
-  if (u_tau != 0.) u_plus = u_tan / u_tau;
+  if (u_tau != 0.) u_plus = div_rn(u_tan, u_tau);
   else flag_error(M.ctl, ERR_TURB, -1, j, i, u_tau);
-  const double y_plus = fabs(u_tau * dwall / M.kinvisc);
+  const double y_plus = fabs(div_rn(u_tau * dwall, M.kinvisc));
   if (u_plus < 0.1) return 1.e+20;
   if (y_plus < 5.) return y_plus - u_plus;
   if (y_plus < 70.) {
     const double yy = const1 * y_plus;
-    return (one_third * cr_log((1. + yy) / (sqrt(yy * (yy - 1.) + 1.)), T) +
-            sqrt_one_third * (cr_atan(sqrt_one_third * (2. * yy - 1.), T) + pi_six)) / const1 +
+    return div_rn(one_third * cr_log(div_rn(1. + yy, sqrt_rn(yy * (yy - 1.) + 1.)), T) +
+                      sqrt_one_third * (cr_atan(sqrt_one_third * (2. * yy - 1.), T) + pi_six), const1) +
            .25 * const2 * cr_log(1. + const3 * cr_pow(y_plus, 4., T), T) - u_plus;
   }
   return const2 * cr_log(y_plus, T) + C - u_plus;
@@ -64,14 +63,14 @@ __device__ double law_of_the_wall(const DevModel &M, int k, int j, int i, int in
   if (M.gas_giant) return 1.0e-4 * kinvisc;
   double dwall;
   if (index == WALL_U) dwall = 0.5 * (d_wall(M, k, j, i) + d_wall(M, k, j, i - 1));
-  else if (index == WALL_V) dwall = 0.5 * M.m[2 * j] * (d_wall(M, k, j, i) / M.m[2 * j + 1] + d_wall(M, k, j - 1, i) / M.m[2 * j - 1]);
+  else if (index == WALL_V) dwall = 0.5 * M.m[2 * j] * (div_rn(d_wall(M, k, j, i), M.m[2 * j + 1]) + div_rn(d_wall(M, k, j - 1, i), M.m[2 * j - 1]));
   else dwall = d_wall(M, k, j, i);
   if (dwall * u_tan < 0.00023) return 0.01 * kinvisc;
   double dwall_inv = 0.;
-  if (dwall > 0.) dwall_inv = 1. / dwall;
+  if (dwall > 0.) dwall_inv = div_rn(1., dwall);
   else flag_error(M.ctl, ERR_TURB, k, j, i, dwall);
-  const double x1 = sqrt(kinvisc * (1. + 0.01) * u_tan * dwall_inv);
-  const double x2 = sqrt(kinvisc * (1. + 20.) * u_tan * dwall_inv);
+  const double x1 = sqrt_rn(kinvisc * (1. + 0.01) * u_tan * dwall_inv);
+  const double x2 = sqrt_rn(kinvisc * (1. + 20.) * u_tan * dwall_inv);
   double fl = func_utau(M, x1, u_tan, dwall, j, i), f = func_utau(M, x2, u_tan, dwall, j, i), rts, xl;
   if (fabs(fl) < fabs(f)) {
     rts = x1; xl = x2;
@@ -82,7 +81,7 @@ __device__ double law_of_the_wall(const DevModel &M, int k, int j, int i, int in
   double u_tau = 0.;
   int iter;
   for (iter = 0; iter < 30; iter++) {
-    const double dx = (xl - rts) * f / (f - fl);
+    const double dx = div_rn((xl - rts) * f, f - fl);
     xl = rts;
     fl = f;
     rts += dx;
@@ -93,7 +92,7 @@ __device__ double law_of_the_wall(const DevModel &M, int k, int j, int i, int in
       break;
     }
   }
-  if (iter < 30) return dmaxr((u_tau * u_tau * dwall / u_tan) - kinvisc, 0.01 * kinvisc);
+  if (iter < 30) return dmaxr(div_rn(u_tau * u_tau * dwall, u_tan) - kinvisc, 0.01 * kinvisc);
   return 20. * kinvisc;
 }
 
@@ -101,12 +100,12 @@ __device__ double law_of_the_wall(const DevModel &M, int k, int j, int i, int in
 __device__ double invert_fv1(const DevModel &M, double t_vis, int j, int i) {
   const double pi_factor = M_PI * 0.5 / 30.0;
   if (t_vis < 0.) flag_error(M.ctl, ERR_TURB, -1, j, i, t_vis);
-  const double chi = t_vis / M.kinvisc;
+  const double chi = div_rn(t_vis, M.kinvisc);
   if (chi > 30) return t_vis;
   if (chi < 0.4) return M.kinvisc * cr_pow(chi * SA_CV1_3, .25, *M.lt);
   double fv1 = cr_cos(pi_factor * cr_pow(chi, 0.35, *M.lt), *M.lt);
   fv1 = 1.0 - fv1 * fv1;
-  return M.kinvisc * chi / fv1;
+  return div_rn(M.kinvisc * chi, fv1);
 }
 
 // get_kin at h-point (j, i) of layer k of the wind time plane `sel`; i = 0 is the pad (bc_lateral)
@@ -126,157 +125,27 @@ __device__ double tau_wall(const DevModel &M, int index, int j, int i) {
   auto gz = [&](int kk, int jj, int ii) { return M.gz3[M.at(kk, jj, ii)]; };
   if (index == WALL_U) {
     const double rho = .5 * (rho3(j, i) + rho3(j, i - 1));
-    const double dz = .5 * (gz(k, j, i) + gz(k, j, i - 1) - gz(k + 1, j, i) - gz(k + 1, j, i - 1)) / M.grav[2 * j + 1];
+    const double dz = div_rn(.5 * (gz(k, j, i) + gz(k, j, i - 1) - gz(k + 1, j, i) - gz(k + 1, j, i - 1)), M.grav[2 * j + 1]);
     const double kin = .5 * (kin_plane(M, PL_UV, k, j, i) + kin_plane(M, PL_UV, k, j, i - 1));
-    const double u_tan = sqrt(2. * kin);
+    const double u_tan = sqrt_rn(2. * kin);
     const double dc = law_of_the_wall(M, k, j, i, WALL_U, u_tan);
-    return (M.dynvisc + rho * dc) * (U[M.at(k, j, i)] - 0.) / dz;
+    return div_rn((M.dynvisc + rho * dc) * (U[M.at(k, j, i)] - 0.), dz);
   }
   if (index == WALL_V) {
     const double rho = .5 * (rho3(j, i) + rho3(j - 1, i));
-    const double dz = .5 * (gz(k, j, i) + gz(k, j - 1, i) - gz(k + 1, j, i) - gz(k + 1, j - 1, i)) / M.grav[2 * j];
+    const double dz = div_rn(.5 * (gz(k, j, i) + gz(k, j - 1, i) - gz(k + 1, j, i) - gz(k + 1, j - 1, i)), M.grav[2 * j]);
     const double kin = .5 * (kin_plane(M, PL_UV, k, j, i) + kin_plane(M, PL_UV, k, j - 1, i));
-    const double u_tan = sqrt(2. * kin);
+    const double u_tan = sqrt_rn(2. * kin);
     const double dc = law_of_the_wall(M, k, j, i, WALL_V, u_tan);
-    return (M.dynvisc + rho * dc) * (V[M.at(k, j, i)] - 0.) / dz;
+    return div_rn((M.dynvisc + rho * dc) * (V[M.at(k, j, i)] - 0.), dz);
   }
   const double rho = rho3(j, i);
-  const double dz = (gz(k, j, i) - gz(k + 1, j, i)) / M.grav[2 * j + 1];
+  const double dz = div_rn(gz(k, j, i) - gz(k + 1, j, i), M.grav[2 * j + 1]);
   const double kin = kin_plane(M, PL_UV, k, j, i);
-  const double u_tan = sqrt(2. * kin);
+  const double u_tan = sqrt_rn(2. * kin);
   const double dc = law_of_the_wall(M, k, j, i, WALL_H, u_tan);
   const double nu = invert_fv1(M, dc, j, i);
-  return (M.dynvisc + rho * nu) * (u_tan - 0.) / dz;
-}
-
-// stability_factor (:2309-2415) of column (j, i) at the layers, sf[K] = stab_factor[2K], K = 0..nk
-// (the only entries the diffusions read).  The slope limiter runs over kk = 1..2nk in order, each
-// step reading the entry the one before may have zeroed.
-__device__ void stability_layers(const DevModel &M, int j, int i, double *sf) {
-  const int nk = M.nk;
-  if (!M.stab) {
-    for (int k = 0; k <= nk; k++) sf[k] = 1.;
-    return;
-  }
-  const double max_ri = 100.;
-  auto ri2 = [&](int k) { return M.ri2[M.at(k, j, i)]; };
-  auto raw = [&](int kk) -> double {   // Ri[kk] before the limiter
-    if (kk == 1) return limit_range(-max_ri, ri2(1), max_ri);
-    if (kk == 2 * nk + 1) return limit_range(-max_ri, ri2(nk), max_ri);
-    const int k = kk / 2;
-    if ((kk & 1) == 0) return limit_range(-max_ri, ri2(k), max_ri);
-    return limit_range(-max_ri, .5 * (ri2(k) + ri2(k + 1)), max_ri);
-  };
-  auto factor = [&](double r) { return r > 0. ? 1. / (1. + 10. * r * (1. + 8. * r)) : sqrt(1. - 18. * r); };
-  double cur = raw(1);
-  sf[0] = 0.;
-  for (int kk = 1; kk <= 2 * nk; kk++) {
-    double nxt = raw(kk + 1);
-    if (-(nxt - cur) > .9 * max_ri) nxt = 0.;
-    if (((kk + 1) & 1) == 0) sf[(kk + 1) / 2] = factor(nxt);
-    cur = nxt;
-  }
-}
-
-// band_decomp / band_back_sub for m1 = m2 = 1 (Numerical Recipes' bandec/banbks with partial
-// pivoting, zero-based, epic_funcs_util.c:3130-3260): A[i][0..2] holds row i's band
-__device__ void band_decomp3(int n, double (*A)[3], double *al, int *index) {
-  int l = 1;
-  A[0][0] = A[0][1]; A[0][1] = A[0][2]; A[0][2] = 0.;
-  for (int k = 0; k < n; k++) {
-    double tmp = A[k][0];
-    int i = k;
-    if (l < n) l++;
-    for (int j = k + 1; j < l; j++)
-      if (fabs(A[j][0]) > fabs(tmp)) { tmp = A[j][0]; i = j; }
-    index[k] = i;
-    if (tmp == 0.) A[k][0] = 1.e-20;
-    if (i != k)
-      for (int j = 0; j < 3; j++) { const double t = A[k][j]; A[k][j] = A[i][j]; A[i][j] = t; }
-    for (i = k + 1; i < l; i++) {
-      tmp = A[i][0] / A[k][0];
-      al[k] = tmp;
-      for (int j = 1; j < 3; j++) A[i][j - 1] = A[i][j] - tmp * A[k][j];
-      A[i][2] = 0.;
-    }
-  }
-}
-__device__ void band_back_sub3(int n, double (*A)[3], const double *al, const int *index, double *b) {
-  int l = 1;
-  for (int k = 0; k < n; k++) {
-    const int i = index[k];
-    if (i != k) { const double t = b[k]; b[k] = b[i]; b[i] = t; }
-    if (l < n) l++;
-    for (int q = k + 1; q < l; q++) b[q] -= al[k] * b[k];
-  }
-  l = 1;
-  for (int i = n - 1; i >= 0; i--) {
-    double tmp = b[i];
-    for (int k = 1; k < l; k++) tmp -= A[i][k] * b[k + i];
-    b[i] = tmp / A[i][0];
-    if (l < 3) l++;
-  }
-}
-
-// crank_nicolson (epic_funcs_util.c:3643-3787) with tridiag(WITH_PIVOTING): band_decomp,
-// band_back_sub and one band_improve pass (:2994-3120, :3330-3400).  z, A, mu, rho (may be null)
-// and ans are indexed 0..n+1; A[0] or A[n+1] above .99e20 marks a no-flux end.  Returns 0, or the
-// first index j where z does not increase (z[j] <= z[j-1]; the reference exits there).
-// Kept out of line: inlined into the column kernels (nvcc 13.0, sm_103a), the callers' store of
-// the no-flux marker A[0] = 1e20 into their local array was not seen by the solver's read of it
-// (measured: every column then took the flux branch); a call makes the arrays' stores complete.
-__device__ __noinline__ int crank_nicolson(int n, double dt, const double *z, const double *A, const double *mu, const double *rho, double *ans) {
-  double a[TN], b[TN], c[TN], r[TN], Ab[TN][3], al[TN];
-  int idx[TN];
-  const int jstart = A[0] > .99e+20 ? 2 : 1, jend = A[n + 1] > .99e+20 ? n : n + 1;
-  for (int j = jstart; j <= jend; j++)
-    if (z[j] <= z[j - 1]) return j;
-  double coeff3 = (A[0] > .99e+20) ? 0. : mu[0] / (z[1] - z[0]), coeff1, factor;
-  a[0] = 0.;
-  c[n - 1] = 0.;
-  for (int j = 1; j <= n; j++) {
-    coeff1 = coeff3;
-    if (j == 1) {
-      coeff3 = mu[j] / (z[j + 1] - z[j]);
-      factor = rho ? dt / (rho[j] * (z[j + 1] - z[j - 1])) : dt / (z[j + 1] - z[j - 1]);
-      b[j - 1] = 1. + (coeff1 + coeff3) * factor;
-      c[j - 1] = -coeff3 * factor;
-      r[j - 1] = 2. * A[j - 1] * coeff1 * factor + A[j] * (1. - (coeff1 + coeff3) * factor) + A[j + 1] * coeff3 * factor;
-    } else if (j == n) {
-      coeff3 = (A[n + 1] > .99e+20) ? 0. : mu[j] / (z[j + 1] - z[j]);
-      factor = rho ? dt / (rho[j] * (z[j + 1] - z[j - 1])) : dt / (z[j + 1] - z[j - 1]);
-      a[j - 1] = -coeff1 * factor;
-      b[j - 1] = 1. + (coeff1 + coeff3) * factor;
-      r[j - 1] = A[j - 1] * coeff1 * factor + A[j] * (1. - (coeff1 + coeff3) * factor) + 2. * A[j + 1] * coeff3 * factor;
-    } else {
-      coeff3 = mu[j] / (z[j + 1] - z[j]);
-      factor = rho ? dt / (rho[j] * (z[j + 1] - z[j - 1])) : dt / (z[j + 1] - z[j - 1]);
-      a[j - 1] = -coeff1 * factor;
-      b[j - 1] = 1. + (coeff1 + coeff3) * factor;
-      c[j - 1] = -coeff3 * factor;
-      r[j - 1] = A[j - 1] * coeff1 * factor + A[j] * (1. - (coeff1 + coeff3) * factor) + A[j + 1] * coeff3 * factor;
-    }
-  }
-  for (int j = 0; j < n; j++) {
-    Ab[j][0] = a[j];
-    Ab[j][1] = b[j];
-    Ab[j][2] = c[j];
-  }
-  band_decomp3(n, Ab, al, idx);
-  for (int j = 0; j < n; j++) ans[j + 1] = r[j];
-  band_back_sub3(n, Ab, al, idx, ans + 1);
-  // band_improve: the residual of the original band (a, b, c) in binary64, one correction
-  double res[TN];
-  for (int i = 0; i < n; i++) {
-    double sdp = -r[i];
-    if (i > 0) sdp += a[i] * ans[i];
-    sdp += b[i] * ans[i + 1];
-    if (i < n - 1) sdp += c[i] * ans[i + 2];
-    res[i] = sdp;
-  }
-  band_back_sub3(n, Ab, al, idx, res);
-  for (int i = 0; i < n; i++) ans[i + 1] -= res[i];
-  return 0;
+  return div_rn((M.dynvisc + rho * nu) * (u_tan - 0.), dz);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -290,12 +159,12 @@ __device__ double brunt2_iface(const DevModel &M, int k, int j, int i) {
   const double pressure = M.p3[x], temperature = M.t3[x], density = M.rho3[x];
   const double cp = 1004., mu = M.mu_dry;
   const double deltap = 0.001 * pressure, deltaT = 0.001 * temperature;
-  auto dens = [&](double p, double t) { return p * mu / (8.314472e+3 * t); };   // return_density
-  const double drho_dp_T = (dens(pressure + deltap, temperature) - dens(pressure - deltap, temperature)) / (2. * deltap);
-  const double drho_dT_p = (dens(pressure, temperature + deltaT) - dens(pressure, temperature - deltaT)) / (2. * deltaT);
-  const double Drho_Dp = (M.rho2[M.at(k + 1, j, i)] - M.rho2[x]) / (M.p2[M.at(k + 1, j, i)] - M.p2[x]);
+  auto dens = [&](double p, double t) { return div_rn(p * mu, 8.314472e+3 * t); };   // return_density
+  const double drho_dp_T = div_rn(dens(pressure + deltap, temperature) - dens(pressure - deltap, temperature), 2. * deltap);
+  const double drho_dT_p = div_rn(dens(pressure, temperature + deltaT) - dens(pressure, temperature - deltaT), 2. * deltaT);
+  const double Drho_Dp = div_rn(M.rho2[M.at(k + 1, j, i)] - M.rho2[x], M.p2[M.at(k + 1, j, i)] - M.p2[x]);
   const double g = M.grav[2 * j + 1];
-  return g * g * (Drho_Dp - drho_dp_T + temperature / (cp * density * density) * drho_dT_p * drho_dT_p);
+  return g * g * (Drho_Dp - drho_dp_T + div_rn(temperature, cp * density * density) * drho_dT_p * drho_dT_p);
 }
 
 // Everything of a point's update but the three gradient terms, at every point k = 1..nk-1,
@@ -322,65 +191,65 @@ __global__ void k_sa_prep(DevModel M) {
   const int jj = 2 * j, kk = 2 * k + 1;
   const double m_2jp1 = M.m[jj + 1], n_2jp1 = M.n[jj + 1];
   // delta_SA (:2774-2808), for k < nk
-  const double dx = 1. / M.m[jj + 1], dy = 1. / M.n[jj + 1];
-  const double dz = (gz3(k - 1) - gz3(k + 1)) / M.grav[jj + 1];
+  const double dx = div_rn(1., M.m[jj + 1]), dy = div_rn(1., M.n[jj + 1]);
+  const double dz = div_rn(gz3(k - 1) - gz3(k + 1), M.grav[jj + 1]);
   double delta = dminr(dx, dy);
   delta = dminr(delta, dz);
   const double d_tilda = dminr(d_wall(M, k, j, i), 0.65 * delta);
-  const double dz_inv = M.grav[jj + 1] / (gz3(k - 1) - gz3(k + 1));
+  const double dz_inv = div_rn(M.grav[jj + 1], gz3(k - 1) - gz3(k + 1));
   // U on the v-grid (zero on the polar rows) and V on the u-grid, layer k
   auto u2d = [&](int J) -> double {
     if (J == 0 || J == M.nj + 1) return 0.;
     const int JJ = 2 * J;
-    const double mn_v = .5 / (1. / M.mn[JJ - 1] + 1. / M.mn[JJ + 1]);
-    return ((u(k, J, i) + u(k, J, i + 1)) * (1. / M.mn[JJ + 1]) + (u(k, J - 1, i) + u(k, J - 1, i + 1)) * (1. / M.mn[JJ - 1])) * mn_v;
+    const double inv_m = div_rn(1., M.mn[JJ - 1]), inv_p = div_rn(1., M.mn[JJ + 1]), mn_v = div_rn(.5, inv_m + inv_p);
+    return ((u(k, J, i) + u(k, J, i + 1)) * inv_p + (u(k, J - 1, i) + u(k, J - 1, i + 1)) * inv_m) * mn_v;
   };
   auto v2d = [&](int I) -> double {
     if (I == M.ni + 1) I = 1;
-    const double mn_u = .5 / (1. / M.mn[jj] + 1. / M.mn[jj + 2]);
-    return ((v(k, j, I) + v(k, j, I - 1)) * (1. / M.mn[jj]) + (v(k, j + 1, I) + v(k, j + 1, I - 1)) * (1. / M.mn[jj + 2])) * mn_u;
+    const double inv_m = div_rn(1., M.mn[jj]), inv_p = div_rn(1., M.mn[jj + 2]), mn_u = div_rn(.5, inv_m + inv_p);
+    return ((v(k, j, I) + v(k, j, I - 1)) * inv_m + (v(k, j + 1, I) + v(k, j + 1, I - 1)) * inv_p) * mn_u;
   };
   const double s11 = (u(k, j, i + 1) - u(k, j, i)) * m_2jp1;
   const double s22 = (v(k, j + 1, i) - v(k, j, i)) * n_2jp1;
-  const double s33 = (w3(k - 1, j, i) - w3(k + 1, j, i)) / (M.sgth[kk - 2] - M.sgth[kk + 2]);
+  const double s33 = div_rn(w3(k - 1, j, i) - w3(k + 1, j, i), M.sgth[kk - 2] - M.sgth[kk + 2]);
   const double s12 = .5 * ((u2d(j + 1) - u2d(j)) * n_2jp1 + (v2d(i + 1) - v2d(i)) * m_2jp1);
   const double u_var3 = 0.5 * (u(k + 1, j, i) + u(k + 1, j, i + 1));
   const double u_var1 = 0.5 * (u(k - 1, j, i) + u(k - 1, j, i + 1));
   double w_var3 = 0.5 * (w3(k, j, i) + w3(k, j, i + 1));
   double w_var1 = 0.5 * (w3(k, j, i) + w3(k, j, i - 1));
   const long long x = M.at(k, j, i);
-  const double h_rho = M.h3[x] / M.rho3[x];
+  const double h_rho = div_rn(M.h3[x], M.rho3[x]);
   const double s13 = .5 * ((u_var1 - u_var3) * dz_inv + h_rho * (w_var3 - w_var1) * m_2jp1);
   const double v_var3 = 0.5 * (v(k + 1, j, i) + v(k + 1, j + 1, i));
   const double v_var1 = 0.5 * (v(k - 1, j, i) + v(k - 1, j + 1, i));
   w_var3 = 0.5 * (w3(k, j, i) + w3(k, j + 1, i));
   w_var1 = 0.5 * (w3(k, j, i) + w3(k, j - 1, i));
   const double s23 = .5 * ((v_var1 - v_var3) * dz_inv + h_rho * (w_var3 - w_var1) * n_2jp1);
-  const double S = sqrt(2. * (s11 * s11 + s22 * s22 + s33 * s33 + 2. * (s12 * s12 + s13 * s13 + s23 * s23)));
+  const double S = sqrt_rn(2. * (s11 * s11 + s22 * s22 + s33 * s33 + 2. * (s12 * s12 + s13 * s13 + s23 * s23)));
   // the point's own NU_TURB terms
   const double nu = M.nu_turb[x];
-  const double chi = nu / M.kinvisc;
+  const double chi = div_rn(nu, M.kinvisc);
   const double chi3 = cr_pow(chi, 3., T);
-  const double fv1 = chi3 / (chi3 + SA_CV1_3);
-  const double fv2 = 1. - (chi / (1. + chi * fv1));
+  const double fv1 = div_rn(chi3, chi3 + SA_CV1_3);
+  const double fv2 = 1. - div_rn(chi, 1. + chi * fv1);
   const double tmp1 = kappa_2 * d_tilda * d_tilda;
-  const double S_tilda = S + (nu * fv2) / tmp1;
+  const double S_tilda = S + div_rn(nu * fv2, tmp1);
   const double tmp2 = S_tilda * tmp1;
   double fw = 1.;
   if (tmp2 != 0.) {
-    const double r_sa = nu / tmp2;
+    const double r_sa = div_rn(nu, tmp2);
     if (r_sa < 0.) flag_error(M.ctl, ERR_TURB, k, j, i, r_sa);
     else if (r_sa < 10.) {
       const double g_sa = r_sa + cw2 * (cr_pow(r_sa, 6., T) - r_sa);
-      fw = g_sa * cr_pow(((1. + cw3_6) / (cr_pow(g_sa, 6., T) + cw3_6)), (1. / 6.), T);
+      fw = g_sa * cr_pow(div_rn(1. + cw3_6, cr_pow(g_sa, 6., T) + cw3_6), (1. / 6.), T);
     }
   }
   const double brunt2 = brunt2_iface(M, k, j, i);
-  const double brunt = sqrt(fabs(brunt2));
+  const double brunt = sqrt_rn(fabs(brunt2));
   M.work0[x] = cb1 * S_tilda * nu;
-  M.work1[x] = cw1 * fw * cr_pow((nu / d_tilda), 2., T);
+  M.work1[x] = cw1 * fw * cr_pow(div_rn(nu, d_tilda), 2., T);
   M.work2[x] = dz_inv;
-  M.work3[x] = brunt2 < 0. ? nu * cr_exp(-nu / nu_turb_limiter, T) * brunt2 / brunt : 0.;
+  M.work3[x] = brunt2 < 0. ? div_rn(nu * cr_exp(div_rn(-nu, nu_turb_limiter), T) * brunt2, brunt) : 0.;
 }
 
 // One wavefront k + j + i = d of the in-place NU_TURB update: the three gradient terms from the
@@ -486,118 +355,248 @@ __global__ void k_lap_apply(DevModel M, double *var, int k0, const double *gh1, 
   const unsigned r = t / ni, q = r / nr;
   const int i = 1 + (int)(t - r * ni), j = (int)(r - q * nr), k = k0 + (int)q;
   const double m_2jp1 = M.m[2 * j + 1], n_2jp1 = M.n[2 * j + 1];
-  const double m_2j_inv = (j == 0) ? 0. : 1. / M.m[2 * j];
-  const double m_2jp2_inv = (j == M.nj) ? 0. : 1. / M.m[2 * j + 2];
+  const double m_2j_inv = (j == 0) ? 0. : div_rn(1., M.m[2 * j]);
+  const double m_2jp2_inv = (j == M.nj) ? 0. : div_rn(1., M.m[2 * j + 2]);
   const long long x = M.at(k, j, i);
   const double lph = m_2jp1 * ((gh1[x + 1] - gh1[x]) + n_2jp1 * (gh2[M.at(k, j + 1, i)] * m_2jp2_inv - gh2[x] * m_2j_inv));
   write_with_pads(var, M, M.at(k, j, 0), i, var[x] + M.dt * lph);
 }
 
 // ---------------------------------------------------------------------------------------------
-// scalar_vertical_diffusion (:1273-1488), one thread per column j = 0..nj, i = 1..ni
+// The implicit vertical diffusions: scalar_vertical_diffusion (:1273-1488) of THETA and NU_TURB,
+// uv_vertical_diffusion (:1940-2075) of U and V, each through crank_nicolson (epic_funcs_util.c:3643-3787)
+// with tridiag(WITH_PIVOTING): band_decomp and band_back_sub for m1 = m2 = 1 (Numerical Recipes'
+// bandec/banbks, :3130-3260) and one band_improve pass (:2994-3120, :3330-3400).
+//
+// A block takes 32 columns, one per lane, with every array in shared memory as [index][lane].  The
+// heights, diffusivities, bands and the residual are pointwise in the levels, which the warps share;
+// elimination (with row swaps) and back substitution are one warp's, their current rows in registers.
+// One thread per column with its arrays in local memory took 682 us for NU_TURB (with its wall stress)
+// and 176 us for each wind at 128x64x20: a chain of dependent quotients and local-memory round trips
+// with two warps per SM.
+//
+// Arrays of n + 2 values a column (VD_ARRAYS of them): z, A and mu are indexed as crank_nicolson's; once
+// the bands a, b, c, r stand, U0, U1, U2 and al (the decomposition) take the places of z, mu and the
+// two stability arrays, and the answer that of A.
 // ---------------------------------------------------------------------------------------------
 
-__global__ void __launch_bounds__(64) k_theta_vdiff(DevModel M) {
-  if (epic_member(M)) return;
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= (M.nj + 1) * M.ni) return;
-  const int j = t / M.ni, i = 1 + t - j * M.ni;
-  const int nk = M.nk, ks = M.k_sigma;
-  const double gi = M.grav[2 * j + 1];
-  double sf[TN], z[TN], A[TN], dee[TN], ans[TN];
-  stability_layers(M, j, i, sf);
-  A[0] = 1.e+20;
-  z[0] = M.gz3[M.at(nk, j, i)] / gi;
-  for (int k = nk; k >= ks - 2; k--) {
-    const int kay = nk - k + 1;
-    A[kay] = M.theta[M.at(k, j, i)];
-    z[kay] = M.gz3[M.at(k, j, i)] / gi;
+enum { VD_THETA, VD_NU, VD_U, VD_V };
+constexpr int VD_ARRAYS = 10, VD_THREADS = 256;
+
+// stability_factor (:2309-2415) at the layers of column (j, i): s[K] = Ri[2K] as its slope limiter
+// leaves it (K = 1..nk; the only entries the diffusions read).  The limiter runs over kk = 1..2nk in
+// order, each step reading the entry the one before may have zeroed.
+__device__ __forceinline__ void stability_ri(const DevModel &M, int j, int i, int kmin, double *s) {   // s[(K - kmin) * 32], K >= kmin
+  const int nk = M.nk, x = M.at(0, j, i), n2 = (int)M.n2;
+  const double max_ri = 100.;
+  double ri = M.ri2[x + n2], cur = limit_range(-max_ri, ri, max_ri);   // kk = 1
+  for (int k = 1; k <= nk; k++) {
+    double nxt = limit_range(-max_ri, ri, max_ri);   // kk = 2k
+    if (-(nxt - cur) > .9 * max_ri) nxt = 0.;
+    if (k >= kmin) s[(k - kmin) * 32] = nxt;
+    cur = nxt;
+    const double below = M.ri2[x + min(k + 1, nk) * n2];
+    nxt = limit_range(-max_ri, k == nk ? ri : .5 * (ri + below), max_ri);   // kk = 2k+1
+    if (-(nxt - cur) > .9 * max_ri) nxt = 0.;
+    cur = nxt;
+    ri = below;
   }
-  for (int k = nk; k > ks - 2; k--)
-    dee[nk - k + 1] = sf[k] * .5 * (M.dc_theta[M.at(k, j, i)] + M.dc_theta[M.at(k - 1, j, i)]);
-  if (const int bad = crank_nicolson(nk - ks + 2, M.dt, z, A, dee, nullptr, ans)) {   // THETA: z[bad] - z[bad-1] recorded
-    flag_error(M.ctl, ERR_TURB, nk - bad + 1, j, i, z[bad] - z[bad - 1]);
-    return;
-  }
-  for (int k = nk; k >= ks - 1; k--) write_with_pads(M.theta, M, M.at(k, j, 0), i, ans[nk - k + 1]);
+}
+__device__ __forceinline__ double stability_factor(double r) {
+  return r > 0. ? div_rn(1., 1. + 10. * r * (1. + 8. * r)) : sqrt_rn(1. - 18. * r);
 }
 
-__global__ void __launch_bounds__(64) k_nu_vdiff(DevModel M) {
-  if (epic_member(M)) return;
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= (M.nj + 1) * M.ni) return;
-  const int j = t / M.ni, i = 1 + t - j * M.ni;
-  const int nk = M.nk;
-  const double gi = M.grav[2 * j + 1], sigma_inv = 3. / 2.;
-  const double tw = tau_wall(M, WALL_H, j, i);
-  double z[TN], A[TN], dee[TN], ans[TN];
-  auto gz = [&](int k) { return M.gz3[M.at(k, j, i)]; };
-  auto nu = [&](int k) { return M.nu_turb[M.at(k, j, i)]; };
-  A[nk + 2] = 1.e+20;
-  z[nk + 2] = (gz(0) + (gz(0) - gz(1))) / gi;
-  for (int k = nk; k >= 0; k--) {
-    A[nk - k + 1] = nu(k);
-    z[nk - k + 1] = gz(k) / gi;
+// forward elimination's row swaps and multipliers on b[0..n-1], then back substitution, of one column
+__device__ __forceinline__ void vd_solve(int n, const double *U0, const double *U1, const double *U2, const double *al,
+                                         unsigned long long swapped, double *b) {
+  double cur = b[0];
+  for (int k = 0; k < n - 1; k++) {
+    double nxt = b[(k + 1) * 32];
+    if ((swapped >> k) & 1) { const double t = cur; cur = nxt; nxt = t; }
+    nxt -= al[k * 32] * cur;
+    b[k * 32] = cur;
+    cur = nxt;
   }
-  for (int k = nk; k > 0; k--) dee[nk - k + 1] = sigma_inv * (M.kinvisc + .5 * (nu(k) + nu(k - 1)));
-  z[0] = (gz(nk) - (gz(nk - 1) - gz(nk))) / gi;
-  dee[0] = dee[1];
-  A[0] = A[1] - tw * (z[1] - z[0]) / dee[0];
-  if (const int bad = crank_nicolson(nk + 1, M.dt, z, A, dee, nullptr, ans)) {
-    flag_error(M.ctl, ERR_TURB, nk - bad + 1, j, i, z[bad] - z[bad - 1]);
-    return;
+  double x1 = 0., x2 = 0.;
+  for (int i = n - 1; i >= 0; i--) {
+    double t = i == n - 1 ? cur : b[i * 32];
+    if (i < n - 1) t -= U1[i * 32] * x1;
+    if (i < n - 2) t -= U2[i * 32] * x2;
+    t = div_rn(t, U0[i * 32]);
+    b[i * 32] = t;
+    x2 = x1;
+    x1 = t;
   }
-  for (int k = nk; k >= 0; k--) write_with_pads(M.nu_turb, M, M.at(k, j, 0), i, ans[nk - k + 1]);
 }
 
-// ---------------------------------------------------------------------------------------------
-// uv_vertical_diffusion (:1940-2075): the wall stresses of all columns first (tau_surface reads
-// the neighbours' bottom winds, which the columns' solves then change), then one thread per column
-// ---------------------------------------------------------------------------------------------
-
-__global__ void k_tau_wall(DevModel M, int comp, double *tw) {
+// tw: the wall stresses (NU_TURB: WALL_H; U, V: their own)
+__global__ void __launch_bounds__(VD_THREADS) k_vdiff(DevModel M, int what, const double *tw) {
   if (epic_member(M, tw)) return;
-  const int j0 = comp == 0 ? 0 : 1;
+  extern __shared__ double vd[];
+  __shared__ int s_bad[32];
+  __shared__ double s_dz[32];
+  const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5), nw = VD_THREADS / 32;
+  const int j0 = what == VD_V ? 1 : 0, nk = M.nk, ks = M.k_sigma, n2 = (int)M.n2;
+  const int t = (int)blockIdx.x * 32 + lane;
+  const bool live = t < (M.nj + 1 - j0) * M.ni;
+  const int j = j0 + (live ? t / M.ni : 0), i = 1 + (live ? t % M.ni : 0);
+  const int n = what == VD_THETA ? nk - ks + 2 : (what == VD_NU ? nk + 1 : nk - 1), S = 32 * (n + 2);
+  double *z = vd + lane, *A = z + S, *mu = A + S, *a = mu + S, *b = a + S, *c = b + S, *r = c + S, *s0 = r + S, *s1 = s0 + S, *rho = s1 + S;
+  double *U0 = z, *U1 = mu, *U2 = s0, *al = s1, *ans = A, *res = rho;
+  const int col = M.at(0, j, i);
+  const double gi = what == VD_V ? M.grav[2 * j] : M.grav[2 * j + 1];
+  // the neighbouring column of the winds' stencil: (j, i-1) for U, (j-1, i) for V
+  const int jn = what == VD_V ? j - 1 : j, in = what == VD_U ? i - 1 : i, coln = M.at(0, jn, in);
+  const bool wind = what == VD_U || what == VD_V;
+  double *F = what == VD_THETA ? M.theta : (what == VD_NU ? M.nu_turb : (what == VD_U ? M.u : M.v) + plane_offset(M, PL_UV));
+  if (warp == 0) s_bad[lane] = n + 2;
+  // the stability factors' Richardson numbers, from layer kmin on (THETA's diffusion uses ks-1..nk)
+  const int kmin = what == VD_THETA ? ks - 1 : 1;
+  if (live && M.stab && what != VD_NU && warp < (wind ? 2 : 1))
+    stability_ri(M, warp == 0 ? j : jn, warp == 0 ? i : in, kmin, warp == 0 ? s0 : s1);
+  __syncthreads();
+  if (live) {
+    auto gz = [&](int k) { return M.gz3[col + k * n2]; };
+    auto gzm = [&](int k) { return .5 * (M.gz3[col + k * n2] + M.gz3[coln + k * n2]); };
+    auto sf = [&](const double *s, int k) { return M.stab ? stability_factor(s[(k - kmin) * 32]) : 1.; };
+    if (what == VD_THETA) {   // kay = nk - k + 1, k = nk..ks-2
+      for (int kay = warp; kay <= n + 1; kay += nw) {
+        const int k = nk - kay + 1;
+        if (kay == 0) { A[0] = 1.e+20; z[0] = div_rn(gz(nk), gi); continue; }
+        A[kay * 32] = M.theta[col + k * n2];
+        z[kay * 32] = div_rn(gz(k), gi);
+        if (kay <= n) mu[kay * 32] = sf(s0, k) * .5 * (M.dc_theta[col + k * n2] + M.dc_theta[col + (k - 1) * n2]);
+      }
+    } else if (what == VD_NU) {   // kay = nk - k + 1, k = nk..0
+      const double sigma_inv = 3. / 2.;
+      auto nu = [&](int k) { return M.nu_turb[col + k * n2]; };
+      auto dee = [&](int k) { return sigma_inv * (M.kinvisc + .5 * (nu(k) + nu(k - 1))); };
+      for (int kay = warp; kay <= n + 1; kay += nw) {
+        const int k = nk - kay + 1;
+        if (kay == 0) {
+          const double z1 = div_rn(gz(nk), gi), z0 = div_rn(gz(nk) - (gz(nk - 1) - gz(nk)), gi), d = dee(nk);
+          z[0] = z0;
+          mu[0] = d;
+          A[0] = nu(nk) - div_rn(tw[M.at2(j, i)] * (z1 - z0), d);
+        } else if (kay == n + 1) {
+          A[kay * 32] = 1.e+20;
+          z[kay * 32] = div_rn(gz(0) + (gz(0) - gz(1)), gi);
+        } else {
+          A[kay * 32] = nu(k);
+          z[kay * 32] = div_rn(gz(k), gi);
+          if (k > 0) mu[kay * 32] = dee(k);
+        }
+      }
+    } else {   // kay = nk - k, k = nk-1..1
+      auto muk = [&](int k) {
+        return M.dynvisc + .5 * (sf(s0, k) * M.rho2[col + k * n2] * .5 * (M.dc_uv[col + (k - 1) * n2] + M.dc_uv[col + k * n2]) +
+                                 sf(s1, k) * M.rho2[coln + k * n2] * .5 * (M.dc_uv[coln + (k - 1) * n2] + M.dc_uv[coln + k * n2]));
+      };
+      for (int kay = warp; kay <= n + 1; kay += nw) {
+        const int k = nk - kay;
+        if (kay == 0) {
+          const double z1 = div_rn(gzm(nk - 1), gi), z0 = div_rn(gzm(nk), gi), m = muk(nk - 1);
+          z[0] = z0;
+          mu[0] = m;
+          A[0] = F[col + (nk - 1) * n2] - div_rn(tw[M.at2(j, i)] * (z1 - z0), m);
+        } else if (kay == n + 1) {
+          A[kay * 32] = 1.e+20;
+          z[kay * 32] = div_rn(gzm(0), gi);
+        } else {
+          A[kay * 32] = F[col + k * n2];
+          z[kay * 32] = div_rn(gzm(k), gi);
+          rho[kay * 32] = .5 * (M.rho3[col + k * n2] + M.rho3[coln + k * n2]);
+          mu[kay * 32] = muk(k);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // crank_nicolson: A[0] or A[n+1] above .99e20 marks a no-flux end; the first index whose height does
+  // not increase ends the column with an error (the reference exits there)
+  const bool flux0 = !(A[0] > .99e+20), fluxn = !(A[(n + 1) * 32] > .99e+20);
+  const double dt = M.dt;
+  if (live)
+    for (int q = 1 + warp; q <= n + 1; q += nw) {
+      const double dz = z[q * 32] - z[(q - 1) * 32];
+      if (q >= (flux0 ? 1 : 2) && q <= (fluxn ? n + 1 : n) && z[q * 32] <= z[(q - 1) * 32]) atomicMin(&s_bad[lane], q);
+      if (q > n) continue;
+      const double c1 = q == 1 && !flux0 ? 0. : div_rn(mu[(q - 1) * 32], dz);
+      const double c3 = q == n && !fluxn ? 0. : div_rn(mu[q * 32], z[(q + 1) * 32] - z[q * 32]);
+      const double zz = z[(q + 1) * 32] - z[(q - 1) * 32];
+      const double f = div_rn(dt, wind ? rho[q * 32] * zz : zz);
+      a[(q - 1) * 32] = -c1 * f;
+      b[(q - 1) * 32] = 1. + (c1 + c3) * f;
+      c[(q - 1) * 32] = -c3 * f;
+      const double m = A[q * 32] * (1. - (c1 + c3) * f);
+      if (q == 1) r[0] = 2. * A[0] * c1 * f + m + A[64] * c3 * f;
+      else if (q == n) r[(q - 1) * 32] = A[(q - 1) * 32] * c1 * f + m + 2. * A[(q + 1) * 32] * c3 * f;
+      else r[(q - 1) * 32] = A[(q - 1) * 32] * c1 * f + m + A[(q + 1) * 32] * c3 * f;
+    }
+  __syncthreads();
+  const int bad = s_bad[lane];
+  if (warp == 0 && bad <= n + 1) s_dz[lane] = z[bad * 32] - z[(bad - 1) * 32];
+  __syncwarp();
+  unsigned long long swapped = 0;
+  if (warp == 0 && live && bad > n + 1) {
+    double p0 = b[0], p1 = c[0], p2 = 0.;
+    for (int k = 0; k < n; k++) {
+      double q0 = 0., q1 = 0., q2 = 0.;
+      if (k + 1 < n) { q0 = a[(k + 1) * 32]; q1 = b[(k + 1) * 32]; q2 = k + 2 < n ? c[(k + 1) * 32] : 0.; }
+      const bool sw = k + 1 < n && fabs(q0) > fabs(p0);
+      if (sw) {
+        swapped |= 1ull << k;
+        double tt = p0; p0 = q0; q0 = tt;
+        tt = p1; p1 = q1; q1 = tt;
+        tt = p2; p2 = q2; q2 = tt;
+      }
+      if (p0 == 0.) p0 = 1.e-20;
+      U0[k * 32] = p0;
+      U1[k * 32] = p1;
+      U2[k * 32] = p2;
+      ans[(k + 1) * 32] = r[k * 32];
+      if (k + 1 < n) {
+        const double m = div_rn(q0, p0);
+        al[k * 32] = m;
+        p0 = q1 - m * p1;
+        p1 = q2 - m * p2;
+        p2 = 0.;
+      }
+    }
+    vd_solve(n, U0, U1, U2, al, swapped, ans + 32);
+  }
+  __syncthreads();
+  // band_improve: the residual of the original band in binary64, one correction
+  if (live && bad > n + 1)
+    for (int q = warp; q < n; q += nw) {
+      double sdp = -r[q * 32];
+      if (q > 0) sdp += a[q * 32] * ans[q * 32];
+      sdp += b[q * 32] * ans[(q + 1) * 32];
+      if (q < n - 1) sdp += c[q * 32] * ans[(q + 2) * 32];
+      res[q * 32] = sdp;
+    }
+  __syncthreads();
+  if (warp == 0 && live && bad > n + 1) vd_solve(n, U0, U1, U2, al, swapped, res);
+  __syncthreads();
+  if (!live) return;
+  const int top = what == VD_THETA || what == VD_NU ? nk + 1 : nk;   // level = top - kay
+  if (bad <= n + 1) {
+    if (warp == 0) flag_error(M.ctl, ERR_TURB, top - bad, j, i, s_dz[lane]);
+    return;
+  }
+  for (int kay = 1 + warp; kay <= n; kay += nw)
+    write_with_pads(F, M, M.at(top - kay, j, 0), i, ans[kay * 32] - res[(kay - 1) * 32]);
+}
+
+// the wall stresses of all columns: WALL_U, WALL_V (tau_surface reads the neighbours' bottom winds,
+// which the columns' solves then change) or WALL_H
+__global__ void k_tau_wall(DevModel M, int index, double *tw) {
+  if (epic_member(M, tw)) return;
+  const int j0 = index == WALL_V ? 1 : 0;
   const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (t >= (M.nj + 1 - j0) * M.ni) return;
   const int j = j0 + t / M.ni, i = 1 + t - (j - j0) * M.ni;
-  tw[M.at2(j, i)] = tau_wall(M, comp == 0 ? WALL_U : WALL_V, j, i);
-}
-
-__global__ void __launch_bounds__(64) k_wind_vdiff(DevModel M, int comp, const double *tw) {
-  if (epic_member(M, tw)) return;
-  const int j0 = comp == 0 ? 0 : 1;
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= (M.nj + 1 - j0) * M.ni) return;
-  const int j = j0 + t / M.ni, i = 1 + t - (j - j0) * M.ni;
-  const int nk = M.nk;
-  // the neighbouring column of the stencil: (j, i-1) for U, (j-1, i) for V
-  const int jn = comp == 0 ? j : j - 1, in = comp == 0 ? i - 1 : i;
-  const double gi = comp == 0 ? M.grav[2 * j + 1] : M.grav[2 * j];
-  double *W = (comp == 0 ? M.u : M.v) + plane_offset(M, PL_UV);
-  double sf2[TN], sf0[TN], z[TN], A[TN], mu[TN], rho[TN], ans[TN];
-  stability_layers(M, j, i, sf2);
-  stability_layers(M, jn, in, sf0);
-  auto gzm = [&](int k) { return .5 * (M.gz3[M.at(k, j, i)] + M.gz3[M.at(k, jn, in)]); };
-  A[nk] = 1.e+20;
-  z[nk] = gzm(0) / gi;
-  for (int k = nk - 1; k >= 1; k--) {
-    const int kay = nk - k;
-    A[kay] = W[M.at(k, j, i)];
-    z[kay] = gzm(k) / gi;
-    rho[kay] = .5 * (M.rho3[M.at(k, j, i)] + M.rho3[M.at(k, jn, in)]);
-  }
-  for (int k = nk - 1; k >= 1; k--)
-    mu[nk - k] = M.dynvisc + .5 * (sf2[k] * M.rho2[M.at(k, j, i)] * .5 * (M.dc_uv[M.at(k - 1, j, i)] + M.dc_uv[M.at(k, j, i)]) +
-                                   sf0[k] * M.rho2[M.at(k, jn, in)] * .5 * (M.dc_uv[M.at(k - 1, jn, in)] + M.dc_uv[M.at(k, jn, in)]));
-  z[0] = gzm(nk) / gi;
-  mu[0] = mu[1];
-  A[0] = A[1] - tw[M.at2(j, i)] * (z[1] - z[0]) / mu[0];
-  if (const int bad = crank_nicolson(nk - 1, M.dt, z, A, mu, rho, ans)) {
-    flag_error(M.ctl, ERR_TURB, nk - bad, j, i, z[bad] - z[bad - 1]);
-    return;
-  }
-  for (int k = nk - 1; k >= 1; k--) write_with_pads(W, M, M.at(k, j, 0), i, ans[nk - k]);
+  tw[M.at2(j, i)] = tau_wall(M, index, j, i);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -613,7 +612,7 @@ __global__ void k_uvh_coef(DevModel M) {
   const unsigned q = t / w;
   const long long x = M.at(1 + (int)q, 0, 0) + (t - q * w);
   M.work0[x] = M.dynvisc + M.rho3[x] * M.dc_uv[x];
-  M.work1[x] = M.h3[x] / M.rho3[x];
+  M.work1[x] = div_rn(M.h3[x], M.rho3[x]);
 }
 
 // TAU12 on the polar rows, per layer: vorticity(ON_SIGMATHETA, RELATIVE) there (epic_funcs_diag.c:
@@ -646,10 +645,10 @@ __device__ __forceinline__ Stress stress_h(const DevModel &M, int k, int j, int 
   auto Vv = [&](int jj, int ii) { return vv[M.at(k, jj, ii)]; };
   auto H = [&](int jj, int ii) { return hr[M.at(k, jj, ii)]; };
   const int jj = 2 * j;
-  const double rln_inv = 1. / M.rln[jj + 1], m_2jp1 = M.m[jj + 1], n_2jp2 = M.n[jj + 2], n_2jp1 = M.n[jj + 1], n_2j = M.n[jj];
+  const double rln_inv = div_rn(1., M.rln[jj + 1]), m_2jp1 = M.m[jj + 1], n_2jp2 = M.n[jj + 2], n_2jp1 = M.n[jj + 1], n_2j = M.n[jj];
   const double e11 = (U(j, i + 1) - U(j, i)) * m_2jp1 + .5 * (Vv(j, i) + Vv(j + 1, i)) * rln_inv * (M.rln[jj + 2] - M.rln[jj]) * n_2jp1;
   const double e22 = (Vv(j + 1, i) - Vv(j, i)) * n_2jp1;
-  double coeff = .5 / H(j, i);
+  double coeff = div_rn(.5, H(j, i));
   double e33 = coeff * (U(j, i + 1) * (H(j, i + 1) - H(j, i)) * m_2jp1 + U(j, i) * (H(j, i) - H(j, i - 1)) * m_2jp1);
   if (Vv(j + 1, i) != 0.) e33 += coeff * Vv(j + 1, i) * (H(j + 1, i) - H(j, i)) * n_2jp2;
   if (Vv(j, i) != 0.) e33 += coeff * Vv(j, i) * (H(j, i) - H(j - 1, i)) * n_2j;
@@ -657,7 +656,7 @@ __device__ __forceinline__ Stress stress_h(const DevModel &M, int k, int j, int 
   Stress s;
   s.t11 = coeff * (2. * e11 - e22 - e33);
   s.t22 = coeff * (2. * e22 - e11 - e33);
-  s.t33 = (coeff / H(j, i)) * (2. * e33 - e11 - e22);
+  s.t33 = div_rn(coeff, H(j, i)) * (2. * e33 - e11 - e22);
   return s;
 }
 
@@ -669,7 +668,7 @@ __device__ __forceinline__ double stress_12(const DevModel &M, int k, int j, int
   auto c = [&](int jj, int ii) { return cd[M.at(k, jj, ii)] * hr[M.at(k, jj, ii)]; };
   const int jj = 2 * j;
   const double e12 = (vv[M.at(k, j, i)] - vv[M.at(k, j, i - 1)]) * M.m[jj] +
-                     M.rln[jj] * (uu[M.at(k, j, i)] / M.rln[jj + 1] - uu[M.at(k, j - 1, i)] / M.rln[jj - 1]) * M.n[jj];
+                     M.rln[jj] * (div_rn(uu[M.at(k, j, i)], M.rln[jj + 1]) - div_rn(uu[M.at(k, j - 1, i)], M.rln[jj - 1])) * M.n[jj];
   const double coeff = .25 * (c(j, i) + c(j, i - 1) + c(j - 1, i) + c(j - 1, i - 1));
   return coeff * e12;
 }
@@ -687,8 +686,8 @@ __global__ void k_uvh_apply(DevModel M) {
   const Stress s = stress_h(M, k, j, i), sw = stress_h(M, k, j, i - 1);
   {
     const int jj = 2 * j;
-    const double rln_inv = 1. / M.rln[jj + 1], m_2jp1 = M.m[jj + 1], n_2jp1 = M.n[jj + 1];
-    const double h_inv = 2. / (M.hdry[M.at(k, j, i)] + M.hdry[M.at(k, j, i - 1)]);
+    const double rln_inv = div_rn(1., M.rln[jj + 1]), m_2jp1 = M.m[jj + 1], n_2jp1 = M.n[jj + 1];
+    const double h_inv = div_rn(2., M.hdry[M.at(k, j, i)] + M.hdry[M.at(k, j, i - 1)]);
     const double t12n = stress_12(M, k, j + 1, i), t12 = stress_12(M, k, j, i);
     const long long x = tend + M.at(k, j, i);
     M.dudt[x] += h_inv * (m_2jp1 * (s.t11 - sw.t11) +
@@ -698,8 +697,8 @@ __global__ void k_uvh_apply(DevModel M) {
   if (j >= 1) {
     const Stress ss = stress_h(M, k, j - 1, i);
     const int jj = 2 * j;
-    const double rln_inv = 1. / M.rln[jj], m_2j = M.m[jj], n_2j = M.n[jj];
-    const double h_inv = 2. / (M.hdry[M.at(k, j, i)] + M.hdry[M.at(k, j - 1, i)]);
+    const double rln_inv = div_rn(1., M.rln[jj]), m_2j = M.m[jj], n_2j = M.n[jj];
+    const double h_inv = div_rn(2., M.hdry[M.at(k, j, i)] + M.hdry[M.at(k, j - 1, i)]);
     const long long x = tend + M.at(k, j, i);
     M.dvdt[x] += h_inv * (m_2j * (stress_12(M, k, j, i) - stress_12(M, k, j, i - 1)) -
                           n_2j * rln_inv * (M.rln[jj + 1] * s.t22 - M.rln[jj - 1] * ss.t22 - .5 * (s.t11 + ss.t11) * (M.rln[jj + 1] - M.rln[jj - 1])) -
@@ -722,9 +721,9 @@ __global__ void k_dc_layers(DevModel M) {
   const int i = 1 + (int)(t - r * ni), j = (int)(r - q * nr), k = 1 + (int)q;
   const long long x = M.at(k, j, i), row = M.at(k, j, 0);
   const double nu = M.nu_turb[x];
-  double chi3 = nu / M.kinvisc;
+  double chi3 = div_rn(nu, M.kinvisc);
   chi3 *= chi3 * chi3;
-  const double fv1 = chi3 / (chi3 + SA_CV1_3);
+  const double fv1 = div_rn(chi3, chi3 + SA_CV1_3);
   const double turb = fv1 * nu;
   const double v = limit_range(0., turb, M.turb_maxnu2[j]);
   write_with_pads(M.dc_theta, M, row, i, v);
@@ -738,7 +737,7 @@ __global__ void k_dc_bottom(DevModel M) {
   const int j = t / M.ni, i = 1 + t - j * M.ni;
   const int k = M.nk - 1;
   const double kin = kin_plane(M, PL_UV_DIS, k, j, i);
-  const double u_tan = sqrt(2. * kin);
+  const double u_tan = sqrt_rn(2. * kin);
   const double turb = law_of_the_wall(M, k, j, i, WALL_H, u_tan);
   const long long row = M.at(M.nk, j, 0);
   write_with_pads(M.dc_uv, M, row, i, limit_range(0., turb + M.kinvisc, M.turb_maxnu2[j]));
@@ -842,11 +841,21 @@ int launch_scalar_hdiff(const DevModel &M, cudaStream_t s) {
   return launch_restore_nu(M, s);
 }
 
-int launch_scalar_vdiff(const DevModel &M, cudaStream_t s) {
-  const unsigned blocks = nblk((long long)(M.nj + 1) * M.ni, 64);
-  k_theta_vdiff<<<zg(blocks, M), 64, 0, s>>>(M);
+static int launch_vdiff(const DevModel &M, int what, const double *tw, cudaStream_t s) {
+  const int n = what == VD_THETA ? M.nk - M.k_sigma + 2 : (what == VD_NU ? M.nk + 1 : M.nk - 1);
+  const long long cols = (long long)(M.nj + (what == VD_V ? 0 : 1)) * M.ni;
+  k_vdiff<<<zg(nblk(cols, 32), M), VD_THREADS, (size_t)VD_ARRAYS * 32 * (n + 2) * sizeof(double), s>>>(M, what, tw);
+  return 0;
+}
+int launch_tau_wall_h(const DevModel &M, double *tw, cudaStream_t s) {
+  k_tau_wall<<<zg(nblk((long long)(M.nj + 1) * M.ni, 32), M), 32, 0, s>>>(M, WALL_H, tw);
+  return 0;
+}
+
+int launch_scalar_vdiff(const DevModel &M, const double *tw, cudaStream_t s) {
+  launch_vdiff(M, VD_THETA, tw, s);
   launch_set_p2etc(M, 1, s);
-  k_nu_vdiff<<<zg(blocks, M), 64, 0, s>>>(M);
+  launch_vdiff(M, VD_NU, tw, s);
   return launch_restore_nu(M, s);
 }
 
@@ -863,11 +872,16 @@ int launch_uv_hdiff(const DevModel &M, cudaStream_t s) {
 
 int launch_uv_vdiff(const DevModel &M, cudaStream_t s) {
   for (int comp = 0; comp < 2; comp++) {
-    const unsigned blocks = nblk((long long)(M.nj + 1 - comp) * M.ni, 64);
-    k_tau_wall<<<zg(blocks, M), 64, 0, s>>>(M, comp, M.work0);
-    k_wind_vdiff<<<zg(blocks, M), 64, 0, s>>>(M, comp, M.work0);
+    k_tau_wall<<<zg(nblk((long long)(M.nj + 1 - comp) * M.ni, 32), M), 32, 0, s>>>(M, comp == 0 ? WALL_U : WALL_V, M.work0);
+    launch_vdiff(M, comp == 0 ? VD_U : VD_V, M.work0, s);
   }
   return 0;
+}
+
+// the most a launch takes, raised once for the process (models of all sizes)
+int turb_kernels_init() {
+  const int big = (int)((size_t)VD_ARRAYS * 32 * (EPIC_TURB_MAX_NK + 3) * sizeof(double));
+  return cudaFuncSetAttribute(k_vdiff, cudaFuncAttributeMaxDynamicSharedMemorySize, big) == cudaSuccess ? 0 : -1;
 }
 
 int launch_set_diffusion_coef(const DevModel &M, cudaStream_t s) {

@@ -130,7 +130,10 @@ int launch_set_itime(const DevModel &M, long long itime, cudaStream_t s);
 // restore_mass(NU_TURB_INDEX); scratch work0..3 and the model's turbulence arrays
 int launch_source_sink_turb(const DevModel &M, cudaStream_t s);
 int launch_scalar_hdiff(const DevModel &M, cudaStream_t s);
-int launch_scalar_vdiff(const DevModel &M, cudaStream_t s);
+// tw: NU_TURB's wall stresses (launch_tau_wall_h: of the winds, GZ3 and RHO3 alone)
+int launch_tau_wall_h(const DevModel &M, double *tw, cudaStream_t s);
+int launch_scalar_vdiff(const DevModel &M, const double *tw, cudaStream_t s);
+int turb_kernels_init();
 int launch_uv_hdiff(const DevModel &M, cudaStream_t s);
 int launch_uv_vdiff(const DevModel &M, cudaStream_t s);
 int launch_set_diffusion_coef(const DevModel &M, cudaStream_t s);
