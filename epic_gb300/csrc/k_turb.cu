@@ -7,7 +7,8 @@
 //   - source_sink_SA updates NU_TURB in place in K, J, I order (each point reads the new values of
 //     its K-1, J-1 and I-1 neighbours, the old ones of K+1, J+1, I+1).  Its NU_TURB-free part
 //     (strain, wall distance, Brunt-Vaisala frequency) is one pointwise pass; the rest runs as
-//     wavefronts K + J + I = d, one launch each, every point of a front independent of the others;
+//     wavefronts K + J + I = d, every point of a front independent of the others, in one kernel per
+//     model whose blocks form a cluster with a barrier between fronts;
 //   - the Laplacians of laplacian_h are three pointwise passes around the row filter, all layers
 //     at once (each layer's Laplacian reads only its own plane);
 //   - the implicit vertical diffusions take a tile of 32 columns per block: the set-up of the bands and
@@ -252,33 +253,42 @@ __global__ void k_sa_prep(DevModel M) {
   M.work3[x] = brunt2 < 0. ? div_rn(nu * cr_exp(div_rn(-nu, nu_turb_limiter), T) * brunt2, brunt) : 0.;
 }
 
-// One wavefront k + j + i = d of the in-place NU_TURB update: the three gradient terms from the
+// The wavefronts k + j + i = d of the in-place NU_TURB update: the three gradient terms from the
 // neighbours (new at k-1, j-1, i-1; old at k+1, j+1, i+1), summed in the reference's order between
-// the point's own terms
-__global__ void k_sa_wave(DevModel M, int d) {
-  if (epic_member(M)) return;
-  const int nr = M.nj + 1;
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= (M.nk - 1) * nr) return;
-  const int k = 1 + t / nr, j = t - (k - 1) * nr, i = d - k - j;
-  if (i < 1 || i > M.ni) return;
+// the point's own terms.  One cluster of blocks per model, a cluster barrier between fronts: bounded by
+// that chain of nk + nj + ni - 2 fronts (one L2 round trip, the arithmetic and a barrier each), where a
+// launch per front cost 5.5 us (210 launches a step at 128x64x20).  What other blocks have written is
+// read past L1; the old values are what they were when the kernel began, wherever they are cached.
+constexpr int SA_THREADS = 128;
+__global__ void __launch_bounds__(SA_THREADS) k_sa_waves(DevModel M) {
+  if (epic_member(M)) return;   // all blocks of a cluster are one member's
+  const int nr = M.nj + 1, pairs = (M.nk - 1) * nr, ni = M.ni;
   const double cb2 = 0.622, sigma = 2. / 3.;
   double *NU = M.nu_turb;
-  auto nut = [&](int kk, int jj, int ii) { return NU[M.at(kk, jj, ii)]; };
-  const long long x = M.at(k, j, i);
-  const int jj = 2 * j;
-  const double m_2jp1 = M.m[jj + 1], n_2jp2 = M.n[jj + 2], n_2j = M.n[jj];
-  const double nu = NU[x];
-  const double g1 = (nut(k, j, i + 1) - nut(k, j, i - 1)) * m_2jp1 * .5;
-  const double g2 = .5 * ((nut(k, j + 1, i) - nu) * n_2jp2 + (nu - nut(k, j - 1, i)) * n_2j);
-  const double g3 = (nut(k - 1, j, i) - nut(k + 1, j, i)) * M.work2[x];
-  double dnudt = M.work0[x];
-  dnudt += (cb2 / sigma) * (g1 * g1);   // pow(g, 2.), the correctly rounded square
-  dnudt += (cb2 / sigma) * (g2 * g2);
-  dnudt += (cb2 / sigma) * (g3 * g3);
-  dnudt -= M.work1[x];
-  dnudt -= M.work3[x];
-  NU[x] = dmaxr(1.e-4 * M.kinvisc, nu + M.dt * dnudt);
+  const int me = (int)(threadIdx.x * gridDim.x + blockIdx.x), all = (int)(gridDim.x * blockDim.x);   // fronts spread over the blocks
+  for (int d = 2; d <= M.nk - 1 + M.nj + ni; d++) {
+    for (int p = me; p < pairs; p += all) {
+      const int k = 1 + p / nr, j = p - (k - 1) * nr, i = d - k - j;
+      if (i < 1 || i > ni) continue;
+      const int x = M.at(k, j, i), n2 = (int)M.n2, row = M.iadim, jj = 2 * j;
+      const double below = __ldcg(NU + x - n2), south = __ldcg(NU + x - row), west = __ldcg(NU + x - 1);
+      const double nu = __ldcg(NU + x), north = NU[x + row], east = NU[x + 1], above = NU[x + n2];
+      const double w0 = M.work0[x], w1 = M.work1[x], w2 = M.work2[x], w3 = M.work3[x];
+      const double g1 = half_of((east - west) * M.m[jj + 1]);
+      const double g2 = half_of((north - nu) * M.n[jj + 2] + (nu - south) * M.n[jj]);
+      const double g3 = (below - above) * w2;
+      double dnudt = w0;
+      dnudt += (cb2 / sigma) * (g1 * g1);   // pow(g, 2.), the correctly rounded square
+      dnudt += (cb2 / sigma) * (g2 * g2);
+      dnudt += (cb2 / sigma) * (g3 * g3);
+      dnudt -= w1;
+      dnudt -= w3;
+      NU[x] = dmaxr(1.e-4 * M.kinvisc, nu + M.dt * dnudt);
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  }
 }
 
 // The solid-surface block (:2690-2704): NU_TURB(nk) = MAX(1e-4 kinvisc, NU_TURB(nk-1)) (the
@@ -814,12 +824,24 @@ static int launch_pads(const DevModel &M, double *a, int k0, int k1, cudaStream_
   return 0;
 }
 
+// Blocks of the wavefront kernel's cluster: 16 where the GPU can place them (a front of 1235 points at
+// 128x64x20 is then a few per thread's SM), else the portable 8.  Set by turb_kernels_init.
+static int g_sa_cluster = 8;
+
 int launch_source_sink_turb(const DevModel &M, cudaStream_t s) {
   const long long cells = (long long)(M.nk - 1) * (M.nj + 1) * M.ni;
   k_sa_prep<<<zg(nblk(cells, 128), M), 128, 0, s>>>(M);
-  const int fronts_lo = 1 + 0 + 1, fronts_hi = (M.nk - 1) + M.nj + M.ni;
-  const unsigned blocks = nblk((long long)(M.nk - 1) * (M.nj + 1), 128);
-  for (int d = fronts_lo; d <= fronts_hi; d++) k_sa_wave<<<zg(blocks, M), 128, 0, s>>>(M, d);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = zg(dim3((unsigned)g_sa_cluster), M);
+  cfg.blockDim = dim3(SA_THREADS);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)g_sa_cluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_sa_waves, M);
   if (!M.gas_giant) k_sa_bottom<<<zg(nblk((long long)(M.nj + 1) * M.ni, 128), M), 128, 0, s>>>(M);
   return launch_pads(M, M.nu_turb, 0, M.nk + 1, s);
 }
@@ -881,6 +903,23 @@ int launch_uv_vdiff(const DevModel &M, cudaStream_t s) {
 // the most a launch takes, raised once for the process (models of all sizes)
 int turb_kernels_init() {
   const int big = (int)((size_t)VD_ARRAYS * 32 * (EPIC_TURB_MAX_NK + 3) * sizeof(double));
+  static const int cluster = [] {   // a property of the device type, found once
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(SA_THREADS);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 16;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    const bool ok = cudaFuncSetAttribute(k_sa_waves, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&n, k_sa_waves, &cfg) == cudaSuccess && n >= 1;
+    cudaGetLastError();
+    return ok ? 16 : 8;
+  }();
+  g_sa_cluster = cluster;
   return cudaFuncSetAttribute(k_vdiff, cudaFuncAttributeMaxDynamicSharedMemorySize, big) == cudaSuccess ? 0 : -1;
 }
 
