@@ -22,6 +22,12 @@ enum TuneGroup { TB_UV_CORE = 0, TB_PGRAD, TB_HSU, TB_VISC, TB_DIAG, TB_UPDATE, 
 
 namespace epic {
 
+// Quantities of the latitude rows that the stencils divide or convert once per cell otherwise, made at
+// model creation in each compute type (k_row_tables) with the expressions of the kernels: row j's h
+// point is half-level 2j+1, its v point 2j.
+enum RowTab { RT_NINV_H, RT_MINV_V, RT_MINV_H, RT_MNINV_H, RT_MNINV_V, RT_MNPV, RT_GDX, RT_GDY, RT_M_H, RT_M_V, RT_N_V, RT_MN_H, RT_F_V,
+              RT_COUNT = 16 };
+
 constexpr int SCRATCH_SETS = 3;   // work0..3, once per branch of the step that uses them concurrently
 constexpr int TABLE_SETS = 4;     // ptable, once per field of the 3-D filter
 constexpr int SCRATCH_VOLUMES = 3 + 4 * SCRATCH_SETS;   // gz, unity, old and the sets of work0..3
@@ -67,6 +73,8 @@ struct DevModel {
   const double *sgth, *dsgth, *dsgth_inv, *h_min, *t_sponge_inv;
   const double *high_lat_h, *high_lat_pv;   // [(nj+3)*(ni+2)] 2-D like the reference
   const double *h_coef, *v_coef;            // d2dy2 coefficients, 3 per row
+  const double *rt64;                       // RowTab of rows 0..nj+1, RT_COUNT values each, in binary64 ...
+  const float *rt32;                        // ... and in binary32
   const double *tw;                         // realft/four1 twiddles (see k_filter.cu)
   const double *coslat;                     // cos(lat[2j+1] deg), j = 0..nj, from the host libm
   const double *coslat4;                    // pow(coslat[j], 4.) correctly rounded (t_rad's cos^4)
@@ -457,17 +465,23 @@ template <class R> __device__ __forceinline__ R rmin(R x, R y) { return x < y ? 
 // a / b: the IEEE quotient (binary64 on the integer pipe)
 template <class R> __device__ __forceinline__ R qdiv(R a, R b) { return a / b; }
 template <> __device__ __forceinline__ double qdiv<double>(double a, double b) { return div_rn(a, b); }
-// x / 2 in the compute type: binary64 on the integer pipe (the exponent less one; zeros as they are,
-// magnitudes at the ends of the range by the multiplication)
-static __device__ __noinline__ double half_cold(double x) { return .5 * x; }
-template <class R> __device__ __forceinline__ R half_of(R x) { return R(.5) * x; }
-template <> __device__ __forceinline__ double half_of<double>(double x) {
-  const int hi = __double2hiint(x), lo = __double2loint(x);
-  const unsigned e = (unsigned)hi & 0x7ff00000u;
-  const bool zero = (((unsigned)hi << 1) | (unsigned)lo) == 0u;
-  if (!zero && e - 0x00200000u >= 0x7fd00000u) return half_cold(x);
-  return __hiloint2double(zero ? hi : hi - 0x00100000, lo);
+// x 2^-E in the compute type: binary64 on the integer pipe (the exponent less E; zeros as they are,
+// magnitudes at the ends of the range by the multiplication).  The rare branch holds no call, so that
+// loads after it can be issued before it.
+template <int E, class R> __device__ __forceinline__ R scale_down(R x) {
+  if constexpr (std::is_same_v<R, double>) {
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    const unsigned e = (unsigned)hi & 0x7ff00000u;
+    const bool zero = (((unsigned)hi << 1) | (unsigned)lo) == 0u;
+    double r = __hiloint2double(zero ? hi : hi - (E << 20), lo);
+    if (!zero && e - ((unsigned)(E + 1) << 20) >= 0x7ff00000u - ((unsigned)(E + 1) << 20)) r = (1. / (1 << E)) * x;
+    return r;
+  } else {
+    return R(1. / (1 << E)) * x;
+  }
 }
+template <class R> __device__ __forceinline__ R half_of(R x) { return scale_down<1>(x); }
+
 template <class R> struct RMath;
 template <> struct RMath<double> {
   static __device__ __forceinline__ double log(const DevModel &M, double x) { return xlog(M, x); }
@@ -537,6 +551,10 @@ __device__ __forceinline__ R hsu_face(R w, R w_up, R a_u, R a_d, R ap_d, R d_up,
 // the predictor's flux: the upwind cell's value carried by w (the other side's term is zero)
 template <class R>
 __device__ __forceinline__ R hsu_upwind(R w, R a_minus, R a_plus) { return w * (is_neg(w) ? a_minus : a_plus); }
+
+template <class R> __device__ __forceinline__ R rt(const DevModel &M, int j, int q);
+template <> __device__ __forceinline__ double rt<double>(const DevModel &M, int j, int q) { return M.rt64[j * RT_COUNT + q]; }
+template <> __device__ __forceinline__ float rt<float>(const DevModel &M, int j, int q) { return M.rt32[j * RT_COUNT + q]; }
 
 struct Trip { double x, y, z; };
 

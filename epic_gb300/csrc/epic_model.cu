@@ -612,7 +612,7 @@ size_t model_pool_bytes(const epic_grid &g) {
   return rnd(sizeof(Ctl)) + (n_state3 + n_scratch3) * rnd(n3 * 8) + 3 * rnd(n2 * 8) + rnd((size_t)epic::TABLE_SETS * (g.nj + 3) * (g.nk + 2) * 3 * 8) +
          rnd(ni1 * 8) + 10 * rnd(nj1 * 8) + 3 * rnd(nk1 * 8) + rnd((g.nk + 2) * 8) + rnd((g.k_sponge + 1) * 8) +
          2 * rnd(3 * (g.nj + 2) * 8) + rnd(ntw * 8) + rnd(ntw * 4) + 2 * rnd((g.nj + 1) * 8) + rnd(sizeof(epic::MathTable)) +
-         rnd(32 * sizeof(float2)) + rnd(((size_t)epic::TH_N * epic::TH_M + 4 * epic::TH_M + epic::TH_N) * 8) +
+         rnd(32 * sizeof(float2)) + rnd((size_t)(g.nj + 2) * epic::RT_COUNT * 8) + rnd((size_t)(g.nj + 2) * epic::RT_COUNT * 4) + rnd(((size_t)epic::TH_N * epic::TH_M + 4 * epic::TH_M + epic::TH_N) * 8) +
          (g.turbulence ? 4 * rnd(n3 * 8) + rnd(2 * (size_t)(g.nk + 2) * 8) + rnd((size_t)(g.nj + 1) * 8) : 0) + 4096;
 }
 
@@ -762,6 +762,8 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
   double *coslat4 = carve<double>(p, g->nj + 1);
   epic::MathTable *lt = carve<epic::MathTable>(p, 1);
   float2 *exp2tab = carve<float2>(p, 32);
+  d.rt64 = carve<double>(p, (size_t)(g->nj + 2) * epic::RT_COUNT);
+  d.rt32 = carve<float>(p, (size_t)(g->nj + 2) * epic::RT_COUNT);
   double *thermo_d = carve<double>(p, (size_t)epic::TH_N * epic::TH_M + 4 * epic::TH_M + epic::TH_N);
   if (d.turb) {   // the turbulence closure: NU_TURB, the three diffusivities (one stride apart, as
                   // relocate_field expects), scratch and a row table
@@ -854,6 +856,7 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
       return set_error(EPIC_ERR_NOMEM, "epic_model_create: %s", why);
     }
   }
+  epic::launch_row_tables(d, m->stream);
   epic::filter_kernels_init(g->ni);
   epic::column_kernels_init(g->nk);
   epic::column_acc_kernels_init();

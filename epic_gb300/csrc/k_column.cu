@@ -866,28 +866,29 @@ __global__ void __launch_bounds__(CT_THREADS, 4) k_pgrad_vars_column_mixed(DevMo
   }
 }
 
-// store_pgrad_vars, horizontal part of DZDT3 (epic_funcs_diag.c:3924-3945) plus bc_lateral.
-template <class R>
+// store_pgrad_vars, horizontal part of DZDT3 (epic_funcs_diag.c:3924-3945) plus bc_lateral, layers 1..nk,
+// rows 0..nj: a row's northern term is the next one's southern.
+template <class R, int ROWS>
 __global__ void k_pgrad_dzdt(DevModel M) {
   if (epic_member(M)) return;
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int ni = M.ni, nk = M.nk;
-  if (t >= nk * (M.nj + 1) * ni) return;
-  const int i = 1 + t % ni;
-  const int j = (t / ni) % (M.nj + 1);
-  const int k = 1 + t / (ni * (M.nj + 1));
-  const int jj = 2 * j;
-  const Ctl *c = M.ctl;
-  const double *U = M.u + (long long)c->it_uv * M.n3, *V = M.v + (long long)c->it_uv * M.n3;
-  const R gdx_inv3 = qdiv(R(.5) * cv<R>(M.m[jj + 1]), cv<R>(M.grav[jj + 1]));
-  const R gdy_inv2 = qdiv(R(.5) * cv<R>(M.n[jj]), cv<R>(M.grav[jj]));
-  const R gdy_inv4 = qdiv(R(.5) * cv<R>(M.n[jj + 2]), cv<R>(M.grav[jj + 2]));
-  const double *G = M.gz3;
-  const long long x = M.at(k, j, i);
+  March s;
+  if (!march<ROWS>(M, 1, M.nk, 0, M.nj, s)) return;
+  const int k = s.k, i = s.i;
+  const long long off = plane_offset(M, PL_UV);
+  const double *U = M.u + off, *V = M.v + off, *G = M.gz3;
   // geopotential differences are formed in FP64 in both forms
-  const R add = cv<R>(V[x]) * cv<R>(G[x] - G[M.at(k, j - 1, i)]) * gdy_inv2 + cv<R>(V[M.at(k, j + 1, i)]) * cv<R>(G[M.at(k, j + 1, i)] - G[x]) * gdy_inv4 +
-                cv<R>(U[x]) * cv<R>(G[x] - G[M.at(k, j, i - 1)]) * gdx_inv3 + cv<R>(U[M.at(k, j, i + 1)]) * cv<R>(G[M.at(k, j, i + 1)] - G[x]) * gdx_inv3;
-  write_with_pads(M.dzdt3, M, M.at(k, j, 0), i, M.dzdt3[x] + to_d(add));
+  auto north = [&](int j) { return cv<R>(V[M.at(k, j, i)]) * cv<R>(G[M.at(k, j, i)] - G[M.at(k, j - 1, i)]) * rt<R>(M, j, RT_GDY); };
+  R ts = north(s.j0);
+#pragma unroll
+  for (int q = 0; q < ROWS; q++) {
+    const int j = s.j0 + q;
+    if (ROWS > 1 && j > s.j1) break;
+    const int x = M.at(k, j, i);
+    const R gdx = rt<R>(M, j, RT_GDX), tn = north(j + 1);
+    const R add = ts + tn + cv<R>(U[x]) * cv<R>(G[x] - G[x - 1]) * gdx + cv<R>(U[x + 1]) * cv<R>(G[x + 1] - G[x]) * gdx;
+    write_with_pads(M.dzdt3, M, x - i, i, M.dzdt3[x] + to_d(add));
+    ts = tn;
+  }
 }
 
 // Monotone fix of the filtered GZ copy, epic_timestep.c:182-195 (the zonal filter of planes
@@ -1156,7 +1157,7 @@ int launch_store_pgrad_vars(const DevModel &M, cudaStream_t s, bool early, bool 
   return dzdt ? launch_pgrad_dzdt(M, s) : 0;
 }
 int launch_pgrad_dzdt(const DevModel &M, cudaStream_t s) {
-  EPIC_LAUNCH_R(M.mixed, k_pgrad_dzdt, epic_blocks((long long)M.nk * (M.nj + 1) * M.ni, TB(M, TB_UPDATE)), TB(M, TB_UPDATE), 0, s, M);
+  EPIC_MARCH(M.mixed, k_pgrad_dzdt, M.nk, M.nj + 1, TB(M, TB_UPDATE), s, M);
   return 0;
 }
 int launch_gz_monotone(const DevModel &M, cudaStream_t s) { k_gz_monotone<<<zg(ncol_blocks(M, TB(M, TB_COLUMN)), M), TB(M, TB_COLUMN), 0, s>>>(M); return 0; }

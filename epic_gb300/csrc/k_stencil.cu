@@ -35,6 +35,29 @@ static inline unsigned cells_blocks(const DevModel &M, int nkk, int njj, int th)
 }
 __device__ __forceinline__ int wrap_i(const DevModel &M, int i) { return i == 0 ? M.ni : (i == M.ni + 1 ? 1 : i); }
 
+template <class R>
+__global__ void k_row_tables(DevModel M, R *out) {
+  const int j = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (j > M.nj + 1) return;
+  const bool h = j <= M.nj, v = j >= 1 && j <= M.nj;   // rows with an h point, v points off the poles
+  auto inv = [&](const double *a, int jj) { return qdiv(R(1.), cv<R>(a[jj])); };
+  R *t = out + j * RT_COUNT;
+  const int jj = 2 * j;
+  t[RT_NINV_H] = h ? inv(M.n, jj + 1) : R(0.);
+  t[RT_MINV_V] = fabs(M.lat[jj]) == 90. ? R(0.) : inv(M.m, jj);
+  t[RT_MINV_H] = h ? inv(M.m, jj + 1) : R(0.);
+  t[RT_MNINV_H] = h ? inv(M.mn, jj + 1) : R(0.);
+  t[RT_MNINV_V] = cv<R>(M.mn_inv[jj]);
+  t[RT_MNPV] = v ? qdiv(R(.5), inv(M.mn, jj - 1) + inv(M.mn, jj + 1)) : R(0.);
+  t[RT_GDX] = h ? qdiv(R(.5) * cv<R>(M.m[jj + 1]), cv<R>(M.grav[jj + 1])) : R(0.);
+  t[RT_GDY] = qdiv(R(.5) * cv<R>(M.n[jj]), cv<R>(M.grav[jj]));
+  t[RT_M_H] = h ? cv<R>(M.m[jj + 1]) : R(0.);
+  t[RT_M_V] = cv<R>(M.m[jj]);
+  t[RT_N_V] = cv<R>(M.n[jj]);
+  t[RT_MN_H] = h ? cv<R>(M.mn[jj + 1]) : R(0.);
+  t[RT_F_V] = cv<R>(M.f[jj]);
+}
+
 // memset of DUDT, DVDT(it_uv_tend), epic_timestep.c:107-108
 __global__ void k_zero_tend(DevModel M) {
   if (epic_member(M)) return;
@@ -50,88 +73,134 @@ __global__ void k_zero_tend(DevModel M) {
 // epic_funcs_diag.c:2694-2847) and the PV averages of include/epic_pv_schemes.h:48-61.
 // ---------------------------------------------------------------------------------------------
 
-// UH(j,i) for j = 0..nj (0 above), periodic in i
+// UH(j,i), j = 0..nj, of wind value u between h-points h0 = H(j,i) and hm = H(j,i-1)
 template <class R>
-__device__ __forceinline__ R uh_at(const DevModel &M, const double *Uk, const double *Hk, int j, int i) {
-  if (j < 0 || j > M.nj) return R(0.);
-  i = wrap_i(M, i);
-  const R havg = R(.5) * (cv<R>(Hk[M.at2(j, i)]) + cv<R>(Hk[M.at2(j, i - 1)]));
-  return cv<R>(Uk[M.at2(j, i)]) * havg * qdiv(R(1.), cv<R>(M.n[2 * j + 1]));
-}
-// VH(j,i) for j = 1..nj (0 at the poles), periodic in i
-template <class R>
-__device__ __forceinline__ R vh_at(const DevModel &M, const double *Vk, const double *Hk, int j, int i) {
-  if (j < 1 || j > M.nj) return R(0.);
-  i = wrap_i(M, i);
-  const R havg = R(.5) * (cv<R>(Hk[M.at2(j, i)]) + cv<R>(Hk[M.at2(j - 1, i)]));
-  return cv<R>(Vk[M.at2(j, i)]) * havg * qdiv(R(1.), cv<R>(M.m[2 * j]));
-}
+__device__ __forceinline__ R uh_of(const DevModel &M, int j, R u, R h0, R hm) { return u * half_of(h0 + hm) * rt<R>(M, j, RT_NINV_H); }
 
-// Kinetic energy per mass on the h grid, planes k = 1..nk-1, into work0 (with pads).
-template <class R>
+// Kinetic energy per mass on the h grid, planes k = 1..nk-1, into work0 (with pads): kin_at up the rows,
+// where a row's northern v terms are the next one's southern.
+template <class R, int ROWS>
 __global__ void k_uv_kin(DevModel M) {
   if (epic_member(M)) return;
-  Cell c;
-  if (!cell3(M, 1, M.nk - 1, 0, M.nj + 1, c)) return;
-  const long long off = plane_offset(M, PL_UV);
-  const double *Uk = M.u + off + c.k * M.n2, *Vk = M.v + off + c.k * M.n2;
-  write_with_pads(M.work0, M, M.at(c.k, c.j, 0), c.i, kin_at<R>(M, Uk, Vk, c.j, c.i));
+  March s;
+  if (!march<ROWS>(M, 1, M.nk - 1, 0, M.nj, s)) return;
+  const int k = s.k, i = s.i, nj = M.nj;
+  const long long off = plane_offset(M, PL_UV) + k * M.n2;
+  const double *Uk = M.u + off, *Vk = M.v + off;
+  auto u = [&](int j, int ii) { return cv<R>(Uk[M.at2(j, ii)]); };
+  // v^2/mn of row j at the cell and of the mean of its neighbours
+  auto vv = [&](int j, R &own, R &mean) {
+    const R v0 = cv<R>(Vk[M.at2(j, i)]), vm = half_of(cv<R>(Vk[M.at2(j, i + 1)]) + cv<R>(Vk[M.at2(j, i - 1)])), w = rt<R>(M, j, RT_MNINV_V);
+    own = v0 * v0 * w;
+    mean = vm * vm * w;
+  };
+  R us_w = R(0.), us_e = R(0.), u_w = u(s.j0, i), u_e = u(s.j0, i + 1), vs, vsm;
+  if (s.j0 > 0) { us_w = u(s.j0 - 1, i); us_e = u(s.j0 - 1, i + 1); }
+  vv(s.j0, vs, vsm);
+#pragma unroll
+  for (int q = 0; q < ROWS; q++) {
+    const int j = s.j0 + q;
+    if (ROWS > 1 && j > s.j1) break;
+    R un_w = R(0.), un_e = R(0.), vn, vnm;
+    if (j < nj) { un_w = u(j + 1, i); un_e = u(j + 1, i + 1); }
+    vv(j + 1, vn, vnm);
+    const R mn1 = rt<R>(M, j, RT_MN_H);
+    R kin = scale_down<2>(u_w * u_w + u_e * u_e + mn1 * (vs + vn));
+    if (j != 0 && j != nj) {
+      const R u2 = half_of(un_w + us_w), u4 = half_of(un_e + us_e);
+      const R kin_s = scale_down<2>(u2 * u2 + u4 * u4 + mn1 * (vsm + vnm));
+      kin = (R(5.) / R(6.)) * kin + (R(1.) / R(6.)) * kin_s;
+    }
+    write_with_pads(M.work0, M, M.at(k, j, 0), i, to_d(kin));
+    us_w = u_w; us_e = u_e; u_w = un_w; u_e = un_e; vs = vn; vsm = vnm;
+  }
 }
 
-// DVDT += (PV*UH terms + KIN(j-1)-KIN(j))*n, then the vertical advection of V.
-template <class R>
+// DVDT += (PV*UH terms + KIN(j-1)-KIN(j))*n, then the vertical advection of V, rows 1..nj.
+template <class R, int ROWS>
 __global__ void k_uv_core_v(DevModel M) {
   if (epic_member(M)) return;
-  Cell c;
-  if (!cell3(M, 1, M.nk - 1, 1, M.nj, c)) return;
-  const int k = c.k, j = c.j, i = c.i;
+  March s;
+  if (!march<ROWS>(M, 1, M.nk - 1, 1, M.nj, s)) return;
+  const int k = s.k, i = s.i, n2 = (int)M.n2, ie = i == M.ni ? 1 : i + 1;   // UH is periodic in i
   const long long off = plane_offset(M, PL_UV);
-  const double *U = M.u + off, *V = M.v + off;
-  const double *Uk = U + k * M.n2, *Hk = M.h3 + k * M.n2;
-  const double *PV = M.pv3 + k * M.n2, *KIN = M.work0 + k * M.n2;
+  const double *V = M.v + off, *Uk = M.u + off + k * M.n2, *Hk = M.h3 + k * M.n2;
+  const double *PV = M.pv3 + k * M.n2, *KIN = M.work0 + k * M.n2, *W = M.w3 + k * M.n2;
   double *D = M.dvdt + plane_offset(M, PL_UV_TEND);
   auto pv = [&](int jj, int ii) { return cv<R>(PV[M.at2(jj, ii)]); };
-  const R ga = (pv(j, i) + pv(j, i + 1) + pv(j + 1, i + 1));
-  const R de = (pv(j, i) + pv(j + 1, i) + pv(j, i + 1));
-  const R al = (pv(j - 1, i) + pv(j, i) + pv(j, i + 1));
-  const R be = (pv(j, i) + pv(j, i + 1) + pv(j - 1, i + 1));
-  const R core = ((-ga * uh_at<R>(M, Uk, Hk, j, i + 1) - de * uh_at<R>(M, Uk, Hk, j, i) - al * uh_at<R>(M, Uk, Hk, j - 1, i) -
-                   be * uh_at<R>(M, Uk, Hk, j - 1, i + 1)) * (R(1.) / R(12.)) +
-                  cv<R>(KIN[M.at2(j - 1, i)]) - cv<R>(KIN[M.at2(j, i)])) * cv<R>(M.n[2 * j]);
-  const long long x = M.at(k, j, i);
-  double d = D[x] + to_d(core);
+  auto uh = [&](int jj, R &c, R &e) {   // UH(jj,i), UH(jj,i+1)
+    const R hc = cv<R>(Hk[M.at2(jj, i)]);
+    c = uh_of<R>(M, jj, cv<R>(Uk[M.at2(jj, i)]), hc, cv<R>(Hk[M.at2(jj, i - 1)]));
+    // the row's last cell takes column 1, whose western neighbour is column 0
+    e = uh_of<R>(M, jj, cv<R>(Uk[M.at2(jj, ie)]), cv<R>(Hk[M.at2(jj, ie)]), ie == 1 ? cv<R>(Hk[M.at2(jj, 0)]) : hc);
+  };
   const int kk = 2 * k + 1;
-  d -= to_d(R(.5) * (cv<R>(M.w3[x]) + cv<R>(M.w3[M.at(k, j - 1, i)])) * (cv<R>(V[M.at(k - 1, j, i)]) - cv<R>(V[M.at(k + 1, j, i)])) /
-                (cv<R>(M.sgth[kk - 2]) - cv<R>(M.sgth[kk + 2])));
-  D[x] = d;
+  const R dsg = cv<R>(M.sgth[kk - 2]) - cv<R>(M.sgth[kk + 2]);
+  R uhs_c, uhs_e, pc = pv(s.j0, i), pe = pv(s.j0, i + 1), ps_e = pv(s.j0 - 1, i + 1), ps = pv(s.j0 - 1, i) + pc;
+  R kin_s = cv<R>(KIN[M.at2(s.j0 - 1, i)]), w_s = cv<R>(W[M.at2(s.j0 - 1, i)]);
+  uh(s.j0 - 1, uhs_c, uhs_e);
+#pragma unroll
+  for (int q = 0; q < ROWS; q++) {
+    const int j = s.j0 + q;
+    if (ROWS > 1 && j > s.j1) break;
+    const int x2 = M.at2(j, i), x = x2 + k * n2;
+    const R pn = pv(j + 1, i), pn_e = pv(j + 1, i + 1), pp = pc + pe, pcn = pc + pn;
+    const R ga = pp + pn_e, de = pcn + pe, al = ps + pe, be = pp + ps_e;
+    R uh_c, uh_e;
+    uh(j, uh_c, uh_e);
+    const R kin = cv<R>(KIN[x2]), w = cv<R>(W[x2]);
+    const R core = ((-ga * uh_e - de * uh_c - al * uhs_c - be * uhs_e) * (R(1.) / R(12.)) + kin_s - kin) * rt<R>(M, j, RT_N_V);
+    double d = D[x] + to_d(core);
+    d -= to_d(qdiv(half_of(w + w_s) * (cv<R>(V[x - n2]) - cv<R>(V[x + n2])), dsg));
+    D[x] = d;
+    ps = pcn; ps_e = pe; pc = pn; pe = pn_e; uhs_c = uh_c; uhs_e = uh_e; kin_s = kin; w_s = w;
+  }
 }
 
-// DUDT += (PV*VH terms + KIN(i-1)-KIN(i))*m with the filtered KIN, then the vertical advection of U.
-template <class R>
+// DUDT += (PV*VH terms + KIN(i-1)-KIN(i))*m with the filtered KIN, then the vertical advection of U,
+// rows 0..nj.
+template <class R, int ROWS>
 __global__ void k_uv_core_u(DevModel M) {
   if (epic_member(M)) return;
-  Cell c;
-  if (!cell3(M, 1, M.nk - 1, 0, M.nj + 1, c)) return;
-  const int k = c.k, j = c.j, i = c.i;
+  March s;
+  if (!march<ROWS>(M, 1, M.nk - 1, 0, M.nj, s)) return;
+  const int k = s.k, i = s.i, n2 = (int)M.n2, nj = M.nj, iw = i == 1 ? M.ni : i - 1;   // VH is periodic in i
   const long long off = plane_offset(M, PL_UV);
-  const double *U = M.u + off, *V = M.v + off;
-  const double *Vk = V + k * M.n2, *Hk = M.h3 + k * M.n2;
-  const double *PV = M.pv3 + k * M.n2, *KIN = M.work0 + k * M.n2;
+  const double *U = M.u + off, *Vk = M.v + off + k * M.n2, *Hk = M.h3 + k * M.n2;
+  const double *PV = M.pv3 + k * M.n2, *KIN = M.work0 + k * M.n2, *W = M.w3 + k * M.n2;
   double *D = M.dudt + plane_offset(M, PL_UV_TEND);
   auto pv = [&](int jj, int ii) { return cv<R>(PV[M.at2(jj, ii)]); };
-  const R al = (pv(j, i) + pv(j + 1, i) + pv(j + 1, i + 1));
-  const R be = (pv(j + 1, i - 1) + pv(j + 1, i) + pv(j, i));
-  const R ga = (pv(j, i - 1) + pv(j, i) + pv(j + 1, i));
-  const R de = (pv(j, i) + pv(j + 1, i) + pv(j, i + 1));
-  const R core = ((al * vh_at<R>(M, Vk, Hk, j + 1, i) + be * vh_at<R>(M, Vk, Hk, j + 1, i - 1) + ga * vh_at<R>(M, Vk, Hk, j, i - 1) +
-                   de * vh_at<R>(M, Vk, Hk, j, i)) * (R(1.) / R(12.)) +
-                  cv<R>(KIN[M.at2(j, i - 1)]) - cv<R>(KIN[M.at2(j, i)])) * cv<R>(M.m[2 * j + 1]);
-  const long long x = M.at(k, j, i);
-  double d = D[x] + to_d(core);
+  auto h = [&](int jj, int ii) { return cv<R>(Hk[M.at2(jj, ii)]); };
+  // VH(jj,ii) on rows 1..nj between h-points hn = H(jj,ii) and hs = H(jj-1,ii); 0 at the poles
+  auto vh = [&](int jj, int ii, R hn, R hs) { return cv<R>(Vk[M.at2(jj, ii)]) * half_of(hn + hs) * rt<R>(M, jj, RT_MINV_V); };
   const int kk = 2 * k + 1;
-  d -= to_d(R(.5) * (cv<R>(M.w3[x]) + cv<R>(M.w3[M.at(k, j, i - 1)])) * (cv<R>(U[M.at(k - 1, j, i)]) - cv<R>(U[M.at(k + 1, j, i)])) /
-                (cv<R>(M.sgth[kk - 2]) - cv<R>(M.sgth[kk + 2])));
-  D[x] = d;
+  const R dsg = cv<R>(M.sgth[kk - 2]) - cv<R>(M.sgth[kk + 2]);
+  R pc = pv(s.j0, i), pw = pv(s.j0, i - 1), pe = pv(s.j0, i + 1), hc = h(s.j0, i), hw = h(s.j0, iw), vs_c = R(0.), vs_w = R(0.);
+  if (s.j0 >= 1) {
+    vs_c = vh(s.j0, i, hc, h(s.j0 - 1, i));
+    vs_w = vh(s.j0, iw, hw, h(s.j0 - 1, iw));
+  }
+#pragma unroll
+  for (int q = 0; q < ROWS; q++) {
+    const int j = s.j0 + q;
+    if (ROWS > 1 && j > s.j1) break;
+    const int x2 = M.at2(j, i), x = x2 + k * n2;
+    const R pn = pv(j + 1, i), pn_w = pv(j + 1, i - 1), pn_e = pv(j + 1, i + 1), pcn = pc + pn;
+    const R al = pcn + pn_e, be = pn_w + pn + pc, ga = pw + pc + pn, de = pcn + pe;
+    R vn_c = R(0.), vn_w = R(0.), hn = R(0.), hn_w = R(0.);
+    if (j < nj) {
+      hn = h(j + 1, i);
+      hn_w = h(j + 1, iw);
+      vn_c = vh(j + 1, i, hn, hc);
+      vn_w = vh(j + 1, iw, hn_w, hw);
+    }
+    const R core = ((al * vn_c + be * vn_w + ga * vs_w + de * vs_c) * (R(1.) / R(12.)) + cv<R>(KIN[x2 - 1]) - cv<R>(KIN[x2])) *
+                   rt<R>(M, j, RT_M_H);
+    double d = D[x] + to_d(core);
+    d -= to_d(qdiv(half_of(cv<R>(W[x2]) + cv<R>(W[x2 - 1])) * (cv<R>(U[x - n2]) - cv<R>(U[x + n2])), dsg));
+    D[x] = d;
+    pc = pn; pw = pn_w; pe = pn_e; hc = hn; hw = hn_w; vs_c = vn_c; vs_w = vn_w;
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -229,18 +298,19 @@ struct Pow2 { float c; };
 template <class R>
 __device__ __forceinline__ R operator*(Pow2 s, R x) { return R(s.c) * x; }
 __device__ __forceinline__ dfl operator*(Pow2 s, dfl x) { return dfl(s.c * x.hi, s.c * x.lo); }
+__device__ __forceinline__ double operator*(Pow2 s, double x) { return s.c == .5f ? scale_down<1>(x) : (s.c == .25f ? scale_down<2>(x) : s.c * x); }
 
 // The four quarter sums and two half sums of a face (lon_face, lat_face): in the FP64 form in
 // the reference's order; the mixed forms share the pair each two of them have in common.
 template <class R, class G>
 __device__ __forceinline__ void face_sums(G gz, R &zb0, R &zb2, R &zt0, R &zt2, R &zb, R &zt) {
   if constexpr (std::is_same_v<R, double>) {
-    zb0 = R(.25) * (gz(1, 1) + gz(1, 0) + gz(2, 1) + gz(2, 0));
-    zb2 = R(.25) * (gz(1, 1) + gz(1, 2) + gz(2, 1) + gz(2, 2));
-    zt0 = R(.25) * (gz(1, 1) + gz(1, 0) + gz(0, 1) + gz(0, 0));
-    zt2 = R(.25) * (gz(1, 1) + gz(1, 2) + gz(0, 1) + gz(0, 2));
-    zb = R(.5) * (gz(1, 1) + gz(2, 1));
-    zt = R(.5) * (gz(1, 1) + gz(0, 1));
+    zb0 = Pow2{.25f} * (gz(1, 1) + gz(1, 0) + gz(2, 1) + gz(2, 0));
+    zb2 = Pow2{.25f} * (gz(1, 1) + gz(1, 2) + gz(2, 1) + gz(2, 2));
+    zt0 = Pow2{.25f} * (gz(1, 1) + gz(1, 0) + gz(0, 1) + gz(0, 0));
+    zt2 = Pow2{.25f} * (gz(1, 1) + gz(1, 2) + gz(0, 1) + gz(0, 2));
+    zb = Pow2{.5f} * (gz(1, 1) + gz(2, 1));
+    zt = Pow2{.5f} * (gz(1, 1) + gz(0, 1));
   } else {
     const R sb = gz(1, 1) + gz(2, 1), st = gz(1, 1) + gz(0, 1);
     zb0 = Pow2{.25f} * (sb + gz(1, 0) + gz(2, 0));
@@ -373,31 +443,52 @@ __device__ __forceinline__ LatFace<R> lat_face(const DevModel &M, const R (&z)[3
   return f;
 }
 
-template <class R>
+// In the FP64 form each thread marches up ROWS rows, a row's north face being the next one's
+// south; the mixed forms take one row (their differences are relative to the row's own cell).
+template <class R, int ROWS>
 __global__ void k_pgrad_lat(DevModel M) {
   if (epic_member(M)) return;
-  Cell c;
-  if (!cell3(M, 1, M.nk - 1, 1, M.nj, c)) return;
-  const int k = c.k, j = c.j, i = c.i;
+  static_assert(std::is_same_v<R, double> || ROWS == 1);
+  March strip;
+  if (!march<ROWS>(M, 1, M.nk - 1, 1, M.nj, strip)) return;
+  const int k = strip.k, i = strip.i;
   const R DLOGZ_TOL = R(1.e-2);
-  const PgradRef<R> ref(M, k, j, i);
   R z[3][2][3], p[2][2][3];
+  LatFace<R> s, n;
 #pragma unroll
-  for (int a = 0; a < 3; a++)
+  for (int q_ = 0; q_ < ROWS; q_++) {
+  const int j = strip.j0 + q_;
+  if (ROWS > 1 && j > strip.j1) break;
+  const PgradRef<R> ref(M, k, j, i);
+  const bool first = q_ == 0;
+  auto load = [&](int b) {
 #pragma unroll
-    for (int b = 0; b < 2; b++)
+    for (int a = 0; a < 3; a++)
 #pragma unroll
       for (int q = 0; q < 3; q++) z[a][b][q] = ref.z(M.at(k + a - 1, j + b - 1, i + q - 1));
 #pragma unroll
-  for (int a = 0; a < 2; a++)
-#pragma unroll
-    for (int b = 0; b < 2; b++)
+    for (int a = 0; a < 2; a++)
 #pragma unroll
       for (int q = 0; q < 3; q++) p[a][b][q] = ref.p(M.at(k + a, j + b - 1, i + q - 1));
+  };
+  if (first) {
+    load(0);
+    s = lat_face<R>(M, z, p, 0, j - 1);
+  } else {
+    s = n;
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        z[a][0][q] = z[a][1][q];
+        if (a < 2) p[a][0][q] = p[a][1][q];
+      }
+  }
+  load(1);
+  n = lat_face<R>(M, z, p, 1, j);
   // z(level k+a-1, row j+b-1, column i+q-1), pp(level k+a, row j+b-1, column i+q-1)
   auto gz = [&](int a, int b, int q) { return z[a][b][q]; };
   auto pp = [&](int a, int b, int q) { return p[a][b][q]; };
-  const LatFace<R> s = lat_face<R>(M, z, p, 0, j - 1), n = lat_face<R>(M, z, p, 1, j);
   const R rho = Pow2{.5f} * (cv<R>(M.rho3[M.at(k, j, i)]) + cv<R>(M.rho3[M.at(k, j - 1, i)]));
   const R rlt = cv<R>(M.rlt[2 * j]);
   const R rlns = s.rln, rlnn = n.rln;
@@ -411,14 +502,14 @@ __global__ void k_pgrad_lat(DevModel M) {
   // centre-column pair (mixed forms; the FP64 form sums in the reference's order)
   R zbe, zte, pbe, pte, zbw, ztw, pbw, ptw;
   if constexpr (std::is_same_v<R, double>) {
-    zbe = R(.125) * (gz(1, 1, 1) + gz(1, 1, 2) + gz(1, 0, 1) + gz(1, 0, 2) + gz(2, 1, 1) + gz(2, 1, 2) + gz(2, 0, 1) + gz(2, 0, 2));
-    zte = R(.125) * (gz(0, 1, 1) + gz(0, 1, 2) + gz(0, 0, 1) + gz(0, 0, 2) + gz(1, 1, 1) + gz(1, 1, 2) + gz(1, 0, 1) + gz(1, 0, 2));
-    pbe = R(.25) * (pp(1, 1, 1) + pp(1, 1, 2) + pp(1, 0, 1) + pp(1, 0, 2));
-    pte = R(.25) * (pp(0, 1, 1) + pp(0, 1, 2) + pp(0, 0, 1) + pp(0, 0, 2));
-    zbw = R(.125) * (gz(1, 1, 1) + gz(1, 1, 0) + gz(1, 0, 1) + gz(1, 0, 0) + gz(2, 1, 1) + gz(2, 1, 0) + gz(2, 0, 1) + gz(2, 0, 0));
-    ztw = R(.125) * (gz(0, 1, 1) + gz(0, 1, 0) + gz(0, 0, 1) + gz(0, 0, 0) + gz(1, 1, 1) + gz(1, 1, 0) + gz(1, 0, 1) + gz(1, 0, 0));
-    pbw = R(.25) * (pp(1, 1, 1) + pp(1, 1, 0) + pp(1, 0, 1) + pp(1, 0, 0));
-    ptw = R(.25) * (pp(0, 1, 1) + pp(0, 1, 0) + pp(0, 0, 1) + pp(0, 0, 0));
+    zbe = scale_down<3>(gz(1, 1, 1) + gz(1, 1, 2) + gz(1, 0, 1) + gz(1, 0, 2) + gz(2, 1, 1) + gz(2, 1, 2) + gz(2, 0, 1) + gz(2, 0, 2));
+    zte = scale_down<3>(gz(0, 1, 1) + gz(0, 1, 2) + gz(0, 0, 1) + gz(0, 0, 2) + gz(1, 1, 1) + gz(1, 1, 2) + gz(1, 0, 1) + gz(1, 0, 2));
+    pbe = Pow2{.25f} * (pp(1, 1, 1) + pp(1, 1, 2) + pp(1, 0, 1) + pp(1, 0, 2));
+    pte = Pow2{.25f} * (pp(0, 1, 1) + pp(0, 1, 2) + pp(0, 0, 1) + pp(0, 0, 2));
+    zbw = scale_down<3>(gz(1, 1, 1) + gz(1, 1, 0) + gz(1, 0, 1) + gz(1, 0, 0) + gz(2, 1, 1) + gz(2, 1, 0) + gz(2, 0, 1) + gz(2, 0, 0));
+    ztw = scale_down<3>(gz(0, 1, 1) + gz(0, 1, 0) + gz(0, 0, 1) + gz(0, 0, 0) + gz(1, 1, 1) + gz(1, 1, 0) + gz(1, 0, 1) + gz(1, 0, 0));
+    pbw = Pow2{.25f} * (pp(1, 1, 1) + pp(1, 1, 0) + pp(1, 0, 1) + pp(1, 0, 0));
+    ptw = Pow2{.25f} * (pp(0, 1, 1) + pp(0, 1, 0) + pp(0, 0, 1) + pp(0, 0, 0));
   } else {
     zbe = Pow2{.5f} * (n.zbne + s.zbne);
     zte = Pow2{.5f} * (n.ztne + s.ztne);
@@ -444,8 +535,8 @@ __global__ void k_pgrad_lat(DevModel M) {
   if (fabs(qdiv(R(2.) * (n.ztn - zts), n.ztn + zts - n.zbn - zbs)) > DLOGZ_TOL) {
     b1 = n.ztne * n.ztnw; b2 = ztse * ztsw; b3 = n.ztne * ztse + n.ztnw * ztsw;
     terms1 = a1 * a1 - b1 - (a2 * a2 - b2);
-    top = Pow2{.5f} * ((n.ptn - pts) * ((rlnn + rlns) * terms1 + (rlnn - rlns) * (b1 + b2 - b3)) + (rlnn + rlns) * terms2 * (n.ztn * pts - zts * n.ptn)) /
-          (n.ztn - zts);
+    top = qdiv(Pow2{.5f} * ((n.ptn - pts) * ((rlnn + rlns) * terms1 + (rlnn - rlns) * (b1 + b2 - b3)) + (rlnn + rlns) * terms2 * (n.ztn * pts - zts * n.ptn)),
+               n.ztn - zts);
   } else {
     top = Pow2{.25f} * (rlnn + rlns) * (pts + n.ptn) * terms2;
   }
@@ -454,8 +545,8 @@ __global__ void k_pgrad_lat(DevModel M) {
   if (fabs(qdiv(R(2.) * (n.zbn - zbs), n.ztn + zts - n.zbn - zbs)) > DLOGZ_TOL) {
     b1 = n.zbne * n.zbnw; b2 = zbse * zbsw; b3 = n.zbne * zbse + n.zbnw * zbsw;
     terms1 = a1 * a1 - b1 - (a2 * a2 - b2);
-    bottom = Pow2{.5f} * ((n.pbn - pbs) * ((rlnn + rlns) * terms1 + (rlnn - rlns) * (b1 + b2 - b3)) + (rlnn + rlns) * terms2 * (n.zbn * pbs - zbs * n.pbn)) /
-             (n.zbn - zbs);
+    bottom = qdiv(Pow2{.5f} * ((n.pbn - pbs) * ((rlnn + rlns) * terms1 + (rlnn - rlns) * (b1 + b2 - b3)) + (rlnn + rlns) * terms2 * (n.zbn * pbs - zbs * n.pbn)),
+                  n.zbn - zbs);
   } else {
     bottom = Pow2{.25f} * (rlnn + rlns) * (pbs + n.pbn) * terms2;
   }
@@ -465,6 +556,7 @@ __global__ void k_pgrad_lat(DevModel M) {
   pgflat = qdiv(pgflat, face_width<R>(M.lat, 2 * j - 1, 2 * j + 1) * rho * rlt * (rlns * (dzs + Pow2{.5f} * dzn) + rlnn * (dzn + Pow2{.5f} * dzs)));
   const long long x = plane_offset(M, PL_UV_TEND) + M.at(k, j, i);
   M.dvdt[x] = M.dvdt[x] + to_d(pgflat);
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -477,10 +569,9 @@ template <class R>
 __device__ __forceinline__ R vm_at(const DevModel &M, const double *V, int kind, int k, int j, int i) {
   if (j < 0 || j > M.nj + 1) return R(0.);
   R v2d;
-  if (kind == 2) v2d = (j >= 1 && j <= M.nj) ? R(.5) * (cv<R>(V[M.at(k, j, i)]) + cv<R>(V[M.at(k - 1, j, i)])) : R(0.);
+  if (kind == 2) v2d = (j >= 1 && j <= M.nj) ? half_of(cv<R>(V[M.at(k, j, i)]) + cv<R>(V[M.at(k - 1, j, i)])) : R(0.);
   else v2d = cv<R>(V[M.at(k, j, i)]);
-  const R mi = (fabs(M.lat[2 * j]) == 90.) ? R(0.) : qdiv(R(1.), cv<R>(M.m[2 * j]));
-  return v2d * mi;
+  return v2d * rt<R>(M, j, RT_MINV_V);
 }
 template <class R>
 __device__ __forceinline__ R hsu_floor(const DevModel &M, int kind, int k) {
@@ -937,47 +1028,49 @@ __global__ void k_zonal_visc_mixed(DevModel M, double *A, int sel, int jbot, int
 // divergence, vorticity, store_diag (epic_funcs_diag.c:3963-4445) and the Richardson number
 // ---------------------------------------------------------------------------------------------
 
-// DIV(j,i) of (UU, VV) on planes k0.., divergence() :4064-4117
-template <class R>
-__device__ __forceinline__ R div_at(const DevModel &M, const double *UU, const double *VV, int k, int j, int i) {
-  const int jj = 2 * j + 1;
-  const R n_inv = qdiv(R(1.), cv<R>(M.n[jj]));
-  const R mn1 = cv<R>(M.mn[jj]);
-  const R m2j_inv = (j == 0) ? R(0.) : qdiv(R(1.), cv<R>(M.m[jj - 1]));
-  const R m2jp2_inv = (j == M.nj) ? R(0.) : qdiv(R(1.), cv<R>(M.m[jj + 1]));
-  return mn1 * ((cv<R>(UU[M.at(k, j, i + 1)]) * n_inv - cv<R>(UU[M.at(k, j, i)]) * n_inv) +
-                (cv<R>(VV[M.at(k, j + 1, i)]) * m2jp2_inv - cv<R>(VV[M.at(k, j, i)]) * m2j_inv));
-}
-
-template <class R>
+// DIV of (UU, VV) on planes k0.., rows 0..nj, divergence() :4064-4117
+template <class R, int ROWS>
 __global__ void k_divergence(DevModel M, const double *UU, const double *VV, int vsel, double *DI, int k0, int nkk) {
   if (epic_member(M, UU, VV, DI)) return;
-  Cell c;
-  if (!cell3(M, k0, nkk, 0, M.nj + 1, c)) return;
+  March s;
+  if (!march<ROWS>(M, k0, nkk, 0, M.nj, s)) return;
   VV += plane_offset(M, vsel);
-  write_with_pads(DI, M, M.at(c.k, c.j, 0), c.i, div_at<R>(M, UU, VV, c.k, c.j, c.i));
+  const int k = s.k, i = s.i;
+  auto vm = [&](int j) { return cv<R>(VV[M.at(k, j, i)]) * rt<R>(M, j, RT_MINV_V); };   // 0 at the poles
+  R vs = vm(s.j0);
+#pragma unroll
+  for (int q = 0; q < ROWS; q++) {
+    const int j = s.j0 + q;
+    if (ROWS > 1 && j > s.j1) break;
+    const int x = M.at(k, j, i);
+    const R n_inv = rt<R>(M, j, RT_NINV_H), vn = vm(j + 1);
+    write_with_pads(DI, M, x - i, i, to_d(rt<R>(M, j, RT_MN_H) * ((cv<R>(UU[x + 1]) * n_inv - cv<R>(UU[x]) * n_inv) + (vn - vs))));
+    vs = vn;
+  }
 }
 
-// Interior potential vorticity, vorticity(ON_SIGMATHETA, POTENTIAL) :4168-4186, planes 0..nk.
-template <class R>
+// Interior potential vorticity, vorticity(ON_SIGMATHETA, POTENTIAL) :4168-4186, planes 0..nk, rows 1..nj.
+template <class R, int ROWS>
 __global__ void k_pv_interior(DevModel M, const double *VV) {
   if (epic_member(M, VV)) return;
-  Cell c;
-  if (!cell3(M, 0, M.nk + 1, 1, M.nj, c)) return;
-  const int k = c.k, j = c.j, i = c.i;
+  March s;
+  if (!march<ROWS>(M, 0, M.nk + 1, 1, M.nj, s)) return;
+  const int k = s.k, i = s.i;
   const double *UU = M.u + plane_offset(M, PL_UV);
-  const double *HH = M.h3;
-  const R f2j = cv<R>(M.f[2 * j]), m2j = cv<R>(M.m[2 * j]), n2j = cv<R>(M.n[2 * j]);
-  const R m_m1_inv = qdiv(R(1.), cv<R>(M.m[2 * j - 1])), m_p1_inv = qdiv(R(1.), cv<R>(M.m[2 * j + 1]));
-  const R mn_m1_inv = qdiv(R(1.), cv<R>(M.mn[2 * j - 1])), mn_p1_inv = qdiv(R(1.), cv<R>(M.mn[2 * j + 1]));
-  const R mn_pv = qdiv(R(.5), mn_m1_inv + mn_p1_inv);
-  const R ze = m2j * ((cv<R>(VV[M.at(k, j, i)]) - cv<R>(VV[M.at(k, j, i - 1)])) +
-                      n2j * (cv<R>(UU[M.at(k, j - 1, i)]) * m_m1_inv - cv<R>(UU[M.at(k, j, i)]) * m_p1_inv));
-  R pv = (ze + f2j);
-  const R h_pv = ((cv<R>(HH[M.at(k, j, i)]) + cv<R>(HH[M.at(k, j, i - 1)])) * mn_p1_inv +
-                  (cv<R>(HH[M.at(k, j - 1, i)]) + cv<R>(HH[M.at(k, j - 1, i - 1)])) * mn_m1_inv) * mn_pv;
-  pv = qdiv(pv, h_pv);
-  write_with_pads(M.pv3, M, M.at(k, j, 0), i, pv);
+  auto um = [&](int j) { return cv<R>(UU[M.at(k, j, i)]) * rt<R>(M, j, RT_MINV_H); };
+  auto hm = [&](int j) { return (cv<R>(M.h3[M.at(k, j, i)]) + cv<R>(M.h3[M.at(k, j, i - 1)])) * rt<R>(M, j, RT_MNINV_H); };
+  R us = um(s.j0 - 1), hs = hm(s.j0 - 1);
+#pragma unroll
+  for (int q = 0; q < ROWS; q++) {
+    const int j = s.j0 + q;
+    if (ROWS > 1 && j > s.j1) break;
+    const int x = M.at(k, j, i);
+    const R un = um(j), hn = hm(j);
+    const R ze = rt<R>(M, j, RT_M_V) * ((cv<R>(VV[x]) - cv<R>(VV[x - 1])) + rt<R>(M, j, RT_N_V) * (us - un));
+    const R h_pv = (hn + hs) * rt<R>(M, j, RT_MNPV);
+    write_with_pads(M.pv3, M, x - i, i, to_d(qdiv(ze + rt<R>(M, j, RT_F_V), h_pv)));
+    us = un; hs = hn;
+  }
 }
 
 // Polar potential vorticity from the circulation of the adjacent u row, :4279-4341.
@@ -1189,36 +1282,49 @@ int launch_zero_tend(const DevModel &M, cudaStream_t s) {
   return 0;
 }
 
-int launch_uv_core(const DevModel &M, cudaStream_t s) {
-  EPIC_LAUNCH_R(M.mixed, k_uv_kin, cells_blocks(M, M.nk - 1, M.nj + 1, TB(M, TB_UV_CORE)), TB(M, TB_UV_CORE), 0, s, M);
-  EPIC_LAUNCH_R(M.mixed, k_uv_core_v, cells_blocks(M, M.nk - 1, M.nj, TB(M, TB_UV_CORE)), TB(M, TB_UV_CORE), 0, s, M);
-  // k_uv_kin wrote KIN on rows 0..nj with their pads
-  launch_filter_planes(M, M.work0, PL_NONE, M.work0, 1, M.nk - 1, 0, s, M.mixed, 0, 1);
-  EPIC_LAUNCH_R(M.mixed, k_uv_core_u, cells_blocks(M, M.nk - 1, M.nj + 1, TB(M, TB_UV_CORE)), TB(M, TB_UV_CORE), 0, s, M);
+int launch_row_tables(const DevModel &M, cudaStream_t s) {
+  const unsigned blocks = epic_blocks(M.nj + 2, 64);
+  k_row_tables<double><<<blocks, 64, 0, s>>>(M, const_cast<double *>(M.rt64));
+  k_row_tables<float><<<blocks, 64, 0, s>>>(M, const_cast<float *>(M.rt32));
   return 0;
 }
 
-// k_pgrad_lon's face exchange: one face per thread of the block
-static size_t lon_smem(const DevModel &M, size_t face_bytes) { return (size_t)TB(M, TB_PGRAD) * face_bytes; }
+int launch_uv_core(const DevModel &M, cudaStream_t s) {
+  const int th = TB(M, TB_UV_CORE);
+  EPIC_MARCH(M.mixed, k_uv_kin, M.nk - 1, M.nj + 1, th, s, M);
+  EPIC_MARCH(M.mixed, k_uv_core_v, M.nk - 1, M.nj, th, s, M);
+  // k_uv_kin wrote KIN on rows 0..nj with their pads
+  launch_filter_planes(M, M.work0, PL_NONE, M.work0, 1, M.nk - 1, 0, s, M.mixed, 0, 1);
+  EPIC_MARCH(M.mixed, k_uv_core_u, M.nk - 1, M.nj + 1, th, s, M);
+  return 0;
+}
 
 int launch_pgrad_poles(const DevModel &M, cudaStream_t s) {
   const int lv = row_sum_levels(M, 2);
   k_gz_pole_rows<<<zg(epic_blocks(M.nk + 1, lv), M), 256, (size_t)2 * lv * (M.ni + 1) * sizeof(double), s>>>(M, lv);
   return 0;
 }
-// FP64 form: binary64; mixed: double-float on the splits; fast mixed: binary32 on the splits
+// FP64 form: binary64; mixed: double-float on the splits; fast mixed: binary32 on the splits.
+// k_pgrad_lon's face exchange wants whole rows in a block (one face per thread in shared memory); the
+// FP64 form takes blocks of a row for it up to 512 columns.
 int launch_pgrad_lon(const DevModel &M, cudaStream_t s) {
-  const dim3 grid = zg(cells_blocks(M, M.nk - 1, M.nj + 1, TB(M, TB_PGRAD)), M);
-  if (!M.mixed) k_pgrad_lon<double><<<grid, TB(M, TB_PGRAD), lon_smem(M, sizeof(LonFace<double>)), s>>>(M);
-  else if (M.col64) k_pgrad_lon<dfl><<<grid, TB(M, TB_PGRAD), lon_smem(M, sizeof(LonFace<dfl>)), s>>>(M);
-  else k_pgrad_lon<float><<<grid, TB(M, TB_PGRAD), 0, s>>>(M);
+  int th = TB(M, TB_PGRAD);
+  if (!M.mixed && M.ni > th && M.ni <= 512) th = M.ni;
+  const dim3 grid = zg(cells_blocks(M, M.nk - 1, M.nj + 1, th), M);
+  if (!M.mixed) k_pgrad_lon<double><<<grid, th, (size_t)th * sizeof(LonFace<double>), s>>>(M);
+  else if (M.col64) k_pgrad_lon<dfl><<<grid, th, (size_t)th * sizeof(LonFace<dfl>), s>>>(M);
+  else k_pgrad_lon<float><<<grid, th, 0, s>>>(M);
   return 0;
 }
 int launch_pgrad_lat(const DevModel &M, cudaStream_t s) {
-  const dim3 grid = zg(cells_blocks(M, M.nk - 1, M.nj, TB(M, TB_PGRAD)), M);
-  if (!M.mixed) k_pgrad_lat<double><<<grid, TB(M, TB_PGRAD), 0, s>>>(M);
-  else if (M.col64) k_pgrad_lat<dfl><<<grid, TB(M, TB_PGRAD), 0, s>>>(M);
-  else k_pgrad_lat<float><<<grid, TB(M, TB_PGRAD), 0, s>>>(M);
+  const int th = TB(M, TB_PGRAD);
+  if (!M.mixed) {
+    EPIC_MARCH_R(double, k_pgrad_lat, M.nk - 1, M.nj, th, s, M);
+    return 0;
+  }
+  const dim3 grid = zg(dim3(epic_blocks((long long)(M.nk - 1) * M.ni, th), M.nj), M);
+  if (M.col64) k_pgrad_lat<dfl, 1><<<grid, th, 0, s>>>(M);
+  else k_pgrad_lat<float, 1><<<grid, th, 0, s>>>(M);
   return 0;
 }
 
@@ -1361,7 +1467,7 @@ int stencil_kernels_init() {
 int launch_divergence_damping(const DevModel &M, cudaStream_t s) {
   if (M.nudiv == 0.) return 0;
   launch_filter_planes(M, M.u, PL_UV_DIS, M.work1, 1, M.nk - 1, 0, s, M.mixed);
-  EPIC_LAUNCH_R(M.mixed, k_divergence, cells_blocks(M, M.nk - 1, M.nj + 1, TB(M, TB_DIAG)), TB(M, TB_DIAG), 0, s, M, M.work1, M.v, PL_UV_DIS, M.work2, 1, M.nk - 1);
+  EPIC_MARCH(M.mixed, k_divergence, M.nk - 1, M.nj + 1, TB(M, TB_DIAG), s, M, M.work1, M.v, PL_UV_DIS, M.work2, 1, M.nk - 1);
   EPIC_LAUNCH_R(M.mixed, k_divdamp_apply, epic_blocks(2LL * (M.nk - 1) * (M.nj + 1) * M.ni, TB(M, TB_UPDATE)), TB(M, TB_UPDATE), 0, s, M);
   return 0;
 }
@@ -1386,7 +1492,7 @@ int launch_diag_filter_u(const DevModel &M, cudaStream_t s) {
   return launch_filter_planes(M, M.u, PL_UV, M.work2, 0, M.nk + 1, 0, s, M.mixed);
 }
 int launch_diag_pv(const DevModel &M, cudaStream_t s) {
-  EPIC_LAUNCH_R(M.mixed, k_pv_interior, cells_blocks(M, M.nk + 1, M.nj, TB(M, TB_DIAG)), TB(M, TB_DIAG), 0, s, M, M.work1);
+  EPIC_MARCH(M.mixed, k_pv_interior, M.nk + 1, M.nj, TB(M, TB_DIAG), s, M, M.work1);
   return 0;
 }
 int launch_diag_pv_poles(const DevModel &M, cudaStream_t s) {
@@ -1395,7 +1501,7 @@ int launch_diag_pv_poles(const DevModel &M, cudaStream_t s) {
   return 0;
 }
 int launch_diag_div(const DevModel &M, cudaStream_t s) {
-  EPIC_LAUNCH_R(M.mixed, k_divergence, cells_blocks(M, M.nk + 1, M.nj + 1, TB(M, TB_DIAG)), TB(M, TB_DIAG), 0, s, M, M.work2, M.v, PL_UV, M.div_uv3, 0, M.nk + 1);
+  EPIC_MARCH(M.mixed, k_divergence, M.nk + 1, M.nj + 1, TB(M, TB_DIAG), s, M, M.work2, M.v, PL_UV, M.div_uv3, 0, M.nk + 1);
   return 0;
 }
 int launch_diag_ri2(const DevModel &M, cudaStream_t s) {

@@ -27,6 +27,40 @@ inline dim3 zg(dim3 g, const DevModel &M) {
   return g;
 }
 
+// Kernels that march up the rows: thread = one column i of one level, ROWS latitude rows from
+// j0 = jlo + blockIdx.y ROWS (per member), carrying what neighbouring rows share -- values already loaded and
+// converted, the products and faces between two rows -- in registers.  As many rows a thread as leave
+// 512 threads per SM, up to 4; a template parameter, so that a single row is straight code.
+inline int march_rows(const DevModel &M, int nkk) {
+  const long long cells = (long long)M.ni * nkk * (M.nj + 1) * (M.nbatch > 1 ? M.nbatch : 1);
+  return cells >= 4LL * 152 * 512 ? 4 : (cells >= 2LL * 152 * 512 ? 2 : 1);
+}
+struct March { int k, i, j0, j1; };
+// rows jlo..jhi; false for a thread without work
+template <int ROWS>
+__device__ __forceinline__ bool march(const DevModel &M, int k0, int nkk, int jlo, int jhi, March &s) {
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, ni = (unsigned)M.ni;
+  s.j0 = jlo + (int)blockIdx.y * ROWS;
+  s.j1 = ROWS == 1 ? s.j0 : min(s.j0 + ROWS - 1, jhi);
+  if (t >= (unsigned)nkk * ni || s.j0 > jhi) return false;
+  s.k = k0 + (int)(t / ni);
+  s.i = 1 + (int)(t - (unsigned)(s.k - k0) * ni);
+  return true;
+}
+#define EPIC_MARCH_R(R, kern, nkk, nrows, block, stream, ...)                                                         \
+  do {                                                                                                                \
+    const int rows_ = march_rows(M, (nkk));                                                                           \
+    const dim3 grid_ = zg(dim3(epic_blocks((long long)(nkk) * M.ni, (block)), epic_blocks((nrows), rows_)), M);       \
+    if (rows_ == 4) kern<R, 4><<<grid_, (block), 0, (stream)>>>(__VA_ARGS__);                                         \
+    else if (rows_ == 2) kern<R, 2><<<grid_, (block), 0, (stream)>>>(__VA_ARGS__);                                    \
+    else kern<R, 1><<<grid_, (block), 0, (stream)>>>(__VA_ARGS__);                                                    \
+  } while (0)
+#define EPIC_MARCH(mixed, kern, nkk, nrows, block, stream, ...)                                                       \
+  do {                                                                                                                \
+    if (mixed) EPIC_MARCH_R(float, kern, nkk, nrows, block, stream, __VA_ARGS__);                                     \
+    else EPIC_MARCH_R(double, kern, nkk, nrows, block, stream, __VA_ARGS__);                                          \
+  } while (0)
+
 // Launch the FP32 (mixed form) or FP64 instantiation of a kernel template over every member
 // (the launcher's `M` sets the batch).
 #define EPIC_LAUNCH_R(mixed, kern, grid, block, smem, stream, ...)                              \
@@ -92,6 +126,8 @@ int launch_advection_prep(const DevModel &M, int phase, cudaStream_t s);
 int column_kernels_init(int nk);
 
 // k_stencil.cu -- horizontal stencils and the time update
+// the row tables (DevModel::rt64, rt32) from the 1-D grid arrays; once per model
+int launch_row_tables(const DevModel &M, cudaStream_t s);
 int launch_zero_tend(const DevModel &M, cudaStream_t s);
 int launch_uv_core(const DevModel &M, cudaStream_t s);
 // uv_pgrad_finite_volume: GZ3's pole rows, then DUDT (lon) and DVDT (lat), independent of each other
