@@ -158,13 +158,10 @@ int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
     case 3: launch_uv_core(M, s); break;
     case 4: launch_uv_drag(M, s); break;
     case 5:
-      launch_meridional_hyperviscosity(M, 2, M.hdry, PL_NONE, s);
-      launch_zonal_hyperviscosity(M, 2, M.hdry, PL_NONE, s);   // then restore_mass, in the same kernel
-      launch_meridional_hyperviscosity(M, 3, M.theta, PL_NONE, s);
-      launch_zonal_hyperviscosity(M, 3, M.theta, PL_NONE, s);
+      launch_hyperviscosity(M, 2, M.hdry, PL_NONE, s);   // then restore_mass, in the same kernel
+      launch_hyperviscosity(M, 3, M.theta, PL_NONE, s);
       if (M.turb) {   // NU_TURB (layers 1..nk on the h-grid), then restore_mass(NU_TURB_INDEX)
-        launch_meridional_hyperviscosity(M, 4, M.nu_turb, PL_NONE, s);
-        launch_zonal_hyperviscosity(M, 4, M.nu_turb, PL_NONE, s);
+        launch_hyperviscosity(M, 4, M.nu_turb, PL_NONE, s);
         launch_restore_nu(M, s);
       }
       break;
@@ -177,17 +174,15 @@ int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
       vertical(M, M.unity, 0, s);
       meridional(M, M.unity, 0, s);
       zonal(M, M.unity, 0, 1, s);
-      launch_advection_prep(M, 1, s);
       vertical(M, M.theta, 1, s);
       meridional(M, M.theta, 1, s);
-      zonal(M, M.theta, 0, M.k_sigma - 1, s);
-      launch_advection_prep(M, 2, s);
+      zonal(M, M.theta, 3, M.k_sigma - 1, s);   // then corrected by UNITY's advection
       if (M.turb) {   // NU_TURB with the same scheme (UNITY stands), before HDRY, epic_flux.c:540-600
-        launch_advection_prep(M, 3, s);
+        launch_advection_prep(M, 1, s);
         vertical(M, M.nu_turb, 3, s);
         meridional(M, M.nu_turb, 3, s);
         zonal(M, M.nu_turb, 2, 1, s);
-        launch_advection_prep(M, 4, s);
+        launch_advection_prep(M, 2, s);
       }
       vertical(M, M.hdry, 2, s);
       meridional(M, M.hdry, 2, s);
@@ -237,10 +232,8 @@ int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
       launch_uv_rotate(M, s);
       break;
     case 15:
-      launch_meridional_hyperviscosity(M, 0, M.u, PL_UV, s);
-      launch_meridional_hyperviscosity(M, 1, M.v, PL_UV, s);
-      launch_zonal_hyperviscosity(M, 0, M.u, PL_UV, s);
-      launch_zonal_hyperviscosity(M, 1, M.v, PL_UV, s);
+      launch_hyperviscosity(M, 0, M.u, PL_UV, s);
+      launch_hyperviscosity(M, 1, M.v, PL_UV, s);
       break;
     case 16:
       launch_diag_filter_v(M, s);
@@ -362,13 +355,10 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
     L.after(3, 0);
   }
   // lane 3: THETA's hyperviscosity; lane 0: HDRY's
-  launch_meridional_hyperviscosity(M3, 3, M.theta, PL_NONE, L[3]);
-  launch_zonal_hyperviscosity(M3, 3, M.theta, PL_NONE, L[3]);
-  launch_meridional_hyperviscosity(M, 2, M.hdry, PL_NONE, L[0]);
-  launch_zonal_hyperviscosity(M, 2, M.hdry, PL_NONE, L[0]);   // then restore_mass, in the same kernel
+  launch_hyperviscosity(M3, 3, M.theta, PL_NONE, L[3]);
+  launch_hyperviscosity(M, 2, M.hdry, PL_NONE, L[0]);   // then restore_mass, in the same kernel
   if (M.turb) {
-    launch_meridional_hyperviscosity(M3, 4, M.nu_turb, PL_NONE, L[3]);
-    launch_zonal_hyperviscosity(M3, 4, M.nu_turb, PL_NONE, L[3]);
+    launch_hyperviscosity(M3, 4, M.nu_turb, PL_NONE, L[3]);
     launch_restore_nu(M, L[3]);
     if (M.turb_v) {
       L.after(0, 3);
@@ -378,18 +368,16 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
     }
   }
   // lane 3: THETA's advection (and NU_TURB's) corrected by UNITY's; lane 0: HDRY's
-  launch_advection_prep(M, 1, L[3]);
   vertical(M3, M.theta, 1, L[3]);
   meridional(M3, M.theta, 1, L[3]);
-  zonal(M3, M.theta, 0, M.k_sigma - 1, L[3]);
   L.after(3, 2);
-  launch_advection_prep(M, 2, L[3]);
+  zonal(M3, M.theta, 3, M.k_sigma - 1, L[3]);
   if (M.turb) {
-    launch_advection_prep(M, 3, L[3]);
+    launch_advection_prep(M, 1, L[3]);
     vertical(M3, M.nu_turb, 3, L[3]);
     meridional(M3, M.nu_turb, 3, L[3]);
     zonal(M3, M.nu_turb, 2, 1, L[3]);
-    launch_advection_prep(M, 4, L[3]);
+    launch_advection_prep(M, 2, L[3]);
   }
   vertical(M, M.hdry, 2, L[0]);
   meridional(M, M.hdry, 2, L[0]);
@@ -433,10 +421,8 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
   if (M.turb && M.turb_v) launch_uv_vdiff(M, L[0]);
   // lane 0: U, lane 1: V; the filtered copies go on in the same lanes
   L.after(1, 0);
-  launch_meridional_hyperviscosity(M, 0, M.u, PL_UV, L[0]);
-  launch_zonal_hyperviscosity(M, 0, M.u, PL_UV, L[0]);
-  launch_meridional_hyperviscosity(M1, 1, M.v, PL_UV, L[1]);
-  launch_zonal_hyperviscosity(M1, 1, M.v, PL_UV, L[1]);
+  launch_hyperviscosity(M, 0, M.u, PL_UV, L[0]);
+  launch_hyperviscosity(M1, 1, M.v, PL_UV, L[1]);
   const cudaEvent_t u_done = L.point(0), v_done = L.point(1);
   launch_diag_filter_u(M, L[0]);
   launch_diag_filter_v(M1, L[1]);

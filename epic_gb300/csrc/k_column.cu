@@ -293,7 +293,9 @@ __global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : 
       for (int k = kf + c.warp; k <= nk; k += c.nw) {
         const long long x = c.base + k * n2;
         const R ffk1 = k == nk ? R(0.) : CT(FF, k + 1);
-        buff[x] = buff[x] + to_d((ffk1 - CT(FF, k)) * dsi(2 * k + 1) * DT);
+        const double before = buff[x];
+        if (kind == 1) M.old[x] = before;   // for the correction by UNITY (advected)
+        buff[x] = before + to_d((ffk1 - CT(FF, k)) * dsi(2 * k + 1) * DT);
       }
   }
 }
@@ -373,7 +375,9 @@ __global__ void __launch_bounds__(CT_THREADS) k_akima_vertical(DevModel M, doubl
     if (c.valid)
       for (int k = kf + c.warp; k <= nk; k += CT_WARPS) {
         const long long x = c.base + k * n2;
-        buff[x] = buff[x] + to_d((CT(FF, k + 1) - CT(FF, k)) * cv<R>(M.dsgth_inv[2 * k + 1]) * DT);
+        const double before = buff[x];
+        if (kind == 1) M.old[x] = before;   // for the correction by UNITY (advected)
+        buff[x] = before + to_d((CT(FF, k + 1) - CT(FF, k)) * cv<R>(M.dsgth_inv[2 * k + 1]) * DT);
       }
   }
 }
@@ -960,24 +964,19 @@ __global__ void k_calc_heating(DevModel M) {
   M.heat3[t] = val;
 }
 
-// advection() bookkeeping around hsu_advection, epic_flux.c:377-435:
-// phase 0: UNITY = 1 over k = 0..nk+1, j = 0..nj, all i;  phase 1: OLD = THETA for k >= k_sigma-1;
-// phase 2: THETA -= OLD*(UNITY-1) for k >= k_sigma-1.
+// advection() bookkeeping around hsu_advection, epic_flux.c:377-435, :569-600:
+// phase 0: UNITY = 1 over k = 0..nk+1, j = 0..nj, all i;  phase 1: OLD = NU_TURB;
+// phase 2: NU_TURB -= OLD*(UNITY-1), floored (THETA's are part of its vertical and zonal passes).
 __global__ void k_advection_prep(DevModel M, int phase) {
   if (epic_member(M)) return;
   const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;   // fewer than n3 < 2^31 cells
   const unsigned w = (unsigned)(M.nj + 1) * (unsigned)M.iadim;
   if (t >= w * (unsigned)(M.nk + 2)) return;
   const unsigned q = t / w;
-  const int k = (int)q;
-  const long long x = M.at(k, 0, 0) + (t - q * w);
+  const long long x = M.at((int)q, 0, 0) + (t - q * w);
   if (phase == 0) M.unity[x] = 1.;
-  else if (phase == 3) M.old[x] = M.nu_turb[x];   // NU_TURB, epic_flux.c:569-600
-  else if (phase == 4) M.nu_turb[x] = dmaxr(1.e-4 * M.kinvisc, M.nu_turb[x] - M.old[x] * (M.unity[x] - 1.));
-  else if (k >= M.k_sigma - 1) {
-    if (phase == 1) M.old[x] = M.theta[x];
-    else M.theta[x] -= M.old[x] * (M.unity[x] - 1.);
-  }
+  else if (phase == 1) M.old[x] = M.nu_turb[x];
+  else M.nu_turb[x] = dmaxr(1.e-4 * M.kinvisc, M.nu_turb[x] - M.old[x] * (M.unity[x] - 1.));
 }
 
 // ---- launchers ----

@@ -10,133 +10,11 @@
 // Compiled without FMA contraction, each filtered row is bit-identical to the reference's.
 #include "device_common.cuh"
 #include "kernels.h"
+#include "row_filter.cuh"
 #include "epic_common.h"
 #include "epic_gb300.h"
 
 namespace epic {
-
-template <class R> struct __align__(2 * sizeof(R)) Cplx { R re, im; };
-
-// Twiddle table layout (pairs), N = ni/2 complex points:
-//   [0, N-1)              four1 isign=+1, stage with half h at offset h-1, entries p = 0..h-1
-//   [N-1, 2N-2)           four1 isign=-1, same layout
-//   [2N-2, 2N-2 + N/2-1)  realft forward post-processing, q = 1..N/2-1
-//   [.., + N/2-1)         realft inverse pre-processing, q = 1..N/2-1
-// The FP64 table holds the recurrence values of the reference; the mixed form reads the same
-// values rounded to float.
-__host__ __device__ inline size_t nr_twiddle_pairs(int ni) {
-  const int N = ni / 2;
-  return 2 * (size_t)(N - 1) + 2 * (size_t)(N / 2 - 1);
-}
-
-// ---- rows by lane groups ----
-//
-// A row belongs to G lanes of one warp (RowShape): 32, or fewer where a row has fewer butterflies, so
-// that a warp instruction is full either way -- a binary64 one costs the pipe the same 16 clocks
-// whatever the number of active lanes.  A block takes `rows` levels of one latitude row, so its rows
-// are all filtered or all not and share what depends on the latitude; a row's passes are separated by
-// __syncwarp alone.  With a block of two warps a row, its passes separated by block barriers and the
-// twiddles copied to shared memory by each, the FP64 form's filters ran at 43-66% of the binary64 pipe
-// with 3 warps resident per scheduler.
-struct RowShape { int G, rows, stride; };   // lanes a row, rows a block, compute-type values a row in shared memory
-struct RowLane {
-  int gl, G, r, k;
-  bool live;   // the row exists (the last block of a launch may have rows to spare)
-};
-__device__ __forceinline__ RowLane row_lane(const RowShape &S, int k0, int kend) {
-  RowLane L;
-  L.G = S.G;
-  L.gl = (int)threadIdx.x & (S.G - 1);
-  L.r = (int)threadIdx.x / S.G;
-  const int k = k0 + (int)blockIdx.y * S.rows + L.r;
-  L.live = k <= kend;
-  L.k = L.live ? k : kend;
-  return L;
-}
-
-template <class R> __device__ __forceinline__ const Cplx<R> *twiddle_table(const DevModel &M);
-template <> __device__ __forceinline__ const Cplx<double> *twiddle_table<double>(const DevModel &M) { return reinterpret_cast<const Cplx<double> *>(M.tw); }
-template <> __device__ __forceinline__ const Cplx<float> *twiddle_table<float>(const DevModel &M) { return reinterpret_cast<const Cplx<float> *>(M.twf); }
-
-// The place of row value e = i-1 among the N complex points in bit-reversed order, which
-// filter_row takes its input in.
-__device__ __forceinline__ int fft_place(int e, int lg) { return 2 * (int)(__brev((unsigned)(e >> 1)) >> (32 - lg)) + (e & 1); }
-__device__ __forceinline__ int fft_log(int ni) { return 31 - __clz(ni / 2); }
-
-// four1's Danielson-Lanczos stages on z (already bit-reversed); tw = this direction's table.  The
-// first stage's only twiddle is (1, 0).
-template <class R>
-__device__ __forceinline__ void four1_stages(Cplx<R> *z, const Cplx<R> *tw, int N, const RowLane &L) {
-  for (int b = L.gl; b < N / 2; b += L.G) {
-    const Cplx<R> u = z[2 * b], v = z[2 * b + 1];
-    z[2 * b] = {u.re + v.re, u.im + v.im};
-    z[2 * b + 1] = {u.re - v.re, u.im - v.im};
-  }
-  __syncwarp();
-  for (int h = 2; h < N; h <<= 1) {
-    const Cplx<R> *wt = tw + (h - 1);
-    for (int b = L.gl; b < N / 2; b += L.G) {
-      const int p = b & (h - 1), i0 = 2 * (b - p) + p, j0 = i0 + h;
-      const Cplx<R> w = wt[p], u = z[i0], v = z[j0];
-      const R tempr = w.re * v.re - w.im * v.im;
-      const R tempi = w.re * v.im + w.im * v.re;
-      z[j0] = {u.re - tempr, u.im - tempi};
-      z[i0] = {u.re + tempr, u.im + tempi};
-    }
-    __syncwarp();
-  }
-}
-
-// Filter a row with weights h(I) = hl[I], I = 1..ni/2+1 (HIGH_LAT(J,I)): z holds the row's values in
-// bit-reversed order (fft_place), on return the filtered row in order, to be multiplied by
-// filter_scale.  Every lane of the warp must call this.  realft forward, the weights and realft
-// inverse (epic_adjust.c:412-456) meet in one pass between the two four1 calls: both split loops and
-// the weights act on the pair (q, N-q).  The reference's factors 1/2 (c1, c2, two per value) and 2/ni
-// are powers of 2, which commute with every rounding in between (the values being far from the ends
-// of the range), so they are left to the one final multiplication.
-template <class R> __device__ __forceinline__ R filter_scale(int ni) { return R(.5) / R(ni); }
-template <class R>
-__device__ __forceinline__ void filter_row(const DevModel &M, Cplx<R> *z, const double *hl, const RowLane &L) {
-  const int N = M.ni / 2, lg = fft_log(M.ni);
-  const Cplx<R> *t4p = twiddle_table<R>(M), *t4m = t4p + (N - 1), *trp = t4p + 2 * (N - 1), *trm = trp + (N / 2 - 1);
-  four1_stages(z, t4p, N, L);
-  for (int q = L.gl; q < N / 2; q += L.G) {
-    if (q == 0) {   // wavenumbers 0 and ni/2 share z[0]; ni/4 has no partner
-      const Cplx<R> a = z[0], b = z[N / 2];
-      const R s = (a.re + a.im) * cv<R>(hl[1]), d = (a.re - a.im) * cv<R>(hl[N + 1]);
-      z[0] = {R(2.) * (s + d), R(2.) * (s - d)};
-      const R h = R(4.) * cv<R>(hl[N / 2 + 1]);
-      if (N > 1) z[N / 2] = {b.re * h, b.im * h};
-      continue;
-    }
-    Cplx<R> a = z[q], b = z[N - q], w = trp[q - 1];
-    R x = a.re + b.re, y = a.im - b.im, s = a.im + b.im, d = a.re - b.re;
-    R ws = w.re * s, id = w.im * d, wd = w.re * d, is = w.im * s;
-    const R hq = cv<R>(hl[q + 1]), hn = cv<R>(hl[N - q + 1]);
-    a = {(x + ws + id) * hq, (y - wd + is) * hq};
-    b = {(x - ws - id) * hn, (-y - wd + is) * hn};
-    w = trm[q - 1];
-    x = a.re + b.re; y = a.im - b.im; s = a.im + b.im; d = a.re - b.re;
-    ws = w.re * s; id = w.im * d; wd = w.re * d; is = w.im * s;
-    z[q] = {x - ws - id, y + wd - is};
-    z[N - q] = {x + ws + id, -y + wd - is};
-  }
-  __syncwarp();
-  for (int k = L.gl; k < N; k += L.G) {
-    const int r = (int)(__brev((unsigned)k) >> (32 - lg));
-    if (r > k) {
-      const Cplx<R> t = z[k];
-      z[k] = z[r];
-      z[r] = t;
-    }
-  }
-  __syncwarp();
-  four1_stages(z, t4m, N, L);
-}
-
-__device__ __forceinline__ bool row_is_filtered(const DevModel &M, int j, int vgrid) {
-  return fabs(M.lat[vgrid ? 2 * j : 2 * j + 1]) >= M.lat0;
-}
 
 // zonal_filter(index, plane, NULL, TWODIM) of planes k0..k0+nplanes-1, from src into dst
 // (dst may equal src).  blockIdx.x = row j + 1, j in -1..nj+1; rows outside the filtered set are
@@ -420,7 +298,7 @@ __global__ void k_varz_filter_rows(DevModel M, double *buff, int sel, int index,
       }
     }
     vz[e] = v;
-    x[filt ? fft_place(e, lg) : e] = dev;
+    x[row_place(filt, e, lg)] = dev;
   }
   __syncwarp();
   if (filt) filter_row<R>(M, reinterpret_cast<Cplx<R> *>(x), (vgrid ? M.high_lat_pv : M.high_lat_h) + M.at2(j, 0), L);
@@ -439,7 +317,7 @@ template <class R>
 __device__ __forceinline__ void zonal_filtered_row(const DevModel &M, const double *buff, int base, int j, R *a, const RowLane &L) {
   const bool filt = row_is_filtered(M, j, 0);   // of the whole block
   const int ni = M.ni, lg = fft_log(ni);
-  for (int e = L.gl; e < ni; e += L.G) a[filt ? fft_place(e, lg) : e] = L.live ? cv<R>(buff[base + e + 1]) : R(1.);
+  for (int e = L.gl; e < ni; e += L.G) a[row_place(filt, e, lg)] = L.live ? cv<R>(buff[base + e + 1]) : R(1.);
   __syncwarp();
   if (!filt) return;
   filter_row<R>(M, reinterpret_cast<Cplx<R> *>(a), M.high_lat_h + M.at2(j, 0), L);
@@ -448,10 +326,20 @@ __device__ __forceinline__ void zonal_filtered_row(const DevModel &M, const doub
   __syncwarp();
 }
 
+// The last word on a cell of an advected field: HDRY (kind 1) takes restore_mass (epic_adjust.c:45-96),
+// which advection() calls next (epic_flux.c:623); THETA (kind 3) loses OLD (UNITY - 1)
+// (epic_flux.c:377-435), OLD being THETA before its advection (the vertical pass keeps it).
+__device__ __forceinline__ double advected(const DevModel &M, int kind, int k, int x, double v) {
+  if (kind == 1) return dmaxr(M.h_min[k], v);
+  if (kind == 3) return v - M.old[x] * (M.unity[x] - 1.);
+  return v;
+}
+
 // Zonal pass of hsu_advection (epic_flux.c:1316-1484), a row per lane group: the fluxes come from a
 // zonally filtered copy of the row, the update goes to the unfiltered field.
-// kind: 0 = interface variable (unity, THETA), 1 = HDRY (layer; u averaged to the layer),
-// 2 = NU_TURB (interface variable with the floor NU_TURB_MIN).
+// kind: 0 = interface variable (unity), 1 = HDRY (layer; u averaged to the layer),
+// 2 = NU_TURB (interface variable with the floor NU_TURB_MIN), 3 = THETA (interface variable, then
+// corrected by UNITY's advection, theta_corrected).
 // Shared arrays by i - 1: a (the filtered row), ff (the flux through the west face), ap (the
 // predicted row); w (the velocity) by i, with the field's own pads.
 template <class R>
@@ -492,17 +380,15 @@ __global__ void k_hsu_zonal(DevModel M, double *buff, int kind, int kstart, RowS
   }
   __syncwarp();
   if (!L.live) return;
-  // HDRY (kind 1): restore_mass (epic_adjust.c:45-96), which advection() calls next
-  // (epic_flux.c:623), on the new value -- the same max per cell, one pass fewer
   for (int e = L.gl; e < ni; e += L.G) {
     const double v = buff[base + e + 1] + to_d((ff[e] - ff[(e + 1) & mask]) * mn1 * DT);
-    write_with_pads(buff, M, base, e + 1, kind == 1 ? dmaxr(M.h_min[k], v) : v);
+    write_with_pads(buff, M, base, e + 1, advected(M, kind, k, base + e + 1, v));
   }
 }
 
 // Zonal pass of akima_advection (epic_flux.c:1826-1932), a row per lane group: the fluxes come from a
 // zonally filtered copy of the row, the update goes to the unfiltered field.
-// kind: 0 = interface variable (unity, THETA), 1 = HDRY (layer; u averaged to the layer).
+// kind: as k_hsu_zonal's (NU_TURB has no floor here).
 // Shared arrays by i - 1: a (the filtered row), dl (the limited slopes), ff (the fluxes).
 template <class R>
 __global__ void k_akima_zonal(DevModel M, double *buff, int kind, int kstart, RowShape S) {
@@ -536,9 +422,9 @@ __global__ void k_akima_zonal(DevModel M, double *buff, int kind, int kstart, Ro
   }
   __syncwarp();
   if (!L.live) return;
-  for (int e = L.gl; e < ni; e += L.G) {   // HDRY (kind 1): restore_mass too
+  for (int e = L.gl; e < ni; e += L.G) {
     const double v = buff[base + e + 1] + to_d((ff[e] - ff[(e + 1) & mask]) * mn1 * DT);
-    write_with_pads(buff, M, base, e + 1, kind == 1 ? dmaxr(M.h_min[k], v) : v);
+    write_with_pads(buff, M, base, e + 1, advected(M, kind, k, base + e + 1, v));
   }
 }
 

@@ -2,6 +2,7 @@
 // named in its comment; thread = one (k, j, i) cell unless stated otherwise.
 #include "device_common.cuh"
 #include "kernels.h"
+#include "row_filter.cuh"
 #include "epic_common.h"
 #include "epic_gb300.h"
 
@@ -209,8 +210,8 @@ __global__ void k_uv_core_u(DevModel M) {
 
 // Row sums in the reference's order (one addition after another) occupy the binary64 pipe for a
 // whole warp instruction per addition whatever the number of active lanes, so the kernels that need
-// them stage several rows in shared memory and sum one row per lane.  Rows lie ni+1 (an odd number
-// of) values apart, which keeps the lanes on different banks.  ROW_SUM_SMEM bounds a block's rows.
+// them stage several rows in shared memory and sum one row per lane.  Rows lie ni+1 or ni+2
+// values apart, which keeps the lanes on different banks or at most two on one.  ROW_SUM_SMEM bounds a block's rows.
 constexpr size_t ROW_SUM_SMEM = 48 * 1024;
 static __device__ __forceinline__ double row_sum(const double *row, int n) {
   double sum = 0.;
@@ -888,15 +889,42 @@ __global__ void k_visc_apply(DevModel M, double *A, int sel, const double *D, in
   write_with_pads(A, M, M.at(c.k, c.j, 0), c.i, A[x] + to_d(cv<R>(M.dt) * cv<R>(sign) * cv<R>(D[x])));
 }
 
+// One row of A (i = 1..ni and its periodic pads) with meridional_hyperviscosity's last order applied:
+// a[i] = A + dt sign D (epic_subgrid.c:650-712), D the zonally filtered second difference.  filter: D is not
+// filtered yet; the row is, in x (ni compute-type values), by the warp's 32 lanes.
+template <class R>
+__device__ __forceinline__ void visc_row(const DevModel &M, const double *A, const double *D, int base, int j, int vgrid, double sign, int filter,
+                                         R *x, double *a, int lane) {
+  const int ni = M.ni, lg = fft_log(ni);
+  const bool filt = filter && row_is_filtered(M, j, vgrid);
+  const R c = cv<R>(M.dt) * cv<R>(sign), scale = filter_scale<R>(ni);
+  if (filt) {
+    for (int e = lane; e < ni; e += 32) x[fft_place(e, lg)] = cv<R>(D[base + e + 1]);
+    __syncwarp();
+    const RowLane L = {lane, 32, 0, 0, true};
+    filter_row<R>(M, reinterpret_cast<Cplx<R> *>(x), (vgrid ? M.high_lat_pv : M.high_lat_h) + M.at2(j, 0), L);
+  }
+  for (int e = lane; e < ni; e += 32) {
+    const R d = filt ? x[e] * scale : cv<R>(D[base + e + 1]);
+    const double v = A[base + e + 1] + to_d(c * d);
+    a[e + 1] = v;
+    if (e == 0) a[ni + 1] = v;
+    if (e == ni - 1) a[0] = v;
+  }
+  __syncwarp();
+}
+
 // zonal_hyperviscosity, epic_subgrid.c:715-808, in the FP64 form: `rows` rows per block, a warp per
 // row at a time; the row means, in the reference's order, by one warp with a row per lane (row_sum).
 // Bound by those additions: with one lane of each row's warp summing it, 4 orders x ni additions a row
-// held the binary64 pipe (71% busy) for 36 us a field at 128x64x20.
-__global__ void __launch_bounds__(256) k_zonal_visc_rows(DevModel M, double *A, int sel, int jbot, int jhalf, int k0, int nkk, int restore, int rows) {
-  if (epic_member(M, A)) return;
-  extern __shared__ double vr[];
+// held the binary64 pipe (71% busy) for 36 us a field at 128x64x20.  The meridional part's filter and
+// last update come first (visc_row), on the row in shared memory: two launches and two passes fewer.
+__global__ void __launch_bounds__(256) k_zonal_visc_rows(DevModel M, double *A, int sel, const double *D, double msign, int filter, int jbot,
+                                                         int jhalf, int k0, int nkk, int restore, int rows) {
+  if (epic_member(M, A, D)) return;
+  extern __shared__ __align__(16) double vr[];
   __shared__ double s_mean[32];
-  const int ni = M.ni, W = ni + 3, lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
+  const int ni = M.ni, W = ni + 2, lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
   const int nr = M.nj - jbot + 1;
   const int row0 = (int)blockIdx.x * rows, nl = min(rows, nr * nkk - row0);
   if (nl <= 0) return;   // a member with fewer rows than the launch
@@ -910,12 +938,11 @@ __global__ void __launch_bounds__(256) k_zonal_visc_rows(DevModel M, double *A, 
   for (int r = w; r < nl; r += nw) {
     int j, k;
     row_at(r, j, k);
-    const int base = M.at(k, j, 0);
-    for (int i = lane; i <= ni + 1; i += 32) a[r * W + i] = h[r * W + i] = A[base + i];
+    visc_row<double>(M, A, D, M.at(k, j, 0), j, jhalf == 0, msign, filter, d + r * W, a + r * W, lane);
+    for (int i = lane; i <= ni + 1; i += 32) h[r * W + i] = a[r * W + i];
   }
   __syncwarp();
   double sign = 1.;
-  bool any_applied = false;
   // fully unrolled so that M.coef[], M.nu[] are indexed by constants (M stays in registers)
 #pragma unroll
   for (int itmp = 2; itmp <= 8; itmp += 2) {
@@ -942,7 +969,6 @@ __global__ void __launch_bounds__(256) k_zonal_visc_rows(DevModel M, double *A, 
       }
     }
     __syncwarp();
-    if (M.nu[itmp] > 0.) any_applied = true;
     sign = -sign;
     double rest = 0.;
 #pragma unroll
@@ -952,22 +978,21 @@ __global__ void __launch_bounds__(256) k_zonal_visc_rows(DevModel M, double *A, 
   }
   // restore (HDRY): restore_mass, which the hyperviscosity step calls next (epic_subgrid.c:240),
   // on the new row -- the same max per cell, one pass fewer
-  if (any_applied || restore)
-    for (int r = w; r < nl; r += nw) {
-      int j, k;
-      row_at(r, j, k);
-      const int base = M.at(k, j, 0);
-      for (int i = lane + 1; i <= ni; i += 32) {
-        const double v = a[r * W + i];
-        write_with_pads(A, M, base, i, restore ? dmaxr(M.h_min[k], v) : v);
-      }
+  for (int r = w; r < nl; r += nw) {
+    int j, k;
+    row_at(r, j, k);
+    const int base = M.at(k, j, 0);
+    for (int i = lane + 1; i <= ni; i += 32) {
+      const double v = a[r * W + i];
+      write_with_pads(A, M, base, i, restore ? dmaxr(M.h_min[k], v) : v);
     }
+  }
 }
 
 // The same in the mixed forms: one warp per row (j, k), blockDim.x / 32 rows per block.  The updated
 // row stays in FP64; the row mean is an FP32 warp reduction.
-__global__ void k_zonal_visc_mixed(DevModel M, double *A, int sel, int jbot, int jhalf, int k0, int restore) {
-  if (epic_member(M, A)) return;
+__global__ void k_zonal_visc_mixed(DevModel M, double *A, int sel, const double *D, double msign, int filter, int jbot, int jhalf, int k0, int restore) {
+  if (epic_member(M, A, D)) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int ni = M.ni, lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
   const int j = jbot + (int)blockIdx.x * nw + w;
@@ -979,8 +1004,7 @@ __global__ void k_zonal_visc_mixed(DevModel M, double *A, int sel, int jbot, int
   double *a = reinterpret_cast<double *>(smraw + w * row_bytes);
   float *hh = reinterpret_cast<float *>(a + (ni + 2)), *d = hh + (ni + 2);
   const unsigned full = 0xffffffffu;
-  for (int i = lane; i <= ni + 1; i += 32) a[i] = A[base + i];
-  __syncwarp();
+  visc_row<float>(M, A, D, (int)base, j, jhalf == 0, msign, filter, d, a, lane);
   // the first second difference is of the field itself: its neighbour differences a(i+1) - a(i) in
   // binary64, one per point (k_d2dy2)
   for (int i = lane; i <= ni; i += 32) hh[i] = d2f(a[i + 1] - a[i]);
@@ -988,7 +1012,6 @@ __global__ void k_zonal_visc_mixed(DevModel M, double *A, int sel, int jbot, int
   const bool taper = fabs(M.lat[2 * j + jhalf]) > M.lat0;
   const double mm = M.m[2 * j + jhalf];
   float sign = 1.f;
-  bool any_applied = false;
   // fully unrolled so that M.coef[], M.nu[] are indexed by constants (M stays in registers)
 #pragma unroll
   for (int itmp = 2; itmp <= 8; itmp += 2) {
@@ -1011,7 +1034,6 @@ __global__ void k_zonal_visc_mixed(DevModel M, double *A, int sel, int jbot, int
       if (M.nu[itmp] > 0.) a[i] += f2d(d2f(M.dt) * sign * v);
     }
     __syncwarp();
-    if (M.nu[itmp] > 0.) any_applied = true;
     sign = -sign;
     double rest = 0.;
 #pragma unroll
@@ -1020,8 +1042,7 @@ __global__ void k_zonal_visc_mixed(DevModel M, double *A, int sel, int jbot, int
     float *t = hh; hh = d; d = t;   // swap roles
   }
   // restore (HDRY): restore_mass too (k_zonal_visc_rows)
-  if (any_applied || restore)
-    for (int i = lane + 1; i <= ni; i += 32) write_with_pads(A, M, base, i, restore ? dmaxr(M.h_min[k], a[i]) : a[i]);
+  for (int i = lane + 1; i <= ni; i += 32) write_with_pads(A, M, base, i, restore ? dmaxr(M.h_min[k], a[i]) : a[i]);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1378,9 +1399,9 @@ static void visc_krange(const DevModel &M, int index, int &k0, int &k1) {
   if (index == 3) k0 = M.k_sigma - 1;
 }
 
-int launch_meridional_hyperviscosity(const DevModel &M, int index, double *var, int sel, cudaStream_t s) {
-  double rest4 = M.nu[4] + M.nu[6] + M.nu[8];
-  if (!(rest4 > 0.)) return 0;
+// meridional_hyperviscosity up to its last order's second difference, which is left in `last` (with its
+// sign) for the zonal kernel to filter and apply
+static void launch_meridional_hyperviscosity(const DevModel &M, int index, double *var, int sel, cudaStream_t s, double *&last, double &last_sign) {
   int k0, k1;
   visc_krange(M, index, k0, k1);
   const int nkk = k1 - k0 + 1;
@@ -1412,46 +1433,54 @@ int launch_meridional_hyperviscosity(const DevModel &M, int index, double *var, 
                     nkk, cur_src == var);
     }
     src_sel = PL_NONE;
+    double rest = 0.;
+    for (int q = itmp + 2; q <= 8; q += 2) rest += M.nu[q];
+    if (!(rest > 0.)) {   // the last order, which is always applied
+      last = dst;
+      last_sign = sign;
+      return;
+    }
     if (M.nu[itmp] > 0.) {
       // k_d2dy2 / k_d2dy2_pair wrote every row of dst with its pads
       launch_filter_planes(M, dst, PL_NONE, dst, k0, nkk, vgrid, s, M.mixed, 0, 1);
       EPIC_LAUNCH_R(M.mixed, k_visc_apply, cells_blocks(M, nkk, vgrid ? M.nj : M.nj + 1, TB(M, TB_VISC)), TB(M, TB_VISC), 0, s, M, var, sel, dst, vgrid, sign, k0, nkk);
     }
     sign = -sign;
-    double rest = 0.;
-    for (int q = itmp + 2; q <= 8; q += 2) rest += M.nu[q];
-    if (!(rest > 0.)) break;
     cur_src = dst;
     which ^= 1;
   }
-  return 0;
 }
 
 constexpr size_t VISC_ROWS_SMEM = 101 * 1024;   // two blocks per SM; 4 rows of EPIC_MAX_NI fit
 
 // index 2 (HDRY) applies restore_mass as well (in the kernel, or alone without hyperviscosity)
-int launch_zonal_hyperviscosity(const DevModel &M, int index, double *var, int sel, cudaStream_t s) {
-  if (M.ni < 2 || !(M.nu[4] + M.nu[6] + M.nu[8] > 0.)) return index == 2 ? launch_restore_mass(M, s) : 0;
+int launch_hyperviscosity(const DevModel &M, int index, double *var, int sel, cudaStream_t s) {
+  if (!(M.nu[4] + M.nu[6] + M.nu[8] > 0.)) return index == 2 ? launch_restore_mass(M, s) : 0;
   int k0, k1;
   visc_krange(M, index, k0, k1);
+  double *D = nullptr, msign = 1.;
+  launch_meridional_hyperviscosity(M, index, var, sel, s, D, msign);
+  // the tensor cores filter whole planes; else the zonal kernel filters each row itself
+  const int filter = !(M.mixed && filter_gemm_usable(M));
+  if (!filter) launch_filter_planes(M, D, PL_NONE, D, k0, k1 - k0 + 1, index == 1, s, 1, 0, 1);
   const int jbot = index == 1 ? 1 : 0, jhalf = index == 1 ? 0 : 1;
   const int nrows = M.nj - jbot + 1, nkk = k1 - k0 + 1;
   if (!M.mixed) {
     // rows per block: a power of 2, the fewest that leave two blocks per SM or fewer (each order's
     // sums are one chain of ni additions per block), up to a warp's lanes and VISC_ROWS_SMEM
-    const size_t row_bytes = (size_t)3 * (M.ni + 3) * sizeof(double);
+    const size_t row_bytes = (size_t)3 * (M.ni + 2) * sizeof(double);
     const long long total = (long long)nrows * nkk * (M.nbatch > 1 ? M.nbatch : 1);
     int rows = 4;
     while (rows < 32 && total > 2LL * 152 * rows && 2 * rows * row_bytes <= VISC_ROWS_SMEM) rows *= 2;
-    k_zonal_visc_rows<<<zg(epic_blocks((long long)nrows * nkk, rows), M), 256, rows * row_bytes, s>>>(M, var, sel, jbot, jhalf, k0, nkk,
-                                                                                                     index == 2, rows);
+    k_zonal_visc_rows<<<zg(epic_blocks((long long)nrows * nkk, rows), M), 256, rows * row_bytes, s>>>(M, var, sel, D, msign, filter, jbot,
+                                                                                                     jhalf, k0, nkk, index == 2, rows);
     return 0;
   }
   const size_t row_bytes = (size_t)(M.ni + 2) * (sizeof(double) + 2 * sizeof(float));
   int rows = (int)((40 * 1024) / row_bytes);
   rows = rows < 1 ? 1 : (rows > 4 ? 4 : rows);
   dim3 grid((nrows + rows - 1) / rows, nkk);
-  k_zonal_visc_mixed<<<zg(grid, M), 32 * rows, rows * row_bytes, s>>>(M, var, sel, jbot, jhalf, k0, index == 2);
+  k_zonal_visc_mixed<<<zg(grid, M), 32 * rows, rows * row_bytes, s>>>(M, var, sel, D, msign, filter, jbot, jhalf, k0, index == 2);
   return 0;
 }
 

@@ -140,8 +140,8 @@ int launch_hsu_meridional(const DevModel &M, double *buff, int kind, cudaStream_
 int launch_akima_vertical(const DevModel &M, double *buff, int kind, cudaStream_t s);
 int launch_akima_meridional(const DevModel &M, double *buff, int kind, cudaStream_t s);
 int launch_akima_zonal(const DevModel &M, double *buff, int kind, int kstart, cudaStream_t s);
-int launch_meridional_hyperviscosity(const DevModel &M, int index, double *var, int sel, cudaStream_t s);
-int launch_zonal_hyperviscosity(const DevModel &M, int index, double *var, int sel, cudaStream_t s);
+// meridional, then zonal hyperviscosity; index: 0 = U, 1 = V, 2 = HDRY (with restore_mass), 3 = THETA, 4 = NU_TURB
+int launch_hyperviscosity(const DevModel &M, int index, double *var, int sel, cudaStream_t s);
 int stencil_kernels_init();
 int launch_divergence_damping(const DevModel &M, cudaStream_t s);
 // the time update: which scheme coefficients this step takes (decide: from the tendency planes of
