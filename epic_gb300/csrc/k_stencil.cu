@@ -220,9 +220,13 @@ static __device__ __forceinline__ double row_sum(const double *row, int n) {
   return sum;
 }
 // levels per block of a kernel that sums `rows` rows of each, one per lane of a warp
+// of which there are nk+1: no more than it takes to have a block per SM
 static int row_sum_levels(const DevModel &M, int rows) {
   const int fit = (int)(ROW_SUM_SMEM / ((size_t)rows * (M.ni + 1) * sizeof(double)));
-  return fit < 1 ? 1 : (fit > 32 / rows ? 32 / rows : fit);
+  const int want = (int)(((long long)(M.nk + 1) * (M.nbatch > 1 ? M.nbatch : 1) + 151) / 152);
+  int lv = fit > 32 / rows ? 32 / rows : fit;
+  lv = lv > want ? want : lv;
+  return lv < 1 ? 1 : lv;
 }
 
 // Pole boundary rows of GZ3 (zonal means of the adjacent row), epic_timestep.c:930-998.
@@ -234,6 +238,7 @@ __global__ void __launch_bounds__(256) k_gz_pole_rows(DevModel M, int lv) {
   extern __shared__ double rows[];   // [lv][2][ni+1]: rows 0 and nj of each level
   __shared__ double avg[32];
   const int ni = M.ni, k0 = (int)blockIdx.x * lv, nl = min(lv, M.nk + 1 - k0);
+#pragma unroll 4
   for (int t = (int)threadIdx.x; t < 2 * nl * ni; t += (int)blockDim.x) {
     const int r = t / ni, i = t - r * ni;
     rows[r * (ni + 1) + i] = M.gz3[M.at(k0 + (r >> 1), (r & 1) ? M.nj : 0, i + 1)];
@@ -923,6 +928,7 @@ __global__ void __launch_bounds__(256) k_zonal_visc_rows(DevModel M, double *A, 
                                                          int jhalf, int k0, int nkk, int restore, int rows) {
   if (epic_member(M, A, D)) return;
   extern __shared__ __align__(16) double vr[];
+  if (filter) prefetch_twiddles<double>(M);
   __shared__ double s_mean[32];
   const int ni = M.ni, W = ni + 2, lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
   const int nr = M.nj - jbot + 1;
@@ -994,6 +1000,7 @@ __global__ void __launch_bounds__(256) k_zonal_visc_rows(DevModel M, double *A, 
 __global__ void k_zonal_visc_mixed(DevModel M, double *A, int sel, const double *D, double msign, int filter, int jbot, int jhalf, int k0, int restore) {
   if (epic_member(M, A, D)) return;
   extern __shared__ __align__(16) unsigned char smraw[];
+  if (filter) prefetch_twiddles<float>(M);
   const int ni = M.ni, lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
   const int j = jbot + (int)blockIdx.x * nw + w;
   const int k = k0 + (int)blockIdx.y;
@@ -1105,6 +1112,7 @@ __global__ void __launch_bounds__(256) k_pv_poles(DevModel M, int lv) {
   const int ni = M.ni, J = M.nj, k0 = (int)blockIdx.x * lv, nl = min(lv, M.nk + 1 - k0);
   const double *UU = M.u + plane_offset(M, PL_UV);
   const double *HH = M.h3;
+#pragma unroll 4
   for (int t = (int)threadIdx.x; t < 4 * nl * ni; t += (int)blockDim.x) {
     const int r = t / ni, i = t - r * ni;
     const double v = ((r & 1) ? HH : UU)[M.at(k0 + (r >> 2), (r & 2) ? J : 0, i + 1)];
@@ -1358,11 +1366,11 @@ int launch_akima_meridional(const DevModel &M, double *buff, int kind, cudaStrea
   return 0;
 }
 
-// The meridional Hsu pass has three forms that give the same bits.  The tile (k_hsu_merid_tile) where
-// its four arrays of nj+2 rows fit MERID_SMEM with 32 columns, or 16 or 8 (64 bytes of a row); the march
-// (k_hsu_meridional, one thread per (k, i, member) walking nj+1 rows) once those threads fill the GPU
-// (large batches); else the four passes, whose threads cover every cell.  The tuning table's
-// TB_HSU_MERID_VARIANT entry overrides the choice (1 march, 2 four passes).
+// The meridional Hsu pass has three forms that give the same bits.  The tile (k_hsu_merid_tile) of 32, 16
+// or 8 columns (64 bytes of a row) where its four arrays of nj+2 rows fit MERID_SMEM, as wide as leaves two
+// blocks per SM; the march (k_hsu_meridional, one thread per (k, i, member) walking nj+1 rows) once those
+// threads fill the GPU (large batches); else the four passes, whose threads cover every cell.  The
+// tuning table's TB_HSU_MERID_VARIANT entry overrides the choice (1 march, 2 four passes).
 constexpr long long HSU_FUSED_MIN_THREADS = 65536;
 constexpr size_t MERID_SMEM = 100 * 1024;   // two blocks per SM
 
@@ -1379,6 +1387,7 @@ int launch_hsu_meridional(const DevModel &M, double *buff, int kind, cudaStream_
   }
   const size_t col = (size_t)4 * (M.nj + 2) * (M.mixed ? sizeof(float) : sizeof(double));
   int TC = 32;
+  while (TC > 8 && (long long)epic_blocks(M.ni, TC) * nkk * (M.nbatch > 1 ? M.nbatch : 1) < 2 * 152) TC /= 2;
   while (TC >= 8 && TC * col > MERID_SMEM) TC /= 2;
   if (variant == 0 && TC >= 8) {
     EPIC_LAUNCH_R(M.mixed, k_hsu_merid_tile, dim3(epic_blocks(M.ni, TC), nkk), 256, TC * col, s, M, buff, kind, k0, TC);
@@ -1416,7 +1425,8 @@ static void launch_meridional_hyperviscosity(const DevModel &M, int index, doubl
   double sign = 1.;
   // the first two passes in one kernel when nothing is applied between them
   const size_t pair_col = (size_t)nrows * (M.mixed ? sizeof(float) : sizeof(double));
-  const int pair_tc = 16 * pair_col <= 48 * 1024 ? 16 : 8;
+  const long long strips = (long long)epic_blocks(M.ni, 16) * nkk * (M.nbatch > 1 ? M.nbatch : 1);
+  const int pair_tc = 16 * pair_col <= 48 * 1024 && strips >= 2 * 152 ? 16 : 8;
   const bool pair = !(M.nu[2] > 0.) && M.nu[4] + M.nu[6] + M.nu[8] > 0. && pair_tc * pair_col <= 48 * 1024;
   for (int itmp = 2; itmp <= 8; itmp += 2) {
     double *dst = bufs[which];

@@ -256,34 +256,59 @@ __global__ void k_sa_prep(DevModel M) {
 // The wavefronts k + j + i = d of the in-place NU_TURB update: the three gradient terms from the
 // neighbours (new at k-1, j-1, i-1; old at k+1, j+1, i+1), summed in the reference's order between
 // the point's own terms.  One cluster of blocks per model, a cluster barrier between fronts: bounded by
-// that chain of nk + nj + ni - 2 fronts (one L2 round trip, the arithmetic and a barrier each), where a
-// launch per front cost 5.5 us (210 launches a step at 128x64x20).  What other blocks have written is
-// read past L1; the old values are what they were when the kernel began, wherever they are cached.
+// that chain of nk + nj + ni - 2 fronts, where a launch per front cost 5.5 us (210 launches a step at
+// 128x64x20).  A thread keeps one (k, j) pair and walks along i with the fronts, so that a front waits
+// only for the two new neighbours of other threads (read past L1, an L2 round trip), the arithmetic that
+// needs them and the barrier: the rest -- old neighbours, which no front before the next but one changes,
+// and the point's own terms -- is loaded a front ahead, its own last value is in a register.  Pairs beyond
+// the cluster's threads take further sweeps over their share with everything loaded in the front.
 constexpr int SA_THREADS = 128;
+struct SaPoint { double north, east, above, w0, w1, w2, w3; };
 __global__ void __launch_bounds__(SA_THREADS) k_sa_waves(DevModel M) {
   if (epic_member(M)) return;   // all blocks of a cluster are one member's
-  const int nr = M.nj + 1, pairs = (M.nk - 1) * nr, ni = M.ni;
-  const double cb2 = 0.622, sigma = 2. / 3.;
+  const int nr = M.nj + 1, pairs = (M.nk - 1) * nr, ni = M.ni, n2 = (int)M.n2, row = M.iadim;
+  const double c = 0.622 / (2. / 3.), floor_nu = 1.e-4 * M.kinvisc;   // cb2 / sigma
   double *NU = M.nu_turb;
   const int me = (int)(threadIdx.x * gridDim.x + blockIdx.x), all = (int)(gridDim.x * blockDim.x);   // fronts spread over the blocks
+  auto load = [&](int x) {
+    SaPoint p;
+    p.north = NU[x + row]; p.east = NU[x + 1]; p.above = NU[x + n2];
+    p.w0 = M.work0[x]; p.w1 = M.work1[x]; p.w2 = M.work2[x]; p.w3 = M.work3[x];
+    return p;
+  };
+  auto update = [&](const SaPoint &p, int x, int jj, double nu, double west) {
+    const double below = __ldcg(NU + x - n2), south = __ldcg(NU + x - row);
+    const double g1 = half_of((p.east - west) * M.m[jj + 1]);
+    const double g2 = half_of((p.north - nu) * M.n[jj + 2] + (nu - south) * M.n[jj]);
+    const double g3 = (below - p.above) * p.w2;
+    double dnudt = p.w0;
+    dnudt += c * (g1 * g1);   // pow(g, 2.), the correctly rounded square
+    dnudt += c * (g2 * g2);
+    dnudt += c * (g3 * g3);
+    dnudt -= p.w1;
+    dnudt -= p.w3;
+    const double v = dmaxr(floor_nu, nu + M.dt * dnudt);
+    NU[x] = v;
+    return v;
+  };
+  const bool mine = me < pairs;
+  const int k0 = mine ? 1 + me / nr : 1, j0 = mine ? me - (k0 - 1) * nr : 0, x0 = M.at(k0, j0, 0);
+  SaPoint next = {};
+  double nu = 0., west = 0.;   // the pair's value at its next i, and the one just written before it
+  if (mine) { next = load(x0 + 1); nu = NU[x0 + 1]; west = NU[x0]; }
   for (int d = 2; d <= M.nk - 1 + M.nj + ni; d++) {
-    for (int p = me; p < pairs; p += all) {
-      const int k = 1 + p / nr, j = p - (k - 1) * nr, i = d - k - j;
-      if (i < 1 || i > ni) continue;
-      const int x = M.at(k, j, i), n2 = (int)M.n2, row = M.iadim, jj = 2 * j;
-      const double below = __ldcg(NU + x - n2), south = __ldcg(NU + x - row), west = __ldcg(NU + x - 1);
-      const double nu = __ldcg(NU + x), north = NU[x + row], east = NU[x + 1], above = NU[x + n2];
-      const double w0 = M.work0[x], w1 = M.work1[x], w2 = M.work2[x], w3 = M.work3[x];
-      const double g1 = half_of((east - west) * M.m[jj + 1]);
-      const double g2 = half_of((north - nu) * M.n[jj + 2] + (nu - south) * M.n[jj]);
-      const double g3 = (below - above) * w2;
-      double dnudt = w0;
-      dnudt += (cb2 / sigma) * (g1 * g1);   // pow(g, 2.), the correctly rounded square
-      dnudt += (cb2 / sigma) * (g2 * g2);
-      dnudt += (cb2 / sigma) * (g3 * g3);
-      dnudt -= w1;
-      dnudt -= w3;
-      NU[x] = dmaxr(1.e-4 * M.kinvisc, nu + M.dt * dnudt);
+    const int i = d - k0 - j0;
+    if (mine && i >= 1 && i <= ni) {
+      const SaPoint p = next;
+      const double now = nu;
+      if (i < ni) { next = load(x0 + i + 1); nu = p.east; }
+      west = update(p, x0 + i, 2 * j0, now, west);
+    }
+    for (int q = me + all; q < pairs; q += all) {
+      const int k = 1 + q / nr, j = q - (k - 1) * nr, iq = d - k - j;
+      if (iq < 1 || iq > ni) continue;
+      const int x = M.at(k, j, iq);
+      update(load(x), x, 2 * j, __ldcg(NU + x), __ldcg(NU + x - 1));
     }
     __syncwarp();
     asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");

@@ -48,6 +48,15 @@ template <class R> __device__ __forceinline__ const Cplx<R> *twiddle_table(const
 template <> __device__ __forceinline__ const Cplx<double> *twiddle_table<double>(const DevModel &M) { return reinterpret_cast<const Cplx<double> *>(M.tw); }
 template <> __device__ __forceinline__ const Cplx<float> *twiddle_table<float>(const DevModel &M) { return reinterpret_cast<const Cplx<float> *>(M.twf); }
 
+// The twiddles into L1, by the lanes of each warp, ahead of the stages that read them: each stage waits for
+// its twiddles between two __syncwarp, an L2 round trip a stage for the first rows of an SM otherwise.
+template <class R>
+__device__ __forceinline__ void prefetch_twiddles(const DevModel &M) {
+  const char *t = reinterpret_cast<const char *>(twiddle_table<R>(M));
+  const int bytes = (int)(nr_twiddle_pairs(M.ni) * sizeof(Cplx<R>));
+  for (int b = 128 * ((int)threadIdx.x & 31); b < bytes; b += 128 * 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(t + b));
+}
+
 // The place of row value e = i-1 among the N complex points in bit-reversed order, which
 // filter_row takes its input in.
 __device__ __forceinline__ int fft_place(int e, int lg) { return 2 * (int)(__brev((unsigned)(e >> 1)) >> (32 - lg)) + (e & 1); }
