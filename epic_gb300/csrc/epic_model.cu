@@ -250,14 +250,26 @@ int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
     case 19: launch_store_pgrad_vars(M, s); break;   // after stage 11: what the pressure gradient reads
     // the turbulence closure (epic_subgrid.c)
     case 21: if (M.turb) launch_source_sink_turb(M, s); break;
-    case 22: if (M.turb) launch_scalar_hdiff(M, s); break;
+    case 22:
+      if (M.turb) {
+        launch_theta_hdiff(M, s);
+        launch_nu_hdiff(M, s);
+      }
+      break;
     case 23:
       if (M.turb) {
         launch_tau_wall_h(M, M.work0, s);
-        launch_scalar_vdiff(M, M.work0, s);
+        launch_theta_vdiff(M, s);
+        launch_nu_vdiff(M, M.work0, s);
       }
       break;
-    case 24: if (M.turb) launch_uv_hdiff(M, s); break;
+    case 24:
+      if (M.turb) {
+        launch_uvh_coef(M, s);
+        for (int q = 0; q < 4; q++) launch_uvh_filter(M, q, s);
+        launch_uvh_apply(M, s);
+      }
+      break;
     case 25: if (M.turb) launch_uv_vdiff(M, s); break;
     default: return set_error(EPIC_ERR_ARG, "unknown stage %d", stage);
   }
@@ -351,21 +363,30 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
     if (M.turb_v) launch_tau_wall_h(M, M2.work0, L[2]);
     launch_source_sink_turb(M, L[0]);
     L.after(0, 1);   // the subgrid diffusion's set_p2etc rewrites P3 and H3, which lane 1 reads
-    if (M.turb_h) launch_scalar_hdiff(M, L[0]);
     L.after(3, 0);
+    if (M.turb_h) {
+      launch_theta_hdiff(M, L[0]);
+      launch_nu_hdiff(M3, L[3]);
+    }
+    L.after(2, 0);
   }
-  // lane 3: THETA's hyperviscosity; lane 0: HDRY's
-  launch_hyperviscosity(M3, 3, M.theta, PL_NONE, L[3]);
-  launch_hyperviscosity(M, 2, M.hdry, PL_NONE, L[0]);   // then restore_mass, in the same kernel
+  // lane 0: HDRY's hyperviscosity, lane 3 THETA's (with the closure lane 2 THETA's, lane 3 NU_TURB's)
   if (M.turb) {
+    launch_hyperviscosity(M2, 3, M.theta, PL_NONE, L[2]);
     launch_hyperviscosity(M3, 4, M.nu_turb, PL_NONE, L[3]);
     launch_restore_nu(M, L[3]);
+  } else {
+    launch_hyperviscosity(M3, 3, M.theta, PL_NONE, L[3]);
+  }
+  launch_hyperviscosity(M, 2, M.hdry, PL_NONE, L[0]);   // then restore_mass, in the same kernel
+  if (M.turb) {
+    L.after(0, 2);
+    L.after(3, 2);
     if (M.turb_v) {
-      L.after(0, 3);
-      L.after(0, 2);
-      launch_scalar_vdiff(M, M2.work0, L[0]);
-      L.after(3, 0);
+      launch_theta_vdiff(M, L[0]);
+      launch_nu_vdiff(M, M2.work0, L[3]);
     }
+    L.after(3, 0);
   }
   // lane 3: THETA's advection (and NU_TURB's) corrected by UNITY's; lane 0: HDRY's
   vertical(M3, M.theta, 1, L[3]);
@@ -411,7 +432,18 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
   L.after(0, 2);
   launch_pgrad_lat(M, L[0]);
   L.after(0, 1);
-  if (M.turb && M.turb_h) launch_uv_hdiff(M, L[0]);
+  if (M.turb && M.turb_h) {
+    L.after(2, 0);
+    launch_uvh_filter(M, 2, L[2]);
+    launch_uvh_filter(M, 3, L[2]);
+    launch_uvh_coef(M, L[0]);
+    L.after(1, 0);
+    launch_uvh_filter(M, 0, L[0]);
+    launch_uvh_filter(M, 1, L[1]);
+    L.after(0, 1);
+    L.after(0, 2);
+    launch_uvh_apply(M, L[0]);
+  }
   launch_divergence_damping(M, L[0]);
   L.after(0, 3);                   // DZDT3 reads the winds before their update
   launch_uv_update(M, L[0]);

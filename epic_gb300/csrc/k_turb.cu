@@ -651,24 +651,36 @@ __global__ void k_uvh_coef(DevModel M) {
 }
 
 // TAU12 on the polar rows, per layer: vorticity(ON_SIGMATHETA, RELATIVE) there (epic_funcs_diag.c:
-// 4279-4290, 4357-4379) times minus the row mean of COEFFD H_RHO, the sums in the reference's order
-__global__ void k_uvh_poles(DevModel M) {
+// 4279-4290, 4357-4379) times minus the row mean of COEFFD H_RHO, the sums in the reference's order.  One
+// block per layer: the four rows staged in shared memory, a row summed per lane (one thread reading both
+// rows of a pole from global memory took 43 us at 128x64x20).
+__global__ void __launch_bounds__(128) k_uvh_poles(DevModel M) {
   if (epic_member(M)) return;
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= 2 * (M.nk - 1)) return;
-  const int k = 1 + t / 2, north = t & 1;
-  const double *uu = M.work2, *cd = M.work0, *hr = M.work1;
-  const int ni = M.ni, jr = north ? M.nj : 0;
-  double ze = 0., coeff = 0.;
-  for (int i = 1; i <= ni; i++) {
-    if (north) ze += uu[M.at(k, jr, i)];
-    else ze -= uu[M.at(k, jr, i)];
+  extern __shared__ double rows[];   // [4][ni+1]: -UU(0), COEFFD H_RHO(0), UU(nj), COEFFD H_RHO(nj)
+  __shared__ double sum[4];
+  const int k = 1 + (int)blockIdx.x, ni = M.ni;
+#pragma unroll 4
+  for (int t = (int)threadIdx.x; t < 4 * ni; t += (int)blockDim.x) {
+    const int r = t / ni, i = t - r * ni, x = M.at(k, (r & 2) ? M.nj : 0, i + 1);
+    rows[r * (ni + 1) + i] = (r & 1) ? M.work0[x] * M.work1[x] : (r == 0 ? -M.work2[x] : M.work2[x]);
   }
-  if (north) ze *= M.mn[2 * (M.nj + 1)] / (M.m[2 * M.nj + 1] * (double)ni);
-  else ze *= M.mn[0] / ((M.m[1]) * (double)ni);
-  for (int i = 1; i <= ni; i++) coeff += cd[M.at(k, jr, i)] * hr[M.at(k, jr, i)];
-  coeff /= ni;
-  M.turb_pole[2 * k + north] = ze * -coeff;
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    const double *row = rows + threadIdx.x * (ni + 1);
+    double s = 0.;
+#pragma unroll 8
+    for (int i = 0; i < ni; i++) s += row[i];
+    sum[threadIdx.x] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    const int north = (int)threadIdx.x;
+    double ze = sum[2 * north], coeff = sum[2 * north + 1];
+    if (north) ze *= M.mn[2 * (M.nj + 1)] / (M.m[2 * M.nj + 1] * (double)ni);
+    else ze *= M.mn[0] / ((M.m[1]) * (double)ni);
+    coeff /= ni;
+    M.turb_pole[2 * k + north] = ze * -coeff;
+  }
 }
 
 struct Stress { double t11, t22, t33; };
@@ -881,9 +893,11 @@ static int laplacian_step(const DevModel &M, double *var, const double *dc, int 
   return 0;
 }
 
-int launch_scalar_hdiff(const DevModel &M, cudaStream_t s) {
+int launch_theta_hdiff(const DevModel &M, cudaStream_t s) {
   laplacian_step(M, M.theta, M.dc_theta, 0, M.k_sigma - 1, s);
-  launch_set_p2etc(M, 1, s);
+  return launch_set_p2etc(M, 1, s);
+}
+int launch_nu_hdiff(const DevModel &M, cudaStream_t s) {
   laplacian_step(M, M.nu_turb, nullptr, 1, 1, s);
   return launch_restore_nu(M, s);
 }
@@ -899,20 +913,29 @@ int launch_tau_wall_h(const DevModel &M, double *tw, cudaStream_t s) {
   return 0;
 }
 
-int launch_scalar_vdiff(const DevModel &M, const double *tw, cudaStream_t s) {
-  launch_vdiff(M, VD_THETA, tw, s);
-  launch_set_p2etc(M, 1, s);
+int launch_theta_vdiff(const DevModel &M, cudaStream_t s) {
+  launch_vdiff(M, VD_THETA, nullptr, s);
+  return launch_set_p2etc(M, 1, s);
+}
+int launch_nu_vdiff(const DevModel &M, const double *tw, cudaStream_t s) {
   launch_vdiff(M, VD_NU, tw, s);
   return launch_restore_nu(M, s);
 }
 
-int launch_uv_hdiff(const DevModel &M, cudaStream_t s) {
+int launch_uvh_coef(const DevModel &M, cudaStream_t s) {
   k_uvh_coef<<<zg(nblk((long long)(M.nj + 1) * M.iadim * (M.nk - 1), 256), M), 256, 0, s>>>(M);
-  launch_filter_planes(M, M.work0, PL_NONE, M.work0, 1, M.nk - 1, 0, s);
-  launch_filter_planes(M, M.work1, PL_NONE, M.work1, 1, M.nk - 1, 0, s);
-  launch_filter_planes(M, M.u, PL_UV_DIS, M.work2, 1, M.nk - 1, 0, s);
-  launch_filter_planes(M, M.v, PL_UV_DIS, M.work3, 1, M.nk - 1, 1, s);
-  k_uvh_poles<<<zg(nblk(2LL * (M.nk - 1), 64), M), 64, 0, s>>>(M);
+  return 0;
+}
+int launch_uvh_filter(const DevModel &M, int which, cudaStream_t s) {
+  switch (which) {
+    case 0: return launch_filter_planes(M, M.work0, PL_NONE, M.work0, 1, M.nk - 1, 0, s);
+    case 1: return launch_filter_planes(M, M.work1, PL_NONE, M.work1, 1, M.nk - 1, 0, s);
+    case 2: return launch_filter_planes(M, M.u, PL_UV_DIS, M.work2, 1, M.nk - 1, 0, s);
+    default: return launch_filter_planes(M, M.v, PL_UV_DIS, M.work3, 1, M.nk - 1, 1, s);
+  }
+}
+int launch_uvh_apply(const DevModel &M, cudaStream_t s) {
+  k_uvh_poles<<<zg(M.nk - 1, M), 128, (size_t)4 * (M.ni + 1) * sizeof(double), s>>>(M);
   k_uvh_apply<<<zg(nblk((long long)(M.nk - 1) * (M.nj + 1) * M.ni, 128), M), 128, 0, s>>>(M);
   return 0;
 }
