@@ -397,7 +397,11 @@ __global__ void k_restore_mass(DevModel M) {
 // set_p2etc, epic_funcs_diag.c:3352-3569 (nq = 0: H2 is HDRY, PDRY3 is P3, HDRY3 is H3).
 // Shared arrays: P (interface pressure), HL (get_h at the layers), TH (THETA), PP (P^(kappa+1),
 // each interface's power computed once for the two layers that share it).
-__global__ void __launch_bounds__(CT_THREADS_WIDE) k_set_p2etc(DevModel M, int update_theta) {
+// THREADS: 256 or 512 a tile (tile_threads), 32 warps per SM either way: the long integer chains of the
+// logarithms, exponentials and quotients want warps more than registers.  With the 114-128 registers the
+// compiler takes by itself (16 warps), 3 steps of 256x128x32 took 17.8 ms; with 64 and a few spills 16.2.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_set_p2etc(DevModel M, int update_theta) {
   if (epic_member(M)) return;
   extern __shared__ double sm[];
   __shared__ double s_lp[32];
@@ -493,7 +497,8 @@ __global__ void __launch_bounds__(CT_THREADS_WIDE) k_set_p2etc(DevModel M, int u
 // the first DZDT3 terms.  Shared arrays: P, R (RHO3), T3, LG (log of successive pressure
 // ratios), GZ (the Leslie-Purser increments, then the running sum in place), Q (P/RHO3, each
 // level's quotient once for the four increments that read it).
-__global__ void __launch_bounds__(CT_THREADS_WIDE) k_pgrad_vars_column(DevModel M) {
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_pgrad_vars_column(DevModel M) {
   if (epic_member(M)) return;
   extern __shared__ double sm[];
   __shared__ double s_rho2_1[32];
@@ -986,11 +991,12 @@ static inline unsigned ncol_blocks(const DevModel &M, int th) { return epic_bloc
 int launch_source_sink(const DevModel &M, cudaStream_t s) { k_source_sink<<<zg(ncol_blocks(M, TB(M, TB_COLUMN)), M), TB(M, TB_COLUMN), 0, s>>>(M); return 0; }
 static inline unsigned ntile_blocks(const DevModel &M) { return epic_blocks((long long)(M.nj + 1) * (M.ni + 2), 32); }
 static inline size_t tile_smem(const DevModel &M, int arrays) { return (size_t)arrays * 32 * (M.nk + 1) * sizeof(double); }
-// 16 warps a tile for the FP64 form's column kernels while the launch has at most a tile per SM:
-// each warp then takes one or two levels of a 20-level column instead of two or three.
+// 16 warps a tile for the FP64 form's column kernels while the launch has at most two tiles per SM (two
+// such blocks fit): each warp then takes one or two levels of a 20-level column instead of two or three.
+// 12 steps of 128x64x20 (265 tiles) 11.45 -> 11.0 ms.
 static inline int tile_threads(const DevModel &M) {
   const long long tiles = (long long)ntile_blocks(M) * (M.nbatch > 1 ? M.nbatch : 1);
-  return !M.mixed && M.nk > CT_WARPS && tiles <= 152 ? CT_THREADS_WIDE : CT_THREADS;
+  return !M.mixed && M.nk > CT_WARPS && tiles <= 2 * 152 ? CT_THREADS_WIDE : CT_THREADS;
 }
 int launch_calc_w(const DevModel &M, cudaStream_t s, bool with_source_sink) {
   EPIC_LAUNCH_R(M.mixed, k_calc_w, ntile_blocks(M), tile_threads(M), tile_smem(M, 6), s, M, (int)with_source_sink);
@@ -1018,7 +1024,8 @@ int launch_restore_mass(const DevModel &M, cudaStream_t s) {
 int launch_set_p2etc(const DevModel &M, int update_theta, cudaStream_t s, bool early) {
   if (M.col64) k_set_p2etc_acc<<<zg(ntile_blocks(M), M), CT_THREADS, tile_smem(M, 4), s>>>(M, update_theta, !early);
   else if (M.mixed) k_set_p2etc_mixed<<<zg(ntile_blocks(M), M), CT_THREADS, tile_smem(M, 3), s>>>(M, update_theta, !early);
-  else k_set_p2etc<<<zg(ntile_blocks(M), M), tile_threads(M), tile_smem(M, 4), s>>>(M, update_theta);
+  else if (tile_threads(M) == CT_THREADS) k_set_p2etc<CT_THREADS><<<zg(ntile_blocks(M), M), CT_THREADS, tile_smem(M, 4), s>>>(M, update_theta);
+  else k_set_p2etc<CT_THREADS_WIDE><<<zg(ntile_blocks(M), M), CT_THREADS_WIDE, tile_smem(M, 4), s>>>(M, update_theta);
   return 0;
 }
 // The gas-giant lower boundary of store_pgrad_vars (epic_funcs_diag.c:3779-3811) with gz_from_u
@@ -1152,7 +1159,8 @@ int launch_store_pgrad_vars(const DevModel &M, cudaStream_t s, bool early, bool 
   }
   if (M.col64) (h2 ? k_pgrad_vars_column_acc_h2 : k_pgrad_vars_column_acc)<<<grid, CT_THREADS, smem, s>>>(M);
   else if (M.mixed) (h2 ? k_pgrad_vars_column_mixed<true, true> : k_pgrad_vars_column_mixed<true, false>)<<<grid, CT_THREADS, smem, s>>>(M);
-  else k_pgrad_vars_column<<<grid, tile_threads(M), tile_smem(M, 6), s>>>(M);
+  else if (tile_threads(M) == CT_THREADS) k_pgrad_vars_column<CT_THREADS><<<grid, CT_THREADS, tile_smem(M, 6), s>>>(M);
+  else k_pgrad_vars_column<CT_THREADS_WIDE><<<grid, CT_THREADS_WIDE, tile_smem(M, 6), s>>>(M);
   return dzdt ? launch_pgrad_dzdt(M, s) : 0;
 }
 int launch_pgrad_dzdt(const DevModel &M, cudaStream_t s) {
@@ -1177,8 +1185,10 @@ int column_kernels_init(int) {
   const int hv = (int)(4 * 32 * (EPIC_MAX_NK + 2) * sizeof(double));
   if (cudaFuncSetAttribute(k_calc_w<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
       cudaFuncSetAttribute(k_calc_w<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
-      cudaFuncSetAttribute(k_set_p2etc, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
-      cudaFuncSetAttribute(k_pgrad_vars_column, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
+      cudaFuncSetAttribute(k_set_p2etc<CT_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
+      cudaFuncSetAttribute(k_set_p2etc<CT_THREADS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
+      cudaFuncSetAttribute(k_pgrad_vars_column<CT_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
+      cudaFuncSetAttribute(k_pgrad_vars_column<CT_THREADS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
       cudaFuncSetAttribute(k_set_p2etc_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
       cudaFuncSetAttribute(k_pgrad_vars_column_mixed<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
       cudaFuncSetAttribute(k_pgrad_vars_column_mixed<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||

@@ -924,7 +924,7 @@ __device__ __forceinline__ void visc_row(const DevModel &M, const double *A, con
 // Bound by those additions: with one lane of each row's warp summing it, 4 orders x ni additions a row
 // held the binary64 pipe (71% busy) for 36 us a field at 128x64x20.  The meridional part's filter and
 // last update come first (visc_row), on the row in shared memory: two launches and two passes fewer.
-__global__ void __launch_bounds__(256) k_zonal_visc_rows(DevModel M, double *A, int sel, const double *D, double msign, int filter, int jbot,
+__global__ void __launch_bounds__(256, 3) k_zonal_visc_rows(DevModel M, double *A, int sel, const double *D, double msign, int filter, int jbot,
                                                          int jhalf, int k0, int nkk, int restore, int rows) {
   if (epic_member(M, A, D)) return;
   extern __shared__ __align__(16) double vr[];
