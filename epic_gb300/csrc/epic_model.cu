@@ -147,6 +147,19 @@ int check_launch(const char *what) {
   return EPIC_OK;
 }
 
+// GZ3 filtered into its copy GZ, the rows the tensor-core filter leaves alone on stream `rest`.
+// The 3-D filter's profiles interpolate in the filtered GZ: filtering GZ itself in FP32
+// makes the mixed form's V error after a day grow from 4e-5 to 7e-5 (leapfrog: 1.7e-4 ->
+// 1.6e-3).  The mixed forms filter it on the tensor cores as GZ - GZ(i=1) per row (FP32
+// rounding of the zonal variations only) where the operator product applies, the FP64 form
+// in binary64.
+void launch_gz_filter(const DevModel &M, cudaStream_t s, cudaStream_t rest) {
+  using namespace epic;
+  const int tensor = M.mixed && filter_gemm_usable(M);
+  launch_filter_rest(M, M.gz3, PL_NONE, M.gz, 0, M.nk, 0, rest, tensor);
+  launch_filter_planes(M, M.gz3, PL_NONE, M.gz, 0, M.nk, 0, s, tensor, tensor, tensor);
+}
+
 // One reference-function stage of the step, in the reference's call order, for a model or
 // (M.batch set) for every member of a batch.
 int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
@@ -198,13 +211,7 @@ int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
     // error after a day ~2x larger); EPIC_PREC_MIXED_FAST keeps the FP32 kernel.
     case 7: launch_store_pgrad_vars(M, s, true); break;
     case 8:   // from GZ3 into its copy GZ (epic_timestep.c:176-195)
-      // The 3-D filter's profiles interpolate in the filtered GZ: filtering GZ itself in FP32
-      // makes the mixed form's V error after a day grow from 4e-5 to 7e-5 (leapfrog: 1.7e-4 ->
-      // 1.6e-3).  The mixed forms filter it on the tensor cores as GZ - GZ(i=1) per row (FP32
-      // rounding of the zonal variations only) where the operator product applies, the FP64 form
-      // in binary64.
-      if (M.mixed && filter_gemm_usable(M)) launch_filter_planes(M, M.gz3, PL_NONE, M.gz, 0, M.nk, 0, s, 1, 1);
-      else launch_filter_planes(M, M.gz3, PL_NONE, M.gz, 0, M.nk, 0, s);
+      launch_gz_filter(M, s, s);
       launch_gz_monotone(M, s);
       break;
     case 9:
@@ -236,10 +243,10 @@ int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
       launch_hyperviscosity(M, 1, M.v, PL_UV, s);
       break;
     case 16:
-      launch_diag_filter_v(M, s);
+      launch_diag_filter_v(M, s, s);
       launch_diag_pv(M, s);
       launch_diag_pv_poles(M, s);
-      launch_diag_filter_u(M, s);
+      launch_diag_filter_u(M, s, s);
       launch_diag_div(M, s);
       launch_diag_ri2(M, s);
       if (M.turb) launch_set_diffusion_coef(M, s);
@@ -350,8 +357,12 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
   launch_zero_tend(M, L[1]);
   launch_uv_decide(M, L[1]);
   launch_advection_prep(M, 0, L[2]);   // UNITY = 1
-  launch_calc_w(M, L[0], true);        // source_sink and calc_w: THETA, W3
-  L.fork();
+  // source_sink and calc_w (THETA, W3) on THETA's lane; HDRY's hyperviscosity needs neither
+  const int w_lane = M.turb ? 0 : 3;
+  launch_calc_w(M, L[w_lane], true);
+  const cudaEvent_t w_done = L.point(w_lane);
+  for (int q = 0; q < LANES; q++)
+    if (q != w_lane && (q != 0 || M.turb)) L.after(q, w_done);
   // lane 1: DUDT, DVDT of uv_core and uv_drag
   launch_uv_core(M1, L[1]);
   launch_uv_drag(M1, L[1]);
@@ -400,6 +411,7 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
     zonal(M3, M.nu_turb, 2, 1, L[3]);
     launch_advection_prep(M, 2, L[3]);
   }
+  L.after(0, w_done);
   vertical(M, M.hdry, 2, L[0]);
   meridional(M, M.hdry, 2, L[0]);
   zonal(M, M.hdry, 1, 1, L[0]);   // then restore_mass, in the same kernel
@@ -407,8 +419,10 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
   launch_set_p2etc(M, 0, L[0], true);
   L.after(0, 3);
   launch_store_pgrad_vars(M, L[0], true);
-  int rc = run_stage_on(M, L[0], 8);   // the filtered GZ
-  if (rc) return rc;
+  L.after(1, 0);
+  launch_gz_filter(M, L[0], L[1]);
+  L.after(0, 1);
+  launch_gz_monotone(M, L[0]);
   // the 3-D filter: lane 1 DUDT, lane 2 DVDT, lane 3 THETA (and NU_TURB), lane 0 HDRY
   L.fork();
   launch_varz_filter(M1, M.dudt, PL_UV_TEND, 0, 1, M.nk, L[1]);
@@ -422,12 +436,12 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
   L.after(0, 3);
   launch_set_p2etc(M, 1, L[0]);
   launch_store_pgrad_vars(M, L[0], false, false);
-  launch_pgrad_poles(M, L[0]);
-  L.after(3, 0);
-  launch_pgrad_dzdt(M, L[3]);      // the rest of store_pgrad_vars
-  launch_calc_heating(M, L[3]);    // of P3 and T3
-  // lane 1: DUDT's pressure gradient, lane 0: DVDT's
+  // lane 1: DUDT's pressure gradient, which alone reads GZ3's pole rows, lane 0: DVDT's
   L.after(1, 0);
+  launch_pgrad_poles(M, L[1]);
+  L.after(3, 1);
+  launch_pgrad_dzdt(M, L[3]);      // the rest of store_pgrad_vars (the pole rows against V = 0)
+  launch_calc_heating(M, L[3]);    // of P3 and T3
   launch_pgrad_lon(M, L[1]);
   L.after(0, 2);
   launch_pgrad_lat(M, L[0]);
@@ -456,15 +470,19 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
   launch_hyperviscosity(M, 0, M.u, PL_UV, L[0]);
   launch_hyperviscosity(M1, 1, M.v, PL_UV, L[1]);
   const cudaEvent_t u_done = L.point(0), v_done = L.point(1);
-  launch_diag_filter_u(M, L[0]);
-  launch_diag_filter_v(M1, L[1]);
   L.after(2, u_done);
+  L.after(3, v_done);
+  launch_diag_filter_u(M, L[0], L[2]);
+  launch_diag_filter_v(M1, L[1], L[3]);
+  const cudaEvent_t u_rest = L.point(2), v_rest = L.point(3);
   launch_diag_pv_poles(M, L[2]);
   L.after(2, v_done);
   launch_diag_ri2(M, L[2]);
   L.after(0, v_done);
+  L.after(0, u_rest);
   launch_diag_div(M, L[0]);
   L.after(1, u_done);
+  L.after(1, v_rest);
   launch_diag_pv(M1, L[1]);
   if (M.turb) {   // of the winds and NU_TURB
     L.after(3, u_done);

@@ -39,7 +39,7 @@ __global__ void k_source_sink(DevModel M) {
 // source_sink = 1: the step's source_sink (k_source_sink) first, in the same pass over the
 // columns: THETA(k >= k_sigma-1) += dt*HEAT3/EXNER3 in binary64, written back and then used.
 template <class R>
-__global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : CT_THREADS, std::is_same_v<R, double> ? 2 : 3) k_calc_w(DevModel M, int source_sink) {
+__global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : CT_THREADS, std::is_same_v<R, double> ? 2 : 4) k_calc_w(DevModel M, int source_sink) {
   if (epic_member(M)) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   R *sm = reinterpret_cast<R *>(smraw);

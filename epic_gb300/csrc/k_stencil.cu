@@ -997,7 +997,7 @@ __global__ void __launch_bounds__(256, 3) k_zonal_visc_rows(DevModel M, double *
 
 // The same in the mixed forms: one warp per row (j, k), blockDim.x / 32 rows per block.  The updated
 // row stays in FP64; the row mean is an FP32 warp reduction.
-__global__ void k_zonal_visc_mixed(DevModel M, double *A, int sel, const double *D, double msign, int filter, int jbot, int jhalf, int k0, int restore) {
+__global__ void __launch_bounds__(128, 8) k_zonal_visc_mixed(DevModel M, double *A, int sel, const double *D, double msign, int filter, int jbot, int jhalf, int k0, int restore) {
   if (epic_member(M, A, D)) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   if (filter) prefetch_twiddles<float>(M);
@@ -1505,7 +1505,8 @@ int stencil_kernels_init() {
 
 int launch_divergence_damping(const DevModel &M, cudaStream_t s) {
   if (M.nudiv == 0.) return 0;
-  launch_filter_planes(M, M.u, PL_UV_DIS, M.work1, 1, M.nk - 1, 0, s, M.mixed);
+  launch_filter_rest(M, M.u, PL_UV_DIS, M.work1, 1, M.nk - 1, 0, s, M.mixed);
+  launch_filter_planes(M, M.u, PL_UV_DIS, M.work1, 1, M.nk - 1, 0, s, M.mixed, 0, 1);
   EPIC_MARCH(M.mixed, k_divergence, M.nk - 1, M.nj + 1, TB(M, TB_DIAG), s, M, M.work1, M.v, PL_UV_DIS, M.work2, 1, M.nk - 1);
   EPIC_LAUNCH_R(M.mixed, k_divdamp_apply, epic_blocks(2LL * (M.nk - 1) * (M.nj + 1) * M.ni, TB(M, TB_UPDATE)), TB(M, TB_UPDATE), 0, s, M);
   return 0;
@@ -1524,11 +1525,13 @@ int launch_uv_rotate(const DevModel &M, cudaStream_t s) {
   return 0;
 }
 
-int launch_diag_filter_v(const DevModel &M, cudaStream_t s) {
-  return launch_filter_planes(M, M.v, PL_UV, M.work1, 0, M.nk + 1, 1, s, M.mixed);
+int launch_diag_filter_v(const DevModel &M, cudaStream_t s, cudaStream_t rest) {
+  launch_filter_rest(M, M.v, PL_UV, M.work1, 0, M.nk + 1, 1, rest, M.mixed);
+  return launch_filter_planes(M, M.v, PL_UV, M.work1, 0, M.nk + 1, 1, s, M.mixed, 0, 1);
 }
-int launch_diag_filter_u(const DevModel &M, cudaStream_t s) {
-  return launch_filter_planes(M, M.u, PL_UV, M.work2, 0, M.nk + 1, 0, s, M.mixed);
+int launch_diag_filter_u(const DevModel &M, cudaStream_t s, cudaStream_t rest) {
+  launch_filter_rest(M, M.u, PL_UV, M.work2, 0, M.nk + 1, 0, rest, M.mixed);
+  return launch_filter_planes(M, M.u, PL_UV, M.work2, 0, M.nk + 1, 0, s, M.mixed, 0, 1);
 }
 int launch_diag_pv(const DevModel &M, cudaStream_t s) {
   EPIC_MARCH(M.mixed, k_pv_interior, M.nk + 1, M.nj, TB(M, TB_DIAG), s, M, M.work1);

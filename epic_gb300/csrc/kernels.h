@@ -73,10 +73,13 @@ __device__ __forceinline__ bool march(const DevModel &M, int k0, int nkk, int jl
 // fp32: filter in FP32 (the mixed forms; on the tensor cores for ni a multiple of 128).
 // shift (tensor-core path only): filter x - x(i=1) of each row and add x(i=1) back in binary64,
 // for fields whose zonal variations are small beside their value (the geopotential).
-// pads_set: an in-place call whose rows 0..nj(+1) already carry their periodic pads (the
-// tensor-core path then touches the filtered rows only).
+// filtered_rows_only: on the tensor-core path only the rows the filter changes are written (an in-place
+// call whose rows 0..nj(+1) already carry their periodic pads, or one beside launch_filter_rest).
 int launch_filter_planes(const DevModel &M, const double *src, int src_sel, double *dst, int k0, int nplanes, int vgrid, cudaStream_t s,
-                         int fp32 = 0, int shift = 0, int pads_set = 0);
+                         int fp32 = 0, int shift = 0, int filtered_rows_only = 0);
+// The other rows of an out-of-place call (the tensor-core path; nothing on the others): copied, with their
+// pads, on a stream of their own choice.
+int launch_filter_rest(const DevModel &M, const double *src, int src_sel, double *dst, int k0, int nplanes, int vgrid, cudaStream_t s, int fp32);
 int launch_varz_filter(const DevModel &M, double *buff, int sel, int index, int kstart, int kend, cudaStream_t s);
 int launch_hsu_zonal(const DevModel &M, double *buff, int kind, int kstart, cudaStream_t s);
 int filter_kernels_init(int ni);
@@ -151,8 +154,8 @@ int launch_uv_update(const DevModel &M, cudaStream_t s);
 int launch_uv_rotate(const DevModel &M, cudaStream_t s);
 // store_diag: the filtered copies of V (into work1) and U (into work2), PV3 from the first with its
 // polar values, DIV_UV3 from the second, RI2
-int launch_diag_filter_v(const DevModel &M, cudaStream_t s);
-int launch_diag_filter_u(const DevModel &M, cudaStream_t s);
+int launch_diag_filter_v(const DevModel &M, cudaStream_t s, cudaStream_t rest);   // rest: launch_filter_rest's stream
+int launch_diag_filter_u(const DevModel &M, cudaStream_t s, cudaStream_t rest);
 int launch_diag_pv(const DevModel &M, cudaStream_t s);
 int launch_diag_pv_poles(const DevModel &M, cudaStream_t s);
 int launch_diag_div(const DevModel &M, cudaStream_t s);
