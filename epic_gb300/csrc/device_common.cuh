@@ -35,18 +35,19 @@ constexpr int SCRATCH_VOLUMES = 3 + 4 * SCRATCH_SETS;   // gz, unity, old and th
 // Time-plane indices and step counters live on the device so that one captured CUDA graph
 // serves every step (the reference rotates IT_ZERO/IT_MINUS1/IT_MINUS2 on the host,
 // src/shared/epic_timestep.c:257-274).
+// What every kernel reads before its first useful load comes first, in one cache line.
 struct Ctl {
   int it_zero, it_minus1, it_minus2;
   int it_uv, it_uv_dis, it_uv_tend;
+  int halted;                          // set between steps once err_code is set: every kernel of the
+                                       // model then returns at entry (the reference stops the run at
+                                       // its first epic_error); cleared by an upload
   long long itime, model_time;
   int err_code, err_k, err_j, err_i;   // first model error (0 = none)
   double err_val;
   double ab[2][3];                     // Adams-Bashforth coefficients chosen for u, v this step
   float2 abf[2][3];                    // the same as double-floats (the mixed forms' update)
   int lf_first[2];                     // leapfrog: forward (Euler) first step for u, v
-  int halted;                          // set between steps once err_code is set: every kernel of the
-                                       // model then returns at entry (the reference stops the run at
-                                       // its first epic_error); cleared by an upload
 };
 
 enum ErrCode { ERR_NONE = 0, ERR_GZ_MONOTONE = 1, ERR_CALC_W_P = 2, ERR_PCHIP_X = 3, ERR_NONFINITE = 4, ERR_TIMEOUT = 5,
@@ -72,6 +73,10 @@ struct DevModel {
   const double *lon, *lat, *rln, *rlt, *f, *m, *n, *mn, *grav, *mn_inv;
   const double *sgth, *dsgth, *dsgth_inv, *h_min, *t_sponge_inv;
   const double *high_lat_h, *high_lat_pv;   // [(nj+3)*(ni+2)] 2-D like the reference
+  int filt_south_h, filt_north_h, filt_south_v, filt_north_v;   // the rows that the zonal filter changes, |lat| >=
+                                            // lat0: j up to filt_south and from filt_north on, h rows and v rows
+                                            // (scalars: a run-time index would put a kernel's DevModel in memory)
+  int filt_bands;                           // 0: not two such bands (row_is_filtered compares the latitude)
   const double *h_coef, *v_coef;            // d2dy2 coefficients, 3 per row
   const double *rt64;                       // RowTab of rows 0..nj+1, RT_COUNT values each, in binary64 ...
   const float *rt32;                        // ... and in binary32

@@ -743,6 +743,19 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
     d.dfc[epic::DFC_LOG_P0] = split(std::log(d.press0));
   }
 
+  // |lat| >= lat0 holds on a band of rows at each pole, latitudes ascending; else the kernels compare
+  d.filt_bands = 1;
+  for (int v = 0; v < 2; v++) {
+    auto filtered = [&](int j) { return std::fabs(g->lat[v ? 2 * j : 2 * j + 1]) >= g->lat0; };
+    int a = v, b = g->nj;
+    while (a <= g->nj && filtered(a)) a++;
+    while (b >= a && filtered(b)) b--;
+    for (int j = a; j <= b; j++)
+      if (filtered(j)) d.filt_bands = 0;
+    (v ? d.filt_south_v : d.filt_south_h) = a - 1;
+    (v ? d.filt_north_v : d.filt_north_h) = b + 1;
+  }
+
   HostTables T;
   filter_tables(*g, L, T);
   visc_tables(*g, T);

@@ -38,12 +38,13 @@ __global__ void k_filter_planes(DevModel M, const double *src, int src_sel, doub
     }
     return;
   }
-  prefetch_twiddles<R>(M);
+  const double *hl = (vgrid ? M.high_lat_pv : M.high_lat_h) + M.at2(j, 0);
+  warm_filter<R>(M, hl);
   R *x = reinterpret_cast<R *>(smraw) + L.r * S.stride;
   const int lg = fft_log(ni);
   for (int e = L.gl; e < ni; e += L.G) x[fft_place(e, lg)] = L.live ? cv<R>(src[base + e + 1]) : R(0.);
   __syncwarp();
-  filter_row<R>(M, reinterpret_cast<Cplx<R> *>(x), (vgrid ? M.high_lat_pv : M.high_lat_h) + M.at2(j, 0), L);
+  filter_row<R>(M, reinterpret_cast<Cplx<R> *>(x), hl, L);
   if (!L.live) return;
   const R scale = filter_scale<R>(ni);
   for (int e = L.gl; e < ni; e += L.G) write_with_pads(dst, M, base, e + 1, to_d(x[e] * scale));
@@ -265,7 +266,7 @@ __global__ void k_varz_filter_rows(DevModel M, double *buff, int sel, int index,
   // The mixed forms leave unfiltered rows untouched (their subtract-and-add-back is the identity
   // up to one rounding); the FP64 form repeats the reference's arithmetic on them.
   if (!filt && !exact) return;
-  if (filt) prefetch_twiddles<R>(M);
+  if (filt) warm_filter<R>(M, (vgrid ? M.high_lat_pv : M.high_lat_h) + M.at2(j, 0));
   VarzKnot *kn = reinterpret_cast<VarzKnot *>(smd);
   VarzInterval *iv = reinterpret_cast<VarzInterval *>(smd);
   double *knot = smd + (size_t)(M.nk + 2) * (sizeof(VarzInterval) / 8);
@@ -352,7 +353,7 @@ __global__ void k_hsu_zonal(DevModel M, double *buff, int kind, int kstart, RowS
   const int j = (int)blockIdx.x;
   if (j > M.nj) return;   // a member with fewer rows than the launch (batches of mixed sizes)
   const RowLane L = row_lane(S, kstart, M.nk);
-  if (row_is_filtered(M, j, 0)) prefetch_twiddles<R>(M);
+  if (row_is_filtered(M, j, 0)) warm_filter<R>(M, M.high_lat_h + M.at2(j, 0));
   const int k = L.k, base = M.at(k, j, 0);
   R *a = reinterpret_cast<R *>(smraw) + L.r * S.stride, *ff = a + ni, *ap = ff + ni, *w = ap + ni;
   const R DT = cv<R>(M.dt);
@@ -401,7 +402,7 @@ __global__ void k_akima_zonal(DevModel M, double *buff, int kind, int kstart, Ro
   const int j = (int)blockIdx.x;
   if (j > M.nj) return;   // a member with fewer rows than the launch (batches of mixed sizes)
   const RowLane L = row_lane(S, kstart, M.nk);
-  if (row_is_filtered(M, j, 0)) prefetch_twiddles<R>(M);
+  if (row_is_filtered(M, j, 0)) warm_filter<R>(M, M.high_lat_h + M.at2(j, 0));
   const int k = L.k, base = M.at(k, j, 0), mask = ni - 1;
   R *a = reinterpret_cast<R *>(smraw) + L.r * S.stride, *dl = a + ni, *ff = dl + ni;
   const R DT = cv<R>(M.dt);

@@ -928,7 +928,7 @@ __global__ void __launch_bounds__(256, 3) k_zonal_visc_rows(DevModel M, double *
                                                          int jhalf, int k0, int nkk, int restore, int rows) {
   if (epic_member(M, A, D)) return;
   extern __shared__ __align__(16) double vr[];
-  if (filter) prefetch_twiddles<double>(M);
+  if (filter) warm_filter<double>(M, nullptr);
   __shared__ double s_mean[32];
   const int ni = M.ni, W = ni + 2, lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
   const int nr = M.nj - jbot + 1;
@@ -1000,7 +1000,7 @@ __global__ void __launch_bounds__(256, 3) k_zonal_visc_rows(DevModel M, double *
 __global__ void __launch_bounds__(128, 8) k_zonal_visc_mixed(DevModel M, double *A, int sel, const double *D, double msign, int filter, int jbot, int jhalf, int k0, int restore) {
   if (epic_member(M, A, D)) return;
   extern __shared__ __align__(16) unsigned char smraw[];
-  if (filter) prefetch_twiddles<float>(M);
+  if (filter) warm_filter<float>(M, nullptr);
   const int ni = M.ni, lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
   const int j = jbot + (int)blockIdx.x * nw + w;
   const int k = k0 + (int)blockIdx.y;

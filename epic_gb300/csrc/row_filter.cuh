@@ -48,13 +48,19 @@ template <class R> __device__ __forceinline__ const Cplx<R> *twiddle_table(const
 template <> __device__ __forceinline__ const Cplx<double> *twiddle_table<double>(const DevModel &M) { return reinterpret_cast<const Cplx<double> *>(M.tw); }
 template <> __device__ __forceinline__ const Cplx<float> *twiddle_table<float>(const DevModel &M) { return reinterpret_cast<const Cplx<float> *>(M.twf); }
 
-// The twiddles into L1, by the lanes of each warp, ahead of the stages that read them: each stage waits for
-// its twiddles between two __syncwarp, an L2 round trip a stage for the first rows of an SM otherwise.
+// The twiddles and a row's weights (if any) into L1, a cache line per lane of each warp, ahead of the
+// stages that read them: each stage waits for its twiddles between two __syncwarp, an L2 round trip a
+// stage for the first rows of an SM otherwise.  Plain loads whose values nobody waits for.
+__device__ __forceinline__ void touch(const char *p, int bytes) {
+  for (int b = 128 * ((int)threadIdx.x & 31); b < bytes; b += 128 * 32) {
+    unsigned v;
+    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(v) : "l"(p + b));
+  }
+}
 template <class R>
-__device__ __forceinline__ void prefetch_twiddles(const DevModel &M) {
-  const char *t = reinterpret_cast<const char *>(twiddle_table<R>(M));
-  const int bytes = (int)(nr_twiddle_pairs(M.ni) * sizeof(Cplx<R>));
-  for (int b = 128 * ((int)threadIdx.x & 31); b < bytes; b += 128 * 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(t + b));
+__device__ __forceinline__ void warm_filter(const DevModel &M, const double *hl) {
+  touch(reinterpret_cast<const char *>(twiddle_table<R>(M)), (int)(nr_twiddle_pairs(M.ni) * sizeof(Cplx<R>)));
+  if (hl) touch(reinterpret_cast<const char *>(hl), (M.ni / 2 + 2) * 8);
 }
 
 // The place of row value e = i-1 among the N complex points in bit-reversed order, which
@@ -134,7 +140,8 @@ __device__ __forceinline__ void filter_row(const DevModel &M, Cplx<R> *z, const 
 }
 
 __device__ __forceinline__ bool row_is_filtered(const DevModel &M, int j, int vgrid) {
-  return fabs(M.lat[vgrid ? 2 * j : 2 * j + 1]) >= M.lat0;
+  if (!M.filt_bands) return fabs(M.lat[vgrid ? 2 * j : 2 * j + 1]) >= M.lat0;
+  return vgrid ? j <= M.filt_south_v || j >= M.filt_north_v : j <= M.filt_south_h || j >= M.filt_north_h;
 }
 
 // The place of row value e = i-1 for filter_row, or in order for a row that is not filtered.
