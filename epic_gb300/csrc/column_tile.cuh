@@ -108,13 +108,16 @@ template <class R>
 __device__ __forceinline__ R f_and_g_sigma_r(const DevModel &M, R s, R &g) {
   const R ss = mconst<R>(M, DFC_SIGMA_SIGMA, M.sigma_sigma), z0 = mconst<R>(M, DFC_ZETA0, M.zeta0),
           z1 = mconst<R>(M, DFC_ZETA1, M.zeta1);
-  if (s <= ss) g = R(0.);
-  else if (s >= R(1.)) g = R(1.);
-  else g = mconst<R>(M, DFC_G_COEFF, M.g_coeff) * (R(1.) - RMath<R>::exp(M, -mconst<R>(M, DFC_ALPHA, M.alpha) * (s - ss)));
-  if (s < R(0.)) return z0;
-  if (s <= ss) return z0 + s * (z1 - z0);
-  if (s < R(1.)) return (R(1.) - g) * (z0 + s * (z1 - z0));
-  return R(0.);
+  if (s <= ss) {
+    g = R(0.);
+    return s < R(0.) ? z0 : z0 + s * (z1 - z0);
+  }
+  if (s >= R(1.)) {
+    g = R(1.);
+    return R(0.);
+  }
+  g = mconst<R>(M, DFC_G_COEFF, M.g_coeff) * (R(1.) - RMath<R>::exp(M, -mconst<R>(M, DFC_ALPHA, M.alpha) * (s - ss)));
+  return (R(1.) - g) * (z0 + s * (z1 - z0));
 }
 
 // d(return_sigmatheta)/dp at fixed theta and pbot, from f_sigma/g_sigma's derivatives:

@@ -293,13 +293,19 @@ __device__ __forceinline__ double f_sigma(const DevModel &M, double s) {
   if (s < 1.) return (1. - g_sigma(M, s)) * (M.zeta0 + s * (M.zeta1 - M.zeta0));
   return 0.;
 }
-// f_sigma(s), with g_sigma(s) returned in g: one exponential serves both.
+// f_sigma(s), with g_sigma(s) returned in g: one exponential and each comparison (a binary64 operation)
+// serve both.
 __device__ __forceinline__ double f_and_g_sigma(const DevModel &M, double s, double &g) {
-  g = g_sigma(M, s);
-  if (s < 0.) return M.zeta0;
-  if (s <= M.sigma_sigma) return M.zeta0 + s * (M.zeta1 - M.zeta0);
-  if (s < 1.) return (1. - g) * (M.zeta0 + s * (M.zeta1 - M.zeta0));
-  return 0.;
+  if (s <= M.sigma_sigma) {
+    g = 0.;
+    return s < 0. ? M.zeta0 : M.zeta0 + s * (M.zeta1 - M.zeta0);
+  }
+  if (s >= 1.) {
+    g = 1.;
+    return 0.;
+  }
+  g = M.g_coeff * (1. - xexp(M, -M.alpha * (s - M.sigma_sigma)));
+  return (1. - g) * (M.zeta0 + s * (M.zeta1 - M.zeta0));
 }
 __device__ __forceinline__ double return_sigmatheta(const DevModel &M, double theta, double p, double pbot, double ptop) {
   if (p <= ptop) return theta;
@@ -486,6 +492,19 @@ template <int E, class R> __device__ __forceinline__ R scale_down(R x) {
   }
 }
 template <class R> __device__ __forceinline__ R half_of(R x) { return scale_down<1>(x); }
+// 2 x likewise
+template <class R> __device__ __forceinline__ R twice_of(R x) {
+  if constexpr (std::is_same_v<R, double>) {
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    const unsigned e = (unsigned)hi & 0x7ff00000u;
+    const bool zero = (((unsigned)hi << 1) | (unsigned)lo) == 0u;
+    double r = __hiloint2double(zero ? hi : hi + 0x00100000, lo);
+    if (!zero && e - 0x00100000u >= 0x7fd00000u) r = 2. * x;
+    return r;
+  } else {
+    return R(2.) * x;
+  }
+}
 
 template <class R> struct RMath;
 template <> struct RMath<double> {
@@ -543,14 +562,14 @@ template <class R>
 __device__ __forceinline__ R hsu_face(R w, R w_up, R a_u, R a_d, R ap_d, R d_up, R aa, R min_u, R min_d, R c, R DT) {
   const bool neg = is_neg(w);
   const R wu = is_neg(w_up) == neg ? w_up : R(0.);
-  R f = R(.5) * (w * (ap_d + a_u));
+  R f = half_of(w * (ap_d + a_u));
   R what = qsqrt<R>(w * wu);
   what = neg ? -what : what;
   const R mu = fabs(w) * c * DT;
   const R al = qdiv(R(1.) + mu, R(6.));
   R g = qdiv(aa, aa + (a_u - min_u) * (a_d - min_d));
   g = g * g;
-  const R be = R(1.) + (qdiv(R(1.), R(2.) * al) - R(1.)) * g;
+  const R be = R(1.) + (qdiv(R(1.), twice_of(al)) - R(1.)) * g;
   return f + -al * (w * be * (ap_d - a_u) - what * (R(1.) - g) * d_up);
 }
 // the predictor's flux: the upwind cell's value carried by w (the other side's term is zero)

@@ -102,16 +102,17 @@ __global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : 
         const R df2 = P2 * CT(DV, k);
         const R df3 = P3 * CT(DV, k + 1);
         CT(DS, k) = -qdiv(qdiv(df0 * (dz21 * dz21 * dz21 * (dz31 + dz32)), dz10 * dz20 * dz30) +
-                            qdiv(df1 * (dz21 * (dz21 * (dz21 + R(2.) * (dz10 - dz31)) - R(6.) * dz10 * dz31)), dz10 * dz31) +
-                            qdiv(df2 * (dz21 * (dz21 * (dz21 + R(2.) * (dz32 - dz20)) - R(6.) * dz20 * dz32)), dz20 * dz32) +
+                            qdiv(df1 * (dz21 * (dz21 * (dz21 + twice_of(dz10 - dz31)) - R(6.) * dz10 * dz31)), dz10 * dz31) +
+                            qdiv(df2 * (dz21 * (dz21 * (dz21 + twice_of(dz32 - dz20)) - R(6.) * dz20 * dz32)), dz20 * dz32) +
                             qdiv(df3 * (dz21 * dz21 * dz21 * (dz10 + dz20)), dz30 * dz31 * dz32),
                         R(12.));
       }
       if constexpr (std::is_same_v<R, double>) {
         // dF/dp by a centred difference of return_sigmatheta at fixed theta and pbot
         const R dp = p3 * M.eps13;
-        R p2 = rmax(p3 - dp * R(.5), ptop);
-        const R p4 = rmin(p3 + dp * R(.5), pbot);
+        const R half_dp = half_of(dp);
+        R p2 = rmax(p3 - half_dp, ptop);
+        const R p4 = rmin(p3 + half_dp, pbot);
         if (p2 < psigma && p4 >= psigma) p2 = p3;
         if (!(p2 < p4)) flag_error(M.ctl, ERR_CALC_W_P, k, c.j, c.i, p2);
         CT(DF, k) = qdiv(sigmatheta_lp<R>(M, theta3, p2, pbot, ptop, lp) - sigmatheta_lp<R>(M, theta3, p4, pbot, ptop, lp), p2 - p4);
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : 
   auto wa = [&](int k) { return CT(WA, k); };
   // W3 at the layer's middle, 0 in the top and bottom layers
   auto w_layer = [&](int k) {
-    return (k == 1 || k == nk) ? R(0.) : R(.5) * (cv<R>(M.w3[c.base + k * n2]) + cv<R>(M.w3[c.base + (k - 1) * n2]));
+    return (k == 1 || k == nk) ? R(0.) : half_of(cv<R>(M.w3[c.base + k * n2]) + cv<R>(M.w3[c.base + (k - 1) * n2]));
   };
   if (c.valid)
     for (int k = (layer ? kf : kf - 1) + c.warp; k <= nk; k += c.nw) CT(WA, k) = cv<R>(buff[c.base + k * n2]);
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : 
         const R au = wa(u), ad = wa(d), auu = edge ? R(0.) : wa(neg ? k - 1 : k + 2);
         R t;
         if (edge) t = fabs(neg ? ad - au : -au + ad) + ep;
-        else t = fabs((neg ? ad : auu) - R(2.) * au + (neg ? auu : ad)) + ep;
+        else t = fabs((neg ? ad : auu) - twice_of(au) + (neg ? auu : ad)) + ep;
         auto amin = [&](int q) { return layer ? cv<R>(M.h_min[q]) : cv<R>(1.e-3 * M.kinvisc); };   // HDRY's and NU_TURB's floors
         CT(FF, k) = hsu_face<R>(w, CT(W, neg ? k - 1 : k + 1), au, ad, CT(PR, d), edge ? R(0.) : CT(PR, u) - auu, t * t, amin(u), amin(d),
                                 dsi(2 * k + 1), DT);
@@ -274,7 +275,7 @@ __global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : 
       R tmp;
       if (k == 0) tmp = fabs(wa(k + 1) - wa(k)) + ep;
       else if (k == nk) tmp = fabs(-wa(k) + wkm1) + ep;
-      else tmp = fabs(wa(k + 1) - R(2.) * wa(k) + wkm1) + ep;
+      else tmp = fabs(wa(k + 1) - twice_of(wa(k)) + wkm1) + ep;
       return tmp * tmp;
     };
     if (c.valid)
@@ -304,7 +305,7 @@ __global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : 
 template <class R>
 __device__ __forceinline__ R akima_dela(R d0, R d1) {
   const R tmp = d0 * d1;
-  return (tmp > R(0.)) ? qdiv(R(2.) * tmp, d0 + d1) : R(0.);
+  return (tmp > R(0.)) ? qdiv(twice_of(tmp), d0 + d1) : R(0.);
 }
 
 // Vertical pass of akima_advection, epic_flux.c:1549-1744 (mass fluxes through the model top
@@ -343,7 +344,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_akima_vertical(DevModel M, doubl
     if (c.valid)
       for (int k = kf - 1 + c.warp; k <= nk; k += CT_WARPS) {
         if (k == kf - 1 || k == nk) { CT(FF, k) = R(0.); continue; }   // mass_flux_top, mass_flux_bot
-        const R aval = R(.5) * (wa(k) + wa(k + 1)) - qdiv(CT(DL, k) - CT(DL, k + 1), R(6.));
+        const R aval = half_of(wa(k) + wa(k + 1)) - qdiv(CT(DL, k) - CT(DL, k + 1), R(6.));
         CT(FF, k) = CT(W, k) * aval;
       }
     __syncthreads();
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_akima_vertical(DevModel M, doubl
     if (c.valid)
       for (int k = kf + c.warp; k <= nk + 1; k += CT_WARPS) {
         if (k == nk + 1) { CT(FF, k) = R(0.); continue; }
-        const R aval = R(.5) * (wa(k - 1) + wa(k)) - qdiv(CT(DL, k - 1) - CT(DL, k), R(6.));
+        const R aval = half_of(wa(k - 1) + wa(k)) - qdiv(CT(DL, k - 1) - CT(DL, k), R(6.));
         CT(FF, k) = CT(W, k) * aval;
       }
     __syncthreads();
@@ -550,8 +551,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_pgrad_vars_column(D
       const double dz20 = dz21 + dz10, dz30 = dz32 + dz20, dz31 = dz32 + dz21;
       const double df0 = CT(Q, k + 1), df1 = CT(Q, k), df2 = CT(Q, k - 1), df3 = CT(Q, k - 2);
       CT(GZ, k - 1) = -qdiv(qdiv(df0 * (dz21 * dz21 * dz21 * (dz31 + dz32)), dz10 * dz20 * dz30) +
-                              qdiv(df1 * (dz21 * (dz21 * (dz21 + 2. * (dz10 - dz31)) - 6. * dz10 * dz31)), dz10 * dz31) +
-                              qdiv(df2 * (dz21 * (dz21 * (dz21 + 2. * (dz32 - dz20)) - 6. * dz20 * dz32)), dz20 * dz32) +
+                              qdiv(df1 * (dz21 * (dz21 * (dz21 + twice_of(dz10 - dz31)) - 6. * dz10 * dz31)), dz10 * dz31) +
+                              qdiv(df2 * (dz21 * (dz21 * (dz21 + twice_of(dz32 - dz20)) - 6. * dz20 * dz32)), dz20 * dz32) +
                               qdiv(df3 * (dz21 * dz21 * dz21 * (dz10 + dz20)), dz30 * dz31 * dz32),
                           12.);
     }

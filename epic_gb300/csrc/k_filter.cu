@@ -379,7 +379,7 @@ __global__ void k_hsu_zonal(DevModel M, double *buff, int kind, int kstart, RowS
     const bool neg = is_neg(v);   // from cell e west to e-1, else from e-1 east to e
     const int west = (e - 1) & mask, u = neg ? e : west, d = neg ? west : e, uu = (neg ? e + 1 : e - 2) & mask;
     const R au = a[u], ad = a[d], auu = a[uu];
-    const R t = fabs((neg ? ad : auu) - R(2.) * au + (neg ? auu : ad)) + R(1.e-10);
+    const R t = fabs((neg ? ad : auu) - twice_of(au) + (neg ? auu : ad)) + R(1.e-10);
     ff[e] = hsu_face<R>(v, w[neg ? e + 2 : e], au, ad, ap[d], ap[u] - auu, t * t, a_min, a_min, mn1, DT);
   }
   __syncwarp();
@@ -413,7 +413,7 @@ __global__ void k_akima_zonal(DevModel M, double *buff, int kind, int kstart, Ro
   for (int e = L.gl; e < ni; e += L.G) {
     const R d0 = a[e] - a[(e - 1) & mask], d1 = a[(e + 1) & mask] - a[e];
     const R tmp = d0 * d1;
-    dl[e] = (tmp > R(0.)) ? qdiv(R(2.) * tmp, d0 + d1) : R(0.);
+    dl[e] = (tmp > R(0.)) ? qdiv(twice_of(tmp), d0 + d1) : R(0.);
   }
   __syncwarp();
   for (int e = L.gl; e < ni; e += L.G) {

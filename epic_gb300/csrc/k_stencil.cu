@@ -403,7 +403,7 @@ __global__ void k_pgrad_lon(DevModel M) {
   const R rlns = cv<R>(M.rln[2 * j]), rlnn = cv<R>(M.rln[2 * j + 2]);
   R a1 = e.ztne + e.ztse, a2 = w.ztne + w.ztse;
   R terms2 = R(3.) * (a1 - a2), top, bottom;
-  if (fabs(qdiv(R(2.) * (e.zte - w.zte), e.zte + w.zte - e.zbe - w.zbe)) > DLOGZ_TOL) {
+  if (fabs(qdiv(twice_of(e.zte - w.zte), e.zte + w.zte - e.zbe - w.zbe)) > DLOGZ_TOL) {
     const R b1 = e.ztne * e.ztse, b2 = w.ztne * w.ztse;
     const R terms1 = a1 * a1 - b1 - (a2 * a2 - b2);
     top = qdiv(-terms1 * (w.pte - e.pte) + terms2 * (e.zte * w.pte - w.zte * e.pte), e.zte - w.zte);
@@ -413,7 +413,7 @@ __global__ void k_pgrad_lon(DevModel M) {
   a1 = e.zbne + e.zbse;
   a2 = w.zbne + w.zbse;
   terms2 = R(3.) * (a1 - a2);
-  if (fabs(qdiv(R(2.) * (e.zbe - w.zbe), e.zte + w.zte - e.zbe - w.zbe)) > DLOGZ_TOL) {
+  if (fabs(qdiv(twice_of(e.zbe - w.zbe), e.zte + w.zte - e.zbe - w.zbe)) > DLOGZ_TOL) {
     const R b1 = e.zbne * e.zbse, b2 = w.zbne * w.zbse;
     const R terms1 = a1 * a1 - b1 - (a2 * a2 - b2);
     bottom = qdiv(-terms1 * (w.pbe - e.pbe) + terms2 * (e.zbe * w.pbe - w.zbe * e.pbe), e.zbe - w.zbe);
@@ -538,7 +538,7 @@ __global__ void k_pgrad_lat(DevModel M) {
   R top, bottom;
   a1 = n.ztne + n.ztnw; a2 = ztse + ztsw;
   terms2 = R(3.) * (a1 - a2);
-  if (fabs(qdiv(R(2.) * (n.ztn - zts), n.ztn + zts - n.zbn - zbs)) > DLOGZ_TOL) {
+  if (fabs(qdiv(twice_of(n.ztn - zts), n.ztn + zts - n.zbn - zbs)) > DLOGZ_TOL) {
     b1 = n.ztne * n.ztnw; b2 = ztse * ztsw; b3 = n.ztne * ztse + n.ztnw * ztsw;
     terms1 = a1 * a1 - b1 - (a2 * a2 - b2);
     top = qdiv(Pow2{.5f} * ((n.ptn - pts) * ((rlnn + rlns) * terms1 + (rlnn - rlns) * (b1 + b2 - b3)) + (rlnn + rlns) * terms2 * (n.ztn * pts - zts * n.ptn)),
@@ -548,7 +548,7 @@ __global__ void k_pgrad_lat(DevModel M) {
   }
   a1 = n.zbne + n.zbnw; a2 = zbse + zbsw;
   terms2 = R(3.) * (a1 - a2);
-  if (fabs(qdiv(R(2.) * (n.zbn - zbs), n.ztn + zts - n.zbn - zbs)) > DLOGZ_TOL) {
+  if (fabs(qdiv(twice_of(n.zbn - zbs), n.ztn + zts - n.zbn - zbs)) > DLOGZ_TOL) {
     b1 = n.zbne * n.zbnw; b2 = zbse * zbsw; b3 = n.zbne * zbse + n.zbnw * zbsw;
     terms1 = a1 * a1 - b1 - (a2 * a2 - b2);
     bottom = qdiv(Pow2{.5f} * ((n.pbn - pbs) * ((rlnn + rlns) * terms1 + (rlnn - rlns) * (b1 + b2 - b3)) + (rlnn + rlns) * terms2 * (n.zbn * pbs - zbs * n.pbn)),
@@ -594,7 +594,7 @@ __device__ __forceinline__ R hsu_merid_flux(const DevModel &M, R w, R w_up, int 
   const R au = a(u), ad = a(d), auu = edge ? R(0.) : a(uu);
   R t;
   if (edge) t = fabs(neg ? ad - au : -au + ad) + R(1.e-10);
-  else t = fabs((neg ? ad : auu) - R(2.) * au + (neg ? auu : ad)) + R(1.e-10);
+  else t = fabs((neg ? ad : auu) - twice_of(au) + (neg ? auu : ad)) + R(1.e-10);
   return hsu_face<R>(w, w_up, au, ad, ap(d), edge ? R(0.) : ap(u) - auu, t * t, a_min, a_min, cv<R>(M.mn[2 * j]), DT);
 }
 
@@ -772,7 +772,7 @@ __global__ void __launch_bounds__(256) k_hsu_merid_tile(DevModel M, double *A, i
 template <class R>
 __device__ __forceinline__ R akima_mean(R d0, R d1) {   // the dela of akima_advection
   const R tmp = d0 * d1;
-  return (tmp > R(0.)) ? qdiv(R(2.) * tmp, d0 + d1) : R(0.);
+  return (tmp > R(0.)) ? qdiv(twice_of(tmp), d0 + d1) : R(0.);
 }
 
 template <class R>
@@ -787,9 +787,9 @@ __global__ void k_akima_merid_flux(DevModel M, const double *A, int kind, int k0
   const R dl_j = akima_mean<R>(deltaa(j), deltaa(j + 1));
   const R dl_jm = akima_mean<R>(deltaa(j - 1), deltaa(j));
   const double *V = M.v + plane_offset(M, PL_UV);
-  const R v2d = kind == 2 ? R(.5) * (cv<R>(V[M.at(k, j, i)]) + cv<R>(V[M.at(k - 1, j, i)])) : cv<R>(V[M.at(k, j, i)]);
+  const R v2d = kind == 2 ? half_of(cv<R>(V[M.at(k, j, i)]) + cv<R>(V[M.at(k - 1, j, i)])) : cv<R>(V[M.at(k, j, i)]);
   const R m_2j_inv = (fabs(M.lat[2 * j]) == 90.) ? R(0.) : qdiv(R(1.), cv<R>(M.m[2 * j]));
-  const R aval = R(.5) * (a(j) + a(j - 1)) - qdiv(dl_j - dl_jm, R(6.));
+  const R aval = half_of(a(j) + a(j - 1)) - qdiv(dl_j - dl_jm, R(6.));
   write_with_pads(M.work3, M, M.at(k, j, 0), i, to_d(v2d * aval * m_2j_inv));
 }
 
@@ -958,7 +958,7 @@ __global__ void __launch_bounds__(256, 3) k_zonal_visc_rows(DevModel M, double *
       const double mm = M.m[2 * j + jhalf];
       const double dc = fabs(M.lat[2 * j + jhalf]) > M.lat0 ? M.coef[itmp] * M.m0 * M.m0 : M.coef[itmp] * mm * mm;
       const double *hr = h + r * W;
-      for (int i = lane + 1; i <= ni; i += 32) d[r * W + i] = dc * (hr[i - 1] - 2. * hr[i] + hr[i + 1]);
+      for (int i = lane + 1; i <= ni; i += 32) d[r * W + i] = dc * (hr[i - 1] - twice_of(hr[i]) + hr[i + 1]);
     }
     __syncthreads();
     if ((int)threadIdx.x < nl) s_mean[threadIdx.x] = row_sum(d + (int)threadIdx.x * W + 1, ni) / ni;
@@ -1148,8 +1148,8 @@ __global__ void k_ri2(DevModel M) {
   const double *U = M.u + off, *V = M.v + off;
   auto u = [&](int kk, int jj, int ii) { return cv<R>(U[M.at(kk, jj, ii)]); };
   auto v = [&](int kk, int jj, int ii) { return cv<R>(V[M.at(kk, jj, ii)]); };
-  R dudz2 = R(.5) * (u(k - 1, j, i) + u(k - 1, j, i + 1) - u(k, j, i) - u(k, j, i + 1));
-  R dvdz2 = R(.5) * (v(k - 1, j, i) + v(k - 1, j + 1, i) - v(k, j, i) + v(k, j + 1, i));
+  R dudz2 = half_of(u(k - 1, j, i) + u(k - 1, j, i + 1) - u(k, j, i) - u(k, j, i + 1));
+  R dvdz2 = half_of(v(k - 1, j, i) + v(k - 1, j + 1, i) - v(k, j, i) + v(k, j + 1, i));
   dudz2 *= dudz2;
   dvdz2 *= dvdz2;
   R ri;
@@ -1159,8 +1159,8 @@ __global__ void k_ri2(DevModel M) {
     const R cp = R(1004.), mu = cv<R>(M.mu_dry);
     const R deltap = R(0.001) * pressure, deltaT = R(0.001) * temperature;
     auto dens = [&](R p, R t) { return qdiv(p * mu, R(8.314472e+3) * t); };   // return_density
-    const R drho_dp_T = qdiv(dens(pressure + deltap, temperature) - dens(pressure - deltap, temperature), R(2.) * deltap);
-    const R drho_dT_p = qdiv(dens(pressure, temperature + deltaT) - dens(pressure, temperature - deltaT), R(2.) * deltaT);
+    const R drho_dp_T = qdiv(dens(pressure + deltap, temperature) - dens(pressure - deltap, temperature), twice_of(deltap));
+    const R drho_dT_p = qdiv(dens(pressure, temperature + deltaT) - dens(pressure, temperature - deltaT), twice_of(deltaT));
     const R Drho_Dp = qdiv(cv<R>(M.rho3[x]) - cv<R>(M.rho3[M.at(k - 1, j, i)]), cv<R>(M.p3[x]) - cv<R>(M.p3[M.at(k - 1, j, i)]));
     const R g = cv<R>(M.grav[2 * j + 1]);
     const R brunt2 = g * g * (Drho_Dp - drho_dp_T + qdiv(temperature, cp * density * density) * drho_dT_p * drho_dT_p);

@@ -109,7 +109,7 @@ __device__ __forceinline__ void filter_row(const DevModel &M, Cplx<R> *z, const 
     if (q == 0) {   // wavenumbers 0 and ni/2 share z[0]; ni/4 has no partner
       const Cplx<R> a = z[0], b = z[N / 2];
       const R s = (a.re + a.im) * cv<R>(hl[1]), d = (a.re - a.im) * cv<R>(hl[N + 1]);
-      z[0] = {R(2.) * (s + d), R(2.) * (s - d)};
+      z[0] = {twice_of(s + d), twice_of(s - d)};
       const R h = R(4.) * cv<R>(hl[N / 2 + 1]);
       if (N > 1) z[N / 2] = {b.re * h, b.im * h};
       continue;
