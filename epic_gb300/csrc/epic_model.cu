@@ -202,14 +202,14 @@ int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
       zonal(M, M.hdry, 1, 1, s);   // then restore_mass, in the same kernel
       // Its P2 is recomputed (stage 11) before the pressure gradient.  EPIC_PREC_MIXED runs the
       // double-float kernel here too: it writes the interfaces' logarithms that stage 7 reads.
-      launch_set_p2etc(M, 0, s, true);
+      launch_set_p2etc(M, 0, s, M.mixed);   // alone, the FP64 form's stages write all that the reference's do
       break;
     }
     // GZ3 for the filtered copy (stage 8).  The copy places the 3-D filter's profiles (stages 9
     // and 10), which pass column-to-column rounding noise of GZ3 into the filtered fields, so
     // EPIC_PREC_MIXED computes it in double-float like stage 19 (the FP32 kernel made the wind
     // error after a day ~2x larger); EPIC_PREC_MIXED_FAST keeps the FP32 kernel.
-    case 7: launch_store_pgrad_vars(M, s, true); break;
+    case 7: launch_store_pgrad_vars(M, s, M.mixed); break;
     case 8:   // from GZ3 into its copy GZ (epic_timestep.c:176-195)
       launch_gz_filter(M, s, s);
       launch_gz_monotone(M, s);

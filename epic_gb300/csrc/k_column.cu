@@ -396,13 +396,15 @@ __global__ void k_restore_mass(DevModel M) {
 }
 
 // set_p2etc, epic_funcs_diag.c:3352-3569 (nq = 0: H2 is HDRY, PDRY3 is P3, HDRY3 is H3).
+// layers = 0: P3 and HDRY only (the step's call inside advection, whose P2 and H3 stage 11 rewrites before
+// anything reads them): no power.
 // Shared arrays: P (interface pressure), HL (get_h at the layers), TH (THETA), PP (P^(kappa+1),
 // each interface's power computed once for the two layers that share it).
 // THREADS: 256 or 512 a tile (tile_threads), 32 warps per SM either way: the long integer chains of the
 // logarithms, exponentials and quotients want warps more than registers.  With the 114-128 registers the
 // compiler takes by itself (16 warps), 3 steps of 256x128x32 took 17.8 ms; with 64 and a few spills 16.2.
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_set_p2etc(DevModel M, int update_theta) {
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_set_p2etc(DevModel M, int update_theta, int layers) {
   if (epic_member(M)) return;
   extern __shared__ double sm[];
   __shared__ double s_lp[32];
@@ -442,7 +444,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_set_p2etc(DevModel 
         CT(HL, k) = hl;
         M.hdry[x] = dmaxr(M.h_min[k], hl);
       }
-      CT(PP, k) = xpow(M, pk, kp1);
+      if (layers) CT(PP, k) = xpow(M, pk, kp1);
       if (update_theta && k < ks - 1) {   // the diagnostic THETA above k_sigma-1
         const double sigma = qdiv(xlog(M, qdiv(pk, pbot)), lp);
         double gs;
@@ -453,7 +455,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_set_p2etc(DevModel 
       }
     }
   __syncthreads();
-  if (!c.valid) return;
+  if (!c.valid || !layers) return;
   for (int k = 1 + c.warp; k <= nk; k += c.nw) {
     const long long x = c.base + k * n2;
     const double top = CT(P, k - 1), bot = CT(P, k);
@@ -498,7 +500,9 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_set_p2etc(DevModel 
 // the first DZDT3 terms.  Shared arrays: P, R (RHO3), T3, LG (log of successive pressure
 // ratios), GZ (the Leslie-Purser increments, then the running sum in place), Q (P/RHO3, each
 // level's quotient once for the four increments that read it).
-template <int THREADS>
+// FULL = false: GZ3 alone and its check, for the step's call before the filtered-GZ copy, whose other
+// outputs the call after stage 11 rewrites before anything reads them.
+template <int THREADS, bool FULL>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_pgrad_vars_column(DevModel M) {
   if (epic_member(M)) return;
   extern __shared__ double sm[];
@@ -513,15 +517,17 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_pgrad_vars_column(D
       const long long x = c.base + k * n2;
       const double theta = M.theta[x], p = M.p3[x];
       const double t3 = return_temp(M, p, theta);
-      M.t3[x] = t3;
-      M.exner3[x] = qdiv(M.cp * t3, theta);
       const double rho = return_density(p, t3, mu);
-      M.rho3[x] = rho;
+      if (FULL) {
+        M.t3[x] = t3;
+        M.exner3[x] = qdiv(M.cp * t3, theta);
+        M.rho3[x] = rho;
+      }
       CT(P, k) = p;
       CT(R, k) = rho;
-      CT(T3, k) = t3;
+      if (FULL) CT(T3, k) = t3;
       CT(Q, k) = qdiv(p, rho);
-      if (k >= 1) {
+      if (FULL && k >= 1) {
         const double pr = M.p2[x];
         const double t2 = return_temp(M, pr, M.theta2[x]);
         M.t2[x] = t2;
@@ -533,7 +539,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_pgrad_vars_column(D
   __syncthreads();
   if (c.valid) {
     for (int k = c.warp; k < nk; k += c.nw) CT(LG, k) = xlog(M, qdiv(CT(P, k + 1), CT(P, k)));
-    if (c.warp == c.nw - 1) {
+    if (FULL && c.warp == c.nw - 1) {
       M.rho2[c.base] = qdiv(CT(R, 0) * CT(R, 0), s_rho2_1[c.lane]);
       M.theta2[c.base] = M.sgth[0];
       M.t2[c.base] = CT(T3, 0);
@@ -566,18 +572,20 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_pgrad_vars_column(D
   for (int k = c.warp; k <= nk; k += c.nw) {
     const long long x = c.base + k * n2;
     const double gzk = CT(GZ, k);
-    const double old = M.gz3[x];
+    const double old = FULL ? M.gz3[x] : 0.;
     M.gz3[x] = gzk;
-    M.mont3[x] = gzk + return_enthalpy(M, CT(T3, k));
+    if (FULL) M.mont3[x] = gzk + return_enthalpy(M, CT(T3, k));
     if (interior && k >= 1) {
-      // DZDT3 = -(GZ3_new - GZ3_old)/(dt*g) from the third step on, 0 before (:3679-3693, :3897-3909)
-      double dz = 0.;
-      if (itime > 1) {
-        const double dtg_inv = qdiv(-1., M.dt * M.grav[2 * c.j + 1]);
-        dz = (old - gzk) * dtg_inv;
+      if (FULL) {
+        // DZDT3 = -(GZ3_new - GZ3_old)/(dt*g) from the third step on, 0 before (:3679-3693, :3897-3909)
+        double dz = 0.;
+        if (itime > 1) {
+          const double dtg_inv = qdiv(-1., M.dt * M.grav[2 * c.j + 1]);
+          dz = (old - gzk) * dtg_inv;
+        }
+        dz += qdiv(M.w3[x] * M.h3[x], CT(R, k));
+        M.dzdt3[x] = dz;
       }
-      dz += qdiv(M.w3[x] * M.h3[x], CT(R, k));
-      M.dzdt3[x] = dz;
       if (gzk >= CT(GZ, k - 1)) flag_error(M.ctl, ERR_GZ_MONOTONE, k, c.j, c.i, gzk);
     }
   }
@@ -1025,8 +1033,8 @@ int launch_restore_mass(const DevModel &M, cudaStream_t s) {
 int launch_set_p2etc(const DevModel &M, int update_theta, cudaStream_t s, bool early) {
   if (M.col64) k_set_p2etc_acc<<<zg(ntile_blocks(M), M), CT_THREADS, tile_smem(M, 4), s>>>(M, update_theta, !early);
   else if (M.mixed) k_set_p2etc_mixed<<<zg(ntile_blocks(M), M), CT_THREADS, tile_smem(M, 3), s>>>(M, update_theta, !early);
-  else if (tile_threads(M) == CT_THREADS) k_set_p2etc<CT_THREADS><<<zg(ntile_blocks(M), M), CT_THREADS, tile_smem(M, 4), s>>>(M, update_theta);
-  else k_set_p2etc<CT_THREADS_WIDE><<<zg(ntile_blocks(M), M), CT_THREADS_WIDE, tile_smem(M, 4), s>>>(M, update_theta);
+  else if (tile_threads(M) == CT_THREADS) k_set_p2etc<CT_THREADS><<<zg(ntile_blocks(M), M), CT_THREADS, tile_smem(M, 4), s>>>(M, update_theta, !early);
+  else k_set_p2etc<CT_THREADS_WIDE><<<zg(ntile_blocks(M), M), CT_THREADS_WIDE, tile_smem(M, 4), s>>>(M, update_theta, !early);
   return 0;
 }
 // The gas-giant lower boundary of store_pgrad_vars (epic_funcs_diag.c:3779-3811) with gz_from_u
@@ -1153,16 +1161,19 @@ int launch_store_pgrad_vars(const DevModel &M, cudaStream_t s, bool early, bool 
   const dim3 grid = zg(ntile_blocks(M), M);
   const size_t smem = tile_smem(M, 5);
   const bool h2 = M.x_h2 != 0.;
-  if (M.mixed && early) {   // GZ3 alone: no DZDT3, so no horizontal part either
+  if (M.mixed && early) {
     if (M.col64) (h2 ? k_gz3_column_acc_h2 : k_gz3_column_acc)<<<grid, CT_THREADS, smem, s>>>(M);
     else (h2 ? k_pgrad_vars_column_mixed<false, true> : k_pgrad_vars_column_mixed<false, false>)<<<grid, CT_THREADS, smem, s>>>(M);
     return 0;
   }
   if (M.col64) (h2 ? k_pgrad_vars_column_acc_h2 : k_pgrad_vars_column_acc)<<<grid, CT_THREADS, smem, s>>>(M);
   else if (M.mixed) (h2 ? k_pgrad_vars_column_mixed<true, true> : k_pgrad_vars_column_mixed<true, false>)<<<grid, CT_THREADS, smem, s>>>(M);
-  else if (tile_threads(M) == CT_THREADS) k_pgrad_vars_column<CT_THREADS><<<grid, CT_THREADS, tile_smem(M, 6), s>>>(M);
-  else k_pgrad_vars_column<CT_THREADS_WIDE><<<grid, CT_THREADS_WIDE, tile_smem(M, 6), s>>>(M);
-  return dzdt ? launch_pgrad_dzdt(M, s) : 0;
+  else {
+    const bool wide = tile_threads(M) != CT_THREADS;
+    (wide ? (early ? k_pgrad_vars_column<CT_THREADS_WIDE, false> : k_pgrad_vars_column<CT_THREADS_WIDE, true>)
+          : (early ? k_pgrad_vars_column<CT_THREADS, false> : k_pgrad_vars_column<CT_THREADS, true>))<<<grid, tile_threads(M), tile_smem(M, 6), s>>>(M);
+  }
+  return dzdt && !early ? launch_pgrad_dzdt(M, s) : 0;
 }
 int launch_pgrad_dzdt(const DevModel &M, cudaStream_t s) {
   EPIC_MARCH(M.mixed, k_pgrad_dzdt, M.nk, M.nj + 1, TB(M, TB_UPDATE), s, M);
@@ -1188,8 +1199,10 @@ int column_kernels_init(int) {
       cudaFuncSetAttribute(k_calc_w<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
       cudaFuncSetAttribute(k_set_p2etc<CT_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
       cudaFuncSetAttribute(k_set_p2etc<CT_THREADS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
-      cudaFuncSetAttribute(k_pgrad_vars_column<CT_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
-      cudaFuncSetAttribute(k_pgrad_vars_column<CT_THREADS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
+      cudaFuncSetAttribute(k_pgrad_vars_column<CT_THREADS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
+      cudaFuncSetAttribute(k_pgrad_vars_column<CT_THREADS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
+      cudaFuncSetAttribute(k_pgrad_vars_column<CT_THREADS_WIDE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
+      cudaFuncSetAttribute(k_pgrad_vars_column<CT_THREADS_WIDE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
       cudaFuncSetAttribute(k_set_p2etc_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
       cudaFuncSetAttribute(k_pgrad_vars_column_mixed<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||
       cudaFuncSetAttribute(k_pgrad_vars_column_mixed<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) != cudaSuccess ||

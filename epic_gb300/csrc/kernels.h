@@ -113,12 +113,12 @@ int launch_calc_w(const DevModel &M, cudaStream_t s, bool with_source_sink = fal
 int launch_uv_drag(const DevModel &M, cudaStream_t s);
 int launch_hsu_vertical(const DevModel &M, double *buff, int kind, cudaStream_t s);
 int launch_restore_mass(const DevModel &M, cudaStream_t s);
-// early: the calls inside advection (set_p2etc) and before the filtered-GZ copy
+// early: the step's calls inside advection (set_p2etc) and before the filtered-GZ copy
 // (store_pgrad_vars), whose outputs but P3, HDRY and GZ3 stage 11 and stage 19 rewrite before
-// anything reads them.  The mixed forms compute only those there (EPIC_PREC_MIXED with its
+// anything reads them: only those are computed (EPIC_PREC_MIXED with its
 // double-float kernels, which also leave the interfaces' logarithms for store_pgrad_vars:
 // GZ3 places the 3-D filter's profiles, so it needs their accuracy; EPIC_PREC_MIXED_FAST with
-// its FP32 ones).  The FP64 form writes everything in every call, as the reference does.
+// its FP32 ones; the FP64 form in binary64, where a power takes as long as ten products).
 int launch_set_p2etc(const DevModel &M, int update_theta, cudaStream_t s, bool early = false);
 // dzdt: its horizontal part of DZDT3 too (launch_pgrad_dzdt).
 int launch_store_pgrad_vars(const DevModel &M, cudaStream_t s, bool early = false, bool dzdt = true);
