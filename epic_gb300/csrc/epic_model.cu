@@ -259,14 +259,14 @@ int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
     case 21: if (M.turb) launch_source_sink_turb(M, s); break;
     case 22:
       if (M.turb) {
-        launch_theta_hdiff(M, s);
+        launch_theta_hdiff(M, s, false);
         launch_nu_hdiff(M, s);
       }
       break;
     case 23:
       if (M.turb) {
         launch_tau_wall_h(M, M.work0, s);
-        launch_theta_vdiff(M, s);
+        launch_theta_vdiff(M, s, false);
         launch_nu_vdiff(M, M.work0, s);
       }
       break;
@@ -376,7 +376,7 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
     L.after(0, 1);   // the subgrid diffusion's set_p2etc rewrites P3 and H3, which lane 1 reads
     L.after(3, 0);
     if (M.turb_h) {
-      launch_theta_hdiff(M, L[0]);
+      launch_theta_hdiff(M, L[0], true);
       launch_nu_hdiff(M3, L[3]);
     }
     L.after(2, 0);
@@ -394,7 +394,7 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
     L.after(0, 2);
     L.after(3, 2);
     if (M.turb_v) {
-      launch_theta_vdiff(M, L[0]);
+      launch_theta_vdiff(M, L[0], true);
       launch_nu_vdiff(M, M2.work0, L[3]);
     }
     L.after(3, 0);

@@ -893,9 +893,9 @@ static int laplacian_step(const DevModel &M, double *var, const double *dc, int 
   return 0;
 }
 
-int launch_theta_hdiff(const DevModel &M, cudaStream_t s) {
+int launch_theta_hdiff(const DevModel &M, cudaStream_t s, bool early) {
   laplacian_step(M, M.theta, M.dc_theta, 0, M.k_sigma - 1, s);
-  return launch_set_p2etc(M, 1, s);
+  return launch_set_p2etc(M, 1, s, early);
 }
 int launch_nu_hdiff(const DevModel &M, cudaStream_t s) {
   laplacian_step(M, M.nu_turb, nullptr, 1, 1, s);
@@ -913,9 +913,9 @@ int launch_tau_wall_h(const DevModel &M, double *tw, cudaStream_t s) {
   return 0;
 }
 
-int launch_theta_vdiff(const DevModel &M, cudaStream_t s) {
+int launch_theta_vdiff(const DevModel &M, cudaStream_t s, bool early) {
   launch_vdiff(M, VD_THETA, nullptr, s);
-  return launch_set_p2etc(M, 1, s);
+  return launch_set_p2etc(M, 1, s, early);
 }
 int launch_nu_vdiff(const DevModel &M, const double *tw, cudaStream_t s) {
   launch_vdiff(M, VD_NU, tw, s);
