@@ -80,6 +80,8 @@ struct DevModel {
   const double *h_coef, *v_coef;            // d2dy2 coefficients, 3 per row
   const double *rt64;                       // RowTab of rows 0..nj+1, RT_COUNT values each, in binary64 ...
   const float *rt32;                        // ... and in binary32
+  const double *vt64;                       // d2dy2's coefficients times the orders' 2, 4, 6 and 8: 12 a row, h rows
+  const float *vt32;                        // 0..nj+1, then v rows (k_visc_tables), in both compute types
   const double *tw;                         // realft/four1 twiddles (see k_filter.cu)
   const double *coslat;                     // cos(lat[2j+1] deg), j = 0..nj, from the host libm
   const double *coslat4;                    // pow(coslat[j], 4.) correctly rounded (t_rad's cos^4)
@@ -579,6 +581,15 @@ __device__ __forceinline__ R hsu_upwind(R w, R a_minus, R a_plus) { return w * (
 template <class R> __device__ __forceinline__ R rt(const DevModel &M, int j, int q);
 template <> __device__ __forceinline__ double rt<double>(const DevModel &M, int j, int q) { return M.rt64[j * RT_COUNT + q]; }
 template <> __device__ __forceinline__ float rt<float>(const DevModel &M, int j, int q) { return M.rt32[j * RT_COUNT + q]; }
+
+// the three coefficients of d2dy2 of an order (2, 4, 6, 8) at row j
+template <class R> __device__ __forceinline__ const R *visc_coef(const DevModel &M, int vgrid, int order, int j);
+template <> __device__ __forceinline__ const double *visc_coef<double>(const DevModel &M, int vgrid, int order, int j) {
+  return M.vt64 + ((vgrid ? M.nj + 2 : 0) + j) * 12 + 3 * (order / 2 - 1);
+}
+template <> __device__ __forceinline__ const float *visc_coef<float>(const DevModel &M, int vgrid, int order, int j) {
+  return M.vt32 + ((vgrid ? M.nj + 2 : 0) + j) * 12 + 3 * (order / 2 - 1);
+}
 
 struct Trip { double x, y, z; };
 

@@ -648,7 +648,7 @@ size_t model_pool_bytes(const epic_grid &g) {
   return rnd(sizeof(Ctl)) + (n_state3 + n_scratch3) * rnd(n3 * 8) + 3 * rnd(n2 * 8) + rnd((size_t)epic::TABLE_SETS * (g.nj + 3) * (g.nk + 2) * 3 * 8) +
          rnd(ni1 * 8) + 10 * rnd(nj1 * 8) + 3 * rnd(nk1 * 8) + rnd((g.nk + 2) * 8) + rnd((g.k_sponge + 1) * 8) +
          2 * rnd(3 * (g.nj + 2) * 8) + rnd(ntw * 8) + rnd(ntw * 4) + 2 * rnd((g.nj + 1) * 8) + rnd(sizeof(epic::MathTable)) +
-         rnd(32 * sizeof(float2)) + rnd((size_t)(g.nj + 2) * epic::RT_COUNT * 8) + rnd((size_t)(g.nj + 2) * epic::RT_COUNT * 4) + rnd(((size_t)epic::TH_N * epic::TH_M + 4 * epic::TH_M + epic::TH_N) * 8) +
+         rnd(32 * sizeof(float2)) + rnd((size_t)(g.nj + 2) * epic::RT_COUNT * 8) + rnd((size_t)(g.nj + 2) * epic::RT_COUNT * 4) + rnd((size_t)(g.nj + 2) * 24 * 8) + rnd((size_t)(g.nj + 2) * 24 * 4) + rnd(((size_t)epic::TH_N * epic::TH_M + 4 * epic::TH_M + epic::TH_N) * 8) +
          (g.turbulence ? 4 * rnd(n3 * 8) + rnd(2 * (size_t)(g.nk + 2) * 8) + rnd((size_t)(g.nj + 1) * 8) : 0) + 4096;
 }
 
@@ -813,6 +813,8 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
   float2 *exp2tab = carve<float2>(p, 32);
   d.rt64 = carve<double>(p, (size_t)(g->nj + 2) * epic::RT_COUNT);
   d.rt32 = carve<float>(p, (size_t)(g->nj + 2) * epic::RT_COUNT);
+  d.vt64 = carve<double>(p, (size_t)(g->nj + 2) * 24);
+  d.vt32 = carve<float>(p, (size_t)(g->nj + 2) * 24);
   double *thermo_d = carve<double>(p, (size_t)epic::TH_N * epic::TH_M + 4 * epic::TH_M + epic::TH_N);
   if (d.turb) {   // the turbulence closure: NU_TURB, the three diffusivities (one stride apart, as
                   // relocate_field expects), scratch and a row table

@@ -59,6 +59,20 @@ __global__ void k_row_tables(DevModel M, R *out) {
   t[RT_F_V] = cv<R>(M.f[jj]);
 }
 
+// d2dy2's coefficients times the viscosity coefficient of each order that uses them, once per model:
+// the FP64 form's hyperviscosity is bound by the FP64 pipe (19 cycles a warp instruction and SM), and
+// three of a point's products depend on its row alone.  The same products, so the same bits.  12 steps
+// of 128x64x20 10.47 -> 10.23 ms, 3 of
+// 256x128x32 15.2 -> 15.0 ms.
+template <class R>
+__global__ void k_visc_tables(DevModel M, R *out) {
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x), rows = M.nj + 2;
+  if (t >= 24 * rows) return;
+  const int v = t / (12 * rows), j = (t - v * 12 * rows) / 12, q = t % 12, order = 2 * (q / 3) + 2;
+  const double c = order == 2 ? M.coef[2] : (order == 4 ? M.coef[4] : (order == 6 ? M.coef[6] : M.coef[8]));
+  out[t] = j <= (v ? M.nj + 1 : M.nj) ? cv<R>(c) * cv<R>((v ? M.v_coef : M.h_coef)[3 * j + q % 3]) : R(0.);
+}
+
 // memset of DUDT, DVDT(it_uv_tend), epic_timestep.c:107-108
 __global__ void k_zero_tend(DevModel M) {
   if (epic_member(M)) return;
@@ -815,15 +829,13 @@ template <class R>
 __global__ void k_d2dy2(DevModel M, const double *src, int src_sel, double *dst, int vgrid, int order, int k0, int nkk,
                         int of_state) {
   if (epic_member(M, src, dst)) return;
-  // the member's own coefficient (it depends on dt and dy0): order 2, 4, 6 or 8, constant indices
-  const double diff_coef = order == 2 ? M.coef[2] : (order == 4 ? M.coef[4] : (order == 6 ? M.coef[6] : M.coef[8]));
   Cell c;
   const int nrows = vgrid ? M.nj + 2 : M.nj + 1;   // v: j = 0..nj+1, h: j = 0..nj
   if (!cell3(M, k0, nkk, 0, nrows, c)) return;
   src += plane_offset(M, src_sel);
   const int k = c.k, j = c.j, i = c.i, nj = M.nj;
-  const double *cf = (vgrid ? M.v_coef : M.h_coef) + 3 * j;
-  const R a0 = cv<R>(diff_coef) * cv<R>(cf[0]), a1 = cv<R>(diff_coef) * cv<R>(cf[1]), a2 = cv<R>(diff_coef) * cv<R>(cf[2]);
+  const R *cf = visc_coef<R>(M, vgrid, order, j);   // the member's own (they depend on dt and dy0)
+  const R a0 = cf[0], a1 = cf[1], a2 = cf[2];
   auto h = [&](int jj) { return cv<R>(src[M.at(k, jj, i)]); };
   R d;
   const int jlast = vgrid ? nj + 1 : nj;
@@ -850,7 +862,6 @@ template <class R>
 __global__ void __launch_bounds__(256) k_d2dy2_pair(DevModel M, const double *src, int src_sel, double *dst, int vgrid, int k0, int TC) {
   if (epic_member(M, src, dst)) return;
   constexpr bool exact = std::is_same_v<R, double>;
-  const double coef1 = M.coef[2], coef2 = M.coef[4];
   extern __shared__ __align__(16) unsigned char smraw[];
   src += plane_offset(M, src_sel);
   const int tx = (int)threadIdx.x & (TC - 1), ty = (int)threadIdx.x / TC, ny = (int)blockDim.x / TC;
@@ -858,16 +869,15 @@ __global__ void __launch_bounds__(256) k_d2dy2_pair(DevModel M, const double *sr
   const int i = (int)blockIdx.x * TC + tx + 1;
   const int k = k0 + (int)blockIdx.y;
   const int nj = M.nj, jlast = vgrid ? nj + 1 : nj;
-  const double *cfa = vgrid ? M.v_coef : M.h_coef;
   const bool live = i <= M.ni;
   for (int j = ty; j <= jlast; j += ny) {
     R d = R(0.);
     if (live) {
-      const double *cf = cfa + 3 * j;
-      const R a0 = cv<R>(coef1) * cv<R>(cf[0]), a2 = cv<R>(coef1) * cv<R>(cf[2]);
+      const R *cf = visc_coef<R>(M, vgrid, 2, j);
+      const R a0 = cf[0], a2 = cf[2];
       const int m = j == 0 ? 1 : (j == jlast ? j - 1 : j);
       const double hm = src[M.at(k, m, i)];
-      if constexpr (exact) d = a0 * src[M.at(k, m - 1, i)] + coef1 * cf[1] * hm + a2 * src[M.at(k, m + 1, i)];
+      if constexpr (exact) d = a0 * src[M.at(k, m - 1, i)] + cf[1] * hm + a2 * src[M.at(k, m + 1, i)];
       else d = a0 * cv<R>(src[M.at(k, m - 1, i)] - hm) + a2 * cv<R>(src[M.at(k, m + 1, i)] - hm);
     }
     d1[j * TC] = d;
@@ -875,8 +885,8 @@ __global__ void __launch_bounds__(256) k_d2dy2_pair(DevModel M, const double *sr
   __syncthreads();
   if (!live) return;
   for (int j = ty; j <= jlast; j += ny) {
-    const double *cf = cfa + 3 * j;
-    const R a0 = cv<R>(coef2) * cv<R>(cf[0]), a1 = cv<R>(coef2) * cv<R>(cf[1]), a2 = cv<R>(coef2) * cv<R>(cf[2]);
+    const R *cf = visc_coef<R>(M, vgrid, 4, j);
+    const R a0 = cf[0], a1 = cf[1], a2 = cf[2];
     const int m = j == 0 ? 1 : (j == jlast ? j - 1 : j);
     const R d = a0 * d1[(m - 1) * TC] + a1 * d1[m * TC] + a2 * d1[(m + 1) * TC];
     write_with_pads(dst, M, M.at(k, j, 0), i, to_d(d));
@@ -1315,6 +1325,8 @@ int launch_row_tables(const DevModel &M, cudaStream_t s) {
   const unsigned blocks = epic_blocks(M.nj + 2, 64);
   k_row_tables<double><<<blocks, 64, 0, s>>>(M, const_cast<double *>(M.rt64));
   k_row_tables<float><<<blocks, 64, 0, s>>>(M, const_cast<float *>(M.rt32));
+  k_visc_tables<double><<<epic_blocks(24LL * (M.nj + 2), 128), 128, 0, s>>>(M, const_cast<double *>(M.vt64));
+  k_visc_tables<float><<<epic_blocks(24LL * (M.nj + 2), 128), 128, 0, s>>>(M, const_cast<float *>(M.vt32));
   return 0;
 }
 

@@ -129,7 +129,7 @@ int launch_advection_prep(const DevModel &M, int phase, cudaStream_t s);
 int column_kernels_init(int nk);
 
 // k_stencil.cu -- horizontal stencils and the time update
-// the row tables (DevModel::rt64, rt32) from the 1-D grid arrays; once per model
+// the row tables (DevModel::rt64, rt32, vt64, vt32) from the 1-D grid arrays; once per model
 int launch_row_tables(const DevModel &M, cudaStream_t s);
 int launch_zero_tend(const DevModel &M, cudaStream_t s);
 int launch_uv_core(const DevModel &M, cudaStream_t s);
