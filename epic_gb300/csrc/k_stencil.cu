@@ -61,9 +61,8 @@ __global__ void k_row_tables(DevModel M, R *out) {
 
 // d2dy2's coefficients times the viscosity coefficient of each order that uses them, once per model:
 // the FP64 form's hyperviscosity is bound by the FP64 pipe (19 cycles a warp instruction and SM), and
-// three of a point's products depend on its row alone.  The same products, so the same bits.  12 steps
-// of 128x64x20 10.47 -> 10.23 ms, 3 of
-// 256x128x32 15.2 -> 15.0 ms.
+// three of a point's products depend on its row alone.  The same products, so the same bits.
+// 12 steps of 128x64x20 10.47 -> 10.23 ms, 3 of 256x128x32 15.2 -> 15.0 ms.
 template <class R>
 __global__ void k_visc_tables(DevModel M, R *out) {
   const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x), rows = M.nj + 2;
