@@ -28,9 +28,13 @@
 // and a CTA takes several groups of columns in turn.
 //
 // What bounds it: latency on a single model (a few dozen CTAs, each a chain of load, convert, multiply,
-// store), the staging and the plane traffic on a large batch.  So eight warps stage and store while one
-// more brings the operator tiles and issues the products, all through mbarriers (no block barrier in
-// the pipeline), with every tile of a short row and four chunks of plane values on their way at once.
+// store), the staging and the plane traffic on a large batch, the products' shared-memory reads (5 KB
+// each) on a long row.  So eight warps stage and store, one issues the products and one brings the
+// operator tiles, all through mbarriers (no block barrier in the pipeline), with every tile of a short
+// row and four chunks of plane values on their way at once.  With one thread for the tiles and the
+// products, 950 cycles of tile requests came between every 760 of products; an epilogue that reads its
+// row length and pointers again after each store takes twice as long.  A launch on 512x256 x 40 planes
+// 105 -> 63 us, on 64 members of 128x64 x 20 planes 75 -> 55 us, on one such model 12.3 -> 11.3 us.
 //
 // With shift set, each row of each plane is filtered as x - x(1), and x(1) is added back to the
 // output in binary64: the operator passes a constant unchanged (its wavenumber-0 weight is 1), so
@@ -59,7 +63,8 @@ constexpr int FG_M = 128;        // output points per tile (tensor-memory lanes)
 constexpr int FG_KC = 32;        // K elements per staged chunk: one 128-byte swizzle row of FP32
 constexpr int FG_NMAX = 64;      // columns per CTA ((member, plane) pairs), a multiple of 32
 constexpr int FG_STAGE = 256;    // eight staging and epilogue warps: two per 32-lane quarter of tensor memory
-constexpr int FG_THREADS = FG_STAGE + 32;   // and one that issues the operator copies and the products
+constexpr int FG_WARPS = FG_STAGE / 32;
+constexpr int FG_THREADS = FG_STAGE + 64;   // warp FG_WARPS issues the products, the next one the operator copies
 constexpr int FG_BUFS = 4;       // operator tile pairs and chunks of plane values in shared memory, each
 constexpr int FG_GROUPS = 8;     // column groups a CTA takes in turn at most
 constexpr unsigned FG_WAIT_LIMIT = 1u << 20;
@@ -146,8 +151,9 @@ __device__ __forceinline__ void mma_commit(unsigned mbar) {   // arrives once th
 // operator (fop_shared).
 //
 // Steps t count (group, K chunk c, output tile) in order.  The issuing thread waits for step t's
-// operator tiles and chunk, issues the products, commits them to the buffers they read, and refills the
-// operator buffer of step t-1 for step t-1+FG_BUFS; with `resident` (ni = 128, one tile per chunk) the
+// operator tiles and chunk, issues the products and commits them to the buffers they read; the copying
+// thread refills a buffer once the products that read it are done; with `resident` (ni = 128, one tile
+// per chunk) the
 // four buffers are filled once.  The staging threads keep FG_BUFS chunks of their columns' values in
 // registers ahead of the one they convert, across groups.  In place, the CTAs of a cluster have all read
 // a row before any writes it.
@@ -190,20 +196,40 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
   const unsigned a_full = bars_s, a_free = bars_s + 8 * FG_BUFS, b_full = a_free + 8 * FG_BUFS, b_free = b_full + 8 * FG_BUFS;
   const unsigned acc_full = b_free + 8 * FG_BUFS, acc_free = acc_full + 8;
   const uint32_t tcols = (uint32_t)(mts * N) <= 32 ? 32u : 1u << (32 - __clz(mts * N - 1));   // a power of 2 >= 32
-  if (tid == FG_STAGE) {
+  // step t's operator tiles, for offset (128 mt - kc) mod ni, hi then lo
+  const void *const fop = opm.fop_map;
+  const unsigned fop_y = (unsigned)(slot * ntiles * 2 * FG_M);
+  auto load_a = [&](int buf, int c, int mt) {
+    const int tt = (((mt0 + mt) * FG_M - c * FG_KC) & (ni - 1)) / FG_KC, y = (int)fop_y + tt * 2 * FG_M;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a_full + 8 * buf), "r"(2 * FG_A_BYTES) : "memory");
+    tma_tile(a_s + buf * 2 * FG_A_BYTES, fop, y, a_full + 8 * buf);
+    tma_tile(a_s + buf * 2 * FG_A_BYTES + FG_A_BYTES, fop, y + FG_M, a_full + 8 * buf);
+  };
+  // the copying thread's next load: group lg, chunk lc, output tile lmt; a resident operator is loaded once
+  const int steps = ngroups * nchunks * mts, loads = resident ? nchunks : steps;
+  int issued = 0, lc = 0, lmt = 0;
+  auto load_next = [&]() {
+    load_a(issued % FG_BUFS, lc, lmt);
+    issued++;
+    if (++lmt == mts) {
+      lmt = 0;
+      if (++lc == nchunks) lc = 0;
+    }
+  };
+  if (tid == FG_STAGE + 32) {
     fail = 0;
     for (int q = 0; q < FG_BUFS; q++) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(a_full + 8 * q));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(a_free + 8 * q));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(b_full + 8 * q), "r"(FG_STAGE));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(b_full + 8 * q), "r"(FG_WARPS));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b_free + 8 * q));
     }
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(acc_full));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(acc_free), "r"(FG_STAGE));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(acc_free), "r"(FG_WARPS));
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
   __syncwarp();
-  if (warp == FG_STAGE / 32) {
+  if (warp == FG_WARPS) {
     const unsigned dst_s = (unsigned)__cvta_generic_to_shared(&tmem_base);
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_s), "r"(tcols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -230,63 +256,53 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t dtmem = tmem_base;
 
-  if (warp == FG_STAGE / 32) {
-    if (lane == 0) {
+  if (warp >= FG_WARPS) {
+    if (warp == FG_WARPS && lane == 0) {
       const uint32_t idesc = idesc_tf32(N);
-      const int steps = ngroups * nchunks * mts, loads = resident ? nchunks : steps;
-      auto load_a = [&](int t) {   // step t's operator tiles, for offset (128 mt - kc) mod ni, hi then lo
-        const int c = (t / mts) % nchunks, mt = mt0 + t % mts, buf = t % FG_BUFS;
-        const int tt = ((mt * FG_M - c * FG_KC) & (ni - 1)) / FG_KC, y = ((slot * ntiles + tt) * 2) * FG_M;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a_full + 8 * buf), "r"(2 * FG_A_BYTES) : "memory");
-        tma_tile(a_s + buf * 2 * FG_A_BYTES, opm.fop_map, y, a_full + 8 * buf);
-        tma_tile(a_s + buf * 2 * FG_A_BYTES + FG_A_BYTES, opm.fop_map, y + FG_M, a_full + 8 * buf);
-      };
-      int issued = 0;
-      for (; issued < loads && issued < FG_BUFS; issued++) load_a(issued);
+      // every operand lies below 2^18 bytes: a descriptor moves by its address / 16
+      const uint64_t a_desc = smem_desc(a_s), b_desc = smem_desc(a_s + b_off);
+      const uint64_t b_lo = b_bytes >> 4;
+      constexpr uint64_t A_LO = FG_A_BYTES >> 4;
       bool ok = true;
-      int t = 0;
-      for (int n = 0; n < ngroups * nchunks && ok; n++) {   // chunks in order
-        const int gi = n / nchunks, c = n - gi * nchunks, bb = n % FG_BUFS;
-        if (c == 0 && gi > 0) {   // the accumulator read out
+      int t = 0, n = 0;
+      for (int gi = 0; gi < ngroups && ok; gi++) {
+        if (gi > 0) {   // the accumulator read out
           ok = mbar_wait(acc_free, (unsigned)((gi - 1) & 1), &fail);
           asm volatile("tcgen05.fence::after_thread_sync;");
         }
-        ok = ok && mbar_wait(b_full + 8 * bb, (unsigned)((n / FG_BUFS) & 1), &fail);
-        for (int mt = 0; mt < mts && ok; mt++, t++) {
-          const int ab = t % FG_BUFS;
-          ok = mbar_wait(a_full + 8 * ab, resident ? 0u : (unsigned)((t / FG_BUFS) & 1), &fail);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;");
-          const unsigned a_hi = a_s + ab * 2 * FG_A_BYTES, a_lo = a_hi + FG_A_BYTES;
-          const unsigned b_hi = a_s + b_off + bb * 2 * b_bytes, b_lo = b_hi + b_bytes;
-          const uint32_t d_mt = dtmem + (uint32_t)(mt * N);
-          for (int ks = 0; ks < FG_KC / 8; ks++) {   // K = 8 TF32 (32 bytes) per instruction
-            const unsigned koff = (unsigned)ks * 32;
-            mma_tf32(d_mt, smem_desc(a_hi + koff), smem_desc(b_hi + koff), idesc, (c > 0 || ks > 0) ? 1u : 0u);
-            mma_tf32(d_mt, smem_desc(a_hi + koff), smem_desc(b_lo + koff), idesc, 1u);
-            mma_tf32(d_mt, smem_desc(a_lo + koff), smem_desc(b_hi + koff), idesc, 1u);
+        for (int c = 0; c < nchunks && ok; c++, n++) {   // chunks in order
+          const int bb = n % FG_BUFS;
+          const uint64_t b = b_desc + (uint64_t)bb * 2 * b_lo;
+          ok = mbar_wait(b_full + 8 * bb, (unsigned)((n / FG_BUFS) & 1), &fail);
+          for (int mt = 0; mt < mts && ok; mt++, t++) {
+            const int ab = t % FG_BUFS;
+            ok = mbar_wait(a_full + 8 * ab, resident ? 0u : (unsigned)((t / FG_BUFS) & 1), &fail);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            const uint64_t a = a_desc + (uint64_t)ab * 2 * A_LO;
+            const uint32_t d_mt = dtmem + (uint32_t)(mt * N);
+#pragma unroll
+            for (int ks = 0; ks < FG_KC / 8; ks++) {   // K = 8 TF32 (32 bytes) per instruction
+              mma_tf32(d_mt, a + 2 * ks, b + 2 * ks, idesc, ks > 0 ? 1u : (uint32_t)(c > 0));
+              mma_tf32(d_mt, a + 2 * ks, b + b_lo + 2 * ks, idesc, 1u);
+              mma_tf32(d_mt, a + A_LO + 2 * ks, b + 2 * ks, idesc, 1u);
+            }
+            // commits complete in issue order: the accumulator's is the last of a group
+            if (!resident) mma_commit(a_free + 8 * ab);
           }
-          // commits complete in issue order: the accumulator's is the last of a group
-          if (!resident) mma_commit(a_free + 8 * ab);
-          if (mt == mts - 1) {
-            mma_commit(b_free + 8 * bb);
-            if (c == nchunks - 1) mma_commit(acc_full);
-          }
-          if (!resident && t >= 1 && issued < loads) {   // step t-1's buffer, its products done while step t's run
-            const int pb = (t - 1) % FG_BUFS;
-            ok = mbar_wait(a_free + 8 * pb, (unsigned)(((t - 1) / FG_BUFS) & 1), &fail);
-            if (ok) load_a(issued++);
-          }
+          if (ok) mma_commit(b_free + 8 * bb);
         }
+        if (ok) mma_commit(acc_full);
       }
-      // an operator copy whose step was never reached is waited for (bounded by the limit), so that
-      // nothing writes this CTA's shared memory after it is released
-      if (!ok)
-        for (int q = 0; q < issued; q++)
-          if (q + FG_BUFS >= issued) {
-            int none = 0;
-            mbar_wait(a_full + 8 * (q % FG_BUFS), (unsigned)((q / FG_BUFS) & 1), &none);
-          }
+    } else if (warp > FG_WARPS && lane == 0) {
+      while (issued < loads && issued < FG_BUFS) load_next();
+      while (issued < loads && mbar_wait(a_free + 8 * (issued % FG_BUFS), (unsigned)((issued / FG_BUFS - 1) & 1), &fail)) load_next();
+      // the copies in flight are waited for (bounded by the limit) whether or not their steps are reached,
+      // so that nothing writes this CTA's shared memory after it is released
+      for (int q = issued > FG_BUFS ? issued - FG_BUFS : 0; q < issued; q++) {
+        int none = 0;
+        mbar_wait(a_full + 8 * (q % FG_BUFS), (unsigned)((q / FG_BUFS) & 1), &none);
+      }
     }
     __syncwarp();
     if (msplit > 1)
@@ -296,13 +312,14 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
       }
   } else {
     // B[n][e] = x_n(kc + e + 1) - x1_n, zero in idle columns: thread tid converts 4 neighbouring values of
-    // column tid/8 and, for N = 64, of column 32 + tid/8, in every chunk
+    // column tid/8 and, for N = 64, of column 32 + tid/8, in every chunk (a column per warp, whole rows of 256
+    // bytes a load, is slower: four times the stores and row pointers, 64 members 71 -> 80 us a launch)
     constexpr int BQ = FG_NMAX * FG_KC / 4 / FG_STAGE;   // 2
-    const int nq = N * (FG_KC / 4) / FG_STAGE, e0 = 4 * (tid % (FG_KC / 4));
+    const int nq = N * (FG_KC / 4) / FG_STAGE, e0 = 4 * (tid % (FG_KC / 4)), lg_nchunks = 31 - __clz(nchunks);
     const int total = ngroups * nchunks;
     double breg[FG_BUFS][BQ][4];
     auto load_b = [&](int n, double (&bn)[BQ][4]) {
-      const int gi = n / nchunks, kc = (n - gi * nchunks) * FG_KC;
+      const int gi = n >> lg_nchunks, kc = (n & (nchunks - 1)) * FG_KC;
 #pragma unroll
       for (int u = 0; u < BQ; u++) {
         if (u >= nq) break;
@@ -334,20 +351,25 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                 : "r"(taddr));
+            double *row[16];   // read before the stores, which might overlap anything
+#pragma unroll
+            for (int n = 0; n < 16; n++) row[n] = s_dst[gi][cg + n];
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             const int i = (mt0 + mt) * FG_M + (warp & 3) * 32 + lane + 1;
+            const int pad = i == ni ? 0 : (i == 1 ? ni + 1 : i);   // ni is at least FG_M
 #pragma unroll
             for (int n = 0; n < 16; n++) {
-              double *row = s_dst[gi][cg + n];
-              if (row) {
-                const double y = f2d(__uint_as_float(r[n]));
-                write_with_pads(row, Mg, 0, i, shift ? y + s_x1[gi][cg + n] : y);
-              }
+              if (!row[n]) continue;
+              double y = f2d(__uint_as_float(r[n]));
+              if (shift) y += s_x1[gi][cg + n];
+              row[n][i] = y;
+              if (pad != i) row[n][pad] = y;
             }
           }
       }
       asm volatile("tcgen05.fence::before_thread_sync;");
-      mbar_arrive(acc_free);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_free);
     };
     for (int n0 = 0; n0 < total; n0 += FG_BUFS) {
 #pragma unroll
@@ -356,7 +378,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
         if (n >= total) break;
         if (n >= FG_BUFS) mbar_wait(b_free + 8 * q, (unsigned)((n / FG_BUFS - 1) & 1), &fail);
         unsigned char *bh = fg_smem + b_off + q * 2 * b_bytes, *bl = bh + b_bytes;
-        const int gi = n / nchunks;
+        const int gi = n >> lg_nchunks;
 #pragma unroll
         for (int u = 0; u < BQ; u++) {
           if (u >= nq) break;
@@ -372,7 +394,8 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
           *reinterpret_cast<float4 *>(bl + off) = make_float4(b4.x - hv.x, b4.y - hv.y, b4.z - hv.z, b4.w - hv.w);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_arrive(b_full + 8 * q);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_full + 8 * q);
         if (n + FG_BUFS < total) load_b(n + FG_BUFS, breg[q]);
         if (n + 1 == (gi + 1) * nchunks) epilogue(gi);
       }
@@ -391,7 +414,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
     }
     __syncthreads();
   }
-  if (warp == FG_STAGE / 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(dtmem), "r"(tcols));
+  if (warp == FG_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(dtmem), "r"(tcols));
 }
 
 // dynamic shared memory of a CTA with N columns: operator buffers, plane buffers, the alignment slack of
@@ -415,9 +438,11 @@ int launch_filter_planes_gemm(const DevModel &M, const double *src, int src_sel,
   const int units = nch * ((members + G - 1) / G);
   const int sms = g_sms > 0 ? g_sms : 152, mtiles = M.ni / FG_M, rows = (M.nj + 3) / 2;   // about half the rows are filtered
   // one CTA per SM (its buffers fill the shared memory).  Few units: a cluster of CTAs shares a row's
-  // output tiles (each tile's sums are unchanged) until every SM has one.
+  // output tiles (each tile's sums are unchanged) as long as they are all resident at once: a second
+  // round pays the setup, the first loads and the staging of the whole row again (512x256 x 40 planes:
+  // one round of 129 CTAs 70 us, two of 258 half as long each 87 us, before the epilogue above).
   int msplit = 1;
-  while (2 * msplit <= mtiles && (long long)rows * units * msplit < sms) msplit *= 2;
+  while (2 * msplit <= mtiles && (long long)rows * units * msplit * 2 <= sms) msplit *= 2;
   // many units, and the row's operator in the four buffers: a CTA takes several groups
   const int resident = M.ni == FG_KC * FG_BUFS && (M.fop_shared || !M.batch);
   int gs = units;
