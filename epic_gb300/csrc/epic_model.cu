@@ -343,7 +343,8 @@ DevModel with_scratch(const DevModel &M, int ws, int ts) {
 
 // One step (timestep(STEP_PROGS_AND_SYNC_DIAGS), epic_timestep.c:130-390), the stages of
 // run_stage_on in an order of the same dependences.  Scratch: lanes 0, 1 / 3 and 2 hold sets 0, 1
-// and 2 of work0..3 (lane 1's uv_core takes work0 alone, lane 3's scalars work1..3).
+// and 2 of work0..3 (lane 1's uv_core takes work0 alone, lane 3's scalars work1..3; NU_TURB's horizontal
+// diffusion takes set 1 whole, on lane 3 once lane 1 is done with it).
 int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
   using namespace epic;
   Lanes one(s);

@@ -1,13 +1,15 @@
 // log2 and exp2 in 64- and 128-bit fixed point on the integer pipe: the fast paths of the
-// correctly rounded log, exp and pow (dd_math.cuh).
+// correctly rounded log, exp and pow (dd_math.cuh).  Below them div_rn and sqrt_rn, the correctly
+// rounded quotient and root on the same pipe.
 //
-// GB300 retires about two binary64 operations a clock and SM, so one takes a warp 16 clocks; a
-// 32 x 32 -> 64 bit multiply-add takes it one or two.  The double-double fast paths these replace
+// GB300 retires under two binary64 operations a clock and SM: a warp instruction takes 19 clocks (64 in a
+// chain), a 32 x 32 -> 64 bit multiply-add one or two.  The double-double fast paths these replace
 // spend about 125 binary64 operations on a pow (2000 clocks a warp); these spend about 200 integer
 // ones.  Measured on a GB300 (FP64 form): 12 steps of 128x64x20 with its transfers 29.7 -> 20.5 ms, 3
 // steps of 256x128x32 43.3 -> 29.1 ms; the column kernels that evaluate them (set_p2etc,
-// store_pgrad_vars, calc_w) were two thirds of the step.  The results are the same bits: each path only returns a value whose whole error interval
-// rounds to one binary64 number, and leaves the rest to the double-double evaluation.
+// store_pgrad_vars, calc_w) were two thirds of the step.  The results are the same bits: each path only
+// returns a value whose whole error interval rounds to one binary64 number, and leaves the rest to the
+// double-double evaluation.
 //
 // Methods (textbook fixed point): log2(x) = e + log2(c) + log2(1 + r) with a table over the ten
 // leading bits of the significand m of 1/c rounded up to 20 bits, so that 1 + r = m / c is the
