@@ -1072,7 +1072,7 @@ __global__ void __launch_bounds__(256) k_gz_means(DevModel M) {
     const double *v = gm + threadIdx.x * ni;
     double sum = 0.;
     for (int I = 0; I < ni; I++) sum += v[I];
-    M.pv3[(long long)(K + 1) * M.n2 + M.at2(J, (int)threadIdx.x)] = sum / ni;
+    M.pv3[(long long)(K + 1) * M.n2 + M.at2(J, (int)threadIdx.x)] = sum * inv_pow2(ni);
   }
 }
 

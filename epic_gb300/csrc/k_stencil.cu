@@ -228,8 +228,21 @@ __global__ void k_uv_core_u(DevModel M) {
 constexpr size_t ROW_SUM_SMEM = 48 * 1024;
 static __device__ __forceinline__ double row_sum(const double *row, int n) {
   double sum = 0.;
-#pragma unroll 8
-  for (int i = 0; i < n; i++) sum += row[i];
+  if (n < 16) {
+    for (int i = 0; i < n; i++) sum += row[i];
+    return sum;
+  }
+  double b[8], c[8];   // n is a power of 2; the next eight values come while these are added
+#pragma unroll
+  for (int q = 0; q < 8; q++) b[q] = row[q];
+  for (int i = 8; i < n; i += 8) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) c[q] = row[i + q];
+#pragma unroll
+    for (int q = 0; q < 8; q++) sum += b[q], b[q] = c[q];
+  }
+#pragma unroll
+  for (int q = 0; q < 8; q++) sum += b[q];
   return sum;
 }
 // levels per block of a kernel that sums `rows` rows of each, one per lane of a warp
@@ -257,7 +270,7 @@ __global__ void __launch_bounds__(256) k_gz_pole_rows(DevModel M, int lv) {
     rows[r * (ni + 1) + i] = M.gz3[M.at(k0 + (r >> 1), (r & 1) ? M.nj : 0, i + 1)];
   }
   __syncthreads();
-  if ((int)threadIdx.x < 2 * nl) avg[threadIdx.x] = row_sum(rows + (int)threadIdx.x * (ni + 1), ni) / ni;
+  if ((int)threadIdx.x < 2 * nl) avg[threadIdx.x] = row_sum(rows + (int)threadIdx.x * (ni + 1), ni) * inv_pow2(ni);
   __syncthreads();
   for (int t = (int)threadIdx.x; t < 2 * nl * (ni + 2); t += (int)blockDim.x) {
     const int r = t / (ni + 2), i = t - r * (ni + 2);
@@ -933,44 +946,56 @@ __device__ __forceinline__ void visc_row(const DevModel &M, const double *A, con
 // Bound by those additions: with one lane of each row's warp summing it, 4 orders x ni additions a row
 // held the binary64 pipe (71% busy) for 36 us a field at 128x64x20.  The meridional part's filter and
 // last update come first (visc_row), on the row in shared memory: two launches and two passes fewer.
+// A block with filtered rows alone took 24,000 cycles for them before its sums (12,000 each, 8,200 of them
+// additions), beside blocks without any: the rows lie all over the latitudes, the mean is a product with a
+// power of 2, and the coefficients are ready before the rows.  12 steps of 128x64x20 10.24 -> 10.10 ms, 8
+// leapfrog steps of 64x47x13 3.14 -> 2.99 ms, 3 of 256x128x32 15.0 -> 14.8 ms.
 __global__ void __launch_bounds__(256, 3) k_zonal_visc_rows(DevModel M, double *A, int sel, const double *D, double msign, int filter, int jbot,
                                                          int jhalf, int k0, int nkk, int restore, int rows) {
   if (epic_member(M, A, D)) return;
   extern __shared__ __align__(16) double vr[];
   if (filter) warm_filter<double>(M, nullptr);
-  __shared__ double s_mean[32];
+  __shared__ double s_mean[32], s_dc[4][32];
   const int ni = M.ni, W = ni + 2, lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
   const int nr = M.nj - jbot + 1;
-  const int row0 = (int)blockIdx.x * rows, nl = min(rows, nr * nkk - row0);
-  if (nl <= 0) return;   // a member with fewer rows than the launch
+  // row r of block b is the member's row b + r nb, levels fastest: a block's rows lie all over the latitudes,
+  // so every block has its share of the filtered ones
+  const int total = nr * nkk, nb = (total + rows - 1) / rows;
+  if ((int)blockIdx.x >= nb) return;   // a member with fewer rows than the launch
+  const int nl = (total - (int)blockIdx.x + nb - 1) / nb;
   A += plane_offset(M, sel);
   double *a = vr, *h = a + rows * W, *d = h + rows * W;
   auto row_at = [&](int r, int &j, int &k) {
-    const int q = (row0 + r) / nr;
-    k = k0 + q;
-    j = jbot + row0 + r - q * nr;
+    const int at = (int)blockIdx.x + r * nb, q = at / nkk;
+    j = jbot + q;
+    k = k0 + at - q * nkk;
   };
+  if ((int)threadIdx.x < nl) {   // the coefficients, while the rows come
+    int j, k;
+    row_at((int)threadIdx.x, j, k);
+    const double mm = M.m[2 * j + jhalf];
+    const bool taper = fabs(M.lat[2 * j + jhalf]) > M.lat0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) s_dc[q][threadIdx.x] = taper ? M.coef[2 * q + 2] * M.m0 * M.m0 : M.coef[2 * q + 2] * mm * mm;
+  }
   for (int r = w; r < nl; r += nw) {
     int j, k;
     row_at(r, j, k);
     visc_row<double>(M, A, D, M.at(k, j, 0), j, jhalf == 0, msign, filter, d + r * W, a + r * W, lane);
     for (int i = lane; i <= ni + 1; i += 32) h[r * W + i] = a[r * W + i];
   }
-  __syncwarp();
+  __syncthreads();
   double sign = 1.;
   // fully unrolled so that M.coef[], M.nu[] are indexed by constants (M stays in registers)
 #pragma unroll
   for (int itmp = 2; itmp <= 8; itmp += 2) {
     for (int r = w; r < nl; r += nw) {
-      int j, k;
-      row_at(r, j, k);
-      const double mm = M.m[2 * j + jhalf];
-      const double dc = fabs(M.lat[2 * j + jhalf]) > M.lat0 ? M.coef[itmp] * M.m0 * M.m0 : M.coef[itmp] * mm * mm;
+      const double dc = s_dc[itmp / 2 - 1][r];
       const double *hr = h + r * W;
       for (int i = lane + 1; i <= ni; i += 32) d[r * W + i] = dc * (hr[i - 1] - twice_of(hr[i]) + hr[i + 1]);
     }
     __syncthreads();
-    if ((int)threadIdx.x < nl) s_mean[threadIdx.x] = row_sum(d + (int)threadIdx.x * W + 1, ni) / ni;
+    if ((int)threadIdx.x < nl) s_mean[threadIdx.x] = row_sum(d + (int)threadIdx.x * W + 1, ni) * inv_pow2(ni);
     __syncthreads();
     for (int r = w; r < nl; r += nw) {
       const double mean = s_mean[r];
@@ -1135,7 +1160,7 @@ __global__ void __launch_bounds__(256) k_pv_poles(DevModel M, int lv) {
     const int north = t & 1;
     double ze = sum[2 * t], h = sum[2 * t + 1];
     ze *= north ? M.mn[2 * (J + 1)] / (M.m[2 * J + 1] * (double)(M.ni)) : M.mn[0] / ((M.m[1]) * (double)(M.ni));
-    h /= (double)(M.ni);
+    h *= inv_pow2(M.ni);
     pole[t] = (ze + (north ? M.f[2 * (J + 1)] : M.f[0])) / h;
   }
   __syncthreads();

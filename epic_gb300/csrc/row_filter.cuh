@@ -99,7 +99,7 @@ __device__ __forceinline__ void four1_stages(Cplx<R> *z, const Cplx<R> *tw, int 
 // the weights act on the pair (q, N-q).  The reference's factors 1/2 (c1, c2, two per value) and 2/ni
 // are powers of 2, which commute with every rounding in between (the values being far from the ends
 // of the range), so they are left to the one final multiplication.
-template <class R> __device__ __forceinline__ R filter_scale(int ni) { return R(.5) / R(ni); }
+template <class R> __device__ __forceinline__ R filter_scale(int ni) { return cv<R>(.5 * inv_pow2(ni)); }
 template <class R>
 __device__ __forceinline__ void filter_row(const DevModel &M, Cplx<R> *z, const double *hl, const RowLane &L) {
   const int N = M.ni / 2, lg = fft_log(M.ni);
