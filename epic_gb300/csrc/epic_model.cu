@@ -926,6 +926,7 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
 
 extern "C" void epic_model_destroy(epic_model *m) {
   if (!m) return;
+  if (m->stream) cudaStreamSynchronize(m->stream);   // what is in flight first, then what it uses
   if (m->run_graph) cudaGraphExecDestroy(m->run_graph);
   if (m->copy_stream) {
     cudaStreamSynchronize(m->copy_stream);
@@ -935,7 +936,6 @@ extern "C" void epic_model_destroy(epic_model *m) {
   if (m->snap_done) cudaEventDestroy(m->snap_done);
   if (m->snap) cudaFree(m->snap);
   if (m->snap_ctl) cudaFreeHost(m->snap_ctl);
-  if (m->stream) cudaStreamSynchronize(m->stream);
   if (m->pool) cudaFree(m->pool);
   if (m->fop) epic::filter_operator_release(m->fop);
   if (m->stream) cudaStreamDestroy(m->stream);
@@ -1294,7 +1294,12 @@ extern "C" int epic_batch_create(epic_model *const *members, int32_t n, epic_bat
   }
   std::vector<DevModel> host(n);
   for (int i = 0; i < n; i++) host[i] = members[i]->d;
-  e = cudaMemcpy(b->dev_members, host.data(), sizeof(DevModel) * (size_t)n, cudaMemcpyHostToDevice);
+  // On the batch's stream, and waited for: every kernel of the batch follows its members' addresses and
+  // sizes from here.  A cudaMemcpy from pageable memory may return before its bytes arrive, in the order of
+  // the legacy stream, which this non-blocking stream does not follow: under the load of other batches a
+  // launch could then take the descriptions of an earlier batch at the same address.
+  e = cudaMemcpyAsync(b->dev_members, host.data(), sizeof(DevModel) * (size_t)n, cudaMemcpyHostToDevice, b->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
   if (cur != members[0]->device) cudaSetDevice(cur);
   if (e != cudaSuccess) {
     epic_batch_destroy(b);
@@ -1328,9 +1333,9 @@ extern "C" int epic_batch_create(epic_model *const *members, int32_t n, epic_bat
 extern "C" void epic_batch_destroy(epic_batch *b) {
   if (!b) return;
   for (auto *g : b->groups) epic_batch_destroy(g);
+  if (b->stream) cudaStreamSynchronize(b->stream);   // what is in flight first, then what it uses
   if (b->host_ctl) cudaFreeHost(b->host_ctl);
   if (b->run_graph) cudaGraphExecDestroy(b->run_graph);
-  if (b->stream) cudaStreamSynchronize(b->stream);
   if (b->dev_members) cudaFree(b->dev_members);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;

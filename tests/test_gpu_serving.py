@@ -3,7 +3,7 @@ and advanced in per-shape-class batches give each run the bits it gets alone."""
 import numpy as np
 import pytest
 
-from epic_gb300 import EPIC_PREC_MIXED, HSConfig, hs_setup, model_bytes
+from epic_gb300 import EPIC_PREC_MIXED, EPIC_PREC_MIXED_FAST, EPIC_PROFILE_N2, EPIC_SYNC_DIAGS_ONLY, HSConfig, Model, hs_setup, model_bytes
 from epic_gb300.serving import RunRequest, RunServer, latency_summary
 
 pytestmark = pytest.mark.gpu
@@ -37,3 +37,41 @@ def test_serving_rejects_oversized_request(gpu):
     q = RunRequest(0, HSConfig(ni=64, nj=32, nk=10, dt=300), 3)
     with pytest.raises(ValueError, match="budget"):
         RunServer(hbm_budget=1 << 20).serve([q])
+
+
+# sizes whose filters run on the tensor cores, in clusters and with shared operators, beside small grids;
+# jets beside resting columns in one launch class
+STREAM = [((256, 128, 10), 60, True), ((128, 64, 10), 240, False), ((256, 128, 10), 60, True), ((64, 32, 32), 300, False),
+          ((256, 128, 10), 120, False), ((128, 64, 20), 60, True), ((512, 256, 10), 60, True), ((256, 128, 10), 60, True),
+          ((64, 32, 10), 60, True), ((128, 64, 32), 90, False), ((512, 256, 10), 60, False), ((128, 64, 10), 60, True),
+          ((64, 32, 10), 60, True), ((128, 64, 20), 120, False), ((256, 128, 10), 120, False), ((128, 64, 32), 60, True)]
+
+
+@pytest.mark.parametrize("form", [EPIC_PREC_MIXED, EPIC_PREC_MIXED_FAST])
+def test_serving_stream_of_tensor_core_sizes(gpu, form):
+    """Runs join and leave classes whose batches are re-formed while other classes' are in flight, twice
+    over (so that operators, pools and batch descriptions are released and made again): every result
+    equals the run alone."""
+    rng = np.random.default_rng(11)
+    reqs = []
+    for q, ((ni, nj, nk), dt, jet) in enumerate(STREAM):
+        kw = dict(state="jet", profile=EPIC_PROFILE_N2) if jet else {}
+        reqs.append(RunRequest(q, HSConfig(ni=ni, nj=nj, nk=nk, dt=dt, seed=300 + q, **kw), int(rng.integers(12, 49)), 0.01 * q,
+                               1.0 + 0.02 * (q % 5 - 2)))
+    alone = []
+    for r in reqs:
+        ga, f = hs_setup(r.cfg)
+        ga.struct.hs_kf *= r.kf_scale
+        m = Model(ga, form)
+        m.upload(f)
+        m.timestep(EPIC_SYNC_DIAGS_ONLY)
+        m.run(r.steps)
+        m.sync()
+        alone.append(m.download())
+        m.close()
+    for _ in range(2):
+        got = RunServer(hbm_budget=40 << 30, precision=form, round_steps=4, keep_fields=True).serve(reqs)
+        for r, w in zip(got, alone):
+            assert r.error is None, (r.rid, r.error)
+            for k in w.arrays:
+                assert np.array_equal(r.fields.arrays[k], w.arrays[k]), (r.rid, r.shape, k)
