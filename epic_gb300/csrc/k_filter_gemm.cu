@@ -51,6 +51,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include "device_common.cuh"
+#include "filter_pipeline.h"
 #include "kernels.h"
 #include "epic_common.h"
 #include "epic_gb300.h"
@@ -65,7 +66,6 @@ constexpr int FG_NMAX = 64;      // columns per CTA ((member, plane) pairs), a m
 constexpr int FG_STAGE = 256;    // eight staging and epilogue warps: two per 32-lane quarter of tensor memory
 constexpr int FG_WARPS = FG_STAGE / 32;
 constexpr int FG_THREADS = FG_STAGE + 64;   // warp FG_WARPS issues the products, the next one the operator copies
-constexpr int FG_BUFS = 4;       // operator tile pairs and chunks of plane values in shared memory, each
 constexpr int FG_GROUPS = 8;     // column groups a CTA takes in turn at most
 constexpr unsigned FG_WAIT_LIMIT = 1u << 20;
 constexpr unsigned FG_A_BYTES = FG_M * FG_KC * 4;   // one operator tile (hi or lo): 16 KB
@@ -162,8 +162,8 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
                                                                       int units, int gs, int resident) {
   extern __shared__ __align__(16) unsigned char fg_raw[];
   // operator tiles landed / read (per buffer), plane chunk staged / read (per buffer), accumulator
-  // complete / read out
-  __shared__ __align__(8) uint64_t bars[4 * FG_BUFS + 2];
+  // complete / read out, every product done (a CTA that gave up)
+  __shared__ __align__(8) uint64_t bars[4 * FG_BUFS + 3];
   __shared__ uint32_t tmem_base;
   __shared__ volatile int fail;
   __shared__ const double *s_src[FG_GROUPS][FG_NMAX];   // each column's row (i = 0), null when idle
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
   const unsigned a_s = (unsigned)__cvta_generic_to_shared(fg_smem), b_off = FG_BUFS * 2 * FG_A_BYTES;
   const unsigned bars_s = (unsigned)__cvta_generic_to_shared(&bars[0]);
   const unsigned a_full = bars_s, a_free = bars_s + 8 * FG_BUFS, b_full = a_free + 8 * FG_BUFS, b_free = b_full + 8 * FG_BUFS;
-  const unsigned acc_full = b_free + 8 * FG_BUFS, acc_free = acc_full + 8;
+  const unsigned acc_full = b_free + 8 * FG_BUFS, acc_free = acc_full + 8, drained = acc_free + 8;
   const uint32_t tcols = (uint32_t)(mts * N) <= 32 ? 32u : 1u << (32 - __clz(mts * N - 1));   // a power of 2 >= 32
   // step t's operator tiles, for offset (128 mt - kc) mod ni, hi then lo
   const void *const fop = opm.fop_map;
@@ -226,6 +226,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
     }
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(acc_full));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(acc_free), "r"(FG_WARPS));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(drained));
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
   __syncwarp();
@@ -287,10 +288,9 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
               mma_tf32(d_mt, a + 2 * ks, b + b_lo + 2 * ks, idesc, 1u);
               mma_tf32(d_mt, a + A_LO + 2 * ks, b + 2 * ks, idesc, 1u);
             }
-            // commits complete in issue order: the accumulator's is the last of a group
-            if (!resident) mma_commit(a_free + 8 * ab);
+            if (fg_signals_operator(t, loads)) mma_commit(a_free + 8 * ab);
           }
-          if (ok) mma_commit(b_free + 8 * bb);
+          if (ok && fg_signals_chunk(n, ngroups * nchunks)) mma_commit(b_free + 8 * bb);
         }
         if (ok) mma_commit(acc_full);
       }
@@ -401,15 +401,17 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
       }
     }
   }
-  // every wait of the other threads is over; the last group's products were waited for in its epilogue,
-  // unless a wait gave up: then the commits in flight are given their time (bounded)
+  // every wait of the other threads is over, and every signal and product was waited for (the last group's
+  // products in its epilogue) -- unless a wait gave up: then the issuing thread waits (bounded) for all it
+  // has issued, so that nothing arrives in the shared or tensor memory of a CTA that has gone
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   if (fail) {
-    if (tid == 0) {
+    if (tid == FG_STAGE) {
       int none = 0;
-      mbar_wait(acc_full, (unsigned)((ngroups - 1) & 1), &none);
+      mma_commit(drained);
+      mbar_wait(drained, 0u, &none);
       flag_error(Mg.ctl, ERR_TIMEOUT, k0, j, 0, 0.);
     }
     __syncthreads();
