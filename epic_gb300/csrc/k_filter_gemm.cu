@@ -117,6 +117,13 @@ __device__ __forceinline__ void tma_tile(unsigned dst, const void *map, int y, u
       : "memory");
 }
 
+// The operator's tensor map lies in global memory, written by a copy: before a block's first use of it, the
+// accesses through the tensor-map proxy are ordered after that write.  Without it a map made at the address
+// of an operator released earlier might be read as the old one, whose tiles have been freed.
+__device__ __forceinline__ void acquire_tensor_map(const void *map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+}
+
 // Bounded; gives up at once when another wait of the CTA has.
 __device__ __forceinline__ bool mbar_wait(unsigned mbar, unsigned phase, volatile int *fail) {
   for (unsigned it = 0; it < FG_WAIT_LIMIT; it++) {
@@ -295,6 +302,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
         if (ok) mma_commit(acc_full);
       }
     } else if (warp > FG_WARPS && lane == 0) {
+      acquire_tensor_map(fop);
       while (issued < loads && issued < FG_BUFS) load_next();
       while (issued < loads && mbar_wait(a_free + 8 * (issued % FG_BUFS), (unsigned)((issued / FG_BUFS - 1) & 1), &fail)) load_next();
       // the copies in flight are waited for (bounded by the limit) whether or not their steps are reached,

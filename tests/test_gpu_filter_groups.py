@@ -28,3 +28,22 @@ def test_members_equal_single_models(gpu, ni, nj, nk, members):
         want, got = single.download(), models[q].download()
         for n in want.arrays:
             assert np.array_equal(want.arrays[n], got.arrays[n]), f"member {q}: {n}"
+
+
+def test_operators_made_where_others_were_released(gpu):
+    """Operators of different grids made and released in turn: 128x64 and 256x64 have the same number of
+    filtered rows, so that one's tensor map may come to lie where the other's was.  Every pass gives the
+    first one's bits."""
+    grids = [hs_setup(HSConfig(ni=ni, nj=64, nk=5, dt=60, seed=ni, nu4=0.03)) for ni in (128, 256)]
+    want = {}
+    for turn in range(5):
+        for q, (ga, f) in enumerate(grids):
+            m = Model(ga, EPIC_PREC_MIXED)
+            m.upload(f)
+            m.timestep(EPIC_SYNC_DIAGS_ONLY)
+            m.run(2)
+            got = m.download()
+            m.close()   # the last model of the grid: its operator goes
+            w = want.setdefault(q, got)
+            for n in w.arrays:
+                assert np.array_equal(w.arrays[n], got.arrays[n]), (turn, q, n)
