@@ -485,14 +485,16 @@ __global__ void k_filter_rows_unfiltered(DevModel M, const double *src, int src_
 // ---- launchers ----
 
 // The shape of a row kernel whose rows take `stride` values of `elem` bytes each: lanes a row as above;
-// 128 threads a block (or the tuning table's choice), fewer where its rows would take more than 48 KB,
-// so that several blocks share an SM.
+// 128 threads a block (or the tuning table's choice, in whole warps: a warp's lanes all belong to rows that
+// the block's shared memory holds), fewer where its rows would take more than 48 KB, so that several blocks
+// share an SM.
 static RowShape row_shape(const DevModel &M, int stride, size_t elem, unsigned &threads) {
   RowShape S;
   S.G = M.ni >= 128 ? 32 : (M.ni >= 64 ? 16 : 8);
   S.stride = stride;
-  threads = M.tb[TB_ROW] > 0 ? (unsigned)M.tb[TB_ROW] : 128u;
-  while (threads > 32 && threads / (unsigned)S.G * (unsigned)stride * elem > 48 * 1024) threads /= 2;
+  unsigned warps = M.tb[TB_ROW] > 0 ? ((unsigned)M.tb[TB_ROW] + 31u) / 32u : 4u;
+  while (warps > 1 && warps * 32u / (unsigned)S.G * (unsigned)stride * elem > 48 * 1024) warps /= 2;
+  threads = 32u * warps;
   S.rows = (int)threads / S.G;
   return S;
 }

@@ -39,3 +39,21 @@ def test_meridional_forms(gpu, form, nj):
     for n in ("hdry", "theta", "p3", "u"):
         for g in got[1:]:
             assert np.array_equal(got[0].arrays[n], g.arrays[n]), n
+
+
+# block sizes of the row kernels that are no multiple of a warp, or halve to one where a row's values fill
+# a block's share of shared memory
+@pytest.mark.parametrize("form,ni", [(0, 512), (0, 16), (1, 64)])
+def test_row_block_sizes(gpu, form, ni):
+    ga, f = hs_setup(HSConfig(ni=ni, nj=8, nk=5, dt=max(1, 600 // ni), seed=ni, nu4=0.5 * min(1., 16. / ni)**4))
+    got = []
+    for threads in (0, 1, 48, 96, 250):
+        m = Model(ga, form)
+        m.set_tuning([0] * 8 + [threads])
+        m.upload(f)
+        m.timestep(EPIC_SYNC_DIAGS_ONLY)
+        m.run(2)
+        got.append(m.download())
+    for n in got[0].arrays:
+        for g in got[1:]:
+            assert np.array_equal(got[0].arrays[n], g.arrays[n]), n

@@ -4,7 +4,7 @@ CUDA runtime; no GPU is needed)."""
 import pytest
 
 from epic_gb300 import Batch, EPIC_PREC_FP64, EPIC_PREC_MIXED, EPIC_SYNC_DIAGS_ONLY, HSConfig, Model, hs_setup
-from host_library import host_library  # noqa: F401
+from host_library import host_library, host_library_file  # noqa: F401
 
 
 @pytest.mark.parametrize("form,shapes", [(EPIC_PREC_FP64, [(16, 8), (16, 8), (32, 16)]), (EPIC_PREC_MIXED, [(128, 8), (128, 8)])])
