@@ -42,8 +42,8 @@
 // geopotential, ~1e-5 of its value.
 //
 // Every wait is bounded: a CTA whose operator copy or MMA completion does not arrive within the
-// limit records ERR_TIMEOUT, waits (bounded) for what it has in flight, frees its tensor memory
-// and returns.
+// limit waits (bounded) for what it has in flight, records ERR_TIMEOUT in every member whose rows it
+// leaves unwritten, frees its tensor memory and returns.
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -67,7 +67,11 @@ constexpr int FG_STAGE = 256;    // eight staging and epilogue warps: two per 32
 constexpr int FG_WARPS = FG_STAGE / 32;
 constexpr int FG_THREADS = FG_STAGE + 64;   // warp FG_WARPS issues the products, the next one the operator copies
 constexpr int FG_GROUPS = 8;     // column groups a CTA takes in turn at most
-constexpr unsigned FG_WAIT_LIMIT = 1u << 20;
+#ifndef EPIC_FILTER_WAIT_LIMIT
+#define EPIC_FILTER_WAIT_LIMIT (1u << 20)
+#endif
+constexpr unsigned FG_WAIT_LIMIT = EPIC_FILTER_WAIT_LIMIT;   // of the pipeline's waits (a test builds with 0)
+constexpr unsigned FG_DRAIN_LIMIT = 1u << 20;                 // of the waits for what a CTA that gives up has in flight
 constexpr unsigned FG_A_BYTES = FG_M * FG_KC * 4;   // one operator tile (hi or lo): 16 KB
 
 // Byte offset of element (r, e), 0 <= e < 32, in a 128B-swizzled K-major tile of FP32 rows.
@@ -125,8 +129,8 @@ __device__ __forceinline__ void acquire_tensor_map(const void *map) {
 }
 
 // Bounded; gives up at once when another wait of the CTA has.
-__device__ __forceinline__ bool mbar_wait(unsigned mbar, unsigned phase, volatile int *fail) {
-  for (unsigned it = 0; it < FG_WAIT_LIMIT; it++) {
+__device__ __forceinline__ bool mbar_wait(unsigned mbar, unsigned phase, volatile int *fail, unsigned limit = FG_WAIT_LIMIT) {
+  for (unsigned it = 0; it < limit; it++) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}\n"
@@ -173,6 +177,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
   __shared__ __align__(8) uint64_t bars[4 * FG_BUFS + 3];
   __shared__ uint32_t tmem_base;
   __shared__ volatile int fail;
+  __shared__ int s_written[FG_GROUPS];                  // staging warps that have written their share of a group
   __shared__ const double *s_src[FG_GROUPS][FG_NMAX];   // each column's row (i = 0), null when idle
   __shared__ double *s_dst[FG_GROUPS][FG_NMAX];
   __shared__ double s_x1[FG_GROUPS][FG_NMAX];           // the subtracted value of each column's row (shift), else 0
@@ -223,6 +228,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
       if (++lc == nchunks) lc = 0;
     }
   };
+  if (tid < FG_GROUPS) s_written[tid] = 0;
   if (tid == FG_STAGE + 32) {
     fail = 0;
     for (int q = 0; q < FG_BUFS; q++) {
@@ -309,7 +315,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
       // so that nothing writes this CTA's shared memory after it is released
       for (int q = issued > FG_BUFS ? issued - FG_BUFS : 0; q < issued; q++) {
         int none = 0;
-        mbar_wait(a_full + 8 * (q % FG_BUFS), (unsigned)((q / FG_BUFS) & 1), &none);
+        mbar_wait(a_full + 8 * (q % FG_BUFS), (unsigned)((q / FG_BUFS) & 1), &none, FG_DRAIN_LIMIT);
       }
     }
     __syncwarp();
@@ -374,6 +380,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
               if (pad != i) row[n][pad] = y;
             }
           }
+        if (lane == 0) atomicAdd(&s_written[gi], 1);
       }
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
@@ -419,8 +426,12 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
     if (tid == FG_STAGE) {
       int none = 0;
       mma_commit(drained);
-      mbar_wait(drained, 0u, &none);
-      flag_error(Mg.ctl, ERR_TIMEOUT, k0, j, 0, 0.);
+      mbar_wait(drained, 0u, &none, FG_DRAIN_LIMIT);
+    }
+    // every member with a row that this CTA has not written, or not whole
+    for (int t = tid; t < ngroups * G; t += FG_THREADS) {
+      const int gi = t / G, u = u0 + gi * gs, q = (u / nch) * G + t - gi * G;
+      if (s_written[gi] < FG_WARPS && q < members) flag_error(M.batch ? M.batch[q].ctl : M.ctl, ERR_TIMEOUT, k0 + (u % nch) * pc, j, 0, 0.);
     }
     __syncthreads();
   }
