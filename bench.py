@@ -701,7 +701,7 @@ def run_gpu_ensemble(args):
             "launch_shapes": {"autotuned": tuning,
                               "groups": ["uv_core", "pgrad", "hsu_meridional", "hyperviscosity", "diagnostics",
                                          "update", "column", "pointwise", "row_filter",
-                                         "hsu_meridional_form (1 fused march, 2 four passes)"]},
+                                         "hsu_meridional_form (1 fused march, 2 four passes, 3 tiles)"]},
             "clocks": clocks,
             "e2e": {"value": e2e_val, "unit": "cell-steps/s", "h2d_bytes_per_step": state_bytes, "d2h_bytes_per_step": state_bytes,
                     "ms_per_step": e2e_s * 1e3, "host_link_gbs": link,

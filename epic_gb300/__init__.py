@@ -22,7 +22,7 @@ from .abi import (EPIC_ADV_AKIMA, EPIC_ADV_HSU, EPIC_IO_ALL, EPIC_IO_STATE, EPIC
                   EPIC_TURB_SA_DES, EPIC_UV_AB3, EPIC_UV_LEAPFROG, TURB_FIELDS, EpicFields, EpicGrid, EpicHsParams, EpicJetParams, Fields, GridArrays, HSConfig, JetConfig, Layout)
 
 TUNE_GROUPS = 10   # EPIC_TUNE_GROUPS
-TUNE_HSU_MERID_VARIANT = 9   # table entry: 0 automatic (tiles, march or passes), 1 fused march, 2 four passes
+TUNE_HSU_MERID_VARIANT = 9   # table entry: 0 automatic, 1 fused march, 2 four passes, 3 tiles of columns
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "_lib", "libepic_gb300.so")
 _lib = None

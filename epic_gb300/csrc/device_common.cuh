@@ -12,7 +12,7 @@
 
 // kernel groups whose block size the autotuner picks (DevModel::tb)
 enum TuneGroup { TB_UV_CORE = 0, TB_PGRAD, TB_HSU, TB_VISC, TB_DIAG, TB_UPDATE, TB_COLUMN, TB_POINT, TB_ROW,
-                 TB_HSU_MERID_VARIANT,   // not a block size: 0 automatic (tiles, march or passes), 1 fused march, 2 four passes
+                 TB_HSU_MERID_VARIANT,   // not a block size: 0 automatic, else a HsuForm (kernels.h)
                  TB_COUNT };
 #define TB(M, g) ((M).tb[g] > 0 ? (M).tb[g] : 128)
 

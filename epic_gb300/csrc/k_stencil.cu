@@ -1406,27 +1406,37 @@ int launch_akima_meridional(const DevModel &M, double *buff, int kind, cudaStrea
 // or 8 columns (64 bytes of a row) where its four arrays of nj+2 rows fit MERID_SMEM, as wide as leaves two
 // blocks per SM; the march (k_hsu_meridional, one thread per (k, i, member) walking nj+1 rows) once those
 // threads fill the GPU (large batches); else the four passes, whose threads cover every cell.  The
-// tuning table's TB_HSU_MERID_VARIANT entry overrides the choice (1 march, 2 four passes).
+// tuning table's TB_HSU_MERID_VARIANT entry overrides the choice (HsuForm; tiles where they fit, else
+// the four passes).
 constexpr long long HSU_FUSED_MIN_THREADS = 65536;
 constexpr size_t MERID_SMEM = 100 * 1024;   // two blocks per SM
+
+// shared memory of one column of a tile: the field, the velocity, the fluxes and the predicted field
+static size_t merid_column_bytes(const DevModel &M) { return (size_t)4 * (M.nj + 2) * (M.mixed ? sizeof(float) : sizeof(double)); }
+// columns of a tile, 0 where 8 do not fit
+static int merid_tile_columns(const DevModel &M, int nkk) {
+  int TC = 32;
+  while (TC > 8 && (long long)epic_blocks(M.ni, TC) * nkk * (M.nbatch > 1 ? M.nbatch : 1) < 2 * 152) TC /= 2;
+  while (TC >= 8 && TC * merid_column_bytes(M) > MERID_SMEM) TC /= 2;
+  return TC >= 8 ? TC : 0;
+}
+int hsu_meridional_form(const DevModel &M, int nkk) {
+  const int entry = M.tb[TB_HSU_MERID_VARIANT];
+  if (entry == HSU_MARCH || (entry == 0 && (long long)M.ni * nkk * (M.nbatch > 1 ? M.nbatch : 1) >= HSU_FUSED_MIN_THREADS)) return HSU_MARCH;
+  return entry != HSU_PASSES && merid_tile_columns(M, nkk) ? HSU_TILES : HSU_PASSES;
+}
 
 int launch_hsu_meridional(const DevModel &M, double *buff, int kind, cudaStream_t s) {
   const int k0 = kind == 1 ? M.k_sigma - 1 : 1;
   const int nkk = M.nk - k0 + 1;
-  const int th = TB(M, TB_HSU);
-  const int variant = M.tb[TB_HSU_MERID_VARIANT];
-  const bool fused = variant == 1 ||
-                     (variant == 0 && (long long)M.ni * nkk * (M.nbatch > 1 ? M.nbatch : 1) >= HSU_FUSED_MIN_THREADS);
-  if (fused) {
+  const int th = TB(M, TB_HSU), form = hsu_meridional_form(M, nkk);
+  if (form == HSU_MARCH) {
     EPIC_LAUNCH_R(M.mixed, k_hsu_meridional, dim3(epic_blocks(M.ni, th), nkk), th, 0, s, M, buff, kind, k0);
     return 0;
   }
-  const size_t col = (size_t)4 * (M.nj + 2) * (M.mixed ? sizeof(float) : sizeof(double));
-  int TC = 32;
-  while (TC > 8 && (long long)epic_blocks(M.ni, TC) * nkk * (M.nbatch > 1 ? M.nbatch : 1) < 2 * 152) TC /= 2;
-  while (TC >= 8 && TC * col > MERID_SMEM) TC /= 2;
-  if (variant == 0 && TC >= 8) {
-    EPIC_LAUNCH_R(M.mixed, k_hsu_merid_tile, dim3(epic_blocks(M.ni, TC), nkk), 256, TC * col, s, M, buff, kind, k0, TC);
+  if (form == HSU_TILES) {
+    const int TC = merid_tile_columns(M, nkk);
+    EPIC_LAUNCH_R(M.mixed, k_hsu_merid_tile, dim3(epic_blocks(M.ni, TC), nkk), 256, TC * merid_column_bytes(M), s, M, buff, kind, k0, TC);
     return 0;
   }
   EPIC_LAUNCH_R(M.mixed, k_hsu_merid_pred, cells_blocks(M, nkk, M.nj + 2, th), th, 0, s, M, buff, kind, k0);

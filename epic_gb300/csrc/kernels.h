@@ -138,6 +138,8 @@ int launch_pgrad_poles(const DevModel &M, cudaStream_t s);
 int launch_pgrad_lon(const DevModel &M, cudaStream_t s);
 int launch_pgrad_lat(const DevModel &M, cudaStream_t s);
 int launch_hsu_meridional(const DevModel &M, double *buff, int kind, cudaStream_t s);
+enum HsuForm { HSU_MARCH = 1, HSU_PASSES = 2, HSU_TILES = 3 };   // the tuning table's TB_HSU_MERID_VARIANT (0: by size)
+int hsu_meridional_form(const DevModel &M, int nkk);             // the form that nkk planes take
 // akima_advection (epic_flux.c:1502-1940), the other advection scheme: vertical (k_column.cu),
 // meridional (k_stencil.cu) and zonal (k_filter.cu) passes, arguments as their Hsu counterparts
 int launch_akima_vertical(const DevModel &M, double *buff, int kind, cudaStream_t s);

@@ -317,9 +317,11 @@ int32_t epic_batch_kernels_per_step(const epic_batch *b);
  * kernel group, 0 keeping the built-in choice: entries 0-8 are block sizes (uv_core, pgrad, Hsu
  * meridional, hyperviscosity, diagnostics, update, column, pointwise, row filter), entry 9 the
  * form of the meridional Hsu pass (1 one fused march per column of cells, 2 four passes over every
- * cell; by default the fused march once its threads fill the GPU).  Tuned kernels are pointwise,
- * per row or per column, and the two Hsu forms give the same bits, so a table changes no result.  epic_batch_autotune times whole steps
- * of the batch for each candidate (trial_steps timed steps each) and keeps the fastest; the
+ * cell, 3 tiles of columns where they fit; by default the fused march once its threads fill the GPU,
+ * else tiles, else the passes).  Tuned kernels are pointwise, per row or per column, and the three Hsu
+ * forms give the same bits, so a table changes no result.  epic_batch_autotune times whole steps
+ * of the batch, as epic_batch_run replays them, for each candidate (trial_steps timed steps each) and
+ * keeps what is faster than the choice in place; the
  * members must hold a primed state (after epic_batch_timestep(b, EPIC_SYNC_DIAGS_ONLY)), and the
  * trial steps advance it, so tune before uploading the state a run starts from.
  */

@@ -5,7 +5,7 @@ restatement bit for bit."""
 import numpy as np
 import pytest
 
-from epic_gb300 import (EPIC_ADV_AKIMA, EPIC_ADV_HSU, EPIC_PROFILE_N2, EPIC_SYNC_DIAGS_ONLY, HSConfig, Model, TUNE_HSU_MERID_VARIANT,
+from epic_gb300 import (Batch, EPIC_ADV_AKIMA, EPIC_ADV_HSU, EPIC_PROFILE_N2, EPIC_SYNC_DIAGS_ONLY, HSConfig, Model, TUNE_HSU_MERID_VARIANT,
                         hs_setup)
 from test_gpu_parity import _stage_by_stage
 
@@ -54,6 +54,33 @@ def test_row_block_sizes(gpu, form, ni):
         m.timestep(EPIC_SYNC_DIAGS_ONLY)
         m.run(2)
         got.append(m.download())
+    for n in got[0].arrays:
+        for g in got[1:]:
+            assert np.array_equal(got[0].arrays[n], g.arrays[n]), n
+
+
+# the meridional pass's tiles asked for by the tuning table (where they do not fit, the four passes), as a
+# single model and as an autotuned batch
+@pytest.mark.parametrize("form,ni,nj", [(0, 16, 30), (1, 64, 30), (0, 16, 400), (1, 16, 800)])
+def test_meridional_tiles_by_table(gpu, form, ni, nj):
+    ga, f = hs_setup(HSConfig(ni=ni, nj=nj, nk=4, dt=5, seed=nj, state="jet", profile=EPIC_PROFILE_N2))
+    got = []
+    for variant in (0, 3, 2):
+        m = Model(ga, form)
+        m.set_tuning([0] * TUNE_HSU_MERID_VARIANT + [variant])
+        m.upload(f)
+        m.timestep(EPIC_SYNC_DIAGS_ONLY)
+        m.run(2)
+        got.append(m.download())
+    models = [Model(ga, form) for _ in range(2)]
+    b = Batch(models)
+    b.upload([f, f])
+    b.timestep(EPIC_SYNC_DIAGS_ONLY)
+    assert b.autotune(trial_steps=1)[TUNE_HSU_MERID_VARIANT] in (1, 2, 3)
+    b.upload([f, f])
+    b.timestep(EPIC_SYNC_DIAGS_ONLY)
+    b.run(2)
+    got.append(b.download([f.copy(), f.copy()])[1])
     for n in got[0].arrays:
         for g in got[1:]:
             assert np.array_equal(got[0].arrays[n], g.arrays[n]), n

@@ -1,7 +1,7 @@
 """What the library launches, by its host code over a stand-in for the CUDA runtime (no GPU is needed)."""
 import pytest
 
-from epic_gb300 import EPIC_PREC_FP64, EPIC_PREC_MIXED, EPIC_SYNC_DIAGS_ONLY, HSConfig, Model, TUNE_GROUPS, hs_setup
+from epic_gb300 import Batch, EPIC_PREC_FP64, EPIC_PREC_MIXED, EPIC_SYNC_DIAGS_ONLY, HSConfig, Model, TUNE_GROUPS, TUNE_HSU_MERID_VARIANT, hs_setup
 from host_library import host_library, host_library_file, launches  # noqa: F401
 
 ROW_KERNELS = ("k_varz_filter_rows", "k_hsu_zonal", "k_filter_planes")
@@ -28,3 +28,21 @@ def test_row_kernels_take_whole_warps(host_library, ni, form, threads):
         n, _, th, _, _ = launches(host_library, k)
         assert n and th >= 32 and th % 32 == 0, (k, n, th)
     m.close()
+
+
+@pytest.mark.parametrize("ni,nj,form,members", [(64, 32, EPIC_PREC_MIXED, 2), (32, 16, EPIC_PREC_FP64, 8)])
+def test_autotuner_times_the_replayed_step(host_library, ni, nj, form, members):
+    """The tuner's trial steps are replays of the captured step, as Batch.run's are, and every form of the
+    meridional pass is among its candidates: the stand-in's clock counts kernels, of which the tiles take
+    one a field where the march or the passes are no fewer."""
+    models = [_model(ni, nj, 5, form, seed=q) for q in range(members)]
+    b = Batch(models)
+    host_library.fake_reset_counts()
+    table = b.autotune(trial_steps=2)
+    assert host_library.fake_direct_launches() == 0
+    assert host_library.fake_graph_launches() >= 3 * (9 * 4 + 3)   # a warm-up and two timed steps per candidate
+    assert table[TUNE_HSU_MERID_VARIANT] == 3 and table[:8] == [128] * 8
+    host_library.fake_reset_counts()
+    b.run(1)
+    assert launches(host_library, "k_hsu_merid_tile")[0] == 3 and launches(host_library, "k_hsu_merid_pred")[0] == 0
+    b.close()
