@@ -861,20 +861,16 @@ static int launch_pads(const DevModel &M, double *a, int k0, int k1, cudaStream_
   return 0;
 }
 
-// Blocks of the wavefront kernel's cluster: 16 where the GPU can place them (a front of 1235 points at
-// 128x64x20 is then a few per thread's SM), else the portable 8.  Set by turb_kernels_init.
-static int g_sa_cluster = 8;
-
 int launch_source_sink_turb(const DevModel &M, cudaStream_t s) {
   const long long cells = (long long)(M.nk - 1) * (M.nj + 1) * M.ni;
   k_sa_prep<<<zg(nblk(cells, 128), M), 128, 0, s>>>(M);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = zg(dim3((unsigned)g_sa_cluster), M);
+  cfg.gridDim = zg(dim3((unsigned)M.sa_cluster), M);
   cfg.blockDim = dim3(SA_THREADS);
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)g_sa_cluster;
+  at[0].val.clusterDim.x = (unsigned)M.sa_cluster;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
@@ -948,26 +944,25 @@ int launch_uv_vdiff(const DevModel &M, cudaStream_t s) {
   return 0;
 }
 
-// the most a launch takes, raised once for the process (models of all sizes)
-int turb_kernels_init() {
+// On the current device, whose own attributes these are: the most shared memory a launch takes (models of
+// all sizes), and the blocks of the wavefront kernel's cluster -- 16 where the GPU can place them (a front of
+// 1235 points at 128x64x20 is then a few per thread's SM), else the portable 8 -- into *cluster.
+int turb_kernels_init(int *cluster) {
   const int big = (int)((size_t)VD_ARRAYS * 32 * (EPIC_TURB_MAX_NK + 3) * sizeof(double));
-  static const int cluster = [] {   // a property of the device type, found once
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(16);
-    cfg.blockDim = dim3(SA_THREADS);
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 16;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int n = 0;
-    const bool ok = cudaFuncSetAttribute(k_sa_waves, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                    cudaOccupancyMaxActiveClusters(&n, k_sa_waves, &cfg) == cudaSuccess && n >= 1;
-    cudaGetLastError();
-    return ok ? 16 : 8;
-  }();
-  g_sa_cluster = cluster;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(16);
+  cfg.blockDim = dim3(SA_THREADS);
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 16;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  const bool ok = cudaFuncSetAttribute(k_sa_waves, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&n, k_sa_waves, &cfg) == cudaSuccess && n >= 1;
+  cudaGetLastError();
+  *cluster = ok ? 16 : 8;
   return cudaFuncSetAttribute(k_vdiff, cudaFuncAttributeMaxDynamicSharedMemorySize, big) == cudaSuccess ? 0 : -1;
 }
 
