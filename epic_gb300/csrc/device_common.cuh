@@ -133,7 +133,8 @@ struct DevModel {
   long long reloc_n3;  // a launch description's field size of member 0 (whose arrays it carries)
   int fop_shared;      // a batch whose members all filter with member 0's operator tiles (same grid)
   char *pool_base;   // start of the model's device pool (state, scratch and tables)
-  int sa_cluster;    // blocks of the closure's wavefront cluster on the model's device (host side only)
+  int sms;           // the model's device (host side only): its SMs, which the launch rules fill,
+  int sa_cluster;    // and the blocks of the closure's wavefront cluster
   // launch shapes (host side only): threads per block of each kernel group, set by the
   // autotuner; they change no result (every tuned kernel is pointwise or per row)
   int tb[TB_COUNT];

@@ -728,6 +728,10 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
   d.stab = g->stability_factor != 0;
   d.kinvisc = g->kinvisc;
   d.dynvisc = g->dynvisc;
+  if (cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || d.sms < 1) {
+    delete m;
+    return set_error(EPIC_ERR_CUDA, "epic_model_create: SM count of device %d", device);
+  }
   d.mixed = precision != EPIC_PREC_FP64;
   d.col64 = precision == EPIC_PREC_MIXED;
   d.cr = precision == EPIC_PREC_FP64;

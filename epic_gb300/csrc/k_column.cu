@@ -1005,7 +1005,7 @@ static inline size_t tile_smem(const DevModel &M, int arrays) { return (size_t)a
 // 12 steps of 128x64x20 (265 tiles) 11.45 -> 11.0 ms.
 static inline int tile_threads(const DevModel &M) {
   const long long tiles = (long long)ntile_blocks(M) * (M.nbatch > 1 ? M.nbatch : 1);
-  return !M.mixed && M.nk > CT_WARPS && tiles <= 2 * 152 ? CT_THREADS_WIDE : CT_THREADS;
+  return !M.mixed && M.nk > CT_WARPS && tiles <= 2 * M.sms ? CT_THREADS_WIDE : CT_THREADS;
 }
 int launch_calc_w(const DevModel &M, cudaStream_t s, bool with_source_sink) {
   EPIC_LAUNCH_R(M.mixed, k_calc_w, ntile_blocks(M), tile_threads(M), tile_smem(M, 6), s, M, (int)with_source_sink);

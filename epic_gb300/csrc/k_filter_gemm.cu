@@ -442,8 +442,6 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_filter_planes_gemm(DevModel M
 // the swizzle atoms
 size_t filter_gemm_smem_bytes(int n) { return 1024 + (size_t)FG_BUFS * 2 * (FG_A_BYTES + (size_t)n * FG_KC * 4); }
 
-static int g_sms = 0;   // SMs of the device (filter_gemm_init, at model creation: not during a graph capture)
-
 bool filter_gemm_usable(const DevModel &M) { return M.fop_map && M.ni % FG_M == 0 && M.ni <= 8 * FG_M; }
 
 // Columns per CTA: up to 64.  Planes beyond that split into chunks; members of one operator fill the
@@ -457,7 +455,7 @@ int launch_filter_planes_gemm(const DevModel &M, const double *src, int src_sel,
   if (G > members) G = members;
   const int N = ((G * pc + 31) / 32) * 32;
   const int units = nch * ((members + G - 1) / G);
-  const int sms = g_sms > 0 ? g_sms : 152, mtiles = M.ni / FG_M, rows = (M.nj + 3) / 2;   // about half the rows are filtered
+  const int sms = M.sms, mtiles = M.ni / FG_M, rows = (M.nj + 3) / 2;   // about half the rows are filtered
   // one CTA per SM (its buffers fill the shared memory).  Few units: a cluster of CTAs shares a row's
   // output tiles (each tile's sums are unchanged) as long as they are all resident at once: a second
   // round pays the setup, the first loads and the staging of the whole row again (512x256 x 40 planes:
@@ -491,8 +489,6 @@ int launch_filter_planes_gemm(const DevModel &M, const double *src, int src_sel,
 }
 
 int filter_gemm_init(int) {
-  int dev = 0;
-  if (g_sms == 0 && cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
   return cudaFuncSetAttribute(k_filter_planes_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)filter_gemm_smem_bytes(FG_NMAX)) ==
                  cudaSuccess
              ? 0

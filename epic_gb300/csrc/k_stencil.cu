@@ -249,7 +249,7 @@ static __device__ __forceinline__ double row_sum(const double *row, int n) {
 // of which there are nk+1: no more than it takes to have a block per SM
 static int row_sum_levels(const DevModel &M, int rows) {
   const int fit = (int)(ROW_SUM_SMEM / ((size_t)rows * (M.ni + 1) * sizeof(double)));
-  const int want = (int)(((long long)(M.nk + 1) * (M.nbatch > 1 ? M.nbatch : 1) + 151) / 152);
+  const int want = (int)(((long long)(M.nk + 1) * (M.nbatch > 1 ? M.nbatch : 1) + M.sms - 1) / M.sms);
   int lv = fit > 32 / rows ? 32 / rows : fit;
   lv = lv > want ? want : lv;
   return lv < 1 ? 1 : lv;
@@ -1416,7 +1416,7 @@ static size_t merid_column_bytes(const DevModel &M) { return (size_t)4 * (M.nj +
 // columns of a tile, 0 where 8 do not fit
 static int merid_tile_columns(const DevModel &M, int nkk) {
   int TC = 32;
-  while (TC > 8 && (long long)epic_blocks(M.ni, TC) * nkk * (M.nbatch > 1 ? M.nbatch : 1) < 2 * 152) TC /= 2;
+  while (TC > 8 && (long long)epic_blocks(M.ni, TC) * nkk * (M.nbatch > 1 ? M.nbatch : 1) < 2 * M.sms) TC /= 2;
   while (TC >= 8 && TC * merid_column_bytes(M) > MERID_SMEM) TC /= 2;
   return TC >= 8 ? TC : 0;
 }
@@ -1472,7 +1472,7 @@ static void launch_meridional_hyperviscosity(const DevModel &M, int index, doubl
   // the first two passes in one kernel when nothing is applied between them
   const size_t pair_col = (size_t)nrows * (M.mixed ? sizeof(float) : sizeof(double));
   const long long strips = (long long)epic_blocks(M.ni, 16) * nkk * (M.nbatch > 1 ? M.nbatch : 1);
-  const int pair_tc = 16 * pair_col <= 48 * 1024 && strips >= 2 * 152 ? 16 : 8;
+  const int pair_tc = 16 * pair_col <= 48 * 1024 && strips >= 2 * M.sms ? 16 : 8;
   const bool pair = !(M.nu[2] > 0.) && M.nu[4] + M.nu[6] + M.nu[8] > 0. && pair_tc * pair_col <= 48 * 1024;
   for (int itmp = 2; itmp <= 8; itmp += 2) {
     double *dst = bufs[which];
@@ -1527,7 +1527,7 @@ int launch_hyperviscosity(const DevModel &M, int index, double *var, int sel, cu
     const size_t row_bytes = (size_t)3 * (M.ni + 2) * sizeof(double);
     const long long total = (long long)nrows * nkk * (M.nbatch > 1 ? M.nbatch : 1);
     int rows = 4;
-    while (rows < 32 && total > 2LL * 152 * rows && 2 * rows * row_bytes <= VISC_ROWS_SMEM) rows *= 2;
+    while (rows < 32 && total > 2LL * M.sms * rows && 2 * rows * row_bytes <= VISC_ROWS_SMEM) rows *= 2;
     k_zonal_visc_rows<<<zg(epic_blocks((long long)nrows * nkk, rows), M), 256, rows * row_bytes, s>>>(M, var, sel, D, msign, filter, jbot,
                                                                                                      jhalf, k0, nkk, index == 2, rows);
     return 0;

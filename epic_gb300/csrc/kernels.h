@@ -33,7 +33,7 @@ inline dim3 zg(dim3 g, const DevModel &M) {
 // 512 threads per SM, up to 4; a template parameter, so that a single row is straight code.
 inline int march_rows(const DevModel &M, int nkk) {
   const long long cells = (long long)M.ni * nkk * (M.nj + 1) * (M.nbatch > 1 ? M.nbatch : 1);
-  return cells >= 4LL * 152 * 512 ? 4 : (cells >= 2LL * 152 * 512 ? 2 : 1);
+  return cells >= 4LL * M.sms * 512 ? 4 : (cells >= 2LL * M.sms * 512 ? 2 : 1);
 }
 struct March { int k, i, j0, j1; };
 // rows jlo..jhi; false for a thread without work

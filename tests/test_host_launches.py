@@ -30,6 +30,19 @@ def test_row_kernels_take_whole_warps(host_library, ni, form, threads):
     m.close()
 
 
+@pytest.mark.parametrize("sms,rows", [(152, 1), (76, 2), (38, 4)])
+def test_launch_rules_follow_the_device(host_library, sms, rows):
+    """As many rows a thread as leave 512 threads per SM of the model's own device: 90112 cells."""
+    host_library.fake_device(1, sms, 1)
+    host_library.cudaSetDevice(1)
+    m = _model(64, 63, 23)
+    host_library.fake_reset_counts()
+    m.timestep()
+    assert launches(host_library, "k_uv_kin")[4] == -(-64 // rows)
+    m.close()
+    host_library.cudaSetDevice(0)
+
+
 @pytest.mark.parametrize("ni,nj,form,members", [(64, 32, EPIC_PREC_MIXED, 2), (32, 16, EPIC_PREC_FP64, 8)])
 def test_autotuner_times_the_replayed_step(host_library, ni, nj, form, members):
     """The tuner's trial steps are replays of the captured step, as Batch.run's are, and every form of the
