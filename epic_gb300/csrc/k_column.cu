@@ -241,8 +241,9 @@ __global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : 
         if (edge) t = fabs(neg ? ad - au : -au + ad) + ep;
         else t = fabs((neg ? ad : auu) - twice_of(au) + (neg ? auu : ad)) + ep;
         auto amin = [&](int q) { return layer ? cv<R>(M.h_min[q]) : cv<R>(1.e-3 * M.kinvisc); };   // HDRY's and NU_TURB's floors
-        CT(FF, k) = hsu_face<R>(w, CT(W, neg ? k - 1 : k + 1), au, ad, CT(PR, d), edge ? R(0.) : CT(PR, u) - auu, t * t, amin(u), amin(d),
-                                dsi(2 * k + 1), DT);
+        const R apu = CT(PR, u), add = (neg ? k + 1 == nk : k == 1) ? R(0.) : wa(neg ? k + 2 : k - 1);
+        CT(FF, k) = hsu_face<R>(w, CT(W, neg ? k - 1 : k + 1), CT(W, neg ? k + 1 : k - 1), au, ad, add, apu, CT(PR, d), edge ? R(0.) : apu - auu,
+                                t * t, amin(u), amin(d), dsi(2 * k + 1), DT);
       }
     __syncthreads();
     if (c.valid && layer)
@@ -283,11 +284,12 @@ __global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : 
         const R w = CT(W, k);
         const bool neg = is_neg(w);   // from interface k-1 down to k, else from k up to k-1
         const int u = neg ? k - 1 : k, d = neg ? k : k - 1;
-        // no velocity upstream of the last layer's, and none below the first one's interface (for
+        // no velocity beyond the last layer's, and none below the first one's interface (for
         // k = 1 and k - 1 < kf); the predictor keeps the field at interface kf - 1
-        const R w_up = neg ? ((k == 1 || k - 1 < kf) ? R(0.) : CT(W, k - 1)) : (k == nk ? R(0.) : CT(W, k + 1));
+        const R w_m = (k == 1 || k - 1 < kf) ? R(0.) : CT(W, k - 1), w_p = k == nk ? R(0.) : CT(W, k + 1);
+        const R add = neg ? (k == nk ? R(0.) : wa(k + 1)) : (k == kf ? R(0.) : wa(k - 2));
         const R d_up = neg ? (k - 1 == kf - 1 ? R(0.) : CT(PR, k - 1) - wa(k - 2)) : (k == nk ? R(0.) : CT(PR, k) - wa(k + 1));
-        CT(FF, k) = hsu_face<R>(w, w_up, wa(u), wa(d), CT(PR, d), d_up, aa(u), R(0.), R(0.), dsi(2 * k), DT);
+        CT(FF, k) = hsu_face<R>(w, neg ? w_m : w_p, neg ? w_p : w_m, wa(u), wa(d), add, CT(PR, u), CT(PR, d), d_up, aa(u), R(0.), R(0.), dsi(2 * k), DT);
       }
     __syncthreads();
     if (c.valid)

@@ -385,7 +385,9 @@ __global__ void k_hsu_zonal(DevModel M, double *buff, int kind, int kstart, RowS
     const int west = (e - 1) & mask, u = neg ? e : west, d = neg ? west : e, uu = (neg ? e + 1 : e - 2) & mask;
     const R au = a[u], ad = a[d], auu = a[uu];
     const R t = fabs((neg ? ad : auu) - twice_of(au) + (neg ? auu : ad)) + R(1.e-10);
-    return hsu_face<R>(v, w[neg ? e + 2 : e], au, ad, ap[d], ap[u] - auu, t * t, a_min, a_min, mn1, DT);
+    const R apu = ap[u];
+    return hsu_face<R>(v, w[neg ? e + 2 : e], w[neg ? e : e + 2], au, ad, a[(neg ? e - 2 : e + 1) & mask], apu, ap[d], apu - auu, t * t, a_min, a_min,
+                       mn1, DT);
   };
   for (int e = L.gl; e < ni; e += 2 * L.G) {   // two faces at once: each is a chain of ~15 dependent operations
     const int e1 = e + L.G;

@@ -609,10 +609,10 @@ template <class R>
 __device__ __forceinline__ R hsu_floor(const DevModel &M, int kind, int k) {
   return kind == 2 ? cv<R>(M.h_min[k]) : (kind == 3 ? cv<R>(1.e-3 * M.kinvisc) : R(0.));
 }
-// The corrector flux through v row j (1..nj) by velocity w: the rows u and d are upstream and
-// downstream of it, uu the row beyond u.  a, ap: the field and the predicted field by row.
+// The corrector flux through v row j (1..nj) by velocity w (w_s, w_n: rows j-1 and j+1): the rows u and d
+// are upstream and downstream of it, uu the row beyond u.  a, ap: the field and the predicted field by row.
 template <class R, class FA, class FP>
-__device__ __forceinline__ R hsu_merid_flux(const DevModel &M, R w, R w_up, int j, R a_min, R DT, FA a, FP ap) {
+__device__ __forceinline__ R hsu_merid_flux(const DevModel &M, R w, R w_s, R w_n, int j, R a_min, R DT, FA a, FP ap) {
   const int nj = M.nj;
   const bool neg = is_neg(w);            // from row j south to j-1, else from j-1 north to j
   const int u = neg ? j : j - 1, d = neg ? j - 1 : j, uu = neg ? j + 1 : j - 2;
@@ -621,7 +621,9 @@ __device__ __forceinline__ R hsu_merid_flux(const DevModel &M, R w, R w_up, int 
   R t;
   if (edge) t = fabs(neg ? ad - au : -au + ad) + R(1.e-10);
   else t = fabs((neg ? ad : auu) - twice_of(au) + (neg ? auu : ad)) + R(1.e-10);
-  return hsu_face<R>(w, w_up, au, ad, ap(d), edge ? R(0.) : ap(u) - auu, t * t, a_min, a_min, cv<R>(M.mn[2 * j]), DT);
+  const R apu = ap(u), add = (neg ? d == 0 : d == nj) ? R(0.) : a(neg ? j - 2 : j + 1);
+  return hsu_face<R>(w, neg ? w_n : w_s, neg ? w_s : w_n, au, ad, add, apu, ap(d), edge ? R(0.) : apu - auu, t * t, a_min, a_min, cv<R>(M.mn[2 * j]),
+                     DT);
 }
 
 template <class R>
@@ -633,7 +635,7 @@ __global__ void k_hsu_merid_pred(DevModel M, const double *A, int kind, int k0) 
   R ff = R(0.);
   if (c.j >= 1 && c.j <= M.nj) {
     const R w = vm_at<R>(M, V, kind, c.k, c.j, c.i);
-    ff = w * cv<R>(A[M.at(c.k, is_neg(w) ? c.j : c.j - 1, c.i)]);
+    ff = hsu_upwind<R>(w, cv<R>(A[M.at(c.k, c.j, c.i)]), cv<R>(A[M.at(c.k, c.j - 1, c.i)]));
   }
   write_with_pads(M.work1, M, M.at(c.k, c.j, 0), c.i, ff);
 }
@@ -660,8 +662,7 @@ __global__ void k_hsu_merid_corr(DevModel M, const double *A, int kind, int k0) 
     const double *V = M.v + plane_offset(M, PL_UV);
     const double *AP = M.work2;
     const R w = vm_at<R>(M, V, kind, k, j, i);
-    const R w_up = vm_at<R>(M, V, kind, k, is_neg(w) ? j + 1 : j - 1, i);
-    ffv = hsu_merid_flux<R>(M, w, w_up, j, hsu_floor<R>(M, kind, k), cv<R>(M.dt), [&](int jj) { return cv<R>(A[M.at(k, jj, i)]); },
+    ffv = hsu_merid_flux<R>(M, w, vm_at<R>(M, V, kind, k, j - 1, i), vm_at<R>(M, V, kind, k, j + 1, i), j, hsu_floor<R>(M, kind, k), cv<R>(M.dt), [&](int jj) { return cv<R>(A[M.at(k, jj, i)]); },
                             [&](int jj) { return cv<R>(AP[M.at(k, jj, i)]); });
   }
   write_with_pads(M.work3, M, M.at(k, j, 0), i, ffv);
@@ -729,7 +730,7 @@ __global__ void k_hsu_meridional(DevModel M, double *A, int kind, int k0) {
     R ffv_1 = R(0.);
     if (j + 1 <= nj)
       ffv_1 = hsu_merid_flux<R>(
-          M, w_1, is_neg(w_1) ? w_2 : w_0, j + 1, a_min, DT,
+          M, w_1, w_0, w_2, j + 1, a_min, DT,
           [&](int jj) { return jj <= j ? (jj < j ? a_m1 : a_0) : (jj > j + 1 ? a_2 : a_1); }, [&](int jj) { return jj <= j ? ap_0 : ap_1; });
     // the update of row j (k_hsu_merid_update)
     const R da = (ffv_0 - ffv_1) * cv<R>(M.mn[2 * j + 1]) * cv<R>(M.dt);
@@ -778,7 +779,7 @@ __global__ void __launch_bounds__(256) k_hsu_merid_tile(DevModel M, double *A, i
   if (live)
     for (int j = 1 + ty; j <= nj; j += ny) {   // ff of rows 0 and nj+1 stays 0
       const R v = w[j * TC];
-      ff[j * TC] = hsu_merid_flux<R>(M, v, w[(is_neg(v) ? j + 1 : j - 1) * TC], j, a_min, DT, [&](int jj) { return a[jj * TC]; },
+      ff[j * TC] = hsu_merid_flux<R>(M, v, w[(j - 1) * TC], w[(j + 1) * TC], j, a_min, DT, [&](int jj) { return a[jj * TC]; },
                                      [&](int jj) { return ap[jj * TC]; });
     }
   __syncthreads();
