@@ -28,9 +28,19 @@ namespace epic {
 enum RowTab { RT_NINV_H, RT_MINV_V, RT_MINV_H, RT_MNINV_H, RT_MNINV_V, RT_MNPV, RT_GDX, RT_GDY, RT_M_H, RT_M_V, RT_N_V, RT_MN_H, RT_F_V,
               RT_COUNT = 16 };
 
-constexpr int SCRATCH_SETS = 3;   // work0..3, once per branch of the step that uses them concurrently
-constexpr int TABLE_SETS = 4;     // ptable, once per field of the 3-D filter
-constexpr int SCRATCH_VOLUMES = 3 + 4 * SCRATCH_SETS;   // gz, unity, old and the sets of work0..3
+constexpr int SCRATCH_VOLUMES = 8;   // gz, unity, old, work0..3, lp3
+constexpr int TABLE_SETS = 4;        // ptable, once per field of the 3-D filter
+// Which volumes are work0..3 of a branch of the step (scratch_sets).  Concurrent branches keep theirs apart
+// in volumes that nothing else uses at the time, so that they cost a model no memory: GZ until the 3-D
+// filter needs it, OLD before THETA's and after NU_TURB's advection, UNITY after advection, DZDT3 until
+// store_pgrad_vars writes every cell that the branch does (rows 0..nj of layers 1..nk), lp3 in the FP64 form.
+enum ScratchSet { WS_MAIN = 0,      // the model's own
+                  WS_KIN_TURB,      // uv_core beside source_sink_turb: KIN in lp3
+                  WS_UNITY,         // UNITY's Akima fluxes in DZDT3
+                  WS_THETA,         // THETA's hyperviscosity in GZ and OLD, its Akima fluxes in GZ
+                  WS_THETA_TURB,    // THETA's hyperviscosity beside HDRY's and NU_TURB's: in work0 and work3
+                  WS_NU,            // NU_TURB's diffusion and hyperviscosity in GZ, OLD and lp3, its Akima fluxes in GZ
+                  WS_V };           // V's hyperviscosity and filtered copy beside U's: in UNITY and OLD
 
 // Time-plane indices and step counters live on the device so that one captured CUDA graph
 // serves every step (the reference rotates IT_ZERO/IT_MINUS1/IT_MINUS2 on the host,
@@ -104,6 +114,7 @@ struct DevModel {
   int stab;                                 // grid.stability_factor "Collins et al. (2004)" (else "off")
   double kinvisc, dynvisc, max_nu2;         // planet->kinvisc, planet->dynvisc, set_max_nu's max_nu[2]
   double *nu_turb, *dc_uv, *dc_theta, *dc_mass;   // NU_TURB and DIFFUSION_COEF_UV, _THETA, _MASS
+  double *turb_tau;                         // scratch: the wall stresses, one per column
   double *turb_pole;                        // scratch: the polar TAU12 rows of uv_horizontal_diffusion
   const double *turb_maxnu2;                // set_diffusion_coef's taper max_nu[2] MIN(1, (dy0 m)^-2), j = 0..nj
   int mixed;                                // FP32 stencils, advection, hyperviscosity, filter, physics
@@ -116,9 +127,8 @@ struct DevModel {
   double *gz3, *mont3, *heat3, *pv3, *ri2, *div_uv3, *w3, *dzdt3, *u_spinup, *gz_surface;
   // scratch
   double *gz, *unity, *old, *work0, *work1, *work2, *work3, *ptable;
-  int wset, tset;   // which of the SCRATCH_SETS copies of work0..3 and of the TABLE_SETS copies of
-                    // ptable this launch's work0..3 and ptable are (concurrent branches of a step
-                    // keep theirs apart; on a member's own description both are 0)
+  int wset, tset;   // which ScratchSet this launch's work0..3 are and which of the TABLE_SETS copies of
+                    // ptable its ptable is (on a member's own description both are 0)
   float2 *lp3;   // log P3 at every interface as a double-float: written by set_p2etc of the mixed
                  // form (stage 11), read by its store_pgrad_vars (stage 19); P3 does not change
                  // between the two
@@ -148,7 +158,7 @@ struct DevModel {
 // A pointer into member 0's arrays, moved to the same place in member `to`'s arrays.  The pool of
 // a model (epic_model_create) packs the state arrays back to back as planes of n3 values (u and v
 // value planes, the tendency planes, then the single fields), and carves the scratch volumes gz,
-// unity, old and the sets of work0..3 one after another, each rounded up to 256 bytes (and, with the turbulence
+// unity, old, work0..3, lp3 one after another, each rounded up to 256 bytes (and, with the turbulence
 // closure, NU_TURB and the three diffusivities the same way); so the plane (or volume) index and
 // the offset inside it follow from the address by integer arithmetic, and map to the member's
 // pool with its own n3.  A pointer outside these regions (a table) is returned as is.
@@ -191,12 +201,18 @@ __device__ __forceinline__ P *member_ptr(const DevModel &M, const DevModel &mem,
   if (M.hetero) return relocate_field(M, mem, p);
   return (P *)(mem.pool_base + ((const char *)p - M.pool_base));
 }
-// Point work0..3 and ptable of a description that has sets 0 at sets ws and ts; n3: the field size
-// of the model whose arrays it carries.
-__host__ __device__ __forceinline__ void scratch_sets(DevModel &M, int ws, int ts, long long n3) {
+// Point work0..3 and ptable of a description that has its own at sets ws and ts.
+__host__ __device__ __forceinline__ void scratch_sets(DevModel &M, int ws, int ts) {
   if (ws) {
-    const long long st = 4LL * ws * (scratch_stride(n3) / 8);
-    M.work0 += st; M.work1 += st; M.work2 += st; M.work3 += st;
+    double *lp3 = reinterpret_cast<double *>(M.lp3);
+    switch (ws) {
+      case WS_KIN_TURB: M.work0 = lp3; break;
+      case WS_UNITY: M.work3 = M.dzdt3; break;
+      case WS_THETA: M.work1 = M.gz; M.work2 = M.old; M.work3 = M.gz; break;
+      case WS_THETA_TURB: M.work1 = M.work0; M.work2 = M.work3; break;
+      case WS_NU: M.work0 = M.gz; M.work1 = M.old; M.work2 = lp3; M.work3 = M.gz; break;
+      case WS_V: M.work1 = M.unity; M.work2 = M.old; break;
+    }
     M.wset = ws;
   }
   if (ts) {
@@ -211,7 +227,7 @@ __device__ __forceinline__ bool epic_member(DevModel &M, P *&...ptrs) {
     ((ptrs = member_ptr(M, mem, ptrs)), ...);
     const int ws = M.wset, ts = M.tset;
     M = mem;
-    scratch_sets(M, ws, ts, M.n3);
+    scratch_sets(M, ws, ts);
   }
   return M.ctl->halted != 0;
 }

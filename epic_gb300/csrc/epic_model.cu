@@ -265,9 +265,9 @@ int run_stage_on(const DevModel &M, cudaStream_t s, int stage) {
       break;
     case 23:
       if (M.turb) {
-        launch_tau_wall_h(M, M.work0, s);
+        launch_tau_wall_h(M, s);
         launch_theta_vdiff(M, s, false);
-        launch_nu_vdiff(M, M.work0, s);
+        launch_nu_vdiff(M, s);
       }
       break;
     case 24:
@@ -335,21 +335,24 @@ struct Lanes {
 };
 
 // The launch description with work0..3 of set ws and ptable of set ts.
-DevModel with_scratch(const DevModel &M, int ws, int ts) {
+DevModel with_scratch(const DevModel &M, int ws, int ts = 0) {
   DevModel d = M;
-  epic::scratch_sets(d, ws, ts, M.batch ? M.reloc_n3 : M.n3);
+  epic::scratch_sets(d, ws, ts);
   return d;
 }
 
 // One step (timestep(STEP_PROGS_AND_SYNC_DIAGS), epic_timestep.c:130-390), the stages of
-// run_stage_on in an order of the same dependences.  Scratch: lanes 0, 1 / 3 and 2 hold sets 0, 1
-// and 2 of work0..3 (lane 1's uv_core takes work0 alone, lane 3's scalars work1..3; NU_TURB's horizontal
-// diffusion takes set 1 whole, on lane 3 once lane 1 is done with it).
+// run_stage_on in an order of the same dependences.  Scratch: each branch has the ScratchSet that its name
+// says; without the closure uv_core's KIN is in work0, which lane 0 does not use until it has joined.
+// The Hsu pass's form of four launches takes work1..3 themselves: where a field is large enough for it (or the
+// tuning table asks for it) UNITY, HDRY and THETA follow one another there.
 int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
   using namespace epic;
   Lanes one(s);
   Lanes &L = lanes ? *lanes : one;
-  const DevModel M1 = with_scratch(M, 1, 1), M2 = with_scratch(M, 2, 2), M3 = with_scratch(M, 1, 3);
+  const DevModel M_kin = M.turb ? with_scratch(M, WS_KIN_TURB) : M, M_unity = with_scratch(M, WS_UNITY), M_theta = with_scratch(M, WS_THETA),
+                 M_nu = with_scratch(M, WS_NU), M_v = with_scratch(M, WS_V);
+  const bool passes = !M.akima && (hsu_meridional_form(M, M.nk) == HSU_PASSES || hsu_meridional_form(M, M.nk - M.k_sigma + 2) == HSU_PASSES);
   auto vertical = M.akima ? launch_akima_vertical : launch_hsu_vertical;
   auto meridional = M.akima ? launch_akima_meridional : launch_hsu_meridional;
   auto zonal = M.akima ? launch_akima_zonal : launch_hsu_zonal;
@@ -365,30 +368,31 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
   for (int q = 0; q < LANES; q++)
     if (q != w_lane && (q != 0 || M.turb)) L.after(q, w_done);
   // lane 1: DUDT, DVDT of uv_core and uv_drag
-  launch_uv_core(M1, L[1]);
-  launch_uv_drag(M1, L[1]);
+  launch_uv_core(M_kin, L[1]);
+  launch_uv_drag(M, L[1]);
   // lane 2: UNITY advected
-  vertical(M2, M.unity, 0, L[2]);
-  meridional(M2, M.unity, 0, L[2]);
-  zonal(M2, M.unity, 0, 1, L[2]);
+  vertical(M, M.unity, 0, L[2]);
+  meridional(passes ? M : M_unity, M.unity, 0, L[2]);
+  zonal(M, M.unity, 0, 1, L[2]);
+  if (passes) L.after(0, 2);
   if (M.turb) {
-    if (M.turb_v) launch_tau_wall_h(M, M2.work0, L[2]);
+    if (M.turb_v) launch_tau_wall_h(M, L[2]);
     launch_source_sink_turb(M, L[0]);
     L.after(0, 1);   // the subgrid diffusion's set_p2etc rewrites P3 and H3, which lane 1 reads
     L.after(3, 0);
     if (M.turb_h) {
       launch_theta_hdiff(M, L[0], true);
-      launch_nu_hdiff(M3, L[3]);
+      launch_nu_hdiff(M_nu, L[3]);
     }
     L.after(2, 0);
   }
   // lane 0: HDRY's hyperviscosity, lane 3 THETA's (with the closure lane 2 THETA's, lane 3 NU_TURB's)
   if (M.turb) {
-    launch_hyperviscosity(M2, 3, M.theta, PL_NONE, L[2]);
-    launch_hyperviscosity(M3, 4, M.nu_turb, PL_NONE, L[3]);
+    launch_hyperviscosity(with_scratch(M, WS_THETA_TURB), 3, M.theta, PL_NONE, L[2]);
+    launch_hyperviscosity(M_nu, 4, M.nu_turb, PL_NONE, L[3]);
     launch_restore_nu(M, L[3]);
   } else {
-    launch_hyperviscosity(M3, 3, M.theta, PL_NONE, L[3]);
+    launch_hyperviscosity(M_theta, 3, M.theta, PL_NONE, L[3]);
   }
   launch_hyperviscosity(M, 2, M.hdry, PL_NONE, L[0]);   // then restore_mass, in the same kernel
   if (M.turb) {
@@ -396,26 +400,33 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
     L.after(3, 2);
     if (M.turb_v) {
       launch_theta_vdiff(M, L[0], true);
-      launch_nu_vdiff(M, M2.work0, L[3]);
+      launch_nu_vdiff(M, L[3]);
     }
     L.after(3, 0);
   }
   // lane 3: THETA's advection (and NU_TURB's) corrected by UNITY's; lane 0: HDRY's
-  vertical(M3, M.theta, 1, L[3]);
-  meridional(M3, M.theta, 1, L[3]);
+  auto advect_hdry = [&] {
+    L.after(0, w_done);
+    vertical(M, M.hdry, 2, L[0]);
+    meridional(M, M.hdry, 2, L[0]);
+    zonal(M, M.hdry, 1, 1, L[0]);   // then restore_mass, in the same kernel
+  };
+  if (passes) {
+    advect_hdry();
+    L.after(3, 0);
+  }
+  vertical(M, M.theta, 1, L[3]);
+  meridional(passes ? M : M_theta, M.theta, 1, L[3]);
   L.after(3, 2);
-  zonal(M3, M.theta, 3, M.k_sigma - 1, L[3]);
+  zonal(M, M.theta, 3, M.k_sigma - 1, L[3]);
   if (M.turb) {
     launch_advection_prep(M, 1, L[3]);
-    vertical(M3, M.nu_turb, 3, L[3]);
-    meridional(M3, M.nu_turb, 3, L[3]);
-    zonal(M3, M.nu_turb, 2, 1, L[3]);
+    vertical(M, M.nu_turb, 3, L[3]);
+    meridional(passes ? M : M_nu, M.nu_turb, 3, L[3]);
+    zonal(M, M.nu_turb, 2, 1, L[3]);
     launch_advection_prep(M, 2, L[3]);
   }
-  L.after(0, w_done);
-  vertical(M, M.hdry, 2, L[0]);
-  meridional(M, M.hdry, 2, L[0]);
-  zonal(M, M.hdry, 1, 1, L[0]);   // then restore_mass, in the same kernel
+  if (!passes) advect_hdry();
   L.after(0, 1);                  // lane 1 has read P3 and H3
   launch_set_p2etc(M, 0, L[0], true);
   L.after(0, 3);
@@ -426,11 +437,12 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
   launch_gz_monotone(M, L[0]);
   // the 3-D filter: lane 1 DUDT, lane 2 DVDT, lane 3 THETA (and NU_TURB), lane 0 HDRY
   L.fork();
-  launch_varz_filter(M1, M.dudt, PL_UV_TEND, 0, 1, M.nk, L[1]);
-  launch_varz_filter(M2, M.dvdt, PL_UV_TEND, 1, 1, M.nk, L[2]);
-  launch_varz_filter(M3, M.theta, PL_NONE, 3, M.k_sigma - 1, M.nk, L[3]);
+  const DevModel T1 = with_scratch(M, WS_MAIN, 1), T2 = with_scratch(M, WS_MAIN, 2), T3 = with_scratch(M, WS_MAIN, 3);   // tables of their own
+  launch_varz_filter(T1, M.dudt, PL_UV_TEND, 0, 1, M.nk, L[1]);
+  launch_varz_filter(T2, M.dvdt, PL_UV_TEND, 1, 1, M.nk, L[2]);
+  launch_varz_filter(T3, M.theta, PL_NONE, 3, M.k_sigma - 1, M.nk, L[3]);
   if (M.turb) {
-    launch_varz_filter(M3, M.nu_turb, PL_NONE, 4, 0, M.nk, L[3]);
+    launch_varz_filter(T3, M.nu_turb, PL_NONE, 4, 0, M.nk, L[3]);
     launch_restore_nu(M, L[3]);
   }
   launch_varz_filter(M, M.hdry, PL_NONE, 2, 1, M.nk, L[0]);   // then restore_mass, in the same kernel
@@ -469,12 +481,12 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
   // lane 0: U, lane 1: V; the filtered copies go on in the same lanes
   L.after(1, 0);
   launch_hyperviscosity(M, 0, M.u, PL_UV, L[0]);
-  launch_hyperviscosity(M1, 1, M.v, PL_UV, L[1]);
+  launch_hyperviscosity(M_v, 1, M.v, PL_UV, L[1]);
   const cudaEvent_t u_done = L.point(0), v_done = L.point(1);
   L.after(2, u_done);
   L.after(3, v_done);
   launch_diag_filter_u(M, L[0], L[2]);
-  launch_diag_filter_v(M1, L[1], L[3]);
+  launch_diag_filter_v(M_v, L[1], L[3]);
   const cudaEvent_t u_rest = L.point(2), v_rest = L.point(3);
   launch_diag_pv_poles(M, L[2]);
   L.after(2, v_done);
@@ -484,7 +496,7 @@ int enqueue_step_on(const DevModel &M, cudaStream_t s, Lanes *lanes = nullptr) {
   launch_diag_div(M, L[0]);
   L.after(1, u_done);
   L.after(1, v_rest);
-  launch_diag_pv(M1, L[1]);
+  launch_diag_pv(M_v, L[1]);
   if (M.turb) {   // of the winds and NU_TURB
     L.after(3, u_done);
     L.after(3, v_done);
@@ -642,7 +654,7 @@ size_t model_pool_bytes(const epic_grid &g) {
   const size_t n3 = (size_t)L.n3, n2 = (size_t)L.n2;
   const size_t nvp = g.uv_scheme == EPIC_UV_AB3 ? 1 : 2, ntp = g.uv_scheme == EPIC_UV_AB3 ? 3 : 1;
   const size_t n_state3 = 2 * nvp + 2 * ntp + 20;   // u,v planes + tendencies + 20 single fields
-  const size_t n_scratch3 = epic::SCRATCH_VOLUMES + 1;   // gz, unity, old, the sets of work0..3; lp3 (float2)
+  const size_t n_scratch3 = epic::SCRATCH_VOLUMES;   // gz, unity, old, work0..3, lp3 (float2)
   const size_t nj1 = 2 * (g.nj + 1) + 1, ni1 = 2 * (g.ni + 1) + 1, nk1 = 2 * (g.nk + 1) + 1;
   const size_t ntw = epic::twiddle_doubles(g.ni);
   auto rnd = [](size_t b) { return ((b + 255) / 256) * 256; };
@@ -650,7 +662,7 @@ size_t model_pool_bytes(const epic_grid &g) {
          rnd(ni1 * 8) + 10 * rnd(nj1 * 8) + 3 * rnd(nk1 * 8) + rnd((g.nk + 2) * 8) + rnd((g.k_sponge + 1) * 8) +
          2 * rnd(3 * (g.nj + 2) * 8) + rnd(ntw * 8) + rnd(ntw * 4) + 2 * rnd((g.nj + 1) * 8) + rnd(sizeof(epic::MathTable)) +
          rnd(32 * sizeof(float2)) + rnd((size_t)(g.nj + 2) * epic::RT_COUNT * 8) + rnd((size_t)(g.nj + 2) * epic::RT_COUNT * 4) + rnd((size_t)(g.nj + 2) * 24 * 8) + rnd((size_t)(g.nj + 2) * 24 * 4) + rnd(((size_t)epic::TH_N * epic::TH_M + 4 * epic::TH_M + epic::TH_N) * 8) +
-         (g.turbulence ? 4 * rnd(n3 * 8) + rnd(2 * (size_t)(g.nk + 2) * 8) + rnd((size_t)(g.nj + 1) * 8) : 0) + 4096;
+         (g.turbulence ? 4 * rnd(n3 * 8) + rnd(n2 * 8) + rnd(2 * (size_t)(g.nk + 2) * 8) + rnd((size_t)(g.nj + 1) * 8) : 0) + 4096;
 }
 
 }  // namespace
@@ -799,7 +811,6 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
   p += (256 - ((size_t)(p - m->pool) & 255)) & 255;   // the scratch and tables start 256-aligned
   double **s3[] = {&d.gz, &d.unity, &d.old, &d.work0, &d.work1, &d.work2, &d.work3};
   for (double **q : s3) *q = carve<double>(p, n3);
-  for (int q = 0; q < 4 * (epic::SCRATCH_SETS - 1); q++) carve<double>(p, n3);   // work0..3 of the other sets
   d.lp3 = carve<float2>(p, n3);
   d.gz_surface = carve<double>(p, n2);
   double *hlh = carve<double>(p, n2), *hlpv = carve<double>(p, n2);
@@ -831,6 +842,7 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
       epic_model_destroy(m);
       return set_error(EPIC_ERR_STATE, "internal pool layout of the turbulence arrays differs from the batch relocation's");
     }
+    d.turb_tau = carve<double>(p, n2);
     d.turb_pole = carve<double>(p, 2 * (size_t)(g->nk + 2));
     d.turb_maxnu2 = carve<double>(p, (size_t)g->nj + 1);
   }
@@ -841,7 +853,7 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
   // the layout relocate_field (batches of mixed sizes) relies on: packed state planes, then the
   // scratch volumes at one stride
   if ((const char *)d.u_spinup - (const char *)d.u != (long long)(2 * d.nvp + 2 * d.ntp + 19) * d.n3 * 8 ||
-      (const char *)d.lp3 - (const char *)d.gz != epic::SCRATCH_VOLUMES * epic::scratch_stride(d.n3)) {
+      (const char *)d.lp3 - (const char *)d.gz != (epic::SCRATCH_VOLUMES - 1) * epic::scratch_stride(d.n3)) {
     epic_model_destroy(m);
     return set_error(EPIC_ERR_STATE, "internal pool layout differs from the batch relocation's");
   }

@@ -464,9 +464,10 @@ __device__ __forceinline__ void vd_solve(int n, const double *U0, const double *
   }
 }
 
-// tw: the wall stresses (NU_TURB: WALL_H; U, V: their own)
-__global__ void __launch_bounds__(VD_THREADS) k_vdiff(DevModel M, int what, const double *tw) {
-  if (epic_member(M, tw)) return;
+// M.turb_tau: the wall stresses (NU_TURB: WALL_H; U, V: their own)
+__global__ void __launch_bounds__(VD_THREADS) k_vdiff(DevModel M, int what) {
+  if (epic_member(M)) return;
+  const double *tw = M.turb_tau;
   extern __shared__ double vd[];
   __shared__ int s_bad[32];
   __shared__ double s_dz[32];
@@ -625,13 +626,13 @@ __global__ void __launch_bounds__(VD_THREADS) k_vdiff(DevModel M, int what, cons
 
 // the wall stresses of all columns: WALL_U, WALL_V (tau_surface reads the neighbours' bottom winds,
 // which the columns' solves then change) or WALL_H
-__global__ void k_tau_wall(DevModel M, int index, double *tw) {
-  if (epic_member(M, tw)) return;
+__global__ void k_tau_wall(DevModel M, int index) {
+  if (epic_member(M)) return;
   const int j0 = index == WALL_V ? 1 : 0;
   const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (t >= (M.nj + 1 - j0) * M.ni) return;
   const int j = j0 + t / M.ni, i = 1 + t - (j - j0) * M.ni;
-  tw[M.at2(j, i)] = tau_wall(M, index, j, i);
+  M.turb_tau[M.at2(j, i)] = tau_wall(M, index, j, i);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -898,23 +899,23 @@ int launch_nu_hdiff(const DevModel &M, cudaStream_t s) {
   return launch_restore_nu(M, s);
 }
 
-static int launch_vdiff(const DevModel &M, int what, const double *tw, cudaStream_t s) {
+static int launch_vdiff(const DevModel &M, int what, cudaStream_t s) {
   const int n = what == VD_THETA ? M.nk - M.k_sigma + 2 : (what == VD_NU ? M.nk + 1 : M.nk - 1);
   const long long cols = (long long)(M.nj + (what == VD_V ? 0 : 1)) * M.ni;
-  k_vdiff<<<zg(nblk(cols, 32), M), VD_THREADS, (size_t)VD_ARRAYS * 32 * (n + 2) * sizeof(double), s>>>(M, what, tw);
+  k_vdiff<<<zg(nblk(cols, 32), M), VD_THREADS, (size_t)VD_ARRAYS * 32 * (n + 2) * sizeof(double), s>>>(M, what);
   return 0;
 }
-int launch_tau_wall_h(const DevModel &M, double *tw, cudaStream_t s) {
-  k_tau_wall<<<zg(nblk((long long)(M.nj + 1) * M.ni, 32), M), 32, 0, s>>>(M, WALL_H, tw);
+int launch_tau_wall_h(const DevModel &M, cudaStream_t s) {
+  k_tau_wall<<<zg(nblk((long long)(M.nj + 1) * M.ni, 32), M), 32, 0, s>>>(M, WALL_H);
   return 0;
 }
 
 int launch_theta_vdiff(const DevModel &M, cudaStream_t s, bool early) {
-  launch_vdiff(M, VD_THETA, nullptr, s);
+  launch_vdiff(M, VD_THETA, s);
   return launch_set_p2etc(M, 1, s, early);
 }
-int launch_nu_vdiff(const DevModel &M, const double *tw, cudaStream_t s) {
-  launch_vdiff(M, VD_NU, tw, s);
+int launch_nu_vdiff(const DevModel &M, cudaStream_t s) {
+  launch_vdiff(M, VD_NU, s);
   return launch_restore_nu(M, s);
 }
 
@@ -938,8 +939,8 @@ int launch_uvh_apply(const DevModel &M, cudaStream_t s) {
 
 int launch_uv_vdiff(const DevModel &M, cudaStream_t s) {
   for (int comp = 0; comp < 2; comp++) {
-    k_tau_wall<<<zg(nblk((long long)(M.nj + 1 - comp) * M.ni, 32), M), 32, 0, s>>>(M, comp == 0 ? WALL_U : WALL_V, M.work0);
-    launch_vdiff(M, comp == 0 ? VD_U : VD_V, M.work0, s);
+    k_tau_wall<<<zg(nblk((long long)(M.nj + 1 - comp) * M.ni, 32), M), 32, 0, s>>>(M, comp == 0 ? WALL_U : WALL_V);
+    launch_vdiff(M, comp == 0 ? VD_U : VD_V, s);
   }
   return 0;
 }

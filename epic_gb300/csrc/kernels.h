@@ -172,10 +172,9 @@ int launch_set_itime(const DevModel &M, long long itime, cudaStream_t s);
 int launch_source_sink_turb(const DevModel &M, cudaStream_t s);
 int launch_theta_hdiff(const DevModel &M, cudaStream_t s, bool early);   // with the set_p2etc that follows (early: launch_set_p2etc's)
 int launch_nu_hdiff(const DevModel &M, cudaStream_t s);      // with restore_mass
-// tw: NU_TURB's wall stresses (launch_tau_wall_h: of the winds, GZ3 and RHO3 alone)
-int launch_tau_wall_h(const DevModel &M, double *tw, cudaStream_t s);
+int launch_tau_wall_h(const DevModel &M, cudaStream_t s);   // NU_TURB's wall stresses, of the winds, GZ3 and RHO3 alone
 int launch_theta_vdiff(const DevModel &M, cudaStream_t s, bool early);   // with the set_p2etc that follows
-int launch_nu_vdiff(const DevModel &M, const double *tw, cudaStream_t s);   // with restore_mass
+int launch_nu_vdiff(const DevModel &M, cudaStream_t s);   // with restore_mass
 int turb_kernels_init(int *cluster);   // on the current device; *cluster: DevModel::sa_cluster
 // uv_horizontal_diffusion: COEFFD and H_RHO; the filtered copies of them (0, 1: after coef), U and V (2, 3); the rest
 int launch_uvh_coef(const DevModel &M, cudaStream_t s);

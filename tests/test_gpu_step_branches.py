@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from epic_gb300 import (Batch, EPIC_ADV_AKIMA, EPIC_ADV_HSU, EPIC_PREC_FP64, EPIC_PREC_MIXED, EPIC_PREC_MIXED_FAST, EPIC_PROFILE_N2,
-                        EPIC_SYNC_DIAGS_ONLY, EPIC_UV_AB3, EPIC_UV_LEAPFROG, HSConfig, Model, hs_setup)
+                        EPIC_SYNC_DIAGS_ONLY, EPIC_UV_AB3, EPIC_UV_LEAPFROG, HSConfig, Model, TUNE_HSU_MERID_VARIANT, hs_setup)
 
 pytestmark = pytest.mark.gpu
 JET = dict(state="jet", profile=EPIC_PROFILE_N2)
@@ -61,3 +61,20 @@ def test_branches_in_a_mixed_size_batch(gpu, form, turbulence):
     b.sync()
     for m, w in zip(models, want):
         _same(m.download(), w, "batch")
+
+
+# the meridional pass as four launches, whose scratch UNITY, HDRY and THETA take one after another
+@pytest.mark.parametrize("form,extra", [(EPIC_PREC_FP64, dict()), (EPIC_PREC_MIXED, dict()), (EPIC_PREC_FP64, dict(turbulence=True, **JET))])
+@pytest.mark.parametrize("sizes", [[(64, 31)], [(32, 17), (64, 32), (32, 40)]])
+def test_branches_with_four_meridional_passes(gpu, form, extra, sizes):
+    grids = [hs_setup(HSConfig(ni=ni, nj=nj, nk=13, dt=60, seed=q, **extra)) for q, (ni, nj) in enumerate(sizes)]
+    want = [_serial(ga, f, form, 3) for ga, f in grids]
+    models = [Model(ga, form) for ga, _ in grids]
+    b = Batch(models)
+    b.set_tuning([0] * TUNE_HSU_MERID_VARIANT + [2])
+    b.upload([f for _, f in grids])
+    b.timestep(EPIC_SYNC_DIAGS_ONLY)
+    b.run(3)
+    b.sync()
+    for m, w in zip(models, want):
+        _same(m.download(), w, "four passes")

@@ -1,7 +1,7 @@
 """What the library launches, by its host code over a stand-in for the CUDA runtime (no GPU is needed)."""
 import pytest
 
-from epic_gb300 import Batch, EPIC_PREC_FP64, EPIC_PREC_MIXED, EPIC_SYNC_DIAGS_ONLY, HSConfig, Model, TUNE_GROUPS, TUNE_HSU_MERID_VARIANT, hs_setup
+from epic_gb300 import Batch, EPIC_PREC_FP64, EPIC_UV_LEAPFROG, EPIC_PREC_MIXED, EPIC_SYNC_DIAGS_ONLY, HSConfig, Model, TUNE_GROUPS, TUNE_HSU_MERID_VARIANT, hs_setup, model_bytes
 from host_library import host_library, host_library_file, launches  # noqa: F401
 
 ROW_KERNELS = ("k_varz_filter_rows", "k_hsu_zonal", "k_filter_planes")
@@ -76,3 +76,14 @@ def test_wavefront_cluster_on_every_device(host_library):
             assert (n, cluster, gx) == (1, want, want)
             m.close()
     host_library.cudaSetDevice(0)
+
+
+@pytest.mark.parametrize("kw,volumes", [(dict(), 28 + 8), (dict(uv_scheme=EPIC_UV_LEAPFROG), 26 + 8), (dict(turbulence=True), 28 + 8 + 4)])
+@pytest.mark.parametrize("shape", [(64, 32, 20), (256, 128, 32)])
+def test_device_bytes_of_a_model(cuda_lib, shape, kw, volumes):
+    """A model takes its state, eight scratch volumes (gz, unity, old, work0..3, lp3; whatever the branches of
+    a step) and tables of less than a volume: what a serving budget was reckoned with."""
+    ni, nj, nk = shape
+    volume = 8 * (ni + 2) * (nj + 3) * (nk + 2)
+    got = model_bytes(hs_setup(HSConfig(ni=ni, nj=nj, nk=nk, dt=60, **kw))[0], EPIC_PREC_FP64)
+    assert volumes * volume < got < (volumes + 1) * volume
