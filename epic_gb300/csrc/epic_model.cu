@@ -929,7 +929,7 @@ extern "C" int epic_model_create(const epic_grid *g, int32_t precision, epic_mod
   epic::column_kernels_init(g->nk);
   epic::column_acc_kernels_init();
   epic::stencil_kernels_init();
-  epic::turb_kernels_init(&d.sa_cluster);
+  if (d.turb) epic::turb_kernels_init(device, &d.sa_cluster);
   epic::filter_gemm_init(g->ni);
   e = cudaStreamSynchronize(m->stream);
   if (e != cudaSuccess) {

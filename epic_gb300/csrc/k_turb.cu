@@ -14,6 +14,8 @@
 //   - the implicit vertical diffusions take a tile of 32 columns per block: the set-up of the bands and
 //     the residual are pointwise in the levels, the band solver's recurrences one warp's;
 //   - uv_horizontal_diffusion's stresses are recomputed where the wind updates read them.
+#include <map>
+#include <mutex>
 #include "device_common.cuh"
 #include "kernels.h"
 #include "epic_common.h"
@@ -947,23 +949,32 @@ int launch_uv_vdiff(const DevModel &M, cudaStream_t s) {
 
 // On the current device, whose own attributes these are: the most shared memory a launch takes (models of
 // all sizes), and the blocks of the wavefront kernel's cluster -- 16 where the GPU can place them (a front of
-// 1235 points at 128x64x20 is then a few per thread's SM), else the portable 8 -- into *cluster.
-int turb_kernels_init(int *cluster) {
+// 1235 points at 128x64x20 is then a few per thread's SM), else the portable 8 -- into *cluster.  Whether it
+// can is asked once per device.
+int turb_kernels_init(int device, int *cluster) {
+  static std::mutex mu;
+  static std::map<int, bool> places16;
   const int big = (int)((size_t)VD_ARRAYS * 32 * (EPIC_TURB_MAX_NK + 3) * sizeof(double));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(16);
-  cfg.blockDim = dim3(SA_THREADS);
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 16;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  int n = 0;
-  const bool ok = cudaFuncSetAttribute(k_sa_waves, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                  cudaOccupancyMaxActiveClusters(&n, k_sa_waves, &cfg) == cudaSuccess && n >= 1;
+  const bool allowed = cudaFuncSetAttribute(k_sa_waves, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    auto known = places16.find(device);
+    if (known == places16.end()) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(16);
+      cfg.blockDim = dim3(SA_THREADS);
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = 16;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      int n = 0;
+      known = places16.emplace(device, allowed && cudaOccupancyMaxActiveClusters(&n, k_sa_waves, &cfg) == cudaSuccess && n >= 1).first;
+    }
+    *cluster = allowed && known->second ? 16 : 8;
+  }
   cudaGetLastError();
-  *cluster = ok ? 16 : 8;
   return cudaFuncSetAttribute(k_vdiff, cudaFuncAttributeMaxDynamicSharedMemorySize, big) == cudaSuccess ? 0 : -1;
 }
 

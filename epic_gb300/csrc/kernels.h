@@ -175,7 +175,7 @@ int launch_nu_hdiff(const DevModel &M, cudaStream_t s);      // with restore_mas
 int launch_tau_wall_h(const DevModel &M, cudaStream_t s);   // NU_TURB's wall stresses, of the winds, GZ3 and RHO3 alone
 int launch_theta_vdiff(const DevModel &M, cudaStream_t s, bool early);   // with the set_p2etc that follows
 int launch_nu_vdiff(const DevModel &M, cudaStream_t s);   // with restore_mass
-int turb_kernels_init(int *cluster);   // on the current device; *cluster: DevModel::sa_cluster
+int turb_kernels_init(int device, int *cluster);   // on the current device; *cluster: DevModel::sa_cluster
 // uv_horizontal_diffusion: COEFFD and H_RHO; the filtered copies of them (0, 1: after coef), U and V (2, 3); the rest
 int launch_uvh_coef(const DevModel &M, cudaStream_t s);
 int launch_uvh_filter(const DevModel &M, int which, cudaStream_t s);

@@ -61,20 +61,20 @@ def test_autotuner_times_the_replayed_step(host_library, ni, nj, form, members):
     b.close()
 
 
-def test_wavefront_cluster_on_every_device(host_library):
+@pytest.mark.parametrize("clusters", [1, 0])
+def test_wavefront_cluster_on_every_device(host_library, clusters):
     """The wavefront kernel's cluster of 16 blocks needs an attribute that belongs to a device: a model of
     the closure on the second device of a process launches it as one on the first does, and a device that
     cannot place 16 takes 8 beside one that can."""
-    for clusters in (1, 0):
-        host_library.fake_device(1, 152, clusters)
-        for device, want in ((0, 16), (1, 16 if clusters else 8)):
-            assert host_library.cudaSetDevice(device) == 0
-            m = _model(16, 8, 4, turbulence=True)
-            host_library.fake_reset_counts()
-            m.timestep()
-            n, cluster, _, gx, _ = launches(host_library, "k_sa_waves")
-            assert (n, cluster, gx) == (1, want, want)
-            m.close()
+    host_library.fake_device(1, 152, clusters)
+    for device, want in ((0, 16), (1, 16 if clusters else 8), (0, 16), (1, 16 if clusters else 8)):
+        assert host_library.cudaSetDevice(device) == 0
+        m = _model(16, 8, 4, turbulence=True)
+        host_library.fake_reset_counts()
+        m.timestep()
+        n, cluster, _, gx, _ = launches(host_library, "k_sa_waves")
+        assert (n, cluster, gx) == (1, want, want)
+        m.close()
     host_library.cudaSetDevice(0)
 
 
