@@ -207,6 +207,8 @@ __global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : 
   R *WA = sm, *W = WA + 32 * L, *PR = W + 32 * L, *FF = PR + 32 * L;
   auto dsi = [&](int kk) { return cv<R>(M.dsgth_inv[kk]); };
   auto wa = [&](int k) { return CT(WA, k); };
+  unsigned top = 0;
+  auto put_pr = [&](int k, R v) { CT(PR, k) = v; top = max(top, top_bits(v)); };
   // W3 at the layer's middle, 0 in the top and bottom layers
   auto w_layer = [&](int k) {
     return (k == 1 || k == nk) ? R(0.) : half_of(cv<R>(M.w3[c.base + k * n2]) + cv<R>(M.w3[c.base + (k - 1) * n2]));
@@ -215,7 +217,11 @@ __global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : 
     for (int k = (layer ? kf : kf - 1) + c.warp; k <= nk; k += c.nw) CT(WA, k) = cv<R>(buff[c.base + k * n2]);
   if (layer || nuk) {
     if (c.valid && layer)
-      for (int k = kf - 1 + c.warp; k <= nk; k += c.nw) CT(W, k) = cv<R>(M.w3[c.base + k * n2]);
+      for (int k = kf - 1 + c.warp; k <= nk; k += c.nw) {
+        const R w = cv<R>(M.w3[c.base + k * n2]);
+        CT(W, k) = w;
+        top = max(top, top_bits(w));   // the first and the last are in no flux
+      }
     if (c.valid && nuk) {
       for (int k = kf + c.warp; k <= nk; k += c.nw) CT(W, k) = w_layer(k);
       // entry 0 is never loaded for NU_TURB; the corrector reads it only against d2(1) = 0
@@ -226,9 +232,20 @@ __global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : 
       for (int k = kf - 1 + c.warp; k <= nk; k += c.nw)
         CT(FF, k) = (k == kf - 1 || k == nk) ? R(0.) : hsu_upwind<R>(CT(W, k), wa(k), wa(k + 1));
     __syncthreads();
-    if (c.valid)
-      for (int k = kf + c.warp; k <= nk; k += c.nw) CT(PR, k) = wa(k) + (CT(FF, k) - CT(FF, k - 1)) * dsi(2 * k) * DT;
-    __syncthreads();
+    auto predict = [&] {
+      if (c.valid)
+        for (int k = kf + c.warp; k <= nk; k += c.nw) put_pr(k, wa(k) + (CT(FF, k) - CT(FF, k - 1)) * dsi(2 * k) * DT);
+    };
+    predict();
+    const bool odd = __syncthreads_or(top >= NONFINITE_BITS<R>);
+    if (odd) {
+      if (c.valid)
+        for (int k = kf + c.warp; k < nk; k += c.nw)
+          if (hsu_upwind_tainted<R>(CT(W, k), wa(k), wa(k + 1))) CT(FF, k) = quiet_nan<R>();
+      __syncthreads();
+      predict();
+      __syncthreads();
+    }
     // the corrector reads PR, WA and W only, so it rewrites FF in place
     if (c.valid)
       for (int k = kf + c.warp; k < nk; k += c.nw) {
@@ -241,9 +258,14 @@ __global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : 
         if (edge) t = fabs(neg ? ad - au : -au + ad) + ep;
         else t = fabs((neg ? ad : auu) - twice_of(au) + (neg ? auu : ad)) + ep;
         auto amin = [&](int q) { return layer ? cv<R>(M.h_min[q]) : cv<R>(1.e-3 * M.kinvisc); };   // HDRY's and NU_TURB's floors
-        const R apu = CT(PR, u), add = (neg ? k + 1 == nk : k == 1) ? R(0.) : wa(neg ? k + 2 : k - 1);
-        CT(FF, k) = hsu_face<R>(w, CT(W, neg ? k - 1 : k + 1), CT(W, neg ? k + 1 : k - 1), au, ad, add, apu, CT(PR, d), edge ? R(0.) : apu - auu,
-                                t * t, amin(u), amin(d), dsi(2 * k + 1), DT);
+        CT(FF, k) = hsu_face<R>(w, CT(W, neg ? k - 1 : k + 1), au, ad, CT(PR, d), edge ? R(0.) : CT(PR, u) - auu, t * t, amin(u), amin(d),
+                                dsi(2 * k + 1), DT);
+      }
+    if (odd && c.valid)
+      for (int k = kf + c.warp; k < nk; k += c.nw) {
+        const bool neg = is_neg(CT(W, k));
+        const R a_dd = (neg ? k + 1 == nk : k == 1) ? R(0.) : wa(neg ? k + 2 : k - 1);
+        if (hsu_tainted<R>(neg, CT(W, neg ? k - 1 : k + 1), CT(W, neg ? k + 1 : k - 1), a_dd, CT(PR, neg ? k : k + 1))) CT(FF, k) = quiet_nan<R>();
       }
     __syncthreads();
     if (c.valid && layer)
@@ -265,10 +287,25 @@ __global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : 
       for (int k = kf + c.warp; k <= nk + 1; k += c.nw)
         CT(FF, k) = k == nk + 1 ? R(0.) : hsu_upwind<R>(CT(W, k), wa(k - 1), wa(k));
     __syncthreads();
-    if (c.valid)
-      for (int k = kf - 1 + c.warp; k <= nk; k += c.nw)
-        CT(PR, k) = k == kf - 1 ? wa(kf - 1) : wa(k) + (CT(FF, k + 1) - CT(FF, k)) * dsi(2 * k + 1) * DT;
-    __syncthreads();
+    auto predict = [&] {
+      if (c.valid)
+        for (int k = kf - 1 + c.warp; k <= nk; k += c.nw)
+          put_pr(k, k == kf - 1 ? wa(kf - 1) : wa(k) + (CT(FF, k + 1) - CT(FF, k)) * dsi(2 * k + 1) * DT);
+    };
+    predict();
+    const bool odd = __syncthreads_or(top >= NONFINITE_BITS<R>);
+    if (odd) {
+      if (c.valid)
+        for (int k = kf + c.warp; k <= nk; k += c.nw)
+          if (hsu_upwind_tainted<R>(CT(W, k), wa(k - 1), wa(k))) CT(FF, k) = quiet_nan<R>();
+      __syncthreads();
+      predict();
+      __syncthreads();
+    }
+    // no velocity beyond the last layer's, and none below the first one's interface (for
+    // k = 1 and k - 1 < kf); the predictor keeps the field at interface kf - 1
+    auto w_m = [&](int k) { return (k == 1 || k - 1 < kf) ? R(0.) : CT(W, k - 1); };
+    auto w_p = [&](int k) { return k == nk ? R(0.) : CT(W, k + 1); };
     // For THETA (kf > 1) the entry below the first loaded one is the value the reference's
     // static column buffer keeps from the preceding unity advection: 1.0 (epic_flux.c:866-877).
     auto aa = [&](int k) {
@@ -284,12 +321,14 @@ __global__ void __launch_bounds__(std::is_same_v<R, double> ? CT_THREADS_WIDE : 
         const R w = CT(W, k);
         const bool neg = is_neg(w);   // from interface k-1 down to k, else from k up to k-1
         const int u = neg ? k - 1 : k, d = neg ? k : k - 1;
-        // no velocity beyond the last layer's, and none below the first one's interface (for
-        // k = 1 and k - 1 < kf); the predictor keeps the field at interface kf - 1
-        const R w_m = (k == 1 || k - 1 < kf) ? R(0.) : CT(W, k - 1), w_p = k == nk ? R(0.) : CT(W, k + 1);
-        const R add = neg ? (k == nk ? R(0.) : wa(k + 1)) : (k == kf ? R(0.) : wa(k - 2));
         const R d_up = neg ? (k - 1 == kf - 1 ? R(0.) : CT(PR, k - 1) - wa(k - 2)) : (k == nk ? R(0.) : CT(PR, k) - wa(k + 1));
-        CT(FF, k) = hsu_face<R>(w, neg ? w_m : w_p, neg ? w_p : w_m, wa(u), wa(d), add, CT(PR, u), CT(PR, d), d_up, aa(u), R(0.), R(0.), dsi(2 * k), DT);
+        CT(FF, k) = hsu_face<R>(w, neg ? w_m(k) : w_p(k), wa(u), wa(d), CT(PR, d), d_up, aa(u), R(0.), R(0.), dsi(2 * k), DT);
+      }
+    if (odd && c.valid)
+      for (int k = kf + c.warp; k <= nk; k += c.nw) {
+        const bool neg = is_neg(CT(W, k));
+        const R a_dd = neg ? (k == nk ? R(0.) : wa(k + 1)) : (k == kf ? R(0.) : wa(k - 2));
+        if (hsu_tainted<R>(neg, neg ? w_m(k) : w_p(k), neg ? w_p(k) : w_m(k), a_dd, CT(PR, neg ? k - 1 : k))) CT(FF, k) = quiet_nan<R>();
       }
     __syncthreads();
     if (c.valid)

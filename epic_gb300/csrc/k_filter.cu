@@ -377,7 +377,22 @@ __global__ void k_hsu_zonal(DevModel M, double *buff, int kind, int kstart, RowS
   const int mask = ni - 1;   // ni is a power of 2: rows wrap
   for (int e = L.gl; e < ni; e += L.G) ff[e] = hsu_upwind<R>(w[e + 1], a[e], a[(e - 1) & mask]);
   __syncwarp();
-  for (int e = L.gl; e < ni; e += L.G) ap[e] = a[e] + (ff[e] - ff[(e + 1) & mask]) * mn1 * DT;
+  unsigned top = 0;
+  auto predict = [&] {
+    for (int e = L.gl; e < ni; e += L.G) {
+      const R p = a[e] + (ff[e] - ff[(e + 1) & mask]) * mn1 * DT;
+      ap[e] = p;
+      top = max(top, top_bits(p));
+    }
+  };
+  predict();
+  const bool odd = __any_sync(0xffffffffu, top >= NONFINITE_BITS<R>);   // in one of the warp's rows
+  if (odd) {
+    for (int e = L.gl; e < ni; e += L.G)
+      if (hsu_upwind_tainted<R>(w[e + 1], a[e], a[(e - 1) & mask])) ff[e] = quiet_nan<R>();
+    __syncwarp();
+    predict();
+  }
   __syncwarp();
   auto face = [&](int e) {
     const R v = w[e + 1];
@@ -385,9 +400,7 @@ __global__ void k_hsu_zonal(DevModel M, double *buff, int kind, int kstart, RowS
     const int west = (e - 1) & mask, u = neg ? e : west, d = neg ? west : e, uu = (neg ? e + 1 : e - 2) & mask;
     const R au = a[u], ad = a[d], auu = a[uu];
     const R t = fabs((neg ? ad : auu) - twice_of(au) + (neg ? auu : ad)) + R(1.e-10);
-    const R apu = ap[u];
-    return hsu_face<R>(v, w[neg ? e + 2 : e], w[neg ? e : e + 2], au, ad, a[(neg ? e - 2 : e + 1) & mask], apu, ap[d], apu - auu, t * t, a_min, a_min,
-                       mn1, DT);
+    return hsu_face<R>(v, w[neg ? e + 2 : e], au, ad, ap[d], ap[u] - auu, t * t, a_min, a_min, mn1, DT);
   };
   for (int e = L.gl; e < ni; e += 2 * L.G) {   // two faces at once: each is a chain of ~15 dependent operations
     const int e1 = e + L.G;
@@ -395,6 +408,11 @@ __global__ void k_hsu_zonal(DevModel M, double *buff, int kind, int kstart, RowS
     ff[e] = f0;
     if (e1 < ni) ff[e1] = f1;
   }
+  if (odd)
+    for (int e = L.gl; e < ni; e += L.G) {
+      const bool neg = is_neg(w[e + 1]);
+      if (hsu_tainted<R>(neg, w[neg ? e + 2 : e], w[neg ? e : e + 2], a[(neg ? e - 2 : e + 1) & mask], ap[neg ? e : (e - 1) & mask])) ff[e] = quiet_nan<R>();
+    }
   __syncwarp();
   if (!L.live) return;
   for (int e0 = L.gl; e0 < ni; e0 += 4 * L.G) {   // four cells' loads before the first store

@@ -609,10 +609,10 @@ template <class R>
 __device__ __forceinline__ R hsu_floor(const DevModel &M, int kind, int k) {
   return kind == 2 ? cv<R>(M.h_min[k]) : (kind == 3 ? cv<R>(1.e-3 * M.kinvisc) : R(0.));
 }
-// The corrector flux through v row j (1..nj) by velocity w (w_s, w_n: rows j-1 and j+1): the rows u and d
-// are upstream and downstream of it, uu the row beyond u.  a, ap: the field and the predicted field by row.
+// The corrector flux through v row j (1..nj) by velocity w: the rows u and d are upstream and
+// downstream of it, uu the row beyond u.  a, ap: the field and the predicted field by row.
 template <class R, class FA, class FP>
-__device__ __forceinline__ R hsu_merid_flux(const DevModel &M, R w, R w_s, R w_n, int j, R a_min, R DT, FA a, FP ap) {
+__device__ __forceinline__ R hsu_merid_flux(const DevModel &M, R w, R w_up, int j, R a_min, R DT, FA a, FP ap) {
   const int nj = M.nj;
   const bool neg = is_neg(w);            // from row j south to j-1, else from j-1 north to j
   const int u = neg ? j : j - 1, d = neg ? j - 1 : j, uu = neg ? j + 1 : j - 2;
@@ -621,9 +621,14 @@ __device__ __forceinline__ R hsu_merid_flux(const DevModel &M, R w, R w_s, R w_n
   R t;
   if (edge) t = fabs(neg ? ad - au : -au + ad) + R(1.e-10);
   else t = fabs((neg ? ad : auu) - twice_of(au) + (neg ? auu : ad)) + R(1.e-10);
-  const R apu = ap(u), add = (neg ? d == 0 : d == nj) ? R(0.) : a(neg ? j - 2 : j + 1);
-  return hsu_face<R>(w, neg ? w_n : w_s, neg ? w_s : w_n, au, ad, add, apu, ap(d), edge ? R(0.) : apu - auu, t * t, a_min, a_min, cv<R>(M.mn[2 * j]),
-                     DT);
+  return hsu_face<R>(w, w_up, au, ad, ap(d), edge ? R(0.) : ap(u) - auu, t * t, a_min, a_min, cv<R>(M.mn[2 * j]), DT);
+}
+// w_s, w_n: the velocities at rows j-1 and j+1
+template <class R, class FA, class FP>
+__device__ __forceinline__ bool hsu_merid_tainted(const DevModel &M, R w, R w_s, R w_n, int j, FA a, FP ap) {
+  const bool neg = is_neg(w);
+  const R a_dd = (neg ? j == 1 : j == M.nj) ? R(0.) : a(neg ? j - 2 : j + 1);
+  return hsu_tainted<R>(neg, neg ? w_n : w_s, neg ? w_s : w_n, a_dd, ap(neg ? j : j - 1));
 }
 
 template <class R>
@@ -635,7 +640,8 @@ __global__ void k_hsu_merid_pred(DevModel M, const double *A, int kind, int k0) 
   R ff = R(0.);
   if (c.j >= 1 && c.j <= M.nj) {
     const R w = vm_at<R>(M, V, kind, c.k, c.j, c.i);
-    ff = hsu_upwind<R>(w, cv<R>(A[M.at(c.k, c.j, c.i)]), cv<R>(A[M.at(c.k, c.j - 1, c.i)]));
+    const R north = cv<R>(A[M.at(c.k, c.j, c.i)]), south = cv<R>(A[M.at(c.k, c.j - 1, c.i)]);
+    ff = hsu_upwind_tainted<R>(w, north, south) ? quiet_nan<R>() : hsu_upwind<R>(w, north, south);
   }
   write_with_pads(M.work1, M, M.at(c.k, c.j, 0), c.i, ff);
 }
@@ -662,8 +668,11 @@ __global__ void k_hsu_merid_corr(DevModel M, const double *A, int kind, int k0) 
     const double *V = M.v + plane_offset(M, PL_UV);
     const double *AP = M.work2;
     const R w = vm_at<R>(M, V, kind, k, j, i);
-    ffv = hsu_merid_flux<R>(M, w, vm_at<R>(M, V, kind, k, j - 1, i), vm_at<R>(M, V, kind, k, j + 1, i), j, hsu_floor<R>(M, kind, k), cv<R>(M.dt), [&](int jj) { return cv<R>(A[M.at(k, jj, i)]); },
-                            [&](int jj) { return cv<R>(AP[M.at(k, jj, i)]); });
+    const R w_s = vm_at<R>(M, V, kind, k, j - 1, i), w_n = vm_at<R>(M, V, kind, k, j + 1, i);
+    auto a = [&](int jj) { return cv<R>(A[M.at(k, jj, i)]); };
+    auto ap = [&](int jj) { return cv<R>(AP[M.at(k, jj, i)]); };
+    ffv = hsu_merid_flux<R>(M, w, is_neg(w) ? w_n : w_s, j, hsu_floor<R>(M, kind, k), cv<R>(M.dt), a, ap);
+    if (hsu_merid_tainted<R>(M, w, w_s, w_n, j, a, ap)) ffv = quiet_nan<R>();
   }
   write_with_pads(M.work3, M, M.at(k, j, 0), i, ffv);
 }
@@ -696,7 +705,7 @@ __global__ void k_hsu_meridional(DevModel M, double *A, int kind, int k0) {
   const double *V = M.v + plane_offset(M, PL_UV);
   const R DT = cv<R>(M.dt), a_min = hsu_floor<R>(M, kind, k);
   auto ld = [&](int jj) { return A[M.at(k, jj, i)]; };
-  auto ff_of = [&](int jj, R w, R am1, R a0) { return (jj >= 1 && jj <= nj) ? hsu_upwind<R>(w, a0, am1) : R(0.); };
+  auto ff_of = [&](int jj, R w, R am1, R a0) { return (jj >= 1 && jj <= nj) ? (hsu_upwind_tainted<R>(w, a0, am1) ? quiet_nan<R>() : hsu_upwind<R>(w, a0, am1)) : R(0.); };
   auto ap_of = [&](int jj, double ad, R ff0, R ff1) { return cv<R>(ad + to_d((ff0 - ff1) * cv<R>(M.mn[2 * jj + 1]) * DT)); };
   // window at the top of iteration j
   R a_m1 = R(0.), a_0, a_1, a_2;   // A(j-1..j+2)
@@ -728,10 +737,12 @@ __global__ void k_hsu_meridional(DevModel M, double *A, int kind, int k0) {
     }
     // FFV(j+1): the corrector flux of row j+1 (k_hsu_merid_corr), its rows j-1..j+2 in the window
     R ffv_1 = R(0.);
-    if (j + 1 <= nj)
-      ffv_1 = hsu_merid_flux<R>(
-          M, w_1, w_0, w_2, j + 1, a_min, DT,
-          [&](int jj) { return jj <= j ? (jj < j ? a_m1 : a_0) : (jj > j + 1 ? a_2 : a_1); }, [&](int jj) { return jj <= j ? ap_0 : ap_1; });
+    if (j + 1 <= nj) {
+      auto a = [&](int jj) { return jj <= j ? (jj < j ? a_m1 : a_0) : (jj > j + 1 ? a_2 : a_1); };
+      auto ap = [&](int jj) { return jj <= j ? ap_0 : ap_1; };
+      ffv_1 = hsu_merid_flux<R>(M, w_1, is_neg(w_1) ? w_2 : w_0, j + 1, a_min, DT, a, ap);
+      if (hsu_merid_tainted<R>(M, w_1, w_0, w_2, j + 1, a, ap)) ffv_1 = quiet_nan<R>();
+    }
     // the update of row j (k_hsu_merid_update)
     const R da = (ffv_0 - ffv_1) * cv<R>(M.mn[2 * j + 1]) * cv<R>(M.dt);
     write_with_pads(A, M, M.at(k, j, 0), i, ad_0 + to_d(da));
@@ -764,24 +775,44 @@ __global__ void __launch_bounds__(256) k_hsu_merid_tile(DevModel M, double *A, i
   R *a = reinterpret_cast<R *>(smraw) + tx, *w = a + (nj + 2) * TC, *ff = w + (nj + 2) * TC, *ap = ff + (nj + 2) * TC;
   const double *V = M.v + plane_offset(M, PL_UV);
   const R DT = cv<R>(M.dt), a_min = hsu_floor<R>(M, kind, k);
+  unsigned top = 0;
   for (int j = ty; j <= nj + 1; j += ny) {
     a[j * TC] = live && j <= nj ? cv<R>(A[M.at(k, j, i)]) : R(0.);
-    w[j * TC] = live ? vm_at<R>(M, V, kind, k, j, i) : R(0.);
+    const R v = live ? vm_at<R>(M, V, kind, k, j, i) : R(0.);
+    w[j * TC] = v;
+    top = max(top, top_bits(v));   // the poles' velocities are in no flux
   }
   __syncthreads();
   for (int j = ty; j <= nj + 1; j += ny)
     ff[j * TC] = j >= 1 && j <= nj ? hsu_upwind<R>(w[j * TC], a[j * TC], a[(j - 1) * TC]) : R(0.);
   __syncthreads();
-  if (live)
-    for (int j = ty; j <= nj; j += ny)
-      ap[j * TC] = cv<R>(A[M.at(k, j, i)] + to_d((ff[j * TC] - ff[(j + 1) * TC]) * cv<R>(M.mn[2 * j + 1]) * DT));
-  __syncthreads();
+  auto predict = [&] {
+    if (live)
+      for (int j = ty; j <= nj; j += ny) {
+        const R p = cv<R>(A[M.at(k, j, i)] + to_d((ff[j * TC] - ff[(j + 1) * TC]) * cv<R>(M.mn[2 * j + 1]) * DT));
+        ap[j * TC] = p;
+        top = max(top, top_bits(p));
+      }
+  };
+  predict();
+  const bool odd = __syncthreads_or(top >= NONFINITE_BITS<R>);
+  if (odd) {
+    for (int j = 1 + ty; j <= nj; j += ny)
+      if (hsu_upwind_tainted<R>(w[j * TC], a[j * TC], a[(j - 1) * TC])) ff[j * TC] = quiet_nan<R>();
+    __syncthreads();
+    predict();
+    __syncthreads();
+  }
   if (live)
     for (int j = 1 + ty; j <= nj; j += ny) {   // ff of rows 0 and nj+1 stays 0
       const R v = w[j * TC];
-      ff[j * TC] = hsu_merid_flux<R>(M, v, w[(j - 1) * TC], w[(j + 1) * TC], j, a_min, DT, [&](int jj) { return a[jj * TC]; },
+      ff[j * TC] = hsu_merid_flux<R>(M, v, w[(is_neg(v) ? j + 1 : j - 1) * TC], j, a_min, DT, [&](int jj) { return a[jj * TC]; },
                                      [&](int jj) { return ap[jj * TC]; });
     }
+  if (odd && live)
+    for (int j = 1 + ty; j <= nj; j += ny)
+      if (hsu_merid_tainted<R>(M, w[j * TC], w[(j - 1) * TC], w[(j + 1) * TC], j, [&](int jj) { return a[jj * TC]; }, [&](int jj) { return ap[jj * TC]; }))
+        ff[j * TC] = quiet_nan<R>();
   __syncthreads();
   if (live)
     for (int j = ty; j <= nj; j += ny) {
