@@ -190,7 +190,10 @@ __host__ __device__ __forceinline__ double div_rn(double a, double b) {
 
 // ---- square root ----
 
-// A reciprocal square root estimate 2^32 y of v in [1, 4), y within 2^-21.5 of 1/sqrt(v).
+// A reciprocal square root estimate 2^32 y of v in [1, 4), y within 2^-21.5 of 1/sqrt(v), relative: the
+// instruction's documented 2^-22.9, v's rounding to binary32 (2^-25), the product's (2^-24) and the factor
+// 1 - 2^-24 together are below 2^-21.7.  An estimate above the largest 32-bit number becomes that number (the
+// conversion saturates), which is nearer.
 __host__ __device__ __forceinline__ uint32_t rsqrt32(uint32_t v30) {   // v in units of 2^-30
 #ifdef __CUDA_ARCH__
   float y;
@@ -209,14 +212,33 @@ static __host__ __device__ EPIC_COLD double sqrt_cold(double x) {
 #endif
 }
 
+// sqrt(v) of v in [1, 4), in units of 2^-62, rounded to nearest in units of 2^-52, from an estimate y0 of
+// 2^32 / sqrt(v) within 2^-21.5.  One Newton step leaves y within 2^-30 (its own error 2^-42, the dropped bits
+// of v and of v y0 add up to 2^-30 y, the last shift takes 2^-32); s = v y is then within 2^-28 of the
+// root, so v - s^2 is at most 2^-26 and its top 32 bits fit an int; and s + (v - s^2) y / 2 with the exact
+// v - s^2 is off by less than 2^-57 (second order) + 2^-55 (y's error) + 2^-57 (the int's dropped bits), and
+// the sum's rounding adds half a unit: within 0.75 units, so the exact remainder of the result moves it by at most
+// one; a root is never half way.  tests/test_fix_sqrt.py moves the estimate to the ends of its bound.
+__host__ __device__ __forceinline__ uint64_t sqrt_steps(uint64_t v, uint32_t y0) {
+  const uint32_t vh = (uint32_t)(v >> 32);                                                  // 2^-30
+  const uint32_t vy = mulhi32(vh, y0);                                                      // v y0, 2^-30
+  const int t = (int)(((int64_t)1 << 46) - (int64_t)(((uint64_t)vy * y0) >> 16));           // 1 - v y0^2, 2^-46
+  const uint32_t yd = y0 + (uint32_t)(int32_t)(((int64_t)t * (int64_t)(uint64_t)y0) >> 47);
+  const uint32_t y = yd < y0 && t > 0 ? 0xffffffffu : yd;                                   // v = 1: y stays below 1
+  const uint32_t s = mulhi32(vh, y);                                                        // 2^-30
+  const int64_t r = (int64_t)(v - ((uint64_t)s * s << 2));                                  // v - s^2, 2^-62, exact
+  const int64_t d = ((int64_t)(int)(r >> 6) * (int64_t)(uint64_t)y + ((int64_t)1 << 36)) >> 37;   // r y / 2, 2^-52
+  uint64_t q = ((uint64_t)s << 22) + (uint64_t)d;
+  const int64_t rem = (int64_t)((v << 42) - q * q);                                         // 2^-104, small
+  q += rem > (int64_t)q ? 1 : 0;
+  q -= rem <= -(int64_t)q ? 1 : 0;
+  return q;
+}
+
 // sqrt(x) rounded to nearest on the integer pipe: about 45 integer instructions where the binary64
-// pipe takes about ten operations, 16 clocks each.  v in [1, 4) is x over an even power of 2.  The
-// estimate y is refined by one Newton step to 2^-30; s = v y is then within 2^-28 of the root (so that
-// v - s^2 is below 2^-26 and its top 32 bits fit an int), and
-// s + (v - s^2) y / 2 with the exact v - s^2 within 2^-54 of it (second-order term 2^-57, the rest from
-// y's error): within 0.6 units of the last place, so the exact remainder of the result moves it by at
-// most one; a root is never half way.  Zeros are answered here (one side of a split velocity always
-// is); subnormals, negative numbers, infinities and NaN go to the function itself.
+// pipe takes about ten operations, 16 clocks each.  v in [1, 4) is x over an even power of 2.  Zeros are
+// answered here (one side of a split velocity always is); subnormals, negative numbers, infinities and NaN go
+// to the function itself.
 __host__ __device__ __forceinline__ double sqrt_rn(double x) {
   uint64_t u;
 #ifdef __CUDA_ARCH__
@@ -229,19 +251,7 @@ __host__ __device__ __forceinline__ double sqrt_rn(double x) {
   if (!zero && e - 1u >= 2046u) return sqrt_cold(x);
   const uint32_t odd = (e & 1u) ^ 1u;       // an even biased exponent is an odd power of 2
   const uint64_t v = ((u & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull) << (10 + odd);   // 2^-62
-  const uint32_t vh = (uint32_t)(v >> 32);                                                  // 2^-30
-  const uint32_t y0 = rsqrt32(vh);                                                          // 2^-32
-  const uint32_t vy = mulhi32(vh, y0);                                                      // v y0, 2^-30
-  const int t = (int)(((int64_t)1 << 46) - (int64_t)(((uint64_t)vy * y0) >> 16));           // 1 - v y0^2, 2^-46
-  const uint32_t yd = y0 + (uint32_t)(int32_t)(((int64_t)t * (int64_t)(uint64_t)y0) >> 47);
-  const uint32_t y = yd < y0 && t > 0 ? 0xffffffffu : yd;                                   // v = 1: y stays below 1
-  const uint32_t s = mulhi32(vh, y);                                                        // 2^-30
-  const int64_t r = (int64_t)(v - ((uint64_t)s * s << 2));                                  // v - s^2, 2^-62, exact
-  const int64_t d = ((int64_t)(int)(r >> 6) * (int64_t)(uint64_t)y + ((int64_t)1 << 36)) >> 37;   // r y / 2, 2^-52
-  uint64_t q = ((uint64_t)s << 22) + (uint64_t)d;
-  const int64_t rem = (int64_t)((v << 42) - q * q);                                         // 2^-104, small
-  q += rem > (int64_t)q ? 1 : 0;
-  q -= rem <= -(int64_t)q ? 1 : 0;
+  const uint64_t q = sqrt_steps(v, rsqrt32((uint32_t)(v >> 32)));
   const uint64_t w = zero ? u : ((uint64_t)((e + 1021u) >> 1) << 52) + q;
 #ifdef __CUDA_ARCH__
   return __longlong_as_double((long long)w);
