@@ -290,30 +290,13 @@ __device__ __forceinline__ void theta2_intervals(const DevModel &M, int *kay, fl
   }
 }
 
-// get_sigma / get_p_sigma / g_sigma / f_sigma / return_sigmatheta, epic_funcs_diag.c:1238-1314,1751-1770
 // In the drop-in form the transcendentals are correctly rounded (dd_math.cuh) so that they agree
 // with the reference's libm; the mixed form's binary64 kernels take the libdevice functions.
 __device__ __forceinline__ double xlog(const DevModel &M, double x) { return M.cr ? cr_log(x, *M.lt) : ::log(x); }
 __device__ __forceinline__ double xexp(const DevModel &M, double x) { return M.cr ? cr_exp(x, *M.lt) : ::exp(x); }
 __device__ __forceinline__ double xpow(const DevModel &M, double x, double y) { return M.cr ? cr_pow(x, y, *M.lt) : ::pow(x, y); }
-__device__ __forceinline__ double get_sigma(const DevModel &M, double pbot, double p, double ptop) {
-  return div_rn(xlog(M, div_rn(p, pbot)), xlog(M, div_rn(ptop, pbot)));
-}
-__device__ __forceinline__ double get_p_sigma(const DevModel &M, double pbot, double sigma, double ptop) {
-  return pbot * xexp(M, sigma * xlog(M, div_rn(ptop, pbot)));
-}
-__device__ __forceinline__ double g_sigma(const DevModel &M, double s) {
-  if (s <= M.sigma_sigma) return 0.;
-  if (s >= 1.) return 1.;
-  return M.g_coeff * (1. - xexp(M, -M.alpha * (s - M.sigma_sigma)));
-}
-__device__ __forceinline__ double f_sigma(const DevModel &M, double s) {
-  if (s < 0.) return M.zeta0;
-  if (s <= M.sigma_sigma) return M.zeta0 + s * (M.zeta1 - M.zeta0);
-  if (s < 1.) return (1. - g_sigma(M, s)) * (M.zeta0 + s * (M.zeta1 - M.zeta0));
-  return 0.;
-}
-// f_sigma(s), with g_sigma(s) returned in g: one exponential and each comparison (a binary64 operation)
+// f_sigma(s), with g_sigma(s) returned in g (epic_funcs_diag.c:1238-1314, 1751-1770; get_sigma, get_p_sigma and
+// return_sigmatheta are parts of the column kernels): one exponential and each comparison (a binary64 operation)
 // serve both.
 __device__ __forceinline__ double f_and_g_sigma(const DevModel &M, double s, double &g) {
   if (s <= M.sigma_sigma) {
@@ -326,11 +309,6 @@ __device__ __forceinline__ double f_and_g_sigma(const DevModel &M, double s, dou
   }
   g = M.g_coeff * (1. - xexp(M, -M.alpha * (s - M.sigma_sigma)));
   return (1. - g) * (M.zeta0 + s * (M.zeta1 - M.zeta0));
-}
-__device__ __forceinline__ double return_sigmatheta(const DevModel &M, double theta, double p, double pbot, double ptop) {
-  if (p <= ptop) return theta;
-  const double s = get_sigma(M, pbot, p, ptop);
-  return f_sigma(M, s) + g_sigma(M, s) * theta;
 }
 // return_density (ideal gas); return_temp and return_enthalpy below (the ideal gas, or hydrogen)
 // The hydrogen thermodynamics of thermo_setup's tables (x_h2 > 0; normal hydrogen, fpara = 0.25,
@@ -392,12 +370,6 @@ __device__ __forceinline__ double return_enthalpy(const DevModel &M, double t) {
     enthalpy = (M.x_h2) * ((1. - TH_FP) * h0 + (TH_FP) * h1) + (M.x_he * 2.5 + M.x_3 * 3.5) * t;
   }
   return enthalpy * M.rgas;
-}
-// onto_kk(P2_INDEX) at a layer, epic_funcs_diag.c:2601-2618
-__device__ __forceinline__ double layer_p(const DevModel &M, double top, double bot) {
-  if (fcmp(bot, top) == 0) return .5 * (bot + top);
-  const double kp1 = M.kappa + 1.;
-  return xpow(M, div_rn(xpow(M, bot, kp1) - xpow(M, top, kp1), kp1 * (bot - top)), div_rn(1., M.kappa));
 }
 
 // ---- binary64 <-> binary32 conversions on the integer pipe ----
@@ -641,73 +613,6 @@ __device__ __forceinline__ double pchst(double a, double b) {
   if (a < 0.0) return b < 0.0 ? 1.0 : (b == 0.0 ? 0.0 : -1.0);
   return b < 0.0 ? -1.0 : (b == 0.0 ? 0.0 : 1.0);
 }
-// spline_pchip (Fritsch-Carlson PCHIM slopes), epic_funcs_util.c:721-845; returns false if x not increasing
-__device__ __forceinline__ bool spline_pchip(int n, Trip *t) {
-  for (int i = 1; i < n; i++)
-    if (t[i].x <= t[i - 1].x) return false;
-  double h1 = t[1].x - t[0].x;
-  double del1 = (t[1].y - t[0].y) / h1;
-  if (n == 2) { t[0].z = del1; t[1].z = del1; return true; }
-  double h2 = t[2].x - t[1].x;
-  double del2 = (t[2].y - t[1].y) / h2;
-  double hsum = h1 + h2;
-  double w1 = (h1 + hsum) / hsum, w2 = -h1 / hsum;
-  t[0].z = w1 * del1 + w2 * del2;
-  if (pchst(t[0].z, del1) <= 0.0) t[0].z = 0.0;
-  else if (pchst(del1, del2) < 0.0) {
-    const double dmx = 3.0 * del1;
-    if (fabs(dmx) < fabs(t[0].z)) t[0].z = dmx;
-  }
-  for (int i = 2; i <= n - 1; i++) {
-    if (2 < i) {
-      h1 = h2;
-      h2 = t[i].x - t[i - 1].x;
-      hsum = h1 + h2;
-      del1 = del2;
-      del2 = (t[i].y - t[i - 1].y) / h2;
-    }
-    t[i - 1].z = 0.0;
-    if (pchst(del1, del2) > 0.0) {
-      const double hsumt3 = 3.0 * hsum;
-      w1 = (hsum + h1) / hsumt3;
-      w2 = (hsum + h2) / hsumt3;
-      const double dmx = dmaxr(fabs(del1), fabs(del2)), dmn = dminr(fabs(del1), fabs(del2));
-      t[i - 1].z = dmn / (w1 * (del1 / dmx) + w2 * (del2 / dmx));
-    }
-  }
-  w1 = -h2 / hsum;
-  w2 = (h2 + hsum) / hsum;
-  t[n - 1].z = w1 * del1 + w2 * del2;
-  if (pchst(t[n - 1].z, del2) <= 0.0) t[n - 1].z = 0.0;
-  else if (pchst(del1, del2) < 0.0) {
-    const double dmx = 3.0 * del2;
-    if (fabs(dmx) < fabs(t[n - 1].z)) t[n - 1].z = dmx;
-  }
-  return true;
-}
-// splint_pchip, epic_funcs_util.c:926-946
-__device__ __forceinline__ double splint_pchip(double xx, const Trip *t, double h) {
-  const double delta = (t[1].y - t[0].y) / h;
-  const double del1 = (t[0].z - delta) / h;
-  const double del2 = (t[1].z - delta) / h;
-  const double c3 = (del1 + del2) / h;
-  const double c2 = -(del1 + del1 + del2);
-  const double x = xx - t[0].x;
-  return t[0].y + x * (t[0].z + x * (c2 + x * c3));
-}
-// find_place_in_table (ascending tables only), epic_funcs_util.c:2908-2967
-__device__ __forceinline__ int find_place_in_table(int n, const Trip *t, double x, double *dx) {
-  if (fcmp(x, t[0].x) <= 0) { *dx = t[1].x - t[0].x; return 0; }
-  if (fcmp(x, t[n - 1].x) >= 0) { *dx = t[n - 1].x - t[n - 2].x; return n - 2; }
-  int il = -1, iu = n;
-  while (iu - il > 1) {
-    const int im = (iu + il) >> 1;
-    if (fcmp(x, t[im].x) >= 0) il = im; else iu = im;
-  }
-  *dx = t[il + 1].x - t[il].x;
-  return il;
-}
-
 // get_kin (the Suarez-Takacs blend for the Sadourney scheme, epic_funcs_diag.c:2694-2847) at h-point
 // (j, i) of the layer planes Uk, Vk
 template <class R>

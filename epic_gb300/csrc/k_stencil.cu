@@ -34,7 +34,6 @@ __device__ __forceinline__ void cell_kji(const DevModel &M, unsigned t, int &k, 
 static inline unsigned cells_blocks(const DevModel &M, int nkk, int njj, int th) {
   return epic_blocks((long long)nkk * njj * M.ni, th);
 }
-__device__ __forceinline__ int wrap_i(const DevModel &M, int i) { return i == 0 ? M.ni : (i == M.ni + 1 ? 1 : i); }
 
 template <class R>
 __global__ void k_row_tables(DevModel M, R *out) {
