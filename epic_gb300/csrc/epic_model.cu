@@ -310,6 +310,7 @@ struct Lanes {
       if (cudaStreamCreateWithFlags(&lane[q], cudaStreamNonBlocking) != cudaSuccess) {
         while (--q >= 1) cudaStreamDestroy(lane[q]);
         for (int r = 1; r < LANES; r++) lane[r] = lane[0];
+        cudaGetLastError();   // not the step's: it is captured on the one stream
         return false;
       }
     return side = true;

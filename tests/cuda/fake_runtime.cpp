@@ -32,6 +32,7 @@ std::map<std::pair<int, std::string>, std::map<int, int>> attributes;   // of a 
 std::vector<Launch> launches;
 Graph *capturing = nullptr;
 int device = 0, sms[2] = {152, 148}, cluster16[2] = {1, 1};
+int streams_left = 1 << 30;
 long graph_launches = 0, direct_launches = 0;
 double clock_ms = 0.;   // what the GPU has done: a microsecond a kernel of a graph, ten of a direct launch
 
@@ -79,6 +80,7 @@ API long fake_launches(const char *part, unsigned *cluster, unsigned *threads, u
     }
   return n;
 }
+API void fake_streams_left(int n) { streams_left = n; }   // cudaStreamCreate fails after n more
 API void fake_device(int d, int sm_count, int clusters_of_16) { sms[d] = sm_count; cluster16[d] = clusters_of_16; }
 
 // ---- registration and launches ----
@@ -151,6 +153,7 @@ API cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t t) {
 
 // ---- streams, events, graphs ----
 API cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
+  if (streams_left-- <= 0) return note(cudaErrorMemoryAllocation);
   auto *t = new Stream;
   t->device = device;
   streams.insert(t);

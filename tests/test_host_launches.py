@@ -87,3 +87,14 @@ def test_device_bytes_of_a_model(cuda_lib, shape, kw, volumes):
     volume = 8 * (ni + 2) * (nj + 3) * (nk + 2)
     got = model_bytes(hs_setup(HSConfig(ni=ni, nj=nj, nk=nk, dt=60, **kw))[0], EPIC_PREC_FP64)
     assert volumes * volume < got < (volumes + 1) * volume
+
+
+@pytest.mark.parametrize("streams", [0, 1, 2])
+def test_step_is_captured_without_side_streams(host_library, streams):
+    """Where the branches' streams cannot be made the step is still captured, on its one stream."""
+    m = _model(16, 8, 4)
+    host_library.fake_streams_left(streams)
+    host_library.fake_reset_counts()
+    m.run(3)
+    assert host_library.fake_graph_launches() == 3 and host_library.fake_direct_launches() == 0
+    m.close()
