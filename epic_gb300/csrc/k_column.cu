@@ -1230,8 +1230,8 @@ int launch_advection_prep(const DevModel &M, int phase, cudaStream_t s) {
   return 0;
 }
 
-// The tile kernels take (arrays x 32 x (nk+1)) doubles of dynamic shared memory: up to 162 KB
-// at nk = EPIC_MAX_NK, above the 48 KB default.  The limit is raised once to that maximum, so
+// The tile kernels take (arrays x 32 x (nk+1)) doubles of dynamic shared memory: up to 195 KB (six
+// arrays) at nk = EPIC_MAX_NK, above the 48 KB default.  The limit is raised once to that maximum, so
 // models of different sizes in one process never lower it for one another.
 int column_kernels_init(int) {
   const int big = (int)(6 * 32 * (EPIC_MAX_NK + 1) * sizeof(double));
